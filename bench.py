@@ -210,14 +210,12 @@ def algorithmic_bytes(kernel: str, n_tris: int, info: dict, S: int, payload: boo
     if kernel in ("vox_small_winner", "vox_large_occupancy", "vox_large_winner"):
         # vertices of every triangle (36 B) + the task count per item (8 B)
         return n_tris * (36 + 8)
-    if kernel == "pyramid":  # leaf level dominates: read bits, write parent bits + block counts
-        return leaf_words * 4 * (1 + 1 / 8 + 1 / 8)
-    if kernel == "compact":
-        return leaf_words * 4 + info["n_nodes"] * 4
+    if kernel == "bricks":  # marks of every leaf block, and the marked blocks (at least one per 256 voxels)
+        return leaf_words / 8 + info["n_filled"] / 256 * 32
     if kernel == "leaf_payload":
-        return info["n_filled"] * (4 + 4 + tri_bytes + 24)
-    if kernel in ("top_down", "bottom_up"):
-        return info["n_nodes"] * (4 + 4 + 4 + 8 + 8 + 24) + info["n_data"] * 32
+        return info["n_filled"] * (8 + tri_bytes + 32)
+    if kernel == "emit":
+        return leaf_words / 8 + info["n_nodes"] * 24
     return 0.0
 
 

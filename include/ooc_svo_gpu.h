@@ -170,14 +170,13 @@ typedef struct {
   uint32_t large_ctas_per_sm; /* persistent CTAs per SM of the large-triangle kernel (1..16) */
   uint64_t batch_budget;      /* occupancy-pyramid bytes per sub-batch (>= 4096), as ooc_set_batch_budget */
   uint32_t graphs;            /* 1: replay each sub-batch's two launch sequences as CUDA graphs; 0: launch directly */
-  uint32_t light_per_thread;  /* elements each thread of the per-block and per-node kernels takes (1..16) */
+  uint32_t light_per_thread;  /* leaves each thread of the leaf payload kernel takes (1..16)                  */
   uint32_t pdl;               /* 1: each kernel of a launch sequence may start while its predecessor drains
                                  (programmatic dependent launch; it waits for the predecessor's results
                                  before touching memory); 0: it starts when the predecessor has finished */
-  uint32_t persistent;        /* 1: the occupancy passes and the pyramid levels of a sub-batch run as one
-                                 persistent launch whose warps take (stripe, chunk), large-triangle task
-                                 and (stripe, level, block range) units from a device work queue; 0: one
-                                 launch per pass and level */
+  uint32_t persistent;        /* 1: the occupancy passes of a sub-batch run as one persistent launch whose
+                                 warps take (stripe, chunk) and large-triangle task units from a device
+                                 work queue; 0: one launch per pass */
 } ooc_tuning;
 
 int ooc_get_tuning(const ooc_ctx* ctx, ooc_tuning* out);

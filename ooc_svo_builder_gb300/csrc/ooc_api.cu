@@ -132,9 +132,8 @@ struct ooc_ctx {
   float phase_ms[kPhases] = {0, 0, 0, 0, 0, 0};
   unsigned long long launches = 0;
   ooc::LaunchState lstate;  // this context's launch count and timing hooks, installed per API call
-  DevBuf d_tris, d_hist, d_axis, d_bits, d_scan, d_scanpart, d_keys, d_size, d_dsize, d_start, d_dstart,
-      d_cache, d_winners, d_taskoff, d_taskpart, d_counter, d_nodes, d_data, d_recs, d_rootinfo, d_itemmask,
-      d_firstchild, d_itembox, d_leaf, d_touch, d_local, d_taskmap, d_woff;
+  DevBuf d_tris, d_hist, d_axis, d_upper, d_brick, d_innerlocal, d_uppercache, d_winners, d_taskoff,
+      d_taskpart, d_counter, d_nodes, d_data, d_recs, d_itemmask, d_itembox, d_leaf, d_touch, d_local, d_taskmap, d_woff;
   uint64_t max_tasks = 0;  // most large-item warp tasks a sub-batch has had (sizes the task map)
   // persistent phase A (ooc_tuning::persistent): its counters, its task map (all ones
   // between launches: every entry a launch fills is emptied by the warp that reads it)
@@ -612,26 +611,12 @@ struct Placed {  // a stripe after the level counts
 // more than they save).
 constexpr int kMarkDepth = 9;
 
-// Levels 0..Ds of a stripe appended to the buffers: the words of the levels
-// kept zero between builds (the leaf level, and with marks the level above it)
-// to `leaf_words`, the others to `words`, every level's scan entries to
-// `entries` (one per group of kLeafGroup blocks for a marked leaf level).
-int pyramid_levels(int Ds, Level* lv, uint64_t& words, uint64_t& leaf_words, uint64_t& entries, bool marked) {
-  const int zl = marked ? Ds - 1 : Ds;
-  for (int l = 0; l <= Ds; l++) {
-    const uint64_t nbits = 1ull << (3 * l);
-    uint64_t nw = (nbits + 31) / 32;
-    nw = (nw + 7) / 8 * 8;
-    uint64_t& acc = l >= zl ? leaf_words : words;
-    lv[l].off_w = acc;
-    lv[l].off_b = entries;
-    lv[l].nwords = nw;
-    lv[l].nblocks = nw / 8;
-    lv[l].nscan = (l == Ds && marked) ? (lv[l].nblocks + kLeafGroup - 1) / kLeafGroup : lv[l].nblocks;
-    acc += nw;
-    entries += lv[l].nscan;
-  }
-  return Ds;
+// Words of a stripe's whole occupancy pyramid, every level padded to 256-bit blocks: what a
+// stripe counts against the batch budget.
+uint64_t pyramid_words(int Ds) {
+  uint64_t w = 0;
+  for (int l = 0; l <= Ds; l++) w += leaf_words(l);
+  return w;
 }
 
 // CTA prefix of one batched launch: stripe s gets ceil(count(s) / per_cta) CTAs.
@@ -642,10 +627,9 @@ std::vector<uint64_t> cta_prefix(uint32_t n, uint64_t per_cta, F count) {
   return beg;
 }
 
-// A per-block or per-node launch: its CTA prefix and the elements each thread
-// takes.  A thread takes as many elements (up to the tuning's limit) as still
-// leave about 16 CTAs per SM: few CTAs cost parallelism on small levels, many
-// cost the per-CTA staging on large ones.
+// A per-leaf launch: its CTA prefix and the leaves each thread takes.  A thread takes as many
+// (up to the tuning's limit) as still leave about 16 CTAs per SM: few CTAs cost parallelism on
+// small stripes, many cost the per-CTA staging on large ones.
 struct Light {
   std::vector<uint64_t> beg;
   uint32_t ept = 1;
@@ -780,62 +764,74 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   const std::vector<std::pair<uint64_t, cudaEvent_t>>* pieces =
       (n == 1 && !meshes[sb[0].mesh].pieces.empty()) ? &meshes[sb[0].mesh].pieces : nullptr;
   // ---- geometry of every stripe ----
-  std::vector<Pyramid> pyr(n);
+  std::vector<Stripe> stripe(n);
   std::vector<VoxJob> vj(n);
-  std::vector<uint64_t> item_beg(n + 1, 0), touch_beg(n, 0), local_beg(n, 0), woff_beg(n, 0);
-  uint64_t words = 0, leaf_words = 0, blocks = 0, tbytes = 0, nlocal = 0, items = 0, nwoff = 0;
-  int max_depth = 0;
+  std::vector<uint64_t> item_beg(n + 1, 0), leaf_beg(n, 0), touch_beg(n, 0), local_beg(n, 0), upper_beg(n, 0),
+      word_beg(n, 0), brick_beg(n, 0);
+  uint64_t leaf_w = 0, tbytes = 0, nlocal = 0, upper_w = 0, pre_w = 0, bricks = 0, items = 0;
+  int max_upper = 0;
+  bool payload_levels = false;
   for (uint32_t s = 0; s < n; s++) {
     const StripeRef& r = sb[s];
-    const MeshWork& m = meshes[r.mesh];
-    std::memset(&pyr[s], 0, sizeof(Pyramid));
-    pyr[s].depth = m.pl.Ds;
-    pyramid_levels(m.pl.Ds, pyr[s].lv, words, leaf_words, blocks, m.pl.Ds >= kMarkDepth);
+    const Plan& mp = meshes[r.mesh].pl;
+    Stripe& S = stripe[s];
+    std::memset(&S, 0, sizeof(S));
+    S.depth = mp.Ds;
+    S.K = std::min(mp.Ds, kBrickLevels);
+    S.U = S.depth - S.K;
+    S.n_bricks = 1u << (3 * S.U);
+    max_upper = std::max(max_upper, S.U);
+    leaf_beg[s] = leaf_w;
+    leaf_w += leaf_words(S.depth);
     touch_beg[s] = tbytes;
-    tbytes += touch_bytes(pyr[s].lv[m.pl.Ds]);
-    local_beg[s] = nlocal;
-    if (m.pl.Ds >= kMarkDepth) nlocal += pyr[s].lv[m.pl.Ds].nblocks;
-    woff_beg[s] = nwoff;  // the winner pass's bit ranks: payload stripes only
-    if (!m.pl.binary) nwoff += pyr[s].lv[m.pl.Ds].nblocks;
-    max_depth = std::max(max_depth, m.pl.Ds);
+    if (S.depth >= kMarkDepth) tbytes += touch_bytes(S.depth);
+    local_beg[s] = nlocal;  // the ranks of leaf bits: payload stripes only
+    if (!mp.binary) nlocal += leaf_blocks(S.depth);
+    payload_levels = payload_levels || (!mp.binary && mp.levels);
+    upper_beg[s] = upper_w;
+    upper_w += upper_off(S.U + 1);
+    word_beg[s] = pre_w;  // one entry past the last word, in whole groups of eight
+    pre_w += (upper_words(S.U) + 8) / 8 * 8;
+    brick_beg[s] = bricks;
+    bricks += std::max<uint32_t>(S.n_bricks, 32);  // whole words
     item_beg[s] = items;
     items += r.n_items;
   }
   item_beg[n] = items;
-  uint32_t* bits = ensure<uint32_t>(c->d_bits, words * 4);
   // the leaf levels and their block marks are all zero between sub-batches
-  if (leaf_words * 4 > c->d_leaf.cap || tbytes > c->d_touch.cap) c->leaf_zero = false;
-  uint32_t* leaf = ensure<uint32_t>(c->d_leaf, leaf_words * 4);
+  if (leaf_w * 4 > c->d_leaf.cap || tbytes > c->d_touch.cap) c->leaf_zero = false;
+  uint32_t* leaf = ensure<uint32_t>(c->d_leaf, leaf_w * 4);
   uint8_t* touch = ensure<uint8_t>(c->d_touch, tbytes);
-  uint16_t* local = ensure<uint16_t>(c->d_local, nlocal * 2);
-  uint64_t* woff = nwoff ? ensure<uint64_t>(c->d_woff, nwoff * 8) : nullptr;
+  uint32_t* local = nlocal ? ensure<uint32_t>(c->d_local, nlocal * 4) : nullptr;
+  uint64_t* woff = nlocal ? ensure<uint64_t>(c->d_woff, nlocal * 8) : nullptr;
+  uint16_t* inner_local = payload_levels ? ensure<uint16_t>(c->d_innerlocal, nlocal * 2) : nullptr;
   if (!c->leaf_zero) {
     ck(cudaMemsetAsync(leaf, 0, c->d_leaf.cap, st), "memset leaf levels");
     ck(cudaMemsetAsync(touch, 0, c->d_touch.cap, st), "memset leaf marks");
     c->leaf_zero = true;
   }
-  uint32_t* scan = ensure<uint32_t>(c->d_scan, (blocks + 1) * 4);
-  uint32_t* scanpart = ensure<uint32_t>(c->d_scanpart, scan_partials_needed(blocks + 1) * 4);
+  uint32_t* upper = ensure<uint32_t>(c->d_upper, upper_w * 8);         // ubits, then upre
+  uint2* brick = ensure<uint2>(c->d_brick, (pre_w + bricks) * 8 + bricks);  // wpre, then bpre, then bunits
   uint64_t* task_off = ensure<uint64_t>(c->d_taskoff, (items + 1) * 8);
   uint64_t* taskpart = ensure<uint64_t>(c->d_taskpart, scan_partials_needed(items + 1) * 8);
   uint64_t* item_mask = ensure<uint64_t>(c->d_itemmask, items * 8);
   uint64_t* item_box = ensure<uint64_t>(c->d_itembox, items * 8);
   unsigned long long* counter = ensure<unsigned long long>(c->d_counter, 16);
-  uint32_t* d_root = ensure<uint32_t>(c->d_rootinfo, ((uint64_t)n * 16 + 64) * 4);
-  uint32_t* flag = d_root + (uint64_t)n * 16;
 
-  constexpr int kTopPyramidLevel = 5;  // levels 0..5 have at most 512 blocks: one CTA per stripe
   for (uint32_t s = 0; s < n; s++) {
     const StripeRef& r = sb[s];
     const MeshWork& m = meshes[r.mesh];
-    Pyramid& P = pyr[s];
-    P.bits = bits;
-    P.leaf = leaf;
-    P.touch = P.depth >= kMarkDepth ? touch + touch_beg[s] : nullptr;
-    P.zl = P.depth >= kMarkDepth ? P.depth - 1 : P.depth;
-    P.local = P.depth >= kMarkDepth ? local + local_beg[s] : nullptr;
-    P.scan = scan;
-    P.woff = m.pl.binary ? nullptr : woff + woff_beg[s];
+    Stripe& S = stripe[s];
+    S.leaf = leaf + leaf_beg[s];
+    S.touch = S.depth >= kMarkDepth ? touch + touch_beg[s] : nullptr;
+    S.ubits = upper + upper_beg[s];
+    S.upre = upper + upper_w + upper_beg[s];
+    S.wpre = brick + word_beg[s];
+    S.bpre = brick + pre_w + brick_beg[s];
+    S.bunits = reinterpret_cast<uint8_t*>(brick + pre_w + bricks) + brick_beg[s];
+    S.local = m.pl.binary ? nullptr : local + local_beg[s];
+    S.woff = m.pl.binary ? nullptr : woff + local_beg[s];
+    S.inner_local = !m.pl.binary && m.pl.levels ? inner_local + local_beg[s] : nullptr;
     VoxJob& j = vj[s];
     std::memset(&j, 0, sizeof(j));
     uint32_t pa[3], sa[3];
@@ -857,8 +853,11 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     j.unit_div = m.pl.unit_div;
     j.small_vol = c->tuning.small_vol;
     j.lines_per_lane = c->tuning.lines_per_lane;
-    j.leafbits = leaf + P.lv[P.depth].off_w;
-    j.leaftouch = P.touch;
+    j.leafbits = S.leaf;
+    j.leaftouch = S.touch;
+    j.wpre = S.wpre;
+    j.leaflocal = S.local;
+    j.leafwoff = S.woff;
     j.task_off = task_off + item_beg[s];
     j.task_flag = task_off + items;
     j.task_counter = counter;
@@ -866,74 +865,35 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     j.item_box = m.pl.binary ? nullptr : item_box + item_beg[s];
   }
   const std::vector<uint64_t> cp_items = cta_prefix(n, kChunk, [&](uint32_t s) { return sb[s].n_items; });
-  std::vector<Light> cp_pyr;
-  for (int r = 0; r <= max_depth - kTopPyramidLevel - 1; r++)
-    cp_pyr.push_back(light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-      const int l = pyr[s].depth - r;
-      return l > kTopPyramidLevel ? pyr[s].lv[l].nscan : 0;
-    }));
+  const std::vector<uint64_t> cp_bricks = cta_prefix(n, 1, [&](uint32_t s) { return brick_ctas(stripe[s]); });
 
-  // keys of every level, launched as soon as the level counts are back (its prefix needs no count)
-  const Light cp_compact = light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-    const uint64_t upper = pyr[s].lv[pyr[s].depth].off_b - pyr[s].lv[0].off_b;  // compact_elems
-    return (upper + 31) / 32 * 32 + (pyr[s].lv[pyr[s].depth].nscan + 31) / 32 * 32;
-  });
-
-  // persistent phase A: 32-item chunks and pyramid units per stripe, and the
-  // per-stripe counts of units not yet done that its waits read
+  // persistent occupancy passes: the items of every stripe in chunks
   bool persist = c->tuning.persistent != 0 && !pieces;
   if (persist && (c->persist_per_sm < 0 || c->persist_lpl != c->tuning.lines_per_lane)) {
     c->persist_per_sm = persist_ctas_per_sm(c->tuning.lines_per_lane);
     c->persist_lpl = c->tuning.lines_per_lane;
   }
   persist = persist && c->persist_per_sm > 0;
-  constexpr uint32_t kPersistEpt = 32;  // pyramid elements per lane of a unit (1,024 per unit)
-  std::vector<uint64_t> p_chunk, p_unit;
-  std::vector<uint32_t> p_occ, p_pyr;
-  const uint32_t p_levels = (uint32_t)cp_pyr.size();
-  if (persist) {
-    p_chunk = cta_prefix(n, kPersistChunkItems, [&](uint32_t s) { return sb[s].n_items; });
-    p_occ.resize(n);
-    for (uint32_t s = 0; s < n; s++) p_occ[s] = (uint32_t)(p_chunk[s + 1] - p_chunk[s]);
-    p_unit.assign(std::max<uint64_t>((uint64_t)p_levels * (n + 1), 1), 0);  // one entry at least: uploaded as is
-    p_pyr.assign(std::max<uint64_t>((uint64_t)p_levels * n, 1), 0);
-    uint64_t acc = 0;
-    for (uint32_t r = 0; r < p_levels; r++) {
-      for (uint32_t s = 0; s < n; s++) {
-        p_unit[(uint64_t)r * (n + 1) + s] = acc;
-        const int l = pyr[s].depth - (int)r;
-        const uint64_t units = l > kTopPyramidLevel ? (pyr[s].lv[l].nscan + 32 * kPersistEpt - 1) / (32 * kPersistEpt) : 0;
-        p_pyr[(uint64_t)r * n + s] = (uint32_t)units;
-        acc += units;
-      }
-      p_unit[(uint64_t)r * (n + 1) + n] = acc;
-    }
-  }
+  std::vector<uint64_t> p_chunk;
+  if (persist) p_chunk = cta_prefix(n, kPersistChunkItems, [&](uint32_t s) { return sb[s].n_items; });
 
   Uploader up1;
   const size_t o_vj = up1.add(vj.data(), n * sizeof(VoxJob));
-  const size_t o_pyr = up1.add(pyr.data(), n * sizeof(Pyramid));
+  const size_t o_str = up1.add(stripe.data(), n * sizeof(Stripe));
   const size_t o_beg = up1.add(item_beg.data(), (n + 1) * 8);
   const size_t o_cpi = up1.add(cp_items.data(), (n + 1) * 8);
-  std::vector<size_t> o_cpp(cp_pyr.size());
-  for (size_t r = 0; r < cp_pyr.size(); r++) o_cpp[r] = up1.add(cp_pyr[r].beg.data(), (n + 1) * 8);
-  const size_t o_cc = up1.add(cp_compact.beg.data(), (n + 1) * 8);
-  size_t o_pc = 0, o_pu = 0, o_po = 0, o_pp = 0;
-  if (persist) {
-    o_pc = up1.add(p_chunk.data(), (n + 1) * 8);
-    o_pu = up1.add(p_unit.data(), p_unit.size() * 8);
-    o_po = up1.add(p_occ.data(), n * 4);
-    o_pp = up1.add(p_pyr.data(), p_pyr.size() * 4);
-  }
+  const size_t o_cpb = up1.add(cp_bricks.data(), (n + 1) * 8);
+  size_t o_pc = 0;
+  if (persist) o_pc = up1.add(p_chunk.data(), (n + 1) * 8);
   unsigned char* t1 = up1.run(c, c->d_tables1, c->h_tables1, st);
   auto dp1 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t1 + off); };
   const VoxJob* d_vj = reinterpret_cast<const VoxJob*>(t1 + o_vj);
-  const Pyramid* d_pyr = reinterpret_cast<const Pyramid*>(t1 + o_pyr);
+  const Stripe* d_str = reinterpret_cast<const Stripe*>(t1 + o_str);
   const uint64_t* d_beg = reinterpret_cast<const uint64_t*>(t1 + o_beg);
 
-  uint32_t* lvl = ensure_pinned<uint32_t>(c->h_misc, ((uint64_t)n * 16 + 64) * 4);  // level bases, then root info
+  uint32_t* lvl = ensure_pinned<uint32_t>(c->h_misc, ((uint64_t)n * kCountWords + 64) * 4);  // counts of every stripe, then two totals
   uint32_t* lvl_dev = nullptr;  // the same pinned memory as the kernels address it
-  ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&lvl_dev), lvl, 0), "mapped level counts");
+  ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&lvl_dev), lvl, 0), "mapped counts");
   // Warp task -> item map, sized by the items and the most tasks a sub-batch has had.
   // Built once the context has seen a sub-batch with many tasks: with few, the large
   // items' search of the task offsets costs less than the map's launch.
@@ -959,24 +919,16 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       c->pmap_empty = true;
     }
     pj.jobs = d_vj;
-    pj.pyrs = d_pyr;
     pj.item_beg = d_beg;
     pj.n = n;
-    pj.levels = p_levels;
     pj.chunk_beg = dp1(o_pc);
-    pj.unit_beg = dp1(o_pu);
-    pj.ept = kPersistEpt;
-    pj.top_level = kTopPyramidLevel;
-    pj.occ_left = reinterpret_cast<uint32_t*>(t1 + o_po);
-    pj.pyr_left = reinterpret_cast<uint32_t*>(t1 + o_pp);
     pj.ctr = ensure<unsigned long long>(c->d_pctr, kPersistCtrWords * 8);
     pj.map = pmap;
     pj.cap = c->d_pmap.cap / 8;
-    pj.scan_end = scan + blocks;
     pj.lines_per_lane = c->tuning.lines_per_lane;
     c->pmap_empty = false;  // until this launch is known to have ended without a timeout
   }
-  c->leaf_zero = false;  // until the clean at the end of the sub-batch is queued
+  c->leaf_zero = false;  // until the emission at the end of the sub-batch is queued
   run_launches(c, st, 0, [&] {
     if (persist) {
       PhaseScope ph(c, PH_VOX, st);
@@ -1014,64 +966,61 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     }
     {
       PhaseScope ph(c, PH_PYR, st);
-      if (!persist) {
-        for (size_t r = 0; r < cp_pyr.size(); r++)
-          launch_b_pyramid(d_pyr, dp1(o_cpp[r]), n, cp_pyr[r].beg[n], cp_pyr[r].ept, (int)r,
-                           n == 1 ? &pyr[0] : nullptr, st);
-        launch_b_pyramid_top(d_pyr, n, kTopPyramidLevel, scan + blocks, st);
-      }
-      scan_u32_exclusive(scan, blocks + 1, scanpart, st);
+      launch_b_bricks(d_str, dp1(o_cpb), n, cp_bricks[n], n == 1 ? &stripe[0] : nullptr, st);
       // the tasks of the sub-batch (sizes the task maps); the persistent kernel counts them itself
       const uint64_t* tasks = persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTasksWord) : task_off + items;
-      // The level counts go straight into pinned host memory, written by the kernel: a
-      // copy on the copy engine would queue behind the previous sub-batch's copy back,
-      // which the host keeps refilling while it waits, and hold up the whole pipeline.
-      launch_b_level_bases(d_pyr, n, lvl_dev, tasks, reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * 16 + 8),
-                           flag, persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTimeoutWord) : nullptr,
-                           reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * 16 + 12), st);
+      // The counts go straight into pinned host memory, written by the kernel: a copy on the
+      // copy engine would queue behind the previous sub-batch's copy back, which the host
+      // keeps refilling while it waits, and hold up the whole pipeline.
+      launch_b_upper(d_str, n, max_upper, lvl_dev, tasks, reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords),
+                     persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTimeoutWord) : nullptr,
+                     reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords + 2), st);
     }
   }, pieces != nullptr);  // waits on the upload stream are not captured
   wait_level_counts(st, idle);
   if (persist) {
     uint64_t code;
-    std::memcpy(&code, lvl + (uint64_t)n * 16 + 12, 8);
+    std::memcpy(&code, lvl + (uint64_t)n * kCountWords + 2, 8);
     if (code != 0) fail(OOC_ERR_DEVICE, "persistent voxelization: a wait ran out (code " + std::to_string(code) + ")");
     c->pmap_empty = true;
   }
   uint64_t tasks_seen;
-  std::memcpy(&tasks_seen, lvl + (uint64_t)n * 16 + 8, 8);
+  std::memcpy(&tasks_seen, lvl + (uint64_t)n * kCountWords, 8);
   c->max_tasks = std::max(c->max_tasks, tasks_seen);
 
   // ---- counts, placement in the files ----
   std::vector<Placed> pl(n);
-  uint64_t total_nodes = 0, summed = 0;
+  uint64_t total_nodes = 0, total_leaves = 0;
+  std::vector<uint64_t> leaf_at(n, 0), cell_at(n, 0);  // the stripes' places in the per-leaf arrays
+  uint64_t cells = 0;
+  bool any_levels = false;
   for (uint32_t s = 0; s < n; s++) {
-    Pyramid& P = pyr[s];
-    const uint32_t* o = lvl + (uint64_t)s * (kMaxLevels + 1);
-    for (int l = 0; l <= P.depth; l++) {
-      P.lv[l].koff = o[l];
-      P.lv[l].n = (uint64_t)o[l + 1] - o[l];
-    }
+    const uint32_t* o = lvl + (uint64_t)s * kCountWords;
     const MeshWork& m = meshes[sb[s].mesh];
     Placed& q = pl[s];
-    q.total = (uint64_t)o[P.depth + 1] - o[0];
-    q.n_leaf = P.lv[P.depth].n;
+    q.n_leaf = o[0];
     q.empty = q.n_leaf == 0;
     if (!q.empty) {
+      q.total = q.n_leaf;  // a one-voxel stripe is its brick
+      if (stripe[s].depth > 0) {
+        q.total += o[1];
+        for (int l = 0; l <= stripe[s].U; l++) q.total += o[2 + l];
+      }
       q.node_span = q.total - 1;
       q.data_span = (m.pl.binary ? 0 : q.n_leaf) + (m.pl.levels ? q.total - q.n_leaf : 0);
     }
-    total_nodes = std::max<uint64_t>(total_nodes, o[P.depth + 1]);
-    summed += q.total;
+    if (!m.pl.binary) {
+      leaf_at[s] = total_leaves;
+      total_leaves += q.n_leaf;
+    }
+    if (m.pl.levels) {
+      any_levels = true;
+      cell_at[s] = cells;
+      cells += upper_cell(stripe[s].U + (stripe[s].K == kBrickLevels ? 2 : 1), 0);  // with the bricks' children
+    }
+    total_nodes += q.total;
   }
-  // node indices are 32-bit within a sub-batch (the block scan is u32)
-  if (summed != total_nodes) fail(OOC_ERR_LIMIT, "more than 2^32 nodes in one sub-batch; lower the batch budget");
-  // the keys need only the phase-A tables: the GPU compacts while the host lays out the rest
-  uint32_t* keys = ensure<uint32_t>(c->d_keys, total_nodes * 4);
-  {
-    PhaseScope ph(c, PH_PYR, st);
-    launch_b_compact(d_pyr, dp1(o_cc), n, cp_compact.beg[n], cp_compact.ept, keys, n == 1 ? &pyr[0] : nullptr, st);
-  }
+  if (total_nodes >> 32) fail(OOC_ERR_LIMIT, "more than 2^32 nodes in one sub-batch; lower the batch budget");
   // the grouping above the stripes, run ahead on placeholders: where every stripe's records start
   for (uint32_t s = 0; s < n; s++) {
     MeshWork& m = meshes[sb[s].mesh];
@@ -1091,19 +1040,10 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       tb.push(tb.top, ph);
     }
   }
-  // ---- per-node arrays and output windows ----
-  bool any_levels = false, any_payload = false;
-  for (auto& m : meshes) {
-    any_levels = any_levels || m.pl.levels;
-    any_payload = any_payload || !m.pl.binary;
-  }
-  uint32_t* size = ensure<uint32_t>(c->d_size, total_nodes * 4);
-  uint32_t* dsize = ensure<uint32_t>(c->d_dsize, total_nodes * 4);
-  uint32_t* first_child = ensure<uint32_t>(c->d_firstchild, total_nodes * 4);
-  uint32_t* start = ensure<uint32_t>(c->d_start, total_nodes * 4);  // stripe-relative: a stripe spans < 2^32
-  uint32_t* dstart = ensure<uint32_t>(c->d_dstart, total_nodes * 4);
-  float* cache = any_levels ? ensure<float>(c->d_cache, total_nodes * 24) : nullptr;
-  uint32_t* winners = any_payload ? ensure<uint32_t>(c->d_winners, total_nodes * 4) : nullptr;
+  // ---- per-leaf arrays and output windows ----
+  const bool any_payload = total_leaves != 0;
+  float* upper_cache = any_levels ? ensure<float>(c->d_uppercache, cells * 24) : nullptr;
+  unsigned long long* winners = any_payload ? ensure<unsigned long long>(c->d_winners, total_leaves * 8) : nullptr;
   uint64_t out_nodes = 0, out_data = 0;
   if (os.mode == OUT_DEST) {
     // meshes whose last stripe is here get their destination; the others park
@@ -1141,10 +1081,17 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     ensure<uint64_t>(c->d_out_nodes[slot], out_nodes * 24);
     ensure<unsigned char>(c->d_out_data[slot], out_data * 32);
   }
+  uint32_t* hr = ensure_pinned<uint32_t>(c->h_root[slot], ((uint64_t)n * 16 + 1) * 4);
+  uint32_t* hr_dev = nullptr;
+  ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hr_dev), hr, 0), "mapped root info");
+  hr[(uint64_t)n * 16] = 0;  // the layout check flag: the record kernels set it, in host memory
+  auto bricks_of = [&](uint32_t s) -> uint64_t { return lvl[(uint64_t)s * kCountWords + 2 + stripe[s].U]; };  // non-empty
+  uint64_t total_bricks = 0;
+  for (uint32_t s = 0; s < n; s++)
+    if (!pl[s].empty) total_bricks += bricks_of(s);
   std::vector<EmitJob> ej(n);
   for (uint32_t s = 0; s < n; s++) {
     const MeshWork& m = meshes[sb[s].mesh];
-    const Pyramid& P = pyr[s];
     const Placed& q = pl[s];
     EmitJob& e = ej[s];
     std::memset(&e, 0, sizeof(e));
@@ -1157,18 +1104,13 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     e.tris = m.d_tris;
     e.stride = vj[s].stride;
     e.unit_div = m.pl.unit_div;
-    e.keys = keys;
-    e.size = size;
-    e.dsize = dsize;
-    e.first_child = first_child;
-    e.start = start;
-    e.dstart = dstart;
-    e.cache = m.pl.levels ? cache : nullptr;
-    e.leaf_inline = (!m.pl.binary && !m.pl.levels) ? 1 : 0;
+    e.upper_cache = upper_cache ? upper_cache + cell_at[s] * 6 : nullptr;
+    e.root_out = hr_dev + (uint64_t)s * 16;
     e.n_tris = m.resident;
-    e.flag = flag;
+    e.flag = hr_dev + (uint64_t)n * 16;
     e.node_base = q.node_base;
     e.data_base = q.data_base;
+    e.data_span = q.data_span;
     if (os.mode == OUT_DEST && m.dst_ready) {
       e.node_win = static_cast<uint64_t*>(m.dst_nodes);
       e.data_win = static_cast<unsigned char*>(m.dst_data);
@@ -1191,80 +1133,57 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       e.node_win_len = q.node_span;
       e.data_win_len = q.data_span;
     }
+    e.n_leaf = q.n_leaf;
+    // A warp's share: about 1,024 records, as long as 48 warps per SM have one.  Fewer repeat the
+    // warp's search and set-up more often; more leave SMs idle behind the warps of dense bricks.
+    e.bricks_per_warp = (uint32_t)std::max<uint64_t>(
+        1, std::min(q.total ? 1024 * bricks_of(s) / q.total : 1, total_bricks / ((uint64_t)c->num_sms * 48)));
     if (!m.pl.binary) {
-      e.winners = winners + P.lv[P.depth].koff;
-      vj[s].winners = winners + P.lv[P.depth].koff;
-      vj[s].leafscan = scan + P.lv[P.depth].off_b;
-      vj[s].leaflocal = P.local;
-      vj[s].leafscan_base = (uint32_t)P.lv[P.depth].koff;
-      vj[s].leafwoff = P.woff;
+      e.winners = winners + leaf_at[s];
+      vj[s].winners = winners + leaf_at[s];
     }
-    if (q.empty) continue;
-    int ls = 0;
-    while (ls + 1 <= P.depth - 1 && P.lv[ls + 1].n <= 256) ls++;
-    e.l_small = ls;
   }
   auto live = [&](uint32_t s) { return !pl[s].empty; };
   const std::vector<uint64_t> cp_pay = cta_prefix(n, kChunk, [&](uint32_t s) -> uint64_t {
     return meshes[sb[s].mesh].pl.binary ? 0 : sb[s].n_items;
   });
-  // leaf payloads: into the cache with -levels, else straight into the data file
-  // (a depth-0 stripe's one voxel is written with its root)
+  // leaf payloads, straight into the data file
   const Light cp_leafpay = light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-    const Plan& mp = meshes[sb[s].mesh].pl;
-    if (!live(s) || mp.binary) return 0;
-    return (mp.levels || pyr[s].depth >= 1) ? pl[s].n_leaf : 0;
+    return live(s) && !meshes[sb[s].mesh].pl.binary ? pl[s].n_leaf : 0;
   });
   // host output: without -levels the data file is final after the leaf payload pass,
   // so its copy back starts there, beside the node layout
   bool early_data = os.mode == OUT_HOST;
   for (uint32_t s = 0; s < n; s++) early_data = early_data && !meshes[sb[s].mesh].pl.levels;
-  const Light cp_leaves = light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-    return (live(s) && pyr[s].depth >= 1) ? pl[s].n_leaf : 0;  // a depth-0 root is the leaf
+  const std::vector<uint64_t> cp_emit = cta_prefix(n, kTreeWarpsPerCta, [&](uint32_t s) -> uint64_t {
+    return live(s) ? (bricks_of(s) + ej[s].bricks_per_warp - 1) / ej[s].bricks_per_warp : 0;
   });
-  const Light cp_clean = light_prefix(c, n, [&](uint32_t s) -> uint64_t { return touch_bytes(pyr[s].lv[pyr[s].depth]) / 16; });
-  std::vector<Light> cp_bu(max_depth + 1), cp_td(max_depth + 1);
-  for (int r = 1; r <= max_depth; r++)
-    cp_bu[r] = light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-      const int l = pyr[s].depth - r;
-      return (live(s) && l > ej[s].l_small && l >= 0) ? pyr[s].lv[l].n : 0;
-    });
-  for (int l = 0; l <= max_depth; l++)
-    cp_td[l] = light_prefix(c, n, [&](uint32_t s) -> uint64_t {
-      const int last_top = std::min(ej[s].l_small, pyr[s].depth - 2);
-      return (live(s) && l > last_top && l <= pyr[s].depth - 2) ? pyr[s].lv[l + 1].n : 0;  // one thread per child
-    });
+  const std::vector<uint64_t> cp_upper = cta_prefix(n, kChunk, [&](uint32_t s) -> uint64_t {
+    return live(s) ? upper_cell(stripe[s].U, 0) : 0;  // levels 0 .. U-1
+  });
   Uploader up2;
   const size_t o_vj2 = up2.add(vj.data(), n * sizeof(VoxJob));
-  const size_t o_pyr2 = up2.add(pyr.data(), n * sizeof(Pyramid));
   const size_t o_ej = up2.add(ej.data(), n * sizeof(EmitJob));
   const size_t o_cpay = up2.add(cp_pay.data(), (n + 1) * 8);
   const size_t o_clp = up2.add(cp_leafpay.beg.data(), (n + 1) * 8);
-  const size_t o_cl = up2.add(cp_leaves.beg.data(), (n + 1) * 8);
-  const size_t o_cln = up2.add(cp_clean.beg.data(), (n + 1) * 8);
-  std::vector<size_t> o_bu(cp_bu.size(), 0), o_td(cp_td.size(), 0);
-  for (size_t r = 1; r < cp_bu.size(); r++) o_bu[r] = up2.add(cp_bu[r].beg.data(), (n + 1) * 8);
-  for (size_t l = 0; l < cp_td.size(); l++) o_td[l] = up2.add(cp_td[l].beg.data(), (n + 1) * 8);
+  const size_t o_em = up2.add(cp_emit.data(), (n + 1) * 8);
+  const size_t o_un = up2.add(cp_upper.data(), (n + 1) * 8);
   unsigned char* t2 = up2.run(c, c->d_tables2, c->h_tables2, st);
   auto dp2 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t2 + off); };
   const VoxJob* d_vj2 = reinterpret_cast<const VoxJob*>(t2 + o_vj2);
-  const Pyramid* d_pyr2 = reinterpret_cast<const Pyramid*>(t2 + o_pyr2);
   const EmitJob* d_ej = reinterpret_cast<const EmitJob*>(t2 + o_ej);
-  const Pyramid* sp1 = n == 1 ? &pyr[0] : nullptr;  // one-stripe launches take the jobs as parameters
+  const Stripe* sp1 = n == 1 ? &stripe[0] : nullptr;  // one-stripe launches take the jobs as parameters
   const EmitJob* se1 = n == 1 ? &ej[0] : nullptr;
 
-  uint32_t* hr = ensure_pinned<uint32_t>(c->h_root[slot], ((uint64_t)n * 16 + 1) * 4);
-  uint32_t* hr_dev = nullptr;
-  ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hr_dev), hr, 0), "mapped root info");
   if (any_payload) run_launches(c, st, 1, [&] {
     {
       PhaseScope ph(c, PH_VOX, st);
-      ck(cudaMemsetAsync(winners, 0xff, total_nodes * 4, st), "memset winners");
+      ck(cudaMemsetAsync(winners, 0xff, total_leaves * 8, st), "memset winners");
       launch_b_vox_small(d_vj2, dp2(o_cpay), n, cp_pay[n], 1, n == 1 ? &vj[0] : nullptr, st);
       if (tasks_seen)  // the count came back with the level counts
         launch_b_vox_large(d_vj2, d_beg, n, task_off, items, counter, 1, st, c->num_sms, (int)c->tuning.large_block,
                            (int)c->tuning.large_ctas_per_sm, c->tuning.lines_per_lane, task_map, map_cap);
-      launch_b_leaf_payload(d_pyr2, d_ej, dp2(o_clp), n, cp_leafpay.beg[n], cp_leafpay.ept, sp1, se1, st);
+      launch_b_leaf_payload(d_str, d_ej, dp2(o_clp), n, cp_leafpay.beg[n], cp_leafpay.ept, sp1, se1, st);
     }
   });
   // recorded between the two launch sequences: an event recorded inside a captured
@@ -1273,17 +1192,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   run_launches(c, st, 2, [&] {
     {
       PhaseScope ph(c, PH_TREE, st);
-      for (size_t r = 1; r < cp_bu.size(); r++)
-        launch_b_bottom_up(d_pyr2, d_ej, dp2(o_bu[r]), n, cp_bu[r].beg[n], cp_bu[r].ept, (int)r, sp1, se1, st);
-      launch_b_bottom_up_top(d_pyr2, d_ej, n, st);
-      launch_b_top_down_top(d_pyr2, d_ej, n, st);
-      for (size_t l = 0; l < cp_td.size(); l++)
-        launch_b_top_down(d_pyr2, d_ej, dp2(o_td[l]), n, cp_td[l].beg[n], cp_td[l].ept, (int)l, sp1, se1, st);
-      launch_b_top_down_leaves(d_pyr2, d_ej, dp2(o_cl), n, cp_leaves.beg[n], cp_leaves.ept, sp1, se1, st);
-      // into pinned host memory by the kernel, like the level counts: not behind the copy back
-      launch_b_root_info(d_pyr2, d_ej, n, hr_dev, flag, st);
-      // the last reader of the leaf levels is done: zero them for the next sub-batch
-      launch_b_clean_leaves(d_pyr2, dp2(o_cln), n, cp_clean.beg[n], cp_clean.ept, sp1, st);
+      launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, sp1, se1, st);
+      if (any_levels) launch_b_upper_avg(d_str, d_ej, n, max_upper, st);
+      launch_b_upper_nodes(d_str, d_ej, dp2(o_un), n, cp_upper[n], sp1, se1, st);
     }
   });
   c->leaf_zero = true;
@@ -1310,7 +1221,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   out_pending.sb = sb;
   out_pending.pl = pl;
   out_pending.depth.resize(n);
-  for (uint32_t s = 0; s < n; s++) out_pending.depth[s] = pyr[s].depth;
+  for (uint32_t s = 0; s < n; s++) out_pending.depth[s] = stripe[s].depth;
 }
 
 // Hand a sub-batch's stripes to their meshes, in file order.  With `block` it
@@ -1678,9 +1589,7 @@ void build_meshes(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, co
         stream_group(c, st, m, part);
       }
       const uint64_t ibeg = m.pl.P > 1 ? m.part_off[part] - m.group_first_item : 0;
-      Level tmp[kMaxLevels];
-      uint64_t w = 0, b = 0;
-      pyramid_levels(m.pl.Ds, tmp, w, w, b, false);
+      const uint64_t w = pyramid_words(m.pl.Ds);
       // host output: the first sub-batch takes an eighth of the budget, so that the copy
       // back (the longer part of a large build) starts after a short first compute
       const uint64_t cap = (os.mode == OUT_HOST && k == 0) ? budget / 8 : budget;
@@ -1927,10 +1836,9 @@ void ooc_ctx_destroy(ooc_ctx* c) {
   for (cudaStream_t rs : c->ring_stream)
     if (rs) cudaStreamSynchronize(rs);
   if (c->h2d_stream) cudaStreamSynchronize(c->h2d_stream);
-  DevBuf* bufs[] = {&c->d_tris, &c->d_hist, &c->d_axis, &c->d_bits, &c->d_scan, &c->d_scanpart,
-                    &c->d_keys, &c->d_size, &c->d_dsize, &c->d_start, &c->d_dstart, &c->d_cache, &c->d_winners,
-                    &c->d_taskoff, &c->d_taskpart, &c->d_counter, &c->d_nodes, &c->d_data, &c->d_recs,
-                    &c->d_rootinfo, &c->d_itemmask, &c->d_firstchild, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_local,
+  DevBuf* bufs[] = {&c->d_tris, &c->d_hist, &c->d_axis, &c->d_upper, &c->d_brick, &c->d_innerlocal, &c->d_uppercache,
+                    &c->d_winners, &c->d_taskoff, &c->d_taskpart, &c->d_counter, &c->d_nodes,
+                    &c->d_data, &c->d_recs, &c->d_itemmask, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_local,
                     &c->d_taskmap, &c->d_woff, &c->d_pctr, &c->d_pmap, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
                     &c->d_group[1], &c->d_stream_mat, &c->d_stream_part, &c->d_stream_base, &c->d_part_off};
   for (DevBuf* b : bufs)

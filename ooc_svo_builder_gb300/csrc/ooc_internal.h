@@ -17,47 +17,63 @@ namespace ooc {
 constexpr int kMaxStripeDepth = 10;
 constexpr int kMaxLevels = kMaxStripeDepth + 1;
 
-// One level of the per-stripe occupancy pyramid.  Level l has 8^l bits; its
-// words are padded to whole 256-bit blocks (8 words) and each block has a
-// popcount entry in the concatenated scan array.
-struct Level {
-  uint64_t off_w;    // first word of this level in its buffer (`leaf` for the leaf level, `bits` above it)
-  uint64_t off_b;    // first block entry of this level in the scan buffer
-  uint64_t nwords;   // padded word count (multiple of 8)
-  uint64_t nblocks;  // nwords / 8
-  uint64_t nscan;    // scan entries: nblocks, or one per group of 16 blocks for a marked leaf level
-  uint64_t koff;     // first node of this level in the per-node arrays
-  uint64_t n;        // set bits (nodes) at this level, filled after the scan
-};
+// A stripe's octree is cut into bricks: the nodes kBrickLevels levels above the
+// leaves (16^3 voxels, 4,096 leaf bits; a stripe of depth 4 or less is one
+// brick).  A brick's records are one contiguous run of the node file, so one
+// warp lays out and writes a whole brick from its leaf bits, and nothing is
+// stored per node.  Only the bricks and the few nodes above them (the upper
+// levels 0..U, U = depth - K) have arrays:
+//   * ubits: the occupancy bits of the upper levels;
+//   * upre: per upper word, the set bits of its level before it;
+//   * wpre: per level-U word (32 bricks), the leaves and the nodes strictly
+//     between the leaves and the bricks before it;
+//   * bpre: per brick, the same within the word; bunits: its child mask.
+// Every position in the files follows from these by prefix sums: the nodes
+// written before a brick's run are the leaves and inner nodes of earlier bricks
+// and the upper nodes whose parents end before it.
+constexpr int kBrickLevels = 4;
+constexpr int kMaxUpper = kMaxStripeDepth - kBrickLevels;
 
-// The leaf level (with a marked leaf level, also the level above it) lives in
-// its own buffer, which is all zero between builds:
-// the voxelization marks every 256-bit leaf block it sets a bit in (`touch`,
-// one byte per block, written with plain stores), the passes over the leaf
-// level read only marked blocks, and the last kernel of a sub-batch zeroes the
-// marked blocks and the marks.  The levels above the leaf are written in full
-// by the pyramid passes.
-//
-// A marked leaf level has one scan entry per group of kLeafGroup blocks (the
-// group's node count) and, for each marked block, the count of the group's
-// nodes before it (`local`), so the scan never visits unmarked blocks.
-struct Pyramid {
-  int depth;  // Ds: levels 0..Ds, level Ds = voxels of the stripe
-  int zl;     // levels zl..Ds live in `leaf` (Ds, or Ds-1 when the leaf level is marked)
-  Level lv[kMaxLevels];
-  uint32_t* bits;   // words of levels 0..zl-1
-  uint32_t* leaf;   // words of levels zl..Ds, zero between builds outside marked groups
-  uint8_t* touch;   // byte b non-zero: leaf block b may have a set bit (NULL: every block is read)
-  uint16_t* local;  // marked leaf level: nodes of block b's group before block b (written for marked blocks)
-  uint32_t* scan;   // exclusive prefix popcount per 256-bit block, all levels (+1 total)
-  uint64_t* woff;   // leaf level, payload stripes: per block, byte k = set bits in its words 0..k-1
-                    // (written for every block of an unmarked level, for marked blocks otherwise); or NULL
-};
+// First word of upper level l in ubits / upre.  Every level has at least one
+// spare word after its last, so the rank at its end can be read like any other.
+__host__ __device__ inline uint32_t upper_off(int l) {
+  return l < 3 ? 8u * (uint32_t)l : (l == 3 ? 24u : (l == 4 ? 48u : (l == 5 ? 184u : (l == 6 ? 1216u : 9416u))));
+}
+__host__ __device__ inline uint32_t upper_words(int l) { return l < 2 ? 1u : 1u << (3 * l - 5); }
 
-constexpr uint64_t kLeafGroup = 16;  // leaf blocks per scan entry of a marked leaf level
+// Words of the leaf level (whole 256-bit blocks) and its blocks.
+__host__ __device__ inline uint64_t leaf_words(int depth) { return depth < 3 ? 8ull : 1ull << (3 * depth - 5); }
+__host__ __device__ inline uint64_t leaf_blocks(int depth) { return leaf_words(depth) / 8; }
+
+// The leaf levels and the marks live in buffers that are all zero between
+// builds: the voxelization of a stripe of 512^3 voxels and more marks every
+// 256-bit leaf block it sets a bit in (`touch`, one byte per block, written with
+// plain stores), the passes over its leaf level read only marked blocks, and the
+// emission zeroes what it has read.
+struct Stripe {
+  int depth;         // levels 0..depth, level `depth` = voxels of the stripe
+  int K;             // levels below a brick: min(depth, kBrickLevels)
+  int U;             // the bricks' level: depth - K
+  uint32_t n_bricks; // 8^U
+  uint32_t* leaf;    // leaf words
+  uint8_t* touch;    // byte b non-zero: leaf block b has a set bit (NULL: every block is read)
+  uint32_t* ubits;
+  uint32_t* upre;
+  uint2* wpre;       // .x leaves, .y inner nodes below the bricks (upper_words(U) + 1 entries)
+  uint2* bpre;
+  uint8_t* bunits;   // per brick: its child mask (1 for a brick of fewer levels); like bpre, whole words
+  // payload stripes, for the rank of a leaf bit (else NULL):
+  uint32_t* local;   // per leaf block: set bits before it within its 32 bricks (written for marked blocks)
+  uint64_t* woff;    // per leaf block: byte k = set bits in its words 0..k-1
+  uint16_t* inner_local;  // per leaf block, payload stripes with -levels (else NULL): the leaves' parents and nodes of
+                          // 64 leaf bits before it within its brick (written for marked blocks)
+};
 
 // Mark bytes of a stripe's leaf level, padded to 16 bytes.
-__host__ __device__ inline uint64_t touch_bytes(const Level& leaf) { return (leaf.nblocks + 15) / 16 * 16; }
+__host__ __device__ inline uint64_t touch_bytes(int depth) { return (leaf_blocks(depth) + 15) / 16 * 16; }
+
+// Words of a stripe's counts as the host reads them.
+constexpr uint32_t kCountWords = 16;  // [0] leaves, [1] inner nodes below the bricks, [2 + l] nodes of upper level l
 
 // Inputs of the voxelization kernels for one stripe.
 struct VoxJob {
@@ -74,11 +90,10 @@ struct VoxJob {
   uint32_t* leafbits;       // level-Ds words
   uint8_t* leaftouch;       // byte per 256-bit block of leafbits, set when a bit of the block is (may be NULL)
   // pass B (payload winners)
-  const uint32_t* leafscan; // scan entries of level Ds (exclusive, minus its base)
-  const uint16_t* leaflocal;// marked leaf level: Pyramid::local (leafscan then has one entry per group)
-  uint32_t leafscan_base;
-  const uint64_t* leafwoff; // Pyramid::woff of the leaf level (the rank of a bit without a popcount per word)
-  uint32_t* winners;        // per leaf: min triangle index
+  const uint2* wpre;        // Stripe::wpre
+  const uint32_t* leaflocal;// Stripe::local
+  const uint64_t* leafwoff; // Stripe::woff
+  unsigned long long* winners;  // per leaf: min of triangle index << 32 | its local Morton code
   uint64_t* task_off;       // per item: exclusive prefix of warp tasks (n_items + 1)
   uint64_t* task_flag;      // set to 1 by an item with tasks (the sub-batch's task_off[items]); may be NULL
   unsigned long long* task_counter;
@@ -96,15 +111,11 @@ struct EmitJob {
   const float* tris;
   int stride;
   float unit_div;
-  const uint32_t* keys;     // per node: local key (Morton prefix within its level)
-  uint32_t* size;           // per node: nodes in its subtree
-  uint32_t* dsize;          // per node: data records in its subtree
-  uint32_t* start;          // per node: first node written inside its subtree, minus node_base
-  uint32_t* dstart;         // per node: its subtree's first data record, minus data_base
-  float* cache;             // per node: 6 floats (colour, normal); only with -levels
-  uint32_t* first_child;    // per internal node: global index of its first child
-  int leaf_inline;          // payload without -levels: the leaf payload pass writes the leaves' data records
-  const uint32_t* winners;
+  float* upper_cache;       // per cell of the upper levels and the bricks' children (upper_cell): its average; with -levels
+  uint32_t* root_out;       // 7 words for the host: the stripe root's child mask and its average
+  const unsigned long long* winners;  // per leaf: triangle << 32 | local Morton code
+  uint64_t n_leaf;          // leaves of the stripe (payload)
+  uint32_t bricks_per_warp; // of the emission
   uint64_t* node_win;       // node window (3 u64 per record)
   uint64_t node_win_base;   // global node index of node_win[0]
   unsigned char* data_win;  // data window (32 bytes per record)
@@ -115,12 +126,15 @@ struct EmitJob {
   uint32_t* flag;           // set non-zero by a kernel that finds an index out of range
   uint64_t node_base;       // file index of the stripe root's first written descendant
   uint64_t data_base;       // file index of the stripe's first data record
-  int l_small;              // levels 0..l_small (at most 256 nodes each) run in one CTA
+  uint64_t data_span;       // data records of the stripe
 };
 
+// Cell z of upper level l in the upper_cache.
+__host__ __device__ inline uint64_t upper_cell(int l, uint64_t z) { return ((1ull << (3 * l)) - 1) / 7 + z; }
+
 // Threads per CTA of the batched kernels; CTA b of a launch belongs to stripe s
-// when cta_beg[s] <= b < cta_beg[s+1] and handles that stripe's elements
-// kChunk * (b - cta_beg[s]) onward.
+// when cta_beg[s] <= b < cta_beg[s+1] and handles that stripe's elements from
+// its CTA b - cta_beg[s] on.
 constexpr uint32_t kChunk = 256;
 
 // The message ooc_last_error returns for `c` (for failures found outside ooc_api.cu).
@@ -163,7 +177,6 @@ struct LaunchScope {
   LaunchScope& operator=(const LaunchScope&) = delete;
 };
 
-void scan_u32_exclusive(uint32_t* data, uint64_t n, uint32_t* partials, cudaStream_t st);
 // flag_last: data[n-1] is not an input but a flag; zero means every element is zero,
 // and the scan is left out.
 void scan_u64_exclusive(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st, bool flag_last = false);
@@ -215,30 +228,16 @@ void launch_b_task_map(const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const
 void launch_b_vox_large(const VoxJob* jobs, const uint64_t* item_beg, uint32_t n_stripes, const uint64_t* task_off,
                         uint64_t total_items, unsigned long long* counter, int pass, cudaStream_t st, int num_sms,
                         int block, int ctas_per_sm, uint32_t lines_per_lane, const uint64_t* map, uint64_t cap);
-// Level depth - r of each stripe.
-void launch_b_pyramid(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept, int r,
-                      const Pyramid* single, cudaStream_t st);
-// One CTA per stripe: levels min(l_hi, depth) .. 0.
-// Also zeroes *scan_end, the block scan's total entry, before the scan.
-void launch_b_pyramid_top(const Pyramid* pyrs, uint32_t n_stripes, int l_hi, uint32_t* scan_end, cudaStream_t st);
-// The persistent phase-A kernel's inputs (ooc_tuning::persistent).
+// The persistent occupancy kernel's inputs (ooc_tuning::persistent).
 struct PersistJob {
   const VoxJob* jobs;
-  const Pyramid* pyrs;
   const uint64_t* item_beg;   // n + 1: first item of each stripe in the sub-batch
   uint32_t n;                 // stripes
-  uint32_t levels;            // R: pyramid levels below the top ones, at most (over the stripes)
   const uint64_t* chunk_beg;  // n + 1: prefix of 256-item chunks per stripe
-  const uint64_t* unit_beg;   // R x (n + 1): prefix of pyramid units per (level r, stripe), r-major, cumulative
-  uint32_t ept;               // elements per lane of a pyramid unit
-  int top_level;              // levels 0..top_level are the top levels
-  uint32_t* occ_left;         // n: occupancy units of each stripe not yet done (chunks, then its queued tasks)
-  uint32_t* pyr_left;         // R x n: pyramid units of (level r, stripe) not yet done
   unsigned long long* ctr;    // 64 counters, four used: tickets, chunks done, tasks reserved, timeout code
                               // (kCtr* in the kernel), each on its own 128-byte line
   unsigned long long* map;    // cap task entries (item | task << 32), all ones when empty
   uint64_t cap;
-  uint32_t* scan_end;         // the pyramid scan's total entry
   uint32_t lines_per_lane;
 };
 // CTAs of the persistent kernel one SM holds (0 on an error).
@@ -248,35 +247,36 @@ constexpr uint64_t kPersistChunkItems = 256;  // items of a chunk unit
 constexpr uint32_t kPersistCtrWords = 64;     // counters of the persistent kernel
 constexpr uint32_t kPersistTimeoutWord = 48;  // where it records the code of a wait that ran out
 constexpr uint32_t kPersistTasksWord = 32;    // where it counts the tasks it found (queued or not)
-void launch_b_compact(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept, uint32_t* keys,
-                      const Pyramid* single, cudaStream_t st);
-// Zero the marked leaf blocks of every stripe and the marks: one thread per 16 mark bytes.
-void launch_b_clean_leaves(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept,
-                           const Pyramid* single, cudaStream_t st);
-// out[s * (kMaxLevels + 1) + l] = global node index of level l's first node, l = 0..depth+1.
-// Also *tasks_out = *tasks (the large-item task count travels back with the level counts)
-// and *flag = 0 (the layout check flag the record kernels may set).
-// Level counts of every stripe and the task count (and, when `code` is set, the
-// persistent kernel's timeout code) into `out` (pinned host memory in the library's use).
-void launch_b_level_bases(const Pyramid* pyrs, uint32_t n_stripes, uint32_t* out, const uint64_t* tasks,
-                          uint64_t* tasks_out, uint32_t* flag, const uint64_t* code, uint64_t* code_out,
-                          cudaStream_t st);
-void launch_b_leaf_payload(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                           uint64_t ctas, uint32_t ept, const Pyramid* sp, const EmitJob* se, cudaStream_t st);
-// Level depth - r of each stripe.
-void launch_b_bottom_up(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept,
-                        int r, const Pyramid* sp, const EmitJob* se, cudaStream_t st);
-void launch_b_bottom_up_top(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, cudaStream_t st);
-void launch_b_top_down_top(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, cudaStream_t st);
-// Parents of absolute level l.
-void launch_b_top_down(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept,
-                       int l, const Pyramid* sp, const EmitJob* se, cudaStream_t st);
-void launch_b_top_down_leaves(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                              uint64_t ctas, uint32_t ept, const Pyramid* sp, const EmitJob* se, cudaStream_t st);
-// out[s * 16 + 0..6] = stripe s's root child mask and cache.
-// Root information of every stripe, and the layout check flag after it, written into
-// `out` (pinned host memory in the library's use).
-void launch_b_root_info(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, uint32_t* out,
-                        const uint32_t* flag, cudaStream_t st);
+
+// ---- the octree (ooc_tree.cu) ----
+// `single` / `sp`, `se` (may be NULL): the stripe (and emit job) of a one-stripe launch, passed
+// as kernel parameters.
+
+// Leaf and inner-node counts of every brick and word, and the level-U words: CTAs of kBrickCta warps,
+// brick_ctas per stripe.
+constexpr uint32_t kBrickCta = 4;
+inline uint32_t brick_ctas(const Stripe& s) {
+  return s.touch ? (upper_words(s.U) + kBrickCta - 1) / kBrickCta : upper_words(s.U);
+}
+void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const Stripe* single,
+                     cudaStream_t st);
+// One CTA per stripe: the upper levels' words and prefixes, and every stripe's counts (kCountWords each)
+// into `counts` (mapped pinned host memory), then *tasks and, when `code` is set, *code.
+void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts, const uint64_t* tasks,
+                    uint64_t* tasks_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st);
+// The payloads of the stripes' leaves, into the data file: CTAs of kChunk threads, `ept` leaves each.
+void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
+                           uint64_t ctas, uint32_t ept, const Stripe* sp, const EmitJob* se, cudaStream_t st);
+// Every brick's run of records and its own record, and (with `levels`) its averages; zeroes the leaf
+// levels and the marks.  CTAs of kTreeWarpsPerCta warps of EmitJob::bricks_per_warp non-empty bricks each.
+constexpr uint32_t kTreeWarpsPerCta = 8;
+void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
+                   bool levels, const Stripe* sp, const EmitJob* se, cudaStream_t st);
+// Averages of the upper levels above the bricks (-levels): one launch per level of more than 4,096 cells
+// and one for the rest.
+void launch_b_upper_avg(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st);
+// The records of the upper levels above the bricks, and the stripe roots' child masks and averages.
+void launch_b_upper_nodes(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
+                          uint64_t ctas, const Stripe* sp, const EmitJob* se, cudaStream_t st);
 
 }  // namespace ooc

@@ -10,6 +10,7 @@
 
 #include "ooc_device.cuh"
 #include "ooc_internal.h"
+#include "ooc_launch.cuh"
 
 namespace ooc {
 
@@ -22,89 +23,11 @@ LaunchScope::LaunchScope(LaunchState* s) : prev(t_launch) { t_launch = s; }
 LaunchScope::~LaunchScope() { t_launch = prev; }
 
 namespace {
-constexpr unsigned FULL = 0xffffffffu;
-
-// Counts one launch and brackets it with the timing hooks of the calling
-// thread's launch state, when one is installed.
-struct KScope {
-  const char* name;
-  cudaStream_t st;
-  LaunchState* ls;
-  KScope(const char* n, cudaStream_t s) : name(n), st(s), ls(t_launch) {
-    if (!ls) return;
-    ls->launches++;
-    if (ls->hooks.begin) ls->hooks.begin(ls->hooks.user, name, st);
-  }
-  ~KScope() {
-    if (ls && ls->hooks.end) ls->hooks.end(ls->hooks.user, name, st);
-  }
-};
-// Programmatic dependent launch.  Every kernel here first waits until the
-// grid before it on the stream has finished and its memory is visible, then
-// lets the grid after it launch, so that grid's CTAs take the SMs this one's
-// last CTAs free instead of waiting for the whole grid to drain.  Without the
-// launch attribute (launch_k with ooc_tuning::pdl off) both are no-ops.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" :::);
-}
-
-// Launch `k` on `st`, with programmatic stream serialization when the calling
-// thread's launch state asks for it.
-template <typename... P, typename... A>
-void launch_k(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = at;
-  cfg.numAttrs = (t_launch && t_launch->pdl) ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
-}
-
 constexpr int SCAN_THREADS = 256;
-
-inline unsigned grid_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 // ===========================================================================
 // Exclusive scan (three phases: per-CTA reduce, scan of CTA sums, down-sweep)
 // ===========================================================================
-template <typename T>
-__device__ __forceinline__ T warp_inclusive(T v) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const T y = __shfl_up_sync(FULL, v, o);
-    if (lane >= o) v += y;
-  }
-  return v;
-}
-
-// Exclusive scan of one value per thread across the CTA; `total` gets the CTA sum.
-template <typename T>
-__device__ __forceinline__ T block_exclusive(T v, T& total) {
-  __shared__ T warp_sums[33];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const T inc = warp_inclusive(v);
-  if (lane == 31) warp_sums[warp] = inc;
-  __syncthreads();
-  if (warp == 0) {
-    const T w = lane < nw ? warp_sums[lane] : T(0);
-    const T wi = warp_inclusive(w);
-    if (lane < nw) warp_sums[lane] = wi - w;
-    if (lane == 31) warp_sums[32] = wi;
-  }
-  __syncthreads();
-  const T r = inc - v + warp_sums[warp];
-  total = warp_sums[32];
-  __syncthreads();
-  return r;
-}
-
 constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
@@ -455,19 +378,6 @@ __device__ __forceinline__ bool item_box(const VoxJob& j, const TriVerts& tv, in
   return lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2];
 }
 
-// Set bits before bit `b` inside its 256-bit block (`blk` points at the block's 8 words).
-__device__ __forceinline__ uint32_t in_block_rank(const uint32_t* __restrict__ blk, uint64_t b) {
-  const uint4* q = reinterpret_cast<const uint4*>(blk);
-  const uint4 q0 = q[0], q1 = q[1];
-  const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-  const uint32_t wi = (uint32_t)(b >> 5) & 7u;
-  const uint32_t lowmask = (1u << (b & 31)) - 1u;
-  uint32_t r = 0;
-#pragma unroll
-  for (uint32_t k = 0; k < 8; k++) r += __popc(k < wi ? w[k] : (k == wi ? (w[k] & lowmask) : 0u));
-  return r;
-}
-
 // Sets `acc` in leaf word w and marks the word's 256-bit block, so every
 // block with a set bit is marked.  The mark is a plain byte store: threads
 // that mark the same block store the same value, and nothing reads the marks
@@ -477,16 +387,19 @@ __device__ __forceinline__ void set_leaf(const VoxJob& j, uint32_t w, uint32_t a
   if (j.leaftouch) j.leaftouch[w >> 3] = 1;
 }
 
-// Rank of bit `b` among the set bits of the leaf level.
+// Rank of bit `b` among the set bits of the leaf level: the set bits before its
+// 32-brick word, before its block within the word's bricks, before its leaf word
+// within the block (all from the brick pass), and one popcount.
 __device__ __forceinline__ uint32_t leaf_rank(const VoxJob& j, uint32_t b) {
   const uint32_t blk = b >> 8;
-  const uint32_t base = j.leaflocal ? j.leafscan[blk / kLeafGroup] + j.leaflocal[blk] : j.leafscan[blk];
-  if (j.leafwoff) {  // the set bits before the bit's word, from the pyramid pass, and one popcount
-    const uint32_t wi = (b >> 5) & 7u;
-    const uint32_t before = (uint32_t)(j.leafwoff[blk] >> (8 * wi)) & 0xffu;
-    return base - j.leafscan_base + before + __popc(j.leafbits[b >> 5] & ((1u << (b & 31)) - 1u));
-  }
-  return base - j.leafscan_base + in_block_rank(j.leafbits + (uint64_t)blk * 8, b);
+  const uint32_t before = (uint32_t)(j.leafwoff[blk] >> (8 * ((b >> 5) & 7u))) & 0xffu;
+  return j.wpre[b >> 17].x + j.leaflocal[blk] + before + __popc(j.leafbits[b >> 5] & ((1u << (b & 31)) - 1u));
+}
+
+// Offers triangle t to voxel m: the smallest index wins, and the voxel's Morton code
+// travels with it to the leaf payload pass, which then needs no search for it.
+__device__ __forceinline__ void offer(const VoxJob& j, uint32_t m, uint32_t t) {
+  atomicMin(&j.winners[leaf_rank(j, m)], ((unsigned long long)t << 32) | m);
 }
 
 __device__ __forceinline__ uint64_t item_triangle(const VoxJob& j, uint64_t i) {
@@ -555,7 +468,7 @@ __device__ __forceinline__ void vox_line(const VoxJob& j, const TriSetup& s, uin
       }
       acc |= 1u << (m & 31);
     } else {
-      atomicMin(&j.winners[leaf_rank(j, m)], tri);  // pass 0 set this voxel's bit
+      offer(j, m, tri);  // pass 0 set this voxel's bit
     }
   };
   if (!mono) {  // every voxel of the line, complete test
@@ -864,7 +777,7 @@ __device__ __forceinline__ void vox_small_win_item(const VoxJob& j, uint64_t i) 
     const uint32_t col = (q * rz) >> 16, z = q - col * bz;
     const uint32_t x = (col * ry) >> 16, y = col - x * by;
     const uint32_t m = morton_local(lx + x, ly + y, lz + z);
-    atomicMin(&j.winners[leaf_rank(j, m)], t);
+    offer(j, m, t);
   }
 }
 
@@ -949,601 +862,6 @@ __global__ void __launch_bounds__(256, 4) k_vox_large(VoxJob j) {
   }
 }
 
-// ===========================================================================
-// Occupancy pyramid: level l-1 bit i = (byte i of level l != 0); the byte is
-// node i's 8-bit child mask.  Also the popcount of every 256-bit block.
-// ===========================================================================
-__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
-  const uint32_t t = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
-  return ((t >> 7) & 1u) | ((t >> 14) & 2u) | ((t >> 21) & 4u) | ((t >> 28) & 8u);
-}
-
-// First word of level l (levels zl.. live in the buffer kept zero between builds).
-__device__ __forceinline__ uint32_t* level_words(const Pyramid& p, int l) {
-  return (l >= p.zl ? p.leaf : p.bits) + p.lv[l].off_w;
-}
-
-// Whether the leaf blocks under block b of level depth-1 (leaf blocks 8b..8b+7,
-// one word of that block each) are all unmarked, so the block is zero.
-// CG: the loads go to L2 (ld.global.cg), for data that other SMs wrote in the
-// same launch (the persistent phase-A kernel); otherwise plain loads.
-template <bool CG>
-__device__ __forceinline__ uint4 ld4(const uint4* p) {
-  if constexpr (CG) return __ldcg(p);
-  else return *p;
-}
-
-template <bool CG = false>
-__device__ __forceinline__ bool parent_block_empty(const Pyramid& p, uint64_t b) {
-  const unsigned long long* t = reinterpret_cast<const unsigned long long*>(p.touch) + b;
-  if constexpr (CG) return __ldcg(t) == 0ull;
-  else return *t == 0ull;
-}
-
-// Block b of level l (not a marked leaf level): its popcount and parent word.
-template <bool CG = false>
-__device__ __forceinline__ void pyramid_block(const Pyramid& p, int l, uint64_t b) {
-  const Level& L = p.lv[l];
-  if (p.touch && l == p.depth - 1 && parent_block_empty<CG>(p, b)) {
-    p.scan[L.off_b + b] = 0u;
-    if (l > 0) level_words(p, l - 1)[b] = 0u;
-    return;
-  }
-  const uint4* q = reinterpret_cast<const uint4*>(level_words(p, l) + 8 * b);
-  const uint4 q0 = ld4<CG>(q), q1 = ld4<CG>(q + 1);
-  const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-  uint32_t c = 0, pw = 0;
-  uint64_t wo = 0;  // byte k: set bits in words 0..k-1 (at most 224)
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    wo |= (uint64_t)c << (8 * k);
-    c += __popc(w[k]);
-    pw |= nonzero_bytes(w[k]) << (4 * k);
-  }
-  p.scan[L.off_b + b] = c;
-  if (l > 0) level_words(p, l - 1)[b] = pw;
-  if (l == p.depth && p.woff) p.woff[b] = wo;
-}
-
-// Global node index of the first node of block blk of level l: the
-// concatenated scan already counts every node of the shallower levels.
-__device__ __forceinline__ uint64_t block_base(const Pyramid& p, int l, uint64_t blk) {
-  if (l == p.depth && p.touch) return (uint64_t)p.scan[p.lv[l].off_b + blk / kLeafGroup] + p.local[blk];
-  return p.scan[p.lv[l].off_b + blk];
-}
-
-// Global node index of bit `b` of level l.
-__device__ __forceinline__ uint64_t node_index(const Pyramid& p, int l, uint64_t b) {
-  const uint64_t blk = b >> 8;
-  if (l == p.depth && p.woff) {  // the leaf level of a payload stripe: word offsets from the pyramid pass
-    const uint32_t wi = (uint32_t)(b >> 5) & 7u;
-    return block_base(p, l, blk) + ((p.woff[blk] >> (8 * wi)) & 0xffu) +
-           __popc(level_words(p, l)[b >> 5] & ((1u << (b & 31)) - 1u));
-  }
-  return block_base(p, l, blk) + in_block_rank(level_words(p, l) + blk * 8, b);
-}
-
-// A marked leaf level, group q of kLeafGroup blocks: the parent words, the
-// group's node count (its scan entry) and each marked block's offset in it.
-template <bool CG = false>
-__device__ __forceinline__ void leaf_group(const Pyramid& p, uint64_t q) {
-  static_assert(kLeafGroup == 16, "one uint4 of marks per group");
-  const Level& L = p.lv[p.depth];
-  const uint4 m4 = ld4<CG>(reinterpret_cast<const uint4*>(p.touch) + q);
-  uint4* parent = reinterpret_cast<uint4*>(level_words(p, p.depth - 1) + q * kLeafGroup);
-  if (!(m4.x | m4.y | m4.z | m4.w)) {  // the parent words stay zero
-    p.scan[L.off_b + q] = 0u;
-    return;
-  }
-  const uint32_t mw[4] = {m4.x, m4.y, m4.z, m4.w};
-  uint32_t pw[16];
-  uint32_t total = 0;
-#pragma unroll
-  for (int k = 0; k < 16; k++) {
-    pw[k] = 0u;
-    if ((mw[k >> 2] >> (8 * (k & 3))) & 0xffu) {
-      const uint64_t b = q * kLeafGroup + (uint64_t)k;
-      const uint4* w4 = reinterpret_cast<const uint4*>(level_words(p, p.depth) + 8 * b);
-      const uint4 q0 = ld4<CG>(w4), q1 = ld4<CG>(w4 + 1);
-      const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-      uint32_t c = 0;
-      uint64_t wo = 0;
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        wo |= (uint64_t)c << (8 * i);
-        c += __popc(w[i]);
-        pw[k] |= nonzero_bytes(w[i]) << (4 * i);
-      }
-      if (p.woff) p.woff[b] = wo;
-      p.local[b] = (uint16_t)total;
-      total += c;
-    }
-  }
-  parent[0] = make_uint4(pw[0], pw[1], pw[2], pw[3]);
-  parent[1] = make_uint4(pw[4], pw[5], pw[6], pw[7]);
-  parent[2] = make_uint4(pw[8], pw[9], pw[10], pw[11]);
-  parent[3] = make_uint4(pw[12], pw[13], pw[14], pw[15]);
-  p.scan[L.off_b + q] = total;
-}
-
-__device__ __forceinline__ uint32_t child_mask(const Pyramid& p, int l, uint32_t k) {
-  return (level_words(p, l)[k >> 2] >> ((k & 3) * 8)) & 0xffu;
-}
-
-// Keys of block lb of level l, from node index r on.
-__device__ __forceinline__ void block_keys(const uint32_t* __restrict__ words, uint64_t lb, uint64_t r,
-                                           uint32_t* __restrict__ keys) {
-  const uint4* q = reinterpret_cast<const uint4*>(words + 8 * lb);
-  const uint4 q0 = q[0], q1 = q[1];
-  if (!(q0.x | q0.y | q0.z | q0.w | q1.x | q1.y | q1.z | q1.w)) return;
-  const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-  const uint64_t wl0 = lb * 8;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    uint32_t word = w[k];
-    while (word) {
-      const int bit = __ffs(word) - 1;
-      keys[r++] = (uint32_t)(((wl0 + k) << 5) | (uint64_t)bit);
-      word &= word - 1;
-    }
-  }
-}
-
-// Keys of all levels in one launch.  The elements of a stripe are the blocks
-// of levels 0..depth-1 (blocks are 8 aligned words and never straddle two
-// levels), padded to a multiple of 32, then the leaf level's scan entries,
-// padded likewise, so every warp works on one region.  An unmarked leaf level
-// has one element per block.  In a marked leaf level each lane takes a group
-// of kLeafGroup blocks; the warp gathers the marked blocks of its 32 groups and
-// hands them out one per lane.
-__device__ __forceinline__ uint64_t compact_elems(const Pyramid& p) {
-  const uint64_t upper = p.lv[p.depth].off_b - p.lv[0].off_b;
-  return (upper + 31) / 32 * 32 + (p.lv[p.depth].nscan + 31) / 32 * 32;
-}
-
-__device__ __forceinline__ void compact_elem(const Pyramid& p, uint64_t e, uint32_t* __restrict__ keys) {
-  const Level& L = p.lv[p.depth];
-  const uint64_t first = p.lv[0].off_b, upper = L.off_b - first, up32 = (upper + 31) / 32 * 32;
-  if (e >= compact_elems(p)) return;  // whole warps
-  if (e < up32) {
-    if (e >= upper) return;
-    int l = p.depth - 1;  // most upper blocks are on the level above the leaves
-    if (first + e < p.lv[l].off_b) {
-      l = 0;
-      while (p.lv[l + 1].off_b <= first + e) l++;
-    }
-    const uint64_t lb = first + e - p.lv[l].off_b;
-    if (p.touch && l == p.depth - 1 && parent_block_empty(p, lb)) return;
-    block_keys(level_words(p, l), lb, p.scan[first + e], keys);
-    return;
-  }
-  const uint64_t q = e - up32;
-  if (!p.touch) {
-    if (q < L.nblocks) block_keys(level_words(p, p.depth), q, p.scan[L.off_b + q], keys);
-    return;
-  }
-  // marked leaf level: all 32 lanes of the warp are here
-  const int lane = threadIdx.x & 31;
-  uint32_t marked = 0;  // bit k: block k of group q is marked
-  if (q < L.nscan) {
-    const uint4 m4 = reinterpret_cast<const uint4*>(p.touch)[q];
-    marked = nonzero_bytes(m4.x) | (nonzero_bytes(m4.y) << 4) | (nonzero_bytes(m4.z) << 8) | (nonzero_bytes(m4.w) << 12);
-  }
-  const uint32_t cnt = __popc(marked);
-  uint32_t incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += y;
-  }
-  const uint32_t total = __shfl_sync(FULL, incl, 31);
-  const uint64_t q0 = q - (uint64_t)lane;
-  for (uint32_t round = 0; round < total; round += 32) {
-    const uint32_t j = round + (uint32_t)lane;  // this lane's marked block, in warp order
-    uint32_t o = 0;                             // its owner lane: the first with incl > j
-#pragma unroll
-    for (uint32_t st = 16; st; st >>= 1) {
-      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
-      if (t <= j) o += st;
-    }
-    uint32_t m = __shfl_sync(FULL, marked, (int)o);
-    const uint32_t before = __shfl_sync(FULL, incl - cnt, (int)o);
-    if (j < total) {
-      for (uint32_t k = j - before; k; k--) m &= m - 1;
-      const uint64_t qo = q0 + o;
-      const uint64_t blk = qo * kLeafGroup + (uint64_t)(__ffs(m) - 1);
-      block_keys(level_words(p, p.depth), blk, (uint64_t)p.scan[L.off_b + qo] + p.local[blk], keys);
-    }
-  }
-}
-
-// Mark bytes 16i .. 16i+15 of a stripe: zero their marked leaf blocks, the
-// group's 16 parent words, then the marks.  A stripe without marks has its 16
-// leaf blocks zeroed outright.
-__device__ __forceinline__ void clean_touch16(const Pyramid& p, uint64_t i) {
-  if (i * 16 >= touch_bytes(p.lv[p.depth])) return;
-  if (!p.touch) {  // T threads zero the level's 2 x nblocks <= 32 T uint4, coalesced
-    const uint64_t T = touch_bytes(p.lv[p.depth]) / 16, n4 = p.lv[p.depth].nwords / 4;
-    uint4* leaf = reinterpret_cast<uint4*>(level_words(p, p.depth));
-    for (uint64_t q = i; q < n4; q += T) leaf[q] = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  uint4* t4 = reinterpret_cast<uint4*>(p.touch) + i;
-  const uint4 t = *t4;
-  if (!(t.x | t.y | t.z | t.w)) return;
-  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-  *t4 = z;
-  uint4* parent = reinterpret_cast<uint4*>(level_words(p, p.depth - 1) + i * 16);  // the group's 16 parent words
-  parent[0] = z;
-  parent[1] = z;
-  parent[2] = z;
-  parent[3] = z;
-  uint4* leaf = reinterpret_cast<uint4*>(level_words(p, p.depth));
-  const uint32_t tw[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const uint32_t nz = nonzero_bytes(tw[q]);  // bit k: mark byte k of this word is set
-    for (uint32_t m = nz; m; m &= m - 1) {
-      const uint64_t blk = i * 16 + (uint64_t)(4 * q + __ffs(m) - 1);
-      leaf[2 * blk] = z;
-      leaf[2 * blk + 1] = z;
-    }
-  }
-}
-
-// ===========================================================================
-// Leaf payload (voxelizer.cpp:295-299, BarycentricCoords.h, main.cpp:373-382)
-// ===========================================================================
-__device__ void payload_color(const TriVerts& tv, const float n[3], int x, int y, int z, float unit_div,
-                              const float* __restrict__ tr, float col[3]) {
-  const float qx = __fdiv_rn((float)x, unit_div);
-  const float qy = __fdiv_rn((float)y, unit_div);
-  const float qz = __fdiv_rn((float)z, unit_div);
-  const float coeffD = -dot3(tv.v[0][0], tv.v[0][1], tv.v[0][2], n[0], n[1], n[2]);
-  const float nn = __fadd_rn(__fadd_rn(__fmul_rn(n[0], n[0]), __fmul_rn(n[1], n[1])), __fmul_rn(n[2], n[2]));
-  const float k = __fdiv_rn(__fadd_rn(dot3(qx, qy, qz, n[0], n[1], n[2]), coeffD), nn);
-  const float ptx = __fsub_rn(qx, __fmul_rn(k, n[0]));
-  const float pty = __fsub_rn(qy, __fmul_rn(k, n[1]));
-  const float ptz = __fsub_rn(qz, __fmul_rn(k, n[2]));
-  // inverse(mat3(v0, v1, v2)) by adjugate over determinant
-  const float a = tv.v[0][0], b = tv.v[1][0], c = tv.v[2][0];
-  const float d = tv.v[0][1], e = tv.v[1][1], f = tv.v[2][1];
-  const float g = tv.v[0][2], h = tv.v[1][2], i = tv.v[2][2];
-  const float C00 = __fsub_rn(__fmul_rn(e, i), __fmul_rn(f, h));
-  const float C01 = __fsub_rn(__fmul_rn(f, g), __fmul_rn(d, i));
-  const float C02 = __fsub_rn(__fmul_rn(d, h), __fmul_rn(e, g));
-  const float det = __fadd_rn(__fadd_rn(__fmul_rn(a, C00), __fmul_rn(b, C01)), __fmul_rn(c, C02));
-  const float r = __fdiv_rn(1.0f, det);
-  const float C10 = __fsub_rn(__fmul_rn(c, h), __fmul_rn(b, i));
-  const float C11 = __fsub_rn(__fmul_rn(a, i), __fmul_rn(c, g));
-  const float C12 = __fsub_rn(__fmul_rn(b, g), __fmul_rn(a, h));
-  const float C20 = __fsub_rn(__fmul_rn(b, f), __fmul_rn(c, e));
-  const float C21 = __fsub_rn(__fmul_rn(c, d), __fmul_rn(a, f));
-  const float C22 = __fsub_rn(__fmul_rn(a, e), __fmul_rn(b, d));
-  const float i00 = __fmul_rn(C00, r), i10 = __fmul_rn(C01, r), i20 = __fmul_rn(C02, r);
-  const float i01 = __fmul_rn(C10, r), i11 = __fmul_rn(C11, r), i21 = __fmul_rn(C12, r);
-  const float i02 = __fmul_rn(C20, r), i12 = __fmul_rn(C21, r), i22 = __fmul_rn(C22, r);
-  const float bx = __fadd_rn(__fadd_rn(__fmul_rn(i00, ptx), __fmul_rn(i01, pty)), __fmul_rn(i02, ptz));
-  const float by = __fadd_rn(__fadd_rn(__fmul_rn(i10, ptx), __fmul_rn(i11, pty)), __fmul_rn(i12, ptz));
-  const float bz = __fadd_rn(__fadd_rn(__fmul_rn(i20, ptx), __fmul_rn(i21, pty)), __fmul_rn(i22, ptz));
-#pragma unroll
-  for (int q = 0; q < 3; q++) {
-    const float c0 = __ldg(tr + 12 + q), c1 = __ldg(tr + 15 + q), c2 = __ldg(tr + 18 + q);
-    col[q] = __fadd_rn(__fadd_rn(__fmul_rn(bx, c0), __fmul_rn(by, c1)), __fmul_rn(bz, c2));
-  }
-}
-
-// Colour and normal of leaf `li` (its index within the leaf level), local key `key`.
-// Returns false (and flags) if the leaf has no winning triangle.
-__device__ bool leaf_value(const EmitJob& e, uint64_t li, uint32_t key, float out[6]) {
-  uint32_t lx, ly, lz;
-  morton_local_decode(key, lx, ly, lz);
-  const int x = e.origin[0] + (int)lx, y = e.origin[1] + (int)ly, z = e.origin[2] + (int)lz;
-  const uint64_t t = e.winners[li];
-  if (t >= e.n_tris) {  // every set voxel has a passing triangle; anything else is a bug
-    atomicOr(e.flag, 4u);
-    return false;
-  }
-  const float* tr = e.tris + t * 21;
-  const float nx = __ldg(tr + 9), ny = __ldg(tr + 10), nz = __ldg(tr + 11);
-  if (e.color_mode == 1) {  // COLOR_FIXED
-    out[0] = out[1] = out[2] = 1.0f;
-  } else if (e.color_mode == 2) {  // COLOR_LINEAR: mortonToRGB (svo_builder_util.h:14-18)
-    const float fn = (float)e.gridsize;
-    out[0] = __fdiv_rn((float)z, fn);
-    out[1] = __fdiv_rn((float)y, fn);
-    out[2] = __fdiv_rn((float)x, fn);
-  } else if (e.color_mode == 3) {  // COLOR_NORMAL
-    float a = nx, b = ny, c = nz;
-    normalize3(a, b, c);
-    out[0] = __fdiv_rn(__fadd_rn(a, 1.0f), 2.0f);
-    out[1] = __fdiv_rn(__fadd_rn(b, 1.0f), 2.0f);
-    out[2] = __fdiv_rn(__fadd_rn(c, 1.0f), 2.0f);
-  } else {  // COLOR_FROM_MODEL
-    const TriVerts tv = load_verts(e.tris, t, 21);
-    float n[3];
-    tri_normal(tv, n);
-    payload_color(tv, n, x, y, z, e.unit_div, tr, out);
-  }
-  out[3] = nx;
-  out[4] = ny;
-  out[5] = nz;
-  return true;
-}
-
-__device__ __forceinline__ void store_data_record(const EmitJob& e, uint64_t idx, uint64_t morton, const float* v);
-
-// Leaf payloads: with -levels into the per-node cache (the averages need them);
-// without, straight into the data file, where leaf i of the stripe is data record
-// data_base + i (its data records are its leaves in key order), so the data file
-// is final before the node records are laid out.
-__device__ __forceinline__ void leaf_payload(const Pyramid& p, const EmitJob& e, uint64_t i) {
-  const Level& L = p.lv[p.depth];
-  const uint32_t k = e.keys[L.koff + i];
-  float v[6];
-  if (!leaf_value(e, i, k, v)) return;
-  if (e.levels) {
-    float* out = e.cache + (L.koff + i) * 6;
-#pragma unroll
-    for (int q = 0; q < 6; q++) out[q] = v[q];
-  } else {
-    store_data_record(e, e.data_base + i, e.stripe_base + k, v);
-  }
-}
-
-// ===========================================================================
-// Octree layout.  Subtree sizes bottom-up, then top-down the index of the
-// first node / data record written inside every subtree; the reference writes
-// a node's 8-child group when the Morton cursor leaves the node's region, so
-// the node file is the post-order of groups (OctreeBuilder.cpp:58-128).
-// ===========================================================================
-__device__ __forceinline__ void average_children(const EmitJob& e, uint32_t mask, uint64_t c0, bool child_leaf,
-                                                 float out[6]) {
-  // OctreeBuilder.cpp:81-99: sum over the 8 slots in child order (null slots
-  // add zero), divide by the non-null count, normalise the normal.
-  float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  float notnull = 0.0f;
-  uint64_t c = c0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    if ((mask >> k) & 1u) {
-      notnull = __fadd_rn(notnull, 1.0f);
-      if (child_leaf && e.binary) {
-#pragma unroll
-        for (int q = 0; q < 6; q++) acc[q] = __fadd_rn(acc[q], 0.0f);
-      } else {
-        const float* cc = e.cache + c * 6;
-#pragma unroll
-        for (int q = 0; q < 6; q++) acc[q] = __fadd_rn(acc[q], cc[q]);
-      }
-      c++;
-    } else {
-#pragma unroll
-      for (int q = 0; q < 6; q++) acc[q] = __fadd_rn(acc[q], 0.0f);
-    }
-  }
-  out[0] = __fdiv_rn(acc[0], notnull);
-  out[1] = __fdiv_rn(acc[1], notnull);
-  out[2] = __fdiv_rn(acc[2], notnull);
-  float tx = __fdiv_rn(acc[3], notnull), ty = __fdiv_rn(acc[4], notnull), tz = __fdiv_rn(acc[5], notnull);
-  normalize3(tx, ty, tz);
-  out[3] = tx;
-  out[4] = ty;
-  out[5] = tz;
-}
-
-// Subtree node / data counts, first-child index and (-levels) averages of node i of level l.
-__device__ __forceinline__ void bottom_up_node(const Pyramid& p, const EmitJob& e, int l, uint64_t i) {
-  const Level& L = p.lv[l];
-  const uint64_t gi = L.koff + i;
-  const uint32_t k = e.keys[gi];
-  const uint32_t mask = child_mask(p, l + 1, k);
-  const int nch = __popc(mask);
-  const uint64_t c0 = node_index(p, l + 1, (uint64_t)k << 3);
-  const bool child_leaf = (l + 1 == p.depth);
-  uint32_t sz, dsz;
-  if (child_leaf) {
-    sz = 1u + (uint32_t)nch;
-    dsz = (uint32_t)e.levels + (e.binary ? 0u : (uint32_t)nch);
-  } else {
-    sz = 1u;
-    dsz = (uint32_t)e.levels;
-    for (int q = 0; q < nch; q++) {
-      sz += e.size[c0 + q];
-      dsz += e.dsize[c0 + q];
-    }
-  }
-  e.size[gi] = sz;
-  e.dsize[gi] = dsz;
-  e.first_child[gi] = (uint32_t)c0;
-  if (e.levels) average_children(e, mask, c0, child_leaf, e.cache + gi * 6);
-}
-
-__device__ __forceinline__ void store_data_record(const EmitJob& e, uint64_t idx, uint64_t morton, const float* v) {
-  if (idx < e.data_win_base || idx - e.data_win_base >= e.data_win_len) {
-    atomicOr(e.flag, 2u);
-    return;
-  }
-  uint4* dst = reinterpret_cast<uint4*>(e.data_win + (idx - e.data_win_base) * 32);
-  dst[0] = make_uint4((uint32_t)morton, (uint32_t)(morton >> 32), __float_as_uint(v[0]), __float_as_uint(v[1]));
-  dst[1] = make_uint4(__float_as_uint(v[2]), __float_as_uint(v[3]), __float_as_uint(v[4]), __float_as_uint(v[5]));
-}
-
-__device__ __forceinline__ void store_node_record(const EmitJob& e, uint64_t pos, uint64_t r0, uint64_t r1,
-                                                  uint64_t r2) {
-  if (pos < e.node_win_base || pos - e.node_win_base >= e.node_win_len) {
-    atomicOr(e.flag, 1u);
-    return;
-  }
-  uint64_t* rec = e.node_win + (pos - e.node_win_base) * 3;
-  rec[0] = r0;
-  rec[1] = r1;
-  rec[2] = r2;
-}
-
-__device__ __forceinline__ uint64_t child_offsets(uint32_t mask) {
-  uint64_t off = 0;
-  uint32_t r = 0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const uint64_t byte = ((mask >> k) & 1u) ? (uint64_t)(r++) : 0xffull;
-    off |= byte << (8 * k);
-  }
-  return off;
-}
-
-// Node i of level l (internal) writes its children's records: they form one
-// contiguous group at its children_base, in child order (groupNodes,
-// OctreeBuilder.cpp:58-79), and each child's subtree starts where the
-// previous sibling's subtree ended.
-__device__ __forceinline__ void top_down_node(const Pyramid& p, const EmitJob& e, int l, uint64_t i) {
-  const Level& L = p.lv[l];
-  const uint64_t gi = L.koff + i;
-  const uint32_t k = e.keys[gi];
-  const uint32_t mask = child_mask(p, l + 1, k);
-  const int nch = __popc(mask);
-  const uint64_t st = e.node_base + e.start[gi];
-  uint64_t run_d = e.data_base + e.dstart[gi];
-  uint64_t run_s = st;
-  const uint64_t cb = st + (uint64_t)e.size[gi] - 1 - (uint64_t)nch;
-  const uint64_t c0 = e.first_child[gi];
-  const bool child_leaf = (l + 1 == p.depth);
-  if (!child_leaf) {
-    // every child's loads first (they are independent), then the running sums and stores
-    uint32_t kc[8], szc[8], dszc[8], mc[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (j < nch) {
-        kc[j] = e.keys[c0 + j];
-        szc[j] = e.size[c0 + j];
-        dszc[j] = e.dsize[c0 + j];
-      }
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (j < nch) mc[j] = child_mask(p, l + 2, kc[j]);
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (j < nch) {
-        const uint64_t c = c0 + (uint64_t)j;
-        e.start[c] = (uint32_t)(run_s - e.node_base);
-        e.dstart[c] = (uint32_t)(run_d - e.data_base);
-        const uint64_t di = run_d + dszc[j] - 1;
-        store_node_record(e, cb + j, e.levels ? di : 0, run_s + szc[j] - 1 - (uint64_t)__popc(mc[j]),
-                          child_offsets(mc[j]));
-        if (e.levels) store_data_record(e, di, 0, e.cache + c * 6);
-        run_s += szc[j] - 1;
-        run_d += dszc[j];
-      }
-    return;
-  }
-  for (int j = 0; j < nch; j++) {
-    const uint64_t c = c0 + (uint64_t)j;
-    const uint32_t kc = e.keys[c];
-    if (e.binary) {
-      store_node_record(e, cb + j, 1, 0, ~0ull);
-    } else {
-      store_node_record(e, cb + j, run_d, 0, ~0ull);
-      if (!e.leaf_inline) {  // (without -levels the leaf payload pass wrote the data record)
-        float v[6];
-#pragma unroll
-        for (int q = 0; q < 6; q++) v[q] = e.cache[c * 6 + q];
-        store_data_record(e, run_d, e.stripe_base + kc, v);
-      }
-      run_d += 1;
-    }
-  }
-}
-
-// Children of level l+1, one thread per child, two at once (i0 < i1; either may
-// be past the level's end).  A child finds its parent's run starts and adds its
-// earlier siblings' subtree sizes (siblings are consecutive in the key order), so
-// the launch reads and writes the child level contiguously.  Every load of both
-// children is issued before the first store, so their chains of dependent loads
-// overlap.
-__device__ __forceinline__ void top_down_children(const Pyramid& p, const EmitJob& e, int l, uint64_t i0, uint64_t i1) {
-  const Level& C = p.lv[l + 1];
-  if (i0 >= C.n) return;
-  const bool v1 = i1 < C.n;
-  const uint64_t c0 = C.koff + i0, c1 = C.koff + (v1 ? i1 : i0);
-  const uint32_t kc0 = e.keys[c0], kc1 = e.keys[c1];
-  const uint64_t p0 = node_index(p, l, kc0 >> 3), p1 = node_index(p, l, kc1 >> 3);
-  const uint64_t f0 = e.first_child[p0], f1 = e.first_child[p1];
-  const uint32_t pm0 = child_mask(p, l + 1, kc0 >> 3), pm1 = child_mask(p, l + 1, kc1 >> 3);
-  uint64_t rs0 = e.node_base + e.start[p0], rd0 = e.data_base + e.dstart[p0];
-  uint64_t rs1 = e.node_base + e.start[p1], rd1 = e.data_base + e.dstart[p1];
-  const uint64_t cb0 = rs0 + (uint64_t)e.size[p0] - 1 - (uint64_t)__popc(pm0);
-  const uint64_t cb1 = rs1 + (uint64_t)e.size[p1] - 1 - (uint64_t)__popc(pm1);
-  const uint32_t mc0 = child_mask(p, l + 2, kc0), mc1 = child_mask(p, l + 2, kc1);
-  const uint64_t sz0 = e.size[c0], dsz0 = e.dsize[c0], sz1 = e.size[c1], dsz1 = e.dsize[c1];
-  for (uint64_t q = f0; q < c0; q++) {
-    rs0 += (uint64_t)e.size[q] - 1;
-    rd0 += e.dsize[q];
-  }
-  for (uint64_t q = f1; q < c1; q++) {
-    rs1 += (uint64_t)e.size[q] - 1;
-    rd1 += e.dsize[q];
-  }
-  e.start[c0] = (uint32_t)(rs0 - e.node_base);
-  e.dstart[c0] = (uint32_t)(rd0 - e.data_base);
-  const uint64_t di0 = rd0 + dsz0 - 1;
-  store_node_record(e, cb0 + (c0 - f0), e.levels ? di0 : 0, rs0 + sz0 - 1 - (uint64_t)__popc(mc0), child_offsets(mc0));
-  if (e.levels) store_data_record(e, di0, 0, e.cache + c0 * 6);
-  if (!v1) return;
-  e.start[c1] = (uint32_t)(rs1 - e.node_base);
-  e.dstart[c1] = (uint32_t)(rd1 - e.data_base);
-  const uint64_t di1 = rd1 + dsz1 - 1;
-  store_node_record(e, cb1 + (c1 - f1), e.levels ? di1 : 0, rs1 + sz1 - 1 - (uint64_t)__popc(mc1), child_offsets(mc1));
-  if (e.levels) store_data_record(e, di1, 0, e.cache + c1 * 6);
-}
-
-// Leaf records, one thread per leaf: the parent (level depth-1) already knows
-// where its child group and data run start.
-__device__ __forceinline__ void top_down_leaf(const Pyramid& p, const EmitJob& e, uint64_t i) {
-  const Level& L = p.lv[p.depth];
-  const uint64_t gi = L.koff + i;
-  const uint32_t k = e.keys[gi];
-  const uint32_t pk = k >> 3;
-  const uint64_t pidx = node_index(p, p.depth - 1, pk);
-  const uint64_t rank = gi - e.first_child[pidx];
-  const uint32_t pmask = child_mask(p, p.depth, pk);
-  const uint64_t pcb = e.node_base + e.start[pidx] + (uint64_t)e.size[pidx] - 1 - (uint64_t)__popc(pmask);
-  if (e.binary) {
-    store_node_record(e, pcb + rank, 1, 0, ~0ull);
-    return;
-  }
-  const uint64_t di = e.data_base + e.dstart[pidx] + rank;
-  store_node_record(e, pcb + rank, di, 0, ~0ull);
-  if (e.leaf_inline) return;  // the leaf payload pass wrote the data record
-  float v[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) v[q] = e.cache[gi * 6 + q];
-  store_data_record(e, di, e.stripe_base + k, v);
-}
-
-// Stripe root: child mask and payload for the host, and (with -levels, or a
-// one-voxel stripe in payload mode) the root's own data record.
-__device__ void root_info(const Pyramid& p, const EmitJob& e, uint64_t data_base, uint32_t* out) {
-  const uint64_t r0 = p.lv[0].koff;  // global node index of the stripe root
-  float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  if (p.depth >= 1) {
-    if (e.levels)
-      for (int q = 0; q < 6; q++) c[q] = e.cache[r0 * 6 + q];
-  } else if (!e.binary) {
-    if (e.cache) {
-      for (int q = 0; q < 6; q++) c[q] = e.cache[r0 * 6 + q];
-    } else {
-      leaf_value(e, 0, 0, c);
-    }
-  }
-  out[0] = p.depth >= 1 ? child_mask(p, 1, 0) : 0u;
-  for (int q = 0; q < 6; q++) out[1 + q] = __float_as_uint(c[q]);
-  if (p.depth >= 1) {
-    if (e.levels) store_data_record(e, data_base + e.dsize[r0] - 1, 0, c);
-  } else if (!e.binary) {
-    store_data_record(e, data_base, e.stripe_base, c);
-  }
-}
-
 // n words into `dst` (mapped pinned host memory): small results the host waits for
 // travel as the kernel's stores, not as copies queued on the copy engine.
 __global__ void k_copy_words(const uint32_t* __restrict__ src, uint64_t n, uint32_t* __restrict__ dst) {
@@ -1576,35 +894,6 @@ __global__ void k_scatter_to(const uint64_t* __restrict__ src, uint64_t n, int w
 // each CTA one stripe and a run of at most kChunk elements; the CTA copies that
 // stripe's job into shared memory and runs the per-element bodies above.
 // ===========================================================================
-template <typename T>
-__device__ __forceinline__ void stage(T& dst, const T& src) {
-  static_assert(sizeof(T) % 4 == 0, "staged structs are word-sized");
-  const uint32_t* s = reinterpret_cast<const uint32_t*>(&src);
-  uint32_t* d = reinterpret_cast<uint32_t*>(&dst);
-  for (uint32_t q = threadIdx.x; q < sizeof(T) / 4; q += blockDim.x) d[q] = s[q];
-}
-
-// CTA b belongs to the stripe s with cta_beg[s] <= b < cta_beg[s+1]; it is
-// the stripe's CTA b - cta_beg[s] and covers the elements per CTA of its
-// launch from there (kChunk, or kChunk * ept for the per-block and per-node
-// launches, each thread taking one element of every kChunk-wide chunk).
-__device__ __forceinline__ uint32_t cta_stripe(const uint64_t* __restrict__ cta_beg, uint32_t n, uint64_t& cta) {
-  __shared__ uint32_t s_stripe;
-  if (threadIdx.x == 0) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (cta_beg[mid] <= blockIdx.x) lo = mid;
-      else hi = mid;
-    }
-    s_stripe = lo;
-  }
-  __syncthreads();
-  const uint32_t s = s_stripe;
-  cta = (uint64_t)(blockIdx.x - cta_beg[s]);  // the CTA's index within its stripe
-  return s;
-}
-
 // A one-stripe launch (SINGLE) takes the stripe's job as a kernel parameter
 // and indexes elements directly; a batch launch finds its stripe first and
 // stages the job in shared memory.
@@ -1686,212 +975,18 @@ __global__ void __launch_bounds__(256, 4) kb_vox_large(const VoxJob* __restrict_
   }
 }
 
-// Element e of level l: a block, or a group of blocks of a marked leaf level.
-template <bool CG = false>
-__device__ __forceinline__ void pyramid_elem(const Pyramid& p, int l, uint64_t e) {
-  if (l == p.depth && p.touch) leaf_group<CG>(p, e);
-  else pyramid_block<CG>(p, l, e);
-}
-
-// Level depth - r of every stripe that has CTAs in this launch.
-template <bool SINGLE>
-__global__ void __launch_bounds__(kChunk) kb_pyramid(const Pyramid* __restrict__ pyrs,
-                                                     const uint64_t* __restrict__ cta_beg, uint32_t n, int r, uint32_t ept,
-                                                     Pyramid p0) {
-  pdl_enter();
-  if constexpr (SINGLE) {
-    const int l = p0.depth - r;
-    for (uint32_t k = 0; k < ept; k++) {
-      const uint64_t b = ((uint64_t)blockIdx.x * ept + k) * kChunk + threadIdx.x;
-      if (b < p0.lv[l].nscan) pyramid_elem(p0, l, b);
-    }
-  } else {
-    __shared__ Pyramid sp;
-    uint64_t cta;
-    const uint32_t s = cta_stripe(cta_beg, n, cta);
-    stage(sp, pyrs[s]);
-    __syncthreads();
-    const int l = sp.depth - r;
-    for (uint32_t k = 0; k < ept; k++) {
-      const uint64_t b = (cta * ept + k) * kChunk + threadIdx.x;
-      if (b < sp.lv[l].nscan) pyramid_elem(sp, l, b);
-    }
-  }
-}
-
-__global__ void kb_pyramid_top(const Pyramid* __restrict__ pyrs, int l_hi, uint32_t* __restrict__ scan_end) {
-  pdl_enter();
-  if (blockIdx.x == 0 && threadIdx.x == 0) *scan_end = 0u;  // the scan's total entry
-  __shared__ Pyramid sp;
-  stage(sp, pyrs[blockIdx.x]);
-  __syncthreads();
-  for (int l = l_hi < sp.depth ? l_hi : sp.depth; l >= 0; l--) {
-    for (uint64_t b = threadIdx.x; b < sp.lv[l].nblocks; b += blockDim.x) pyramid_block(sp, l, b);
-    // the padding words of level l-1 (levels 0..2 are padded to a whole block)
-    if (l > 0)
-      for (uint64_t w = sp.lv[l].nblocks + threadIdx.x; w < sp.lv[l - 1].nwords; w += blockDim.x)
-        level_words(sp, l - 1)[w] = 0u;
-    __syncthreads();
-  }
-}
-
-// Zero the marked leaf blocks and the marks of every stripe.
-template <bool SINGLE>
-__global__ void __launch_bounds__(kChunk) kb_clean_leaves(const Pyramid* __restrict__ pyrs,
-                                                          const uint64_t* __restrict__ cta_beg, uint32_t n, uint32_t ept,
-                                                          Pyramid p0) {
-  pdl_enter();
-  if constexpr (SINGLE) {
-    for (uint32_t k = 0; k < ept; k++) clean_touch16(p0, ((uint64_t)blockIdx.x * ept + k) * kChunk + threadIdx.x);
-  } else {
-    __shared__ Pyramid sp;
-    uint64_t cta;
-    const uint32_t s = cta_stripe(cta_beg, n, cta);
-    stage(sp, pyrs[s]);
-    __syncthreads();
-    for (uint32_t k = 0; k < ept; k++) clean_touch16(sp, (cta * ept + k) * kChunk + threadIdx.x);
-  }
-}
-
-// Every block of every level of the stripe.
-template <bool SINGLE>
-__global__ void __launch_bounds__(kChunk) kb_compact(const Pyramid* __restrict__ pyrs,
-                                                     const uint64_t* __restrict__ cta_beg, uint32_t n,
-                                                     uint32_t* __restrict__ keys, uint32_t ept, Pyramid p0) {
-  pdl_enter();
-  if constexpr (SINGLE) {
-    for (uint32_t k = 0; k < ept; k++)
-      compact_elem(p0, ((uint64_t)blockIdx.x * ept + k) * kChunk + threadIdx.x, keys);
-  } else {
-    __shared__ Pyramid sp;
-    uint64_t cta;
-    const uint32_t s = cta_stripe(cta_beg, n, cta);
-    stage(sp, pyrs[s]);
-    __syncthreads();
-    for (uint32_t k = 0; k < ept; k++) compact_elem(sp, (cta * ept + k) * kChunk + threadIdx.x, keys);
-  }
-}
-
-// Also copies *tasks to *tasks_out and, when `code` is set, *code to *code_out.
-__global__ void kb_level_bases(const Pyramid* __restrict__ pyrs, uint32_t n_stripes, uint32_t* __restrict__ out,
-                               const uint64_t* __restrict__ tasks, uint64_t* __restrict__ tasks_out,
-                               uint32_t* __restrict__ flag, const uint64_t* __restrict__ code,
-                               uint64_t* __restrict__ code_out) {
-  pdl_enter();
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) {
-    *tasks_out = *tasks;
-    if (code) *code_out = *code;
-    *flag = 0u;  // the layout check flag of the sub-batch's record kernels
-  }
-  if (s >= n_stripes) return;
-  const Pyramid& p = pyrs[s];
-  uint32_t* o = out + (uint64_t)s * (kMaxLevels + 1);
-  for (int l = 0; l <= p.depth; l++) o[l] = p.scan[p.lv[l].off_b];
-  o[p.depth + 1] = p.scan[p.lv[p.depth].off_b + p.lv[p.depth].nscan];
-}
-
-// Kinds of per-node launches that take (Pyramid, EmitJob) pairs.
-enum NodeOp { OP_LEAF_PAYLOAD = 0, OP_BOTTOM_UP = 1, OP_TOP_DOWN = 2, OP_LEAVES = 3 };
-
-template <int OP>
-__device__ __forceinline__ void node_op(const Pyramid& p, const EmitJob& e, int arg, uint64_t i) {
-  if (OP == OP_LEAF_PAYLOAD) {
-    if (i < p.lv[p.depth].n) leaf_payload(p, e, i);
-  } else if (OP == OP_BOTTOM_UP) {
-    const int l = p.depth - arg;  // arg = distance from the leaf level
-    if (i < p.lv[l].n) bottom_up_node(p, e, l, i);
-  } else if (OP == OP_TOP_DOWN) {
-    top_down_children(p, e, arg, i, ~0ull);  // arg = absolute parent level
-  } else {
-    if (i < p.lv[p.depth].n) top_down_leaf(p, e, i);
-  }
-}
-
-template <int OP, bool SINGLE>
-__global__ void __launch_bounds__(kChunk) kb_nodes(const Pyramid* __restrict__ pyrs, const EmitJob* __restrict__ emits,
-                                                   const uint64_t* __restrict__ cta_beg, uint32_t n, int arg, uint32_t ept,
-                                                   Pyramid p0, EmitJob e0) {
-  pdl_enter();
-  if constexpr (SINGLE) {
-    if constexpr (OP == OP_TOP_DOWN) {
-      for (uint32_t k = 0; k < ept; k += 2) {
-        const uint64_t i = ((uint64_t)blockIdx.x * ept + k) * kChunk + threadIdx.x;
-        top_down_children(p0, e0, arg, i, k + 1 < ept ? i + kChunk : ~0ull);
-      }
-    } else {
-      for (uint32_t k = 0; k < ept; k++) node_op<OP>(p0, e0, arg, ((uint64_t)blockIdx.x * ept + k) * kChunk + threadIdx.x);
-    }
-  } else {
-    __shared__ Pyramid sp;
-    __shared__ EmitJob se;
-    uint64_t cta;
-    const uint32_t s = cta_stripe(cta_beg, n, cta);
-    stage(sp, pyrs[s]);
-    stage(se, emits[s]);
-    __syncthreads();
-    if constexpr (OP == OP_TOP_DOWN) {
-      for (uint32_t k = 0; k < ept; k += 2) {
-        const uint64_t i = (cta * ept + k) * kChunk + threadIdx.x;
-        top_down_children(sp, se, arg, i, k + 1 < ept ? i + kChunk : ~0ull);
-      }
-    } else {
-      for (uint32_t k = 0; k < ept; k++) node_op<OP>(sp, se, arg, (cta * ept + k) * kChunk + threadIdx.x);
-    }
-  }
-}
-
-// One CTA per stripe: bottom-up of levels l_small .. 0.
-__global__ void kb_bottom_up_top(const Pyramid* __restrict__ pyrs, const EmitJob* __restrict__ emits) {
-  pdl_enter();
-  __shared__ Pyramid sp;
-  __shared__ EmitJob se;
-  stage(sp, pyrs[blockIdx.x]);
-  stage(se, emits[blockIdx.x]);
-  __syncthreads();
-  if (sp.depth < 1 || sp.lv[sp.depth].n == 0) return;
-  for (int l = se.l_small; l >= 0; l--) {
-    for (uint64_t i = threadIdx.x; i < sp.lv[l].n; i += blockDim.x) bottom_up_node(sp, se, l, i);
-    __syncthreads();
-  }
-}
-
-// One CTA per stripe: the root starts at the stripe's bases; parents of levels 0 .. min(l_small, depth-2).
-__global__ void kb_top_down_top(const Pyramid* __restrict__ pyrs, const EmitJob* __restrict__ emits) {
-  pdl_enter();
-  __shared__ Pyramid sp;
-  __shared__ EmitJob se;
-  stage(sp, pyrs[blockIdx.x]);
-  stage(se, emits[blockIdx.x]);
-  __syncthreads();
-  if (sp.depth < 1 || sp.lv[sp.depth].n == 0) return;
-  if (threadIdx.x == 0) {
-    se.start[sp.lv[0].koff] = 0u;  // the stripe root starts at the stripe's bases
-    se.dstart[sp.lv[0].koff] = 0u;
-  }
-  __syncthreads();
-  const int last = se.l_small < sp.depth - 2 ? se.l_small : sp.depth - 2;
-  for (int l = 0; l <= last; l++) {
-    for (uint64_t i = threadIdx.x; i < sp.lv[l].n; i += blockDim.x) top_down_node(sp, se, l, i);
-    __syncthreads();
-  }
-}
-
 // ===========================================================================
-// Persistent phase A (ooc_tuning::persistent): the occupancy passes and the
-// pyramid levels of every stripe of a sub-batch in one launch.  Each warp
+// Persistent occupancy passes (ooc_tuning::persistent): the small pass and the
+// large-triangle tasks of every stripe of a sub-batch in one launch.  Each warp
 // takes tickets from one counter and runs the unit its ticket names.  Tickets
 // come in this order:
-//   [0, C)          32-item chunks of the small pass, stripe by stripe;
+//   [0, C)          256-item chunks of the small pass, stripe by stripe;
 //   [C, C + T)      warp tasks of large items, in the order the chunks queued
-//                   them (T is final once every chunk is done);
-//   [C + T, + U)    pyramid units, level by level from the leaf level up to the
-//                   top levels: 32 x ept elements of one level of one stripe;
-//   [.., + n)       the top levels of each stripe, one warp each.
-// A unit waits only for units with smaller tickets (its stripe's occupancy, or
-// its stripe's level below), which running warps hold already, so every wait
-// ends whether or not the whole grid is resident.  Each wait is still bounded:
-// past kPersistSpins polls it records its code in ctr[3] and every warp stops.
+//                   them (T is final once every chunk is done).
+// A task waits only for chunks, whose tickets are smaller and held by running
+// warps already, so every wait ends whether or not the whole grid is resident.
+// Each wait is still bounded: past kPersistWaitNs it records its code in the
+// timeout counter and every warp stops.
 // ===========================================================================
 // Counters, each on its own 128-byte line so the polls of waiting warps do not
 // queue behind the ticket atomics.
@@ -1904,12 +999,6 @@ constexpr uint32_t kPersistChunkRounds = 8;          // a chunk is 8 x 32 items
 __device__ __forceinline__ uint64_t ld_acquire(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -1937,21 +1026,6 @@ struct Backoff {
     return true;
   }
 };
-
-// Lane 0: wait until *p is zero; false on a timeout (here or in another warp).
-__device__ __forceinline__ bool persist_wait_zero(const uint32_t* p, unsigned long long* ctr, uint32_t code) {
-  Backoff b;
-  while (ld_acquire(p) != 0u)
-    if (!b.pause(ctr, code)) return false;
-  return true;
-}
-
-// Every lane's writes of the unit reach the GPU scope before lane 0 counts it done.
-__device__ __forceinline__ void persist_done(uint32_t* left, int lane) {
-  __threadfence();
-  __syncwarp();
-  if (lane == 0) atomicSub(left, 1u);
-}
 
 __device__ __forceinline__ uint32_t find_stripe(const uint64_t* __restrict__ beg, uint32_t n, uint64_t x) {
   uint32_t lo = 0, hi = n;  // beg[lo] <= x < beg[hi]
@@ -1993,15 +1067,7 @@ __device__ __forceinline__ void persist_items(const PersistJob& pj, uint32_t s, 
   // stalled the whole grid).  Tasks reserved at or past `cap` have no entry:
   // this warp walks them, and the warps that draw their tickets skip them.
   unsigned long long base = 0;
-  if (lane == 0) {
-    base = atomicAdd(pj.ctr + kCtrTasksQueued, (unsigned long long)total);
-    const uint64_t queued = base >= pj.cap ? 0 : (base + total <= pj.cap ? total : pj.cap - base);
-    if (queued) {
-      // counted before any entry is written, so no task can finish before it
-      atomicAdd(pj.occ_left + s, (uint32_t)queued);
-      __threadfence();
-    }
-  }
+  if (lane == 0) base = atomicAdd(pj.ctr + kCtrTasksQueued, (unsigned long long)total);
   base = __shfl_sync(FULL, base, 0);
   __syncwarp();
   const uint64_t ig = pj.item_beg[s] + i;  // the item's index in the sub-batch
@@ -2026,12 +1092,10 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
   pdl_enter();
   extern __shared__ uint32_t lines_smem[];  // 32 x lines_per_lane per warp
   __shared__ VoxJob s_job[8];
-  __shared__ Pyramid s_pyr[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t* wl = lines_smem + (uint32_t)w * 32u * pj.lines_per_lane;
   const uint64_t C = pj.chunk_beg[pj.n];
-  const uint64_t U = pj.levels ? pj.unit_beg[(uint64_t)pj.levels * (pj.n + 1) - 1] : 0;
-  uint32_t job_s = ~0u, pyr_s = ~0u;  // the stripe staged in s_job[w] / s_pyr[w]
+  uint32_t job_s = ~0u;  // the stripe staged in s_job[w]
   for (;;) {
     unsigned long long t = 0;
     if (lane == 0)
@@ -2050,19 +1114,16 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
         if (i0 >= s_job[w].n_items) break;
         persist_items(pj, s, i0, lane, s_job[w], wl);
       }
-      // this chunk's bits, marks and queued tasks are visible before it counts as done
+      // this chunk's queued tasks are visible before it counts as done
       __threadfence();
       __syncwarp();
-      if (lane == 0) {
-        atomicSub(pj.occ_left + s, 1u);
-        atomicAdd(pj.ctr + kCtrChunksDone, 1ull);
-      }
+      if (lane == 0) atomicAdd(pj.ctr + kCtrChunksDone, 1ull);
       continue;
     }
-    // a queued task, or (once every chunk is done and no task is left) a pyramid unit
+    // a queued task, or (once every chunk is done and no task is left) the end
     const uint64_t u = t - C;
-    // kind 1: task, 2: after the tasks, 3: stop, 4: a task its chunk walks
-    unsigned long long kind = 0, tail = 0, entry = 0;
+    // kind 1: task, 3: stop, 4: a task its chunk walks
+    unsigned long long kind = 0, entry = 0;
     if (lane == 0) {
       Backoff b;
       for (;;) {
@@ -2071,8 +1132,7 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
           break;
         }
         if (ld_acquire(pj.ctr + kCtrChunksDone) == C) {
-          tail = ld_acquire(pj.ctr + kCtrTasksQueued);
-          kind = u < tail ? 1 : 2;
+          kind = u < ld_acquire(pj.ctr + kCtrTasksQueued) ? 1 : 3;
           break;
         }
         if (!b.pause(pj.ctr, 1u)) {
@@ -2094,80 +1154,15 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
     kind = __shfl_sync(FULL, kind, 0);
     if (kind == 3) return;
     if (kind == 4) continue;
-    if (kind == 1) {
-      entry = __shfl_sync(FULL, entry, 0);
-      const uint64_t item = (uint32_t)entry;
-      const uint32_t s = find_stripe(pj.item_beg, pj.n, item);
-      if (s != job_s) {
-        stage_warp(s_job[w], pj.jobs[s], lane);
-        job_s = s;
-      }
-      vox_large_task<0>(s_job[w], item - pj.item_beg[s], entry >> 32, lane, wl);
-      persist_done(pj.occ_left + s, lane);
-      continue;
+    entry = __shfl_sync(FULL, entry, 0);
+    const uint64_t item = (uint32_t)entry;
+    const uint32_t s = find_stripe(pj.item_beg, pj.n, item);
+    if (s != job_s) {
+      stage_warp(s_job[w], pj.jobs[s], lane);
+      job_s = s;
     }
-    const uint64_t v = u - __shfl_sync(FULL, tail, 0);
-    if (v < U) {  // pyramid unit: level r of stripe s
-      uint32_t r = 0;
-      while (v >= pj.unit_beg[(uint64_t)r * (pj.n + 1) + pj.n]) r++;
-      const uint64_t* ub = pj.unit_beg + (uint64_t)r * (pj.n + 1);
-      const uint32_t s = find_stripe(ub, pj.n, v);
-      bool ok = true;
-      if (lane == 0)
-        ok = persist_wait_zero(r == 0 ? pj.occ_left + s : pj.pyr_left + (uint64_t)(r - 1) * pj.n + s, pj.ctr, 3u);
-      if (!__shfl_sync(FULL, ok, 0)) return;
-      __syncwarp();  // the lanes' loads below follow lane 0's acquire
-      if (s != pyr_s) {
-        stage_warp(s_pyr[w], pj.pyrs[s], lane);
-        pyr_s = s;
-      }
-      const Pyramid& P = s_pyr[w];
-      const int l = P.depth - (int)r;
-      const uint64_t e0 = (v - ub[s]) * pj.ept * 32u;
-      for (uint32_t k = 0; k < pj.ept; k++) {
-        const uint64_t e = e0 + (uint64_t)k * 32u + (uint64_t)lane;
-        if (e < P.lv[l].nscan) pyramid_elem<true>(P, l, e);
-      }
-      persist_done(pj.pyr_left + (uint64_t)r * pj.n + s, lane);
-      continue;
-    }
-    if (v - U >= pj.n) return;  // past the last unit
-    // the top levels of stripe s, after its last pyramid unit
-    const uint32_t s = (uint32_t)(v - U);
-    if (s != pyr_s) {
-      stage_warp(s_pyr[w], pj.pyrs[s], lane);
-      pyr_s = s;
-    }
-    const Pyramid& P = s_pyr[w];
-    const int below = P.depth - pj.top_level;  // pyramid levels of the stripe under the top ones
-    bool ok = true;
-    if (lane == 0)
-      ok = persist_wait_zero(below <= 0 ? pj.occ_left + s : pj.pyr_left + (uint64_t)(below - 1) * pj.n + s, pj.ctr,
-                             4u);
-    if (!__shfl_sync(FULL, ok, 0)) return;
-    __syncwarp();
-    if (s == 0 && lane == 0) *pj.scan_end = 0u;  // the scan's total entry
-    for (int l = pj.top_level < P.depth ? pj.top_level : P.depth; l >= 0; l--) {
-      for (uint64_t b = (uint64_t)lane; b < P.lv[l].nblocks; b += 32u) pyramid_block<true>(P, l, b);
-      if (l > 0)
-        for (uint64_t x = P.lv[l].nblocks + (uint64_t)lane; x < P.lv[l - 1].nwords; x += 32u)
-          level_words(P, l - 1)[x] = 0u;
-      __threadfence_block();
-      __syncwarp();
-    }
+    vox_large_task<0>(s_job[w], item - pj.item_beg[s], entry >> 32, lane, wl);
   }
-}
-
-// Root information of every stripe into `out` (16 words each), and the layout
-// check flag after them (out[16 n]).
-__global__ void kb_root_info(const Pyramid* __restrict__ pyrs, const EmitJob* __restrict__ emits, uint32_t n_stripes,
-                             uint32_t* __restrict__ out, const uint32_t* __restrict__ flag) {
-  pdl_enter();
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) out[(uint64_t)n_stripes * 16] = *flag;
-  if (s >= n_stripes) return;
-  if (pyrs[s].lv[pyrs[s].depth].n == 0) return;
-  root_info(pyrs[s], emits[s], emits[s].data_base, out + (uint64_t)s * 16);
 }
 
 }  // namespace
@@ -2177,9 +1172,6 @@ __global__ void kb_root_info(const Pyramid* __restrict__ pyrs, const EmitJob* __
 // ===========================================================================
 uint64_t scan_partials_needed(uint64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
 
-void scan_u32_exclusive(uint32_t* data, uint64_t n, uint32_t* partials, cudaStream_t st) {
-  scan_exclusive<uint32_t>(data, n, partials, st);
-}
 void scan_u64_exclusive(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st, bool flag_last) {
   unsigned long long* d = reinterpret_cast<unsigned long long*>(data);
   scan_exclusive<unsigned long long>(d, n, reinterpret_cast<unsigned long long*>(partials), st,
@@ -2354,107 +1346,6 @@ void launch_b_vox_large(const VoxJob* jobs, const uint64_t* item_beg, uint32_t n
              counter, lines_per_lane, map, cap);
 }
 
-void launch_b_pyramid(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept, int r,
-                      const Pyramid* single, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k(r == 0 ? "pyramid_leaf" : "pyramid", st);
-  Pyramid p0;
-  std::memset(&p0, 0, sizeof(p0));
-  if (single) p0 = *single;
-  if (single) launch_k(kb_pyramid<true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, r, ept, p0);
-  else launch_k(kb_pyramid<false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, r, ept, p0);
-}
-
-void launch_b_pyramid_top(const Pyramid* pyrs, uint32_t n_stripes, int l_hi, uint32_t* scan_end, cudaStream_t st) {
-  if (n_stripes == 0) return;
-  KScope k("pyramid_top", st);
-  launch_k(kb_pyramid_top, dim3(n_stripes), dim3(512), 0, st, pyrs, l_hi, scan_end);
-}
-
-void launch_b_compact(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept,
-                      uint32_t* keys, const Pyramid* single, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k("compact", st);
-  Pyramid p0;
-  std::memset(&p0, 0, sizeof(p0));
-  if (single) p0 = *single;
-  if (single) launch_k(kb_compact<true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, keys, ept, p0);
-  else launch_k(kb_compact<false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, keys, ept, p0);
-}
-
-void launch_b_clean_leaves(const Pyramid* pyrs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, uint32_t ept,
-                           const Pyramid* single, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k("clean_leaves", st);
-  Pyramid p0;
-  std::memset(&p0, 0, sizeof(p0));
-  if (single) p0 = *single;
-  if (single) launch_k(kb_clean_leaves<true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, ept, p0);
-  else launch_k(kb_clean_leaves<false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, cta_beg, n, ept, p0);
-}
-
-void launch_b_level_bases(const Pyramid* pyrs, uint32_t n_stripes, uint32_t* out, const uint64_t* tasks,
-                          uint64_t* tasks_out, uint32_t* flag, const uint64_t* code, uint64_t* code_out,
-                          cudaStream_t st) {
-  if (n_stripes == 0) return;
-  KScope k("level_bases", st);
-  launch_k(kb_level_bases, dim3(grid_for(n_stripes, 128)), dim3(128), 0, st, pyrs, n_stripes, out, tasks, tasks_out,
-           flag, code, code_out);
-}
-
-namespace {
-template <int OP>
-void launch_nodes(const char* name, const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                  uint64_t ctas, uint32_t ept, int arg, const Pyramid* sp, const EmitJob* se, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k(name, st);
-  Pyramid p0;
-  EmitJob e0;
-  std::memset(&p0, 0, sizeof(p0));
-  std::memset(&e0, 0, sizeof(e0));
-  if (sp && se) {
-    p0 = *sp;
-    e0 = *se;
-    launch_k(kb_nodes<OP, true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, emits, cta_beg, n, arg, ept, p0, e0);
-  } else {
-    launch_k(kb_nodes<OP, false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, pyrs, emits, cta_beg, n, arg, ept, p0, e0);
-  }
-}
-}  // namespace
-
-void launch_b_leaf_payload(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                           uint64_t ctas, uint32_t ept, const Pyramid* sp, const EmitJob* se, cudaStream_t st) {
-  launch_nodes<OP_LEAF_PAYLOAD>("leaf_payload", pyrs, emits, cta_beg, n, ctas, ept, 0, sp, se, st);
-}
-
-void launch_b_bottom_up(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                        uint32_t ept, int r, const Pyramid* sp, const EmitJob* se, cudaStream_t st) {
-  launch_nodes<OP_BOTTOM_UP>(r == 1 ? "bottom_up_leaf_parents" : "bottom_up", pyrs, emits, cta_beg, n, ctas, ept, r,
-                             sp, se, st);
-}
-
-void launch_b_bottom_up_top(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, cudaStream_t st) {
-  if (n_stripes == 0) return;
-  KScope k("bottom_up_top", st);
-  launch_k(kb_bottom_up_top, dim3(n_stripes), dim3(256), 0, st, pyrs, emits);
-}
-
-void launch_b_top_down_top(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, cudaStream_t st) {
-  if (n_stripes == 0) return;
-  KScope k("top_down_top", st);
-  launch_k(kb_top_down_top, dim3(n_stripes), dim3(256), 0, st, pyrs, emits);
-}
-
-void launch_b_top_down(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                       uint32_t ept, int l, const Pyramid* sp, const EmitJob* se, cudaStream_t st) {
-  launch_nodes<OP_TOP_DOWN>("top_down", pyrs, emits, cta_beg, n, ctas, ept, l, sp, se, st);
-}
-
-void launch_b_top_down_leaves(const Pyramid* pyrs, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                              uint64_t ctas, uint32_t ept, const Pyramid* sp, const EmitJob* se, cudaStream_t st) {
-  launch_nodes<OP_LEAVES>("top_down_leaves", pyrs, emits, cta_beg, n, ctas, ept, 0, sp, se, st);
-}
-
 int persist_ctas_per_sm(uint32_t lines_per_lane) {
   int per_sm = 0;
   const size_t smem = (size_t)256 * lines_per_lane * 4;
@@ -2466,16 +1357,9 @@ int persist_ctas_per_sm(uint32_t lines_per_lane) {
 }
 
 void launch_b_persist(const PersistJob& pj, int num_sms, int ctas_per_sm, cudaStream_t st) {
-  KScope k("persistent_phase_a", st);
+  KScope k("persistent_occupancy", st);
   const size_t smem = (size_t)256 * pj.lines_per_lane * 4;
   launch_k(kb_persist, dim3((unsigned)(num_sms * ctas_per_sm)), dim3(256), smem, st, pj);
-}
-
-void launch_b_root_info(const Pyramid* pyrs, const EmitJob* emits, uint32_t n_stripes, uint32_t* out,
-                        const uint32_t* flag, cudaStream_t st) {
-  if (n_stripes == 0) return;
-  KScope k("root_info", st);
-  launch_k(kb_root_info, dim3(grid_for(n_stripes, 128)), dim3(128), 0, st, pyrs, emits, n_stripes, out, flag);
 }
 
 }  // namespace ooc

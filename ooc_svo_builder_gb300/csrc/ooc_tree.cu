@@ -1,0 +1,1357 @@
+// The octree of a stripe from its leaf bits: counts per brick, prefixes over the
+// bricks and the levels above them, and the records of both files (sm_103a).
+//
+// Compiled with -fmad=false; FP32 arithmetic additionally goes through the
+// __f*_rn intrinsics so that each operation rounds once, as in the
+// reference's x86-64 build.
+//
+// Layout.  The reference writes a node's group of children when the Morton
+// cursor leaves the node's region (groupNodes, OctreeBuilder.cpp:58-79; the loop
+// of refineBuffers, 112-128), so the node file is the post-order of groups: the
+// record of a node stands in its parent's group, after the groups of every inner
+// node whose region ends earlier.  Positions are therefore counts, and counts are
+// prefix sums of the occupancy bits:
+//   * before a brick's run: the leaves and inner nodes of earlier bricks, and the
+//     upper nodes whose parent's region ends before the brick;
+//   * inside a brick, a node two levels above the leaves (64 leaf bits, one word)
+//     owns a run of its leaves followed by their parents; the runs of eight such
+//     words are followed by those words' own records, and the whole brick by the
+//     records of its children.
+// The data file (-levels) is ordered the same way, an inner node's average
+// standing after its region's records.
+#include <cuda_runtime.h>
+
+#include <cstring>
+
+#include "ooc_device.cuh"
+#include "ooc_internal.h"
+#include "ooc_launch.cuh"
+
+namespace ooc {
+
+namespace {
+
+__device__ __forceinline__ uint32_t nonzero_bytes64(uint64_t v) {
+  return nonzero_bytes((uint32_t)v) | (nonzero_bytes((uint32_t)(v >> 32)) << 4);
+}
+
+
+// Set bits of upper level l before bit `pos` (0 .. 8^l).
+__device__ __forceinline__ uint32_t upper_rank(const Stripe& p, int l, uint32_t pos) {
+  const uint32_t i = upper_off(l) + (pos >> 5);
+  return p.upre[i] + __popc(p.ubits[i] & ((1u << (pos & 31u)) - 1u));
+}
+
+__device__ __forceinline__ uint32_t upper_byte(const Stripe& p, int l, uint32_t parent) {
+  return (p.ubits[upper_off(l) + (parent >> 2)] >> (8u * (parent & 3u))) & 0xffu;
+}
+
+// Leaves (.x) and inner nodes below the bricks (.y) before brick `pos` (0 .. n_bricks).
+__device__ __forceinline__ uint2 brick_prefix(const Stripe& p, uint32_t pos) {
+  const uint32_t w = pos >> 5;
+  uint2 v = p.wpre[w];
+  if (pos & 31u) {
+    const uint2 b = p.bpre[pos];
+    v.x += b.x;
+    v.y += b.y;
+  }
+  return v;
+}
+
+// A check of the layout failed: the host reads the flag and fails the build.
+__device__ __forceinline__ void raise_flag(const EmitJob& e, uint32_t code) {
+  *reinterpret_cast<volatile uint32_t*>(e.flag) = code;
+}
+
+// ===========================================================================
+// Counts per brick and per level-U word (32 bricks).
+//
+// Bound by the latency of the leaf blocks' loads.  A marked leaf level is read
+// only where it has bits: one warp per word, the marked blocks of the word's
+// bricks handed out one per lane, so the lanes stay busy on sparse bricks.  An
+// unmarked level (at most 4,096 bricks) is read whole, and its few words would
+// leave most SMs idle for 16 rounds of loads: the CTA's four warps share a word,
+// eight bricks each (18 -> 10 us at gridsize 256).
+// ===========================================================================
+struct WordCount {
+  uint32_t l, i;  // leaves and inner nodes below the bricks
+};
+
+// Bricks [x0, x0 + 32), lane's brick x0 + lane (those at or past x1 have none): the counts
+// before each brick and its units (bit q: the 512 leaf bits of child q are not all zero; for a
+// brick of fewer levels bit 0: it has a bit); returns the totals.
+__device__ __forceinline__ WordCount count_bricks(const Stripe& p, uint32_t x0, uint32_t x1, int lane, WordCount& before_x,
+                                                  uint32_t& units) {
+  const uint32_t x = x0 + (uint32_t)lane;
+  uint32_t marked = 0;  // bit k: block k of brick x is to be read
+  const uint32_t per = (uint32_t)min((uint64_t)16, leaf_blocks(p.depth));
+  if (x < x1) {
+    if (p.touch) {
+      const uint4 m = reinterpret_cast<const uint4*>(p.touch)[x];
+      marked = nonzero_bytes(m.x) | (nonzero_bytes(m.y) << 4) | (nonzero_bytes(m.z) << 8) | (nonzero_bytes(m.w) << 12);
+    } else {
+      marked = (1u << per) - 1u;
+    }
+  }
+  const uint32_t cnt = __popc(marked);
+  const uint32_t incl = warp_inclusive(cnt), excl = incl - cnt;
+  const uint32_t total = __shfl_sync(FULL, incl, 31);
+  uint32_t carry_l = 0, carry_i = 0;  // leaves, inner nodes of the blocks before this round
+  uint32_t my_l = 0, my_i = 0;        // before brick x
+  uint32_t seen = marked;             // blocks of brick x with a bit
+  for (uint32_t round = 0; round < total; round += 32u) {
+    const uint32_t j = round + (uint32_t)lane;  // this lane's block, in Morton order
+    uint32_t o = 0;                             // its brick: the first lane with incl > j
+#pragma unroll
+    for (uint32_t st = 16; st; st >>= 1) {
+      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
+      if (t <= j) o += st;
+    }
+    uint32_t m = __shfl_sync(FULL, marked, (int)o);
+    const uint32_t before = __shfl_sync(FULL, excl, (int)o);
+    uint32_t l = 0, in = 0;
+    uint64_t blk = 0, wo = 0;
+    if (j < total) {
+      uint32_t k = j - before;
+      if (p.touch) {  // the k-th marked block
+        for (; k; k--) m &= m - 1;
+        k = (uint32_t)__ffs(m) - 1u;
+      }
+      blk = (uint64_t)(x0 + o) * 16u + k;
+      const uint4* q = reinterpret_cast<const uint4*>(p.leaf) + 2 * blk;
+      const uint4 q0 = q[0], q1 = q[1];
+      const uint32_t wd[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        wo |= (uint64_t)l << (8 * i);  // at most 224
+        l += __popc(wd[i]);
+        if (p.K >= 2) in += __popc(nonzero_bytes(wd[i]));
+      }
+      if (p.K >= 3) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) in += (wd[i] | wd[i + 1]) ? 1u : 0u;
+      }
+    }
+    const uint32_t nonempty = __ballot_sync(FULL, l != 0);
+    const uint32_t il = warp_inclusive(l), ii = warp_inclusive(in);
+    const uint32_t el = carry_l + il - l, ei = carry_i + ii - in;
+    if (p.local && j < total) {
+      p.local[blk] = el;
+      p.woff[blk] = wo;
+    }
+    const uint32_t src = excl - round;  // where this lane's brick starts, when it does in this round
+    const uint32_t vl = __shfl_sync(FULL, el, (int)(src & 31u)), vi = __shfl_sync(FULL, ei, (int)(src & 31u));
+    if (excl >= round && src < 32u) {
+      my_l = vl;
+      my_i = vi;
+      if (!p.touch) seen = (nonempty >> src) & marked;
+    }
+    if (p.inner_local) {
+      const uint32_t brick_i = __shfl_sync(FULL, my_i, (int)o);  // before the block's brick
+      if (j < total) p.inner_local[blk] = (uint16_t)(ei - brick_i);
+    }
+    carry_l += __shfl_sync(FULL, il, 31);
+    carry_i += __shfl_sync(FULL, ii, 31);
+  }
+  if (excl >= total) {  // no block in this brick or after it
+    my_l = carry_l;
+    my_i = carry_i;
+    seen = 0;
+  }
+  // units: pairs of blocks
+  units = (seen | (seen >> 1)) & 0x5555u;
+  units = (units | (units >> 1)) & 0x3333u;
+  units = (units | (units >> 2)) & 0x0f0fu;
+  units = (units | (units >> 4)) & 0xffu;
+  if (p.K < kBrickLevels) units = units ? 1u : 0u;
+  const uint32_t c3 = p.K == kBrickLevels ? __popc(units) : 0u;  // they are nodes
+  const uint32_t i3 = warp_inclusive(c3);
+  before_x = WordCount{my_l, my_i + i3 - c3};
+  return WordCount{carry_l, carry_i + __shfl_sync(FULL, i3, 31)};
+}
+
+__device__ __forceinline__ void count_cta(const Stripe& p, uint32_t cta) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t off = upper_off(p.U);
+  WordCount mine;
+  uint32_t units;
+  if (p.touch) {  // one word per warp
+    const uint32_t w = cta * kBrickCta + (uint32_t)warp;
+    if (w >= upper_words(p.U)) return;
+    const WordCount t = count_bricks(p, w * 32u, p.n_bricks, lane, mine, units);
+    const uint32_t bits = __ballot_sync(FULL, units != 0);
+    p.bpre[w * 32u + (uint32_t)lane] = make_uint2(mine.l, mine.i);
+    p.bunits[w * 32u + (uint32_t)lane] = (uint8_t)units;
+    if (lane == 0) {
+      p.ubits[off + w] = bits;
+      p.wpre[w] = make_uint2(t.l, t.i);  // the word's own counts; kb_upper makes them prefixes
+    }
+    return;
+  }
+  // one word per CTA, a quarter of its bricks per warp
+  static_assert(kBrickCta == 4, "a warp takes 8 of a word's 32 bricks");
+  __shared__ WordCount s_t[kBrickCta];
+  __shared__ uint32_t s_bits[kBrickCta];
+  const uint32_t w = cta, x0 = w * 32u + 8u * (uint32_t)warp;
+  const WordCount t = count_bricks(p, x0, min(p.n_bricks, x0 + 8u), lane, mine, units);
+  const uint32_t bits = __ballot_sync(FULL, units != 0);
+  if (lane == 0) {
+    s_t[warp] = t;
+    s_bits[warp] = bits;
+  }
+  __syncthreads();
+  uint32_t l = 0, i = 0, all = 0;
+#pragma unroll
+  for (int k = 0; k < (int)kBrickCta; k++) {
+    if (k < warp) {
+      l += s_t[k].l;
+      i += s_t[k].i;
+    }
+    all |= s_bits[k] << (8 * k);
+  }
+  if (p.local) {  // the blocks' ranks count from the word's start
+    const uint32_t b0 = x0 * 16u, n = (uint32_t)min((uint64_t)128, leaf_blocks(p.depth) - min(leaf_blocks(p.depth), (uint64_t)b0));
+    if (l)
+      for (uint32_t k = (uint32_t)lane; k < n; k += 32u) p.local[b0 + k] += l;
+  }
+  if (lane < 8) {
+    p.bpre[x0 + (uint32_t)lane] = make_uint2(l + mine.l, i + mine.i);
+    p.bunits[x0 + (uint32_t)lane] = (uint8_t)units;
+  }
+  if (warp == kBrickCta - 1 && lane == 0) {
+    p.ubits[off + w] = all;
+    p.wpre[w] = make_uint2(l + t.l, i + t.i);
+  }
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(32 * kBrickCta) kb_bricks(const Stripe* __restrict__ stripes,
+                                                            const uint64_t* __restrict__ cta_beg, uint32_t n, Stripe p0) {
+  pdl_enter();
+  if constexpr (SINGLE) {
+    count_cta(p0, blockIdx.x);
+  } else {
+    __shared__ Stripe sp;
+    uint64_t cta;
+    const uint32_t s = cta_stripe(cta_beg, n, cta);
+    stage(sp, stripes[s]);
+    __syncthreads();
+    count_cta(sp, (uint32_t)cta);
+  }
+}
+
+// Parent word of eight words of a level: bit i is set when byte i is non-zero.
+__device__ __forceinline__ uint32_t parent_word(const uint32_t w[8]) {
+  uint32_t p = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) p |= nonzero_bytes(w[k]) << (4 * k);
+  return p;
+}
+
+// One CTA per stripe: the prefixes of level U, then the levels above it, each
+// thread on eight words.  Latency-bound (a few dependent block scans); levels of
+// 256 words and fewer are left to the first warp, which needs no block barrier.
+template <int T>
+__global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes, uint32_t* __restrict__ counts,
+                                              const uint64_t* __restrict__ tasks, uint64_t* __restrict__ tasks_out,
+                                              const uint64_t* __restrict__ code, uint64_t* __restrict__ code_out) {
+  pdl_enter();
+  __shared__ Stripe sp;
+  __shared__ uint32_t s_words[2][1024];
+  stage(sp, stripes[blockIdx.x]);
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *tasks_out = *tasks;
+    if (code) *code_out = *code;
+  }
+  uint32_t* out = counts + (uint64_t)blockIdx.x * kCountWords;
+  const int U = sp.U;
+  uint32_t W = upper_words(U), off = upper_off(U);
+  uint32_t carry_r = 0, carry_l = 0, carry_i = 0;
+  for (uint32_t base = 0; base < W; base += T * 8u) {
+    const uint32_t i0 = base + threadIdx.x * 8u;
+    uint32_t w[8], r = 0;
+    uint2 li[8];
+    uint32_t sl = 0, si = 0;
+    if (i0 + 8u <= W) {
+      const uint4* q = reinterpret_cast<const uint4*>(sp.ubits + off + i0);
+      const uint4 q0 = q[0], q1 = q[1];
+      w[0] = q0.x, w[1] = q0.y, w[2] = q0.z, w[3] = q0.w, w[4] = q1.x, w[5] = q1.y, w[6] = q1.z, w[7] = q1.w;
+      const uint4* v = reinterpret_cast<const uint4*>(sp.wpre + i0);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint4 t = v[k];
+        li[2 * k] = make_uint2(t.x, t.y);
+        li[2 * k + 1] = make_uint2(t.z, t.w);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        w[k] = i0 + k < W ? sp.ubits[off + i0 + k] : 0u;
+        li[k] = i0 + k < W ? sp.wpre[i0 + k] : make_uint2(0u, 0u);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      r += __popc(w[k]);
+      sl += li[k].x;
+      si += li[k].y;
+    }
+    unsigned long long tot;
+    uint32_t tot_r;
+    const unsigned long long ex = block_exclusive<unsigned long long>((unsigned long long)sl | ((unsigned long long)si << 32), tot);
+    uint32_t run_r = carry_r + block_exclusive<uint32_t>(r, tot_r);
+    uint32_t run_l = carry_l + (uint32_t)ex, run_i = carry_i + (uint32_t)(ex >> 32);
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (i0 + k < W) {
+        sp.upre[off + i0 + k] = run_r;
+        sp.wpre[i0 + k] = make_uint2(run_l, run_i);
+        run_r += __popc(w[k]);
+        run_l += li[k].x;
+        run_i += li[k].y;
+      }
+    if (U > 0 && i0 < W) {
+      const uint32_t pw = parent_word(w);
+      sp.ubits[upper_off(U - 1) + i0 / 8u] = pw;
+      s_words[(U - 1) & 1][i0 / 8u] = pw;
+    }
+    carry_r += tot_r;
+    carry_l += (uint32_t)tot;
+    carry_i += (uint32_t)(tot >> 32);
+  }
+  if (threadIdx.x == 0) {  // the entries past the end
+    sp.ubits[off + W] = 0u;
+    sp.upre[off + W] = carry_r;
+    sp.wpre[W] = make_uint2(carry_l, carry_i);
+    out[0] = carry_l;
+    out[1] = carry_i;
+    out[2 + U] = carry_r;
+  }
+  __syncthreads();
+  for (int l = U - 1; l >= 0; l--) {
+    W = upper_words(l);
+    off = upper_off(l);
+    const bool one_warp = W <= 256u;
+    if (one_warp && threadIdx.x >= 32) return;  // every later level is smaller
+    const uint32_t i0 = threadIdx.x * 8u;
+    uint32_t w[8], r = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      w[k] = i0 + k < W ? s_words[l & 1][i0 + k] : 0u;
+      r += __popc(w[k]);
+    }
+    uint32_t run, tot;
+    if (one_warp) {
+      const uint32_t inc = warp_inclusive(r);
+      run = inc - r;
+      tot = __shfl_sync(FULL, inc, 31);
+    } else {
+      run = block_exclusive<uint32_t>(r, tot);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (i0 + k < W) {
+        sp.upre[off + i0 + k] = run;
+        run += __popc(w[k]);
+      }
+    if (l > 0 && i0 < W) {
+      const uint32_t pw = parent_word(w);
+      sp.ubits[upper_off(l - 1) + i0 / 8u] = pw;
+      s_words[(l - 1) & 1][i0 / 8u] = pw;
+    }
+    if (threadIdx.x == 0) {
+      sp.ubits[off + W] = 0u;
+      sp.upre[off + W] = tot;
+      out[2 + l] = tot;
+    }
+    if (one_warp) __syncwarp();
+    else __syncthreads();
+  }
+}
+
+// ===========================================================================
+// Leaf payload (voxelizer.cpp:295-299, BarycentricCoords.h, main.cpp:373-382)
+// ===========================================================================
+__device__ void payload_color(const TriVerts& tv, const float n[3], int x, int y, int z, float unit_div,
+                              const float* __restrict__ tr, float col[3]) {
+  const float qx = __fdiv_rn((float)x, unit_div);
+  const float qy = __fdiv_rn((float)y, unit_div);
+  const float qz = __fdiv_rn((float)z, unit_div);
+  const float coeffD = -dot3(tv.v[0][0], tv.v[0][1], tv.v[0][2], n[0], n[1], n[2]);
+  const float nn = __fadd_rn(__fadd_rn(__fmul_rn(n[0], n[0]), __fmul_rn(n[1], n[1])), __fmul_rn(n[2], n[2]));
+  const float k = __fdiv_rn(__fadd_rn(dot3(qx, qy, qz, n[0], n[1], n[2]), coeffD), nn);
+  const float ptx = __fsub_rn(qx, __fmul_rn(k, n[0]));
+  const float pty = __fsub_rn(qy, __fmul_rn(k, n[1]));
+  const float ptz = __fsub_rn(qz, __fmul_rn(k, n[2]));
+  // inverse(mat3(v0, v1, v2)) by adjugate over determinant
+  const float a = tv.v[0][0], b = tv.v[1][0], c = tv.v[2][0];
+  const float d = tv.v[0][1], e = tv.v[1][1], f = tv.v[2][1];
+  const float g = tv.v[0][2], h = tv.v[1][2], i = tv.v[2][2];
+  const float C00 = __fsub_rn(__fmul_rn(e, i), __fmul_rn(f, h));
+  const float C01 = __fsub_rn(__fmul_rn(f, g), __fmul_rn(d, i));
+  const float C02 = __fsub_rn(__fmul_rn(d, h), __fmul_rn(e, g));
+  const float det = __fadd_rn(__fadd_rn(__fmul_rn(a, C00), __fmul_rn(b, C01)), __fmul_rn(c, C02));
+  const float r = __fdiv_rn(1.0f, det);
+  const float C10 = __fsub_rn(__fmul_rn(c, h), __fmul_rn(b, i));
+  const float C11 = __fsub_rn(__fmul_rn(a, i), __fmul_rn(c, g));
+  const float C12 = __fsub_rn(__fmul_rn(b, g), __fmul_rn(a, h));
+  const float C20 = __fsub_rn(__fmul_rn(b, f), __fmul_rn(c, e));
+  const float C21 = __fsub_rn(__fmul_rn(c, d), __fmul_rn(a, f));
+  const float C22 = __fsub_rn(__fmul_rn(a, e), __fmul_rn(b, d));
+  const float i00 = __fmul_rn(C00, r), i10 = __fmul_rn(C01, r), i20 = __fmul_rn(C02, r);
+  const float i01 = __fmul_rn(C10, r), i11 = __fmul_rn(C11, r), i21 = __fmul_rn(C12, r);
+  const float i02 = __fmul_rn(C20, r), i12 = __fmul_rn(C21, r), i22 = __fmul_rn(C22, r);
+  const float bx = __fadd_rn(__fadd_rn(__fmul_rn(i00, ptx), __fmul_rn(i01, pty)), __fmul_rn(i02, ptz));
+  const float by = __fadd_rn(__fadd_rn(__fmul_rn(i10, ptx), __fmul_rn(i11, pty)), __fmul_rn(i12, ptz));
+  const float bz = __fadd_rn(__fadd_rn(__fmul_rn(i20, ptx), __fmul_rn(i21, pty)), __fmul_rn(i22, ptz));
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    const float c0 = __ldg(tr + 12 + q), c1 = __ldg(tr + 15 + q), c2 = __ldg(tr + 18 + q);
+    col[q] = __fadd_rn(__fadd_rn(__fmul_rn(bx, c0), __fmul_rn(by, c1)), __fmul_rn(bz, c2));
+  }
+}
+
+// Colour, normal and local Morton code of leaf `li` (its index among the stripe's leaves).
+// Returns false (and flags) if the leaf has no winning triangle.
+__device__ bool leaf_value(const EmitJob& e, uint64_t li, uint32_t& key, float out[6]) {
+  const unsigned long long win = e.winners[li];  // triangle, Morton code
+  key = (uint32_t)win;
+  uint32_t lx, ly, lz;
+  morton_local_decode(key, lx, ly, lz);
+  const int x = e.origin[0] + (int)lx, y = e.origin[1] + (int)ly, z = e.origin[2] + (int)lz;
+  const uint64_t t = win >> 32;
+  if (t >= e.n_tris) {  // every set voxel has a passing triangle; anything else is a bug
+    raise_flag(e, 4u);
+    return false;
+  }
+  const float* tr = e.tris + t * 21;
+  const float nx = __ldg(tr + 9), ny = __ldg(tr + 10), nz = __ldg(tr + 11);
+  if (e.color_mode == 1) {  // COLOR_FIXED
+    out[0] = out[1] = out[2] = 1.0f;
+  } else if (e.color_mode == 2) {  // COLOR_LINEAR: mortonToRGB (svo_builder_util.h:14-18)
+    const float fn = (float)e.gridsize;
+    out[0] = __fdiv_rn((float)z, fn);
+    out[1] = __fdiv_rn((float)y, fn);
+    out[2] = __fdiv_rn((float)x, fn);
+  } else if (e.color_mode == 3) {  // COLOR_NORMAL
+    float a = nx, b = ny, c = nz;
+    normalize3(a, b, c);
+    out[0] = __fdiv_rn(__fadd_rn(a, 1.0f), 2.0f);
+    out[1] = __fdiv_rn(__fadd_rn(b, 1.0f), 2.0f);
+    out[2] = __fdiv_rn(__fadd_rn(c, 1.0f), 2.0f);
+  } else {  // COLOR_FROM_MODEL
+    const TriVerts tv = load_verts(e.tris, t, 21);
+    float n[3];
+    tri_normal(tv, n);
+    payload_color(tv, n, x, y, z, e.unit_div, tr, out);
+  }
+  out[3] = nx;
+  out[4] = ny;
+  out[5] = nz;
+  return true;
+}
+
+__device__ __forceinline__ void store_data_record(const EmitJob& e, uint64_t idx, uint64_t morton, const float* v) {
+  if (idx < e.data_win_base || idx - e.data_win_base >= e.data_win_len) {
+    raise_flag(e, 2u);
+    return;
+  }
+  uint4* dst = reinterpret_cast<uint4*>(e.data_win + (idx - e.data_win_base) * 32);
+  dst[0] = make_uint4((uint32_t)morton, (uint32_t)(morton >> 32), __float_as_uint(v[0]), __float_as_uint(v[1]));
+  dst[1] = make_uint4(__float_as_uint(v[2]), __float_as_uint(v[3]), __float_as_uint(v[4]), __float_as_uint(v[5]));
+}
+
+__device__ __forceinline__ void store_node_record(const EmitJob& e, uint64_t pos, uint64_t r0, uint64_t r1,
+                                                  uint64_t r2) {
+  if (pos < e.node_win_base || pos - e.node_win_base >= e.node_win_len) {
+    raise_flag(e, 1u);
+    return;
+  }
+  uint64_t* rec = e.node_win + (pos - e.node_win_base) * 3;
+  rec[0] = r0;
+  rec[1] = r1;
+  rec[2] = r2;
+}
+
+__device__ __forceinline__ uint64_t child_offsets(uint32_t mask) {
+  uint64_t off = 0;
+  uint32_t r = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const uint64_t byte = ((mask >> k) & 1u) ? (uint64_t)(r++) : 0xffull;
+    off |= byte << (8 * k);
+  }
+  return off;
+}
+
+// OctreeBuilder.cpp:81-99: sum over the 8 slots in child order (null slots add
+// zero), divide by the non-null count, normalise the normal.  `child`: the
+// averages (or leaf values) of the children, one after another; NULL: all zero.
+__device__ __forceinline__ void average_children(uint32_t mask, const float* child, float out[6]) {
+  float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  float notnull = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if ((mask >> k) & 1u) {
+      notnull = __fadd_rn(notnull, 1.0f);
+      if (child) {
+#pragma unroll
+        for (int q = 0; q < 6; q++) c[q] = child[q];
+        child += 6;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q++) acc[q] = __fadd_rn(acc[q], c[q]);
+  }
+  out[0] = __fdiv_rn(acc[0], notnull);
+  out[1] = __fdiv_rn(acc[1], notnull);
+  out[2] = __fdiv_rn(acc[2], notnull);
+  float tx = __fdiv_rn(acc[3], notnull), ty = __fdiv_rn(acc[4], notnull), tz = __fdiv_rn(acc[5], notnull);
+  normalize3(tx, ty, tz);
+  out[3] = tx;
+  out[4] = ty;
+  out[5] = tz;
+}
+
+// The last index w < n of a non-decreasing array with at(w) <= r (at(0) <= r), by the whole
+// warp: every step reads 32 entries at once, so 8,192 words take three dependent loads.
+template <typename F>
+__device__ __forceinline__ uint32_t warp_search(uint32_t n, uint32_t r, int lane, F at) {
+  uint32_t lo = 0, step = 1;
+  while (step * 32u < n) step *= 32u;
+  for (;; step /= 32u) {
+    const uint32_t i = lo + (uint32_t)lane * step;
+    lo += (uint32_t)(__popc(__ballot_sync(FULL, i < n && at(i) <= r)) - 1) * step;
+    if (step == 1) return lo;
+  }
+}
+
+constexpr uint32_t kTreeThreads = 256;
+constexpr uint32_t kTreeWarps = kTreeThreads / 32;
+static_assert(kTreeWarps == kTreeWarpsPerCta, "the host sizes the launches");
+
+// ===========================================================================
+// Leaf payloads, one thread per leaf: the winner pass left every leaf's triangle
+// and Morton code.  The leaf goes straight into the data file: without -levels
+// leaf i of the stripe is its data record i; with -levels the averages of the inner
+// nodes whose regions end before the leaf stand before it too.
+//
+// Bound by the gathers of the winners' 84-byte triangle records.
+// ===========================================================================
+// Inner nodes of the stripe whose regions end before leaf bit `key`.
+__device__ __forceinline__ uint32_t inner_before(const Stripe& p, uint32_t key) {
+  const uint32_t x = p.K == kBrickLevels ? key >> 12 : 0u, blk = key >> 8;
+  uint32_t s = p.wpre[x >> 5].y + p.bpre[x].y + p.inner_local[blk];
+  if (p.K == kBrickLevels) s += __popc(p.bunits[x] & ((1u << ((key >> 9) & 7u)) - 1u));  // nodes of 512 leaf bits
+  for (int l = 1; l <= p.U; l++) s += upper_rank(p, l, x >> (3 * (p.U - l)));
+  const uint4* q = reinterpret_cast<const uint4*>(p.leaf) + 2 * (uint64_t)blk;
+  const uint4 q0 = q[0], q1 = q[1];
+  const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+  const uint32_t wi = (key >> 5) & 7u;
+#pragma unroll
+  for (uint32_t k = 0; k < 8; k++) {  // the block's words before the leaf's, and the bytes before the leaf's
+    const uint32_t v = k < wi ? w[k] : (k == wi ? w[k] & ((1u << (key & 24u)) - 1u) : 0u);
+    if (p.K >= 2) s += __popc(nonzero_bytes(v));
+    if (p.K >= 3 && (k & 1u) && k < (wi & ~1u)) s += (w[k - 1] | w[k]) ? 1u : 0u;  // nodes of 64 leaf bits
+  }
+  return s;
+}
+
+__device__ __forceinline__ void leaf_payload(const Stripe& p, const EmitJob& e, uint64_t i) {
+  if (i >= e.n_leaf) return;
+  float v[6];
+  uint32_t key;
+  if (!leaf_value(e, i, key, v)) return;
+  store_data_record(e, e.data_base + i + (e.levels ? inner_before(p, key) : 0u), e.stripe_base + key, v);
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(kTreeThreads) kb_leaf_payload(const Stripe* __restrict__ stripes,
+                                                                const EmitJob* __restrict__ emits,
+                                                                const uint64_t* __restrict__ cta_beg, uint32_t n,
+                                                                uint32_t ept, Stripe p0, EmitJob e0) {
+  pdl_enter();
+  if constexpr (SINGLE) {
+    for (uint32_t k = 0; k < ept; k++) leaf_payload(p0, e0, ((uint64_t)blockIdx.x * ept + k) * kTreeThreads + threadIdx.x);
+  } else {
+    __shared__ Stripe sp;
+    __shared__ EmitJob se;
+    uint64_t cta;
+    const uint32_t s = cta_stripe(cta_beg, n, cta);
+    stage(sp, stripes[s]);
+    stage(se, emits[s]);
+    __syncthreads();
+    for (uint32_t k = 0; k < ept; k++) leaf_payload(sp, se, (cta * ept + k) * kTreeThreads + threadIdx.x);
+  }
+}
+
+// ===========================================================================
+// Emission: the records of every brick's run and the brick's own.
+//
+// A warp takes consecutive non-empty bricks of the stripe and lays them out in
+// steps of eight units (a unit: 512 leaf bits, a child of a brick), four lanes to
+// a unit, whichever bricks the units belong to, so a step is full on sparse bricks
+// too.  A lane holds 128 leaf bits: two nodes of 64 (a run of their leaves and
+// those leaves' parents, and their own records in the unit's group).  One warp
+// scan gives every position of a step.  The parents of leaves, whose number per
+// lane varies most, are shared out over all lanes.  The records of a step are one
+// run per brick: they are written to shared memory and leave as bulk copies, one
+// per brick, so every sector of the node file is written whole and the copy costs
+// the warp a few instructions (records stored by the lanes themselves took 2.2 times
+// as long on the 20M-triangle soup at gridsize 4096).
+//
+// Bound by latency and issue: about 800 warp instructions per step, DRAM at a
+// third of its rate.  The 20M-triangle soup (651M records, 15.6 GB) takes 6.8 ms;
+// the passes this replaced (keys, subtree sizes bottom-up, positions top-down and
+// leaf records, each over arrays of every node) took 19 ms.  On the 1024^3
+// heightfield it is 41 us instead of 190.
+// ===========================================================================
+// A window holds kWindow records and a gap of up to two slots between the records of eight bricks.
+// CTAs per SM: three (no spills) took 10% longer on the large soups and 10% less on the heightfield,
+// where a warp has one or two bricks; five is within 2% of four.
+constexpr int kEmitCtas = 4;
+constexpr uint32_t kWindow = 128;
+constexpr uint32_t kSlots = kWindow + 16;
+
+// A lane's words as the warp's lanes read them when they share out the step's parents of leaves.
+struct __align__(16) LaneWords {
+  uint64_t a, b;
+  uint32_t m16_gap;  // non-zero bytes of a and b | slots before its brick's records << 16
+  uint32_t c_pk;     // the lane's first record in the step | parents of leaves before it << 16
+  uint32_t base;     // a record's number in the step + this = its position in the stripe
+  uint32_t da;       // -levels: data records of the stripe before a's leaves
+};
+struct __align__(16) WarpScratch {
+  uint64_t win[kSlots * 3];
+  LaneWords words[32];
+  uint32_t gaps[8];
+};
+
+// Bit position of the t-th (from 0) set bit of the 8-bit mask m.
+__device__ __forceinline__ uint32_t select8(uint32_t m, uint32_t t) {
+  uint32_t pos = 0, c = __popc(m & 15u);
+  if (t >= c) {
+    t -= c;
+    pos = 4;
+  }
+  c = __popc((m >> pos) & 3u);
+  if (t >= c) {
+    t -= c;
+    pos += 2;
+  }
+  return pos + (t >= ((m >> pos) & 1u) ? 1u : 0u);
+}
+
+// Bulk copies of shared memory to global memory (both 16-byte aligned, a multiple of 16
+// bytes); a thread's copies since its last commit form a group.
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+               "r"((uint32_t)__cvta_generic_to_shared(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// Shared memory written by this thread becomes visible to its warp's bulk copies.
+__device__ __forceinline__ void bulk_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// Running sum of a node's children (OctreeBuilder.cpp:81-99).  Adding a null slot's zero
+// never changes a sum (no sum is -0), so null slots are skipped.
+struct Sum {
+  float v[6];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int q = 0; q < 6; q++) v[q] = 0.0f;
+  }
+  __device__ __forceinline__ void add(const float* c) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) v[q] = __fadd_rn(v[q], c[q]);
+  }
+  // the colour and normal of a data record
+  __device__ __forceinline__ void add(const uint4& r0, const uint4& r1) {
+    const float c[6] = {__uint_as_float(r0.z), __uint_as_float(r0.w), __uint_as_float(r1.x),
+                        __uint_as_float(r1.y), __uint_as_float(r1.z), __uint_as_float(r1.w)};
+    add(c);
+  }
+  // divided by the children's number, the normal normalised
+  __device__ __forceinline__ void average(uint32_t children) {
+    const float n = (float)children;
+#pragma unroll
+    for (int q = 0; q < 6; q++) v[q] = __fdiv_rn(v[q], n);
+    normalize3(v[3], v[4], v[5]);
+  }
+};
+
+// -levels: the average of n <= 8 children from their data records, child k's at(k); four
+// children's loads at a time.
+template <typename F>
+__device__ __forceinline__ void average_records(const EmitJob& e, uint32_t n, Sum& s, F at) {
+  s.zero();
+  for (uint32_t k0 = 0; k0 < n; k0 += 4) {
+    uint4 r[4][2];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if (k0 + k < n) {
+        const uint64_t i = at(k0 + k) - e.data_win_base;
+        if (i < e.data_win_len) {
+          const uint4* src = reinterpret_cast<const uint4*>(e.data_win + i * 32);
+          r[k][0] = src[0];
+          r[k][1] = src[1];
+        }
+      }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if (k0 + k < n) s.add(r[k][0], r[k][1]);
+  }
+  s.average(n);
+}
+
+// What the layout of word w's bricks needs from memory, lane = brick.  Loaded before the
+// previous word is laid out: the marks come from DRAM, and the word's first use of them would
+// otherwise wait for two loads in a row.
+struct WordIn {
+  uint32_t bits;        // the word
+  uint2 wp, wn, bp;     // leaves and inner nodes before the word, before the next, and before the brick in the word
+  uint32_t units;
+  uint4 marks;
+  uint32_t up, upd;     // upper nodes recorded before the brick's parent's children; averaged before the brick (-levels)
+};
+
+template <bool LEVELS>
+__device__ __forceinline__ WordIn load_word(const Stripe& p, uint32_t w, int lane) {
+  WordIn in;
+  const int U = p.U;
+  const uint32_t x = w * 32u + (uint32_t)lane, off = upper_off(U) + w;
+  in.bits = p.ubits[off];
+  const bool have = (in.bits >> lane) & 1u;
+  in.wp = p.wpre[w];
+  in.wn = p.wpre[w + 1];
+  in.bp = p.bpre[x];
+  in.units = have ? p.bunits[x] : 0u;
+  in.marks = make_uint4(~0u, ~0u, ~0u, ~0u);
+  if (have && p.touch) in.marks = reinterpret_cast<const uint4*>(p.touch)[x];
+  in.up = in.upd = 0;
+  if (U) {
+    const uint32_t pre = p.upre[off];
+    in.up = pre + __popc(in.bits & ((1u << (lane & ~7)) - 1u));
+    if (LEVELS) in.upd = pre + __popc(in.bits & ((1u << lane) - 1u));
+#pragma unroll
+    for (int l = 1; l < kMaxUpper; l++)
+      if (l < U) {
+        const uint32_t anc = x >> (3 * (U - l));
+        const uint32_t i = upper_off(l) + (anc >> 5), ub = p.ubits[i], ur = p.upre[i];
+        in.up += ur + __popc(ub & ((1u << (anc & 24u)) - 1u));  // before its parent's children: whole bytes
+        if (LEVELS) in.upd += ur + __popc(ub & ((1u << (anc & 31u)) - 1u));
+      }
+  }
+  return in;
+}
+
+// The bricks `rem` of word w.
+template <bool LEVELS>
+__device__ __forceinline__ void emit_word(const Stripe& p, const EmitJob& e, uint32_t w, uint32_t rem, const WordIn& in,
+                                          int lane, WarpScratch& sm, const uint64_t* __restrict__ lut) {
+  const uint32_t le = (2u << lane) - 1u, lt = le >> 1;
+  const int K = p.K, U = p.U;
+  const bool pay = !e.binary;
+  uint64_t* const nodes = e.node_win - (int64_t)(e.node_win_base - e.node_base) * 3;  // the stripe's records
+  const uint64_t dbase = e.data_base;
+  // ---- lane = brick x ----
+  const uint32_t x = w * 32u + (uint32_t)lane;
+  bool mine = (rem >> lane) & 1u;
+  const uint2 wn = in.wn;
+  const uint32_t lpre = in.wp.x + in.bp.x, ipre = in.wp.y + in.bp.y;
+  uint32_t units = mine && K ? in.units : 0u;
+  // leaf blocks that may have a bit
+  const uint32_t blocks = nonzero_bytes(in.marks.x) | (nonzero_bytes(in.marks.y) << 4) | (nonzero_bytes(in.marks.z) << 8) |
+                          (nonzero_bytes(in.marks.w) << 12);
+  const uint32_t up = in.up, upd = in.upd;
+  const uint32_t sib = __popc((in.bits >> (lane & ~7)) & ((1u << (lane & 7)) - 1u));
+  const uint32_t start = up + lpre + ipre;  // stripe-relative, like all positions here
+  uint32_t nl = __shfl_down_sync(FULL, lpre, 1), ni = __shfl_down_sync(FULL, ipre, 1);  // before the next brick
+  const uint32_t pend = ((uint32_t)lane | 7u) + 1u;                                      // the parent's end
+  uint32_t pl = __shfl_sync(FULL, lpre, (int)(pend & 31u)), pi = __shfl_sync(FULL, ipre, (int)(pend & 31u));
+  if (lane == 31) nl = wn.x, ni = wn.y;
+  if (pend == 32u) pl = wn.x, pi = wn.y;
+  const uint32_t n3 = K == kBrickLevels ? __popc(units) : 0u;
+  const uint32_t g3 = start + (nl - lpre) + (ni - ipre) - n3;  // where its children's group starts
+  const uint32_t dpre = LEVELS ? (pay ? lpre : 0u) + ipre + upd : 0u;               // data records before its own
+  const uint32_t dtop = LEVELS ? dpre + (pay ? nl - lpre : 0u) + (ni - ipre) : 0u;  // and before its average
+  const uint32_t own_at = up + pl + pi + sib;                                       // its own record
+  // every record of the brick lies in the window (the run from start to g3 + n3, then its own)
+  if (mine && K &&
+      (e.node_base + start < e.node_win_base ||
+       e.node_base + max(g3 + n3, U ? own_at + 1u : 0u) - e.node_win_base > e.node_win_len)) {
+    raise_flag(e, 1u);
+    mine = false;
+    units = 0;
+  }
+  if (U && mine) {  // its own record, in its parent's group
+    uint64_t* t = nodes + (uint64_t)own_at * 3u;
+    t[0] = LEVELS ? dbase + dtop : 0;
+    t[1] = e.node_base + g3;
+    t[2] = lut[units];
+  }
+  const uint32_t cnt = __popc(units);
+  const uint32_t incl = warp_inclusive(cnt), excl = incl - cnt;
+  const uint32_t total = __shfl_sync(FULL, incl, 31);
+  uint32_t carry = 0;          // records | leaves << 16 of the last step's last brick so far
+  uint32_t root_mask = units;  // of a one-brick stripe
+  const uint32_t odd0 = (uint32_t)(reinterpret_cast<uintptr_t>(nodes) >> 3);
+  for (uint32_t g = 0; g < total; g += 8u) {
+    // ---- four lanes = unit u ----
+    const uint32_t u = g + (uint32_t)(lane >> 2);
+    const bool valid = u < total;
+    uint32_t o = 0;  // its brick: the first lane with incl > u
+#pragma unroll
+    for (uint32_t st = 16; st; st >>= 1) {
+      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
+      if (t <= u) o += st;
+    }
+    const uint32_t o_first = __shfl_sync(FULL, excl, (int)o);
+    const uint32_t t3 = u - o_first;  // its number in the brick
+    const uint32_t q = select8(__shfl_sync(FULL, units, (int)o), t3) & 7u;
+    const uint32_t o_blocks = __shfl_sync(FULL, blocks, (int)o), o_start = __shfl_sync(FULL, start, (int)o);
+    const uint32_t o_g3 = __shfl_sync(FULL, g3, (int)o);
+    uint32_t o_lpre = 0, o_dpre = 0;
+    if (!LEVELS && pay) o_lpre = __shfl_sync(FULL, lpre, (int)o);
+    if (LEVELS) o_dpre = __shfl_sync(FULL, dpre, (int)o);
+    const uint32_t xo = w * 32u + o;
+    const uint32_t word = xo * 128u + q * 16u + (uint32_t)(lane & 3) * 4u;  // below 2^25
+    uint64_t a = 0, b = 0;
+    if (valid && ((o_blocks >> (2u * q + (uint32_t)((lane >> 1) & 1))) & 1u) && (K == kBrickLevels || word < leaf_words(p.depth))) {
+      uint4* src = reinterpret_cast<uint4*>(p.leaf + word);
+      const uint4 v = *src;
+      a = (uint64_t)v.x | ((uint64_t)v.y << 32);
+      b = (uint64_t)v.z | ((uint64_t)v.w << 32);
+      if (a | b) *src = make_uint4(0u, 0u, 0u, 0u);  // zero for the next build
+    }
+    const uint32_t ca = __popcll(a), cb = __popcll(b);
+    const uint32_t ma = K >= 2 ? nonzero_bytes64(a) : 0u, mb = K >= 2 ? nonzero_bytes64(b) : 0u;
+    const uint32_t ka = __popc(ma), kb = __popc(mb), kc = ka + kb;
+    const uint32_t bal_a = __ballot_sync(FULL, ca != 0), bal_b = __ballot_sync(FULL, cb != 0);
+    const uint32_t na4 = (bal_a >> (lane & 28)) & 15u, nb4 = (bal_b >> (lane & 28)) & 15u;
+    // the unit's child mask: its lanes' a and b in turn
+    const uint32_t m3 = ((na4 & 1u) | ((na4 & 2u) << 1) | ((na4 & 4u) << 2) | ((na4 & 8u) << 3)) |
+                        (((nb4 & 1u) | ((nb4 & 2u) << 1) | ((nb4 & 4u) << 2) | ((nb4 & 8u) << 3)) << 1);
+    const uint32_t k2 = K >= 3 ? __popc(m3) : 0u;
+    const bool last = (lane & 3) == 3;
+    // records | leaves << 16: of the lane, before it in the step, before it in its brick
+    const uint32_t own = (ca + cb + kc + (last ? k2 : 0u)) | ((ca + cb) << 16);
+    const uint32_t inc = warp_inclusive(own), before = inc - own;
+    const uint32_t head = o_first > g ? o_first - g : 0u;  // the brick's first unit of this step
+    const uint32_t in_brick = before - __shfl_sync(FULL, before, (int)((head * 4u) & 31u)) + (o_first < g ? carry : 0u);
+    const uint32_t brick_end = in_brick + own;
+    carry = __shfl_sync(FULL, brick_end, 31);
+    const uint32_t S = __shfl_sync(FULL, inc, 31) & 0xffffu;  // records of the step
+    const uint32_t c_at = before & 0xffffu;                   // the lane's first record in the step
+    const uint32_t base = o_start + (in_brick & 0xffffu) - c_at;
+    const uint32_t grp = o_start + (__shfl_sync(FULL, brick_end, lane | 3) & 0xffffu) - k2;  // the unit's children's group
+    // the step's records stand brick by brick, brick s's starting at an even or odd word like in the
+    // file: of the two slots before a brick's records one decides the parity
+    const bool is_head = (lane & 3) == 0 && valid && (uint32_t)(lane >> 2) == head;
+    const uint32_t heads = __ballot_sync(FULL, is_head);
+    const uint32_t to_here = (2u << (lane & 28)) - 1u;
+    const uint32_t later = heads & ~to_here;
+    const uint32_t c_next = __shfl_sync(FULL, c_at, later ? __ffs(later) - 1 : 0);
+    const uint32_t s = __popc(heads & to_here) - 1u;
+    const uint32_t gap = 2u * s + ((odd0 + base) & 1u);
+    if (is_head) sm.gaps[s & 7u] = gap;
+    // parents of leaves: before the lane and in the step
+    const uint32_t quad_lt = (1u << (lane & 28)) - 1u;
+    const uint32_t own_recs = K >= 3 ? __popc(bal_a & quad_lt) + __popc(bal_b & quad_lt) : 0u;  // of earlier units' words
+    const uint32_t pk = c_at - (before >> 16) - own_recs;
+    const uint32_t n1 = __shfl_sync(FULL, pk + kc, 31);
+    uint32_t da = 0, db = 0, d3 = 0;  // -levels: data records before a's, b's leaves and before the unit's average
+    if (LEVELS) {
+      const uint32_t in4 = (1u << (lane & 3)) - 1u;
+      da = o_dpre + (in_brick & 0xffffu) - (pay ? 0u : in_brick >> 16) + t3;
+      if (K >= 3) da += __popc(na4 & in4) + __popc(nb4 & in4);  // the words before it in the unit
+      db = da + (pay ? ca : 0u) + ka + (K >= 3 && ca ? 1u : 0u);
+      d3 = db + (pay ? cb : 0u) + kb + (K >= 3 && cb ? 1u : 0u);
+    }
+    const uint32_t has_k = __ballot_sync(FULL, kc != 0);
+    if (kc) sm.words[__popc(has_k & lt)] = LaneWords{a, b, ma | (mb << 8) | (gap << 16), c_at | (pk << 16), base, da};
+    __syncwarp();
+    // item i0 + lane of the step's parents of leaves
+    struct Parent {
+      uint32_t mask, nc;  // its children
+      uint32_t first;     // its first leaf's record in the step
+      uint32_t r;         // its own
+      uint32_t gap, base, d;  // d: -levels, data records before its leaves
+    };
+    auto parent = [&](uint32_t i0) {
+      uint32_t h = 0;
+      if (kc && pk - i0 < 32u) h = 1u << (pk - i0);
+      h = __reduce_or_sync(FULL, h);
+      const uint32_t slot = __popc(__ballot_sync(FULL, kc != 0 && pk < i0)) + __popc(h & le) - 1u;
+      const LaneWords lw = sm.words[slot & 31u];
+      const uint32_t m16 = lw.m16_gap & 0xffffu, ka1 = __popc(m16 & 0xffu);
+      const uint32_t i = i0 + (uint32_t)lane - (lw.c_pk >> 16);  // its number among the owner's
+      const bool in_b = i >= ka1;
+      const uint32_t j = in_b ? i - ka1 : i;  // and among its word's
+      const uint64_t v = in_b ? lw.b : lw.a;
+      const uint32_t k = select8(in_b ? m16 >> 8 : m16 & 0xffu, j) & 7u;
+      const uint32_t ca1 = __popcll(lw.a), l0 = __popcll(v & ((1ull << (8u * k)) - 1ull));
+      const uint32_t word_at = (lw.c_pk & 0xffffu) + (in_b ? ca1 + ka1 : 0u);
+      Parent t;
+      t.mask = (uint32_t)(v >> (8u * k)) & 0xffu;
+      t.nc = __popc(t.mask);
+      t.first = word_at + l0;
+      t.r = word_at + (uint32_t)__popcll(v) + j;
+      t.gap = lw.m16_gap >> 16;
+      t.base = lw.base;
+      t.d = LEVELS ? lw.da + (in_b ? (pay ? ca1 : 0u) + ka1 + (K >= 3 && ca1 ? 1u : 0u) : 0u) + (pay ? l0 : 0u) + j : 0u;
+      return t;
+    };
+    if (LEVELS) {  // the averages, each also a data record; the leaves' records are there already
+      for (uint32_t i0 = 0; i0 < n1; i0 += 32u) {  // of leaves' parents
+        const Parent t = parent(i0);
+        if (i0 + (uint32_t)lane < n1) {
+          Sum sum;
+          if (pay) {
+            average_records(e, t.nc, sum, [&](uint32_t k) { return dbase + t.d + k; });
+          } else {
+            sum.zero();
+            sum.average(t.nc);
+          }
+          store_data_record(e, dbase + t.d + (pay ? t.nc : 0u), 0, sum.v);
+        }
+      }
+      __syncwarp();
+      Sum sa, sb;
+      sa.zero();
+      sb.zero();
+      if (K >= 2) {  // of the lanes' words
+        auto word_average = [&](uint64_t v, uint32_t m8, uint32_t d, Sum& sum) {
+          uint32_t m = m8, at = d;
+          average_records(e, __popc(m8), sum, [&](uint32_t) {
+            at += pay ? __popc((uint32_t)(v >> (8u * ((uint32_t)__ffs(m) - 1u))) & 0xffu) : 0u;
+            m &= m - 1;
+            return dbase + at++;
+          });
+          if (K >= 3) store_data_record(e, dbase + at, 0, sum.v);
+        };
+        if (ka) word_average(a, ma, da, sa);
+        if (kb) word_average(b, mb, db, sb);
+      } else if (ca) {  // the leaves' parent is the stripe root
+        if (pay) average_records(e, ca, sa, [&](uint32_t k) { return dbase + da + k; });
+        else sa.average(ca);
+      }
+      if (K >= 3) {
+        Sum s3;
+        s3.zero();
+#pragma unroll 1
+        for (int k = 0; k < 8; k++) {
+          float c[6];
+#pragma unroll
+          for (int i = 0; i < 6; i++) c[i] = __shfl_sync(FULL, (k & 1) ? sb.v[i] : sa.v[i], (lane & ~3) | (k >> 1));
+          if ((m3 >> k) & 1u) s3.add(c);
+        }
+        sa = s3;
+        if (last && valid) {
+          sa.average(__popc(m3));
+          if (K == kBrickLevels) store_data_record(e, dbase + d3, 0, sa.v);
+        }
+      }
+      // for the brick's average: a child's, or (fewer levels) the brick's own
+      if (K >= 3 ? (last && valid) : lane == 0) {
+        float* c = e.upper_cache + (K == kBrickLevels ? upper_cell(U + 1, (uint64_t)xo * 8u + q) : upper_cell(U, xo)) * 6;
+#pragma unroll
+        for (int i = 0; i < 6; i++) c[i] = sa.v[i];
+      }
+    }
+    if (K < kBrickLevels) {
+      const uint32_t r = K == 3 ? m3 : (K == 2 ? ma : (uint32_t)a & 0xffu);
+      root_mask = __shfl_sync(FULL, r, 0);
+    } else if (last && valid) {  // the unit's own record
+      uint64_t* t = nodes + (uint64_t)(o_g3 + t3) * 3u;
+      t[0] = LEVELS ? dbase + d3 : 0;
+      t[1] = e.node_base + grp;
+      t[2] = lut[m3];
+    }
+    // ---- the records, window by window ----
+    uint32_t next = 0, next_l = 0;  // the first parent whose record (whose last leaf's) is not yet written
+    uint64_t leaf_data = 0;         // payload: the next leaf's data record
+    if (!LEVELS && pay) leaf_data = dbase + __shfl_sync(FULL, o_lpre + (in_brick >> 16), 0);
+    for (uint32_t w0 = 0; w0 < S; w0 += kWindow) {
+      const uint32_t nrec = min(kWindow, S - w0);
+      bulk_wait_read();  // the copies out of the window have read it
+      __syncwarp();
+      uint64_t* const rec = sm.win;
+      {  // every slot a leaf's record, two words at a time
+        const uint32_t n4 = ((nrec + 2u * __popc(heads)) * 3u + 1u) / 2u;
+        uint32_t f = (2u * (uint32_t)lane) % 3u;  // the first word's place in its record; +64 words: one further
+        const uint64_t lead = pay ? 0ull : 1ull;
+        for (uint32_t i = (uint32_t)lane; i < n4; i += 32u) {
+          reinterpret_cast<ulonglong2*>(rec)[i] =
+              make_ulonglong2(f == 0 ? lead : (f == 1 ? 0ull : ~0ull), f == 0 ? 0ull : (f == 1 ? ~0ull : lead));
+          f = f == 2 ? 0u : f + 1u;
+        }
+      }
+      __syncwarp();
+      auto put = [&](uint32_t slot, uint64_t d, uint32_t child, uint32_t mask) {
+        uint64_t* t = rec + slot * 3u;
+        t[0] = d;
+        t[1] = e.node_base + child;
+        t[2] = lut[mask];
+      };
+      while (next < n1) {  // the leaves' parents, in the order of their records
+        const Parent t = parent(next);
+        const bool in = next + (uint32_t)lane < n1 && t.r < w0 + kWindow;
+        if (in) put(t.r - w0 + t.gap, LEVELS ? dbase + t.d + (pay ? t.nc : 0u) : 0, t.base + t.first, t.mask);
+        const uint32_t done = __popc(__ballot_sync(FULL, in));
+        next += done;
+        if (done < 32u) break;
+      }
+      if (K >= 3) {  // the words' own records, in their units' groups
+        const uint32_t gr = grp - base, below = 2u * (uint32_t)(lane & 3);
+        const uint32_t r_a = gr + __popc(m3 & ((1u << below) - 1u)), r_b = gr + __popc(m3 & ((2u << below) - 1u));
+        if (ca && r_a - w0 < kWindow) put(r_a - w0 + gap, LEVELS ? dbase + da + (pay ? ca : 0u) + ka : 0, base + c_at + ca, ma);
+        if (cb && r_b - w0 < kWindow)
+          put(r_b - w0 + gap, LEVELS ? dbase + db + (pay ? cb : 0u) + kb : 0, base + c_at + ca + ka + cb, mb);
+      }
+      if (pay && !LEVELS) {  // a leaf's data record: leaves stand in the order of their records
+        __syncwarp();
+        for (uint32_t i0 = 0; i0 < nrec; i0 += 32u) {
+          const uint32_t r0 = w0 + i0;
+          uint32_t h = 0;
+          if (is_head && c_at - r0 < 32u) h = 1u << (c_at - r0);
+          h = __reduce_or_sync(FULL, h);
+          const uint32_t sg = __popc(__ballot_sync(FULL, is_head && c_at < r0)) + __popc(h & le) - 1u;
+          uint64_t* t = rec + (i0 + (uint32_t)lane + sm.gaps[sg & 7u]) * 3u;
+          const bool is_leaf = i0 + (uint32_t)lane < nrec && t[2] == ~0ull;
+          const uint32_t bal = __ballot_sync(FULL, is_leaf);
+          if (is_leaf) t[0] = leaf_data + __popc(bal & lt);
+          leaf_data += __popc(bal);
+        }
+      }
+      if (LEVELS && pay) {  // with the averages of the parents between them
+        if (K < 2) {
+          for (uint32_t t = 0; t < ca; t++) rec[(c_at + t + gap) * 3u] = dbase + da + t;  // (at most eight records)
+        }
+        while (next_l < n1) {
+          const Parent t = parent(next_l);
+          const bool have = next_l + (uint32_t)lane < n1;
+          if (have)
+            for (uint32_t k = 0; k < t.nc; k++)
+              if (t.first + k - w0 < kWindow) rec[(t.first + k - w0 + t.gap) * 3u] = dbase + t.d + k;
+          const uint32_t done = __popc(__ballot_sync(FULL, have && t.first + t.nc <= w0 + kWindow));
+          next_l += done;
+          if (done < 32u) break;
+        }
+      }
+      bulk_fence();
+      __syncwarp();
+      if (is_head) {
+        const uint32_t r0 = max(c_at, w0), r1 = min(later ? c_next : S, w0 + kWindow);
+        if (r0 < r1) {
+          uint64_t* dst = nodes + (uint64_t)(base + r0) * 3u;
+          const uint64_t* src = rec + (r0 - w0 + gap) * 3u;
+          uint32_t n = (r1 - r0) * 3u;
+          if (reinterpret_cast<uintptr_t>(dst) & 8u) {
+            *dst++ = *src++;
+            n--;
+          }
+          if (n & 1u) dst[n - 1] = src[n - 1];
+          if (n >= 2u) bulk_store(dst, src, (n & ~1u) * 8u);
+        }
+      }
+      bulk_commit();
+    }
+    __syncwarp();  // the lanes' words are free for the next step
+  }
+  if (LEVELS && K) {
+    __syncwarp();
+    if (mine) {
+      float* c = e.upper_cache + upper_cell(U, x) * 6;
+      Sum s4;
+      s4.zero();
+      if (K == kBrickLevels) {  // from its children's averages
+        for (uint32_t m = units; m; m &= m - 1)
+          s4.add(e.upper_cache + upper_cell(U + 1, (uint64_t)x * 8u + (uint32_t)__ffs(m) - 1u) * 6);
+        s4.average(__popc(units));
+#pragma unroll
+        for (int i = 0; i < 6; i++) c[i] = s4.v[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 6; i++) s4.v[i] = c[i];
+      }
+      store_data_record(e, dbase + dtop, 0, s4.v);
+      if (U == 0)
+        for (int i = 0; i < 6; i++) e.root_out[1 + i] = __float_as_uint(s4.v[i]);
+    }
+  }
+  if (mine && p.touch) reinterpret_cast<uint4*>(p.touch)[x] = make_uint4(0u, 0u, 0u, 0u);  // zero for the next build
+  if (U == 0 && lane == 0) {  // the stripe root, which the host writes
+    e.root_out[0] = root_mask;
+    if (K == 0) {  // one voxel
+      p.leaf[0] = 0u;
+      if (pay) {
+        float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        uint32_t key;
+        leaf_value(e, 0, key, c);
+        for (int i = 0; i < 6; i++) e.root_out[1 + i] = __float_as_uint(c[i]);
+      }
+    }
+  }
+}
+
+// The bricks of the stripe's warp i: bricks_per_warp consecutive ones of its non-empty bricks.
+template <bool LEVELS>
+__device__ __forceinline__ void emit_warp(const Stripe& p, const EmitJob& e, uint64_t i, int lane, WarpScratch& sm,
+                                          const uint64_t* __restrict__ lut) {
+  const uint32_t W = upper_words(p.U), off = upper_off(p.U), n = p.upre[off + W];
+  const uint64_t r0 = i * e.bricks_per_warp;
+  if (r0 >= n) return;
+  uint32_t r = (uint32_t)r0;
+  const uint32_t r1 = (uint32_t)min((uint64_t)n, r0 + e.bricks_per_warp);
+  uint32_t w = warp_search(W, r, lane, [&](uint32_t i) { return p.upre[off + i]; });
+  WordIn in = load_word<LEVELS>(p, w, lane);
+  uint32_t rank = p.upre[off + w];  // of the word's first brick
+  for (;;) {
+    const uint32_t mine = rank + __popc(in.bits & ((1u << lane) - 1u));
+    const uint32_t rem = __ballot_sync(FULL, ((in.bits >> lane) & 1u) && mine >= r && mine < r1);
+    rank += __popc(in.bits);
+    uint32_t nw = w;
+    WordIn next = in;
+    const bool more = rank < r1;
+    if (more) {
+      for (nw = w + 1; nw < W; nw += 32u) {  // the next word with a brick: there is one
+        const uint32_t i = nw + (uint32_t)lane;
+        const uint32_t some = __ballot_sync(FULL, i < W && p.ubits[off + i] != 0u);
+        if (some) {
+          nw += (uint32_t)__ffs(some) - 1u;
+          break;
+        }
+      }
+      if (nw < W) next = load_word<LEVELS>(p, nw, lane);
+    }
+    emit_word<LEVELS>(p, e, w, rem, in, lane, sm, lut);
+    if (!more || nw >= W) break;
+    w = nw;
+    in = next;
+  }
+  bulk_wait_all();
+}
+
+template <bool SINGLE, bool LEVELS>
+__global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(const Stripe* __restrict__ stripes,
+                                                                      const EmitJob* __restrict__ emits,
+                                                                      const uint64_t* __restrict__ cta_beg, uint32_t n,
+                                                                      Stripe p0, EmitJob e0) {
+  __shared__ uint64_t lut[256];  // child_offsets of every mask
+  __shared__ WarpScratch ws[kTreeWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  static_assert(kTreeThreads == 256, "one table entry per thread");
+  static_assert(kWindow % 2 == 0 && kSlots % 2 == 0, "windows start on 16 bytes, every window's parity is the same");
+  lut[threadIdx.x] = child_offsets(threadIdx.x);
+  pdl_enter();
+  if constexpr (SINGLE) {
+    __syncthreads();
+    emit_warp<LEVELS>(p0, e0, (uint64_t)blockIdx.x * kTreeWarps + (uint32_t)warp, lane, ws[warp], lut);
+  } else {
+    __shared__ Stripe sp;
+    __shared__ EmitJob se;
+    uint64_t cta;
+    const uint32_t s = cta_stripe(cta_beg, n, cta);
+    stage(sp, stripes[s]);
+    stage(se, emits[s]);
+    __syncthreads();
+    const uint64_t i = cta * kTreeWarps + (uint32_t)warp;
+    if (LEVELS && se.levels) emit_warp<true>(sp, se, i, lane, ws[warp], lut);
+    else emit_warp<false>(sp, se, i, lane, ws[warp], lut);
+  }
+}
+
+// ---- the levels above the bricks ----
+// Average of cell z of level l from the cells of level l + 1.
+__device__ __forceinline__ void average_cell(const Stripe& p, const EmitJob& e, int l, uint32_t z) {
+  if (!((p.ubits[upper_off(l) + (z >> 5)] >> (z & 31u)) & 1u)) return;
+  const uint32_t mask = upper_byte(p, l + 1, z);
+  // the children's averages stand at their cells: gather them in child order
+  float child[48];
+  uint32_t c = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 8; k++)
+    if ((mask >> k) & 1u) {
+      const float* src = e.upper_cache + upper_cell(l + 1, (uint64_t)z * 8u + k) * 6;
+      for (int q = 0; q < 6; q++) child[c * 6 + q] = src[q];
+      c++;
+    }
+  float v[6];
+  average_children(mask, child, v);
+  float* out = e.upper_cache + upper_cell(l, z) * 6;
+#pragma unroll
+  for (int q = 0; q < 6; q++) out[q] = v[q];
+}
+
+// Level l of the stripes that have it above their bricks, one thread per cell (grid.y: the stripes).
+__global__ void __launch_bounds__(256) kb_upper_avg(const Stripe* __restrict__ stripes, const EmitJob* __restrict__ emits,
+                                                    uint32_t n, int l) {
+  pdl_enter();
+  const uint32_t z = blockIdx.x * 256u + threadIdx.x;
+  for (uint32_t s = blockIdx.y; s < n; s += gridDim.y) {
+    const Stripe& p = stripes[s];
+    const EmitJob& e = emits[s];
+    if (e.levels && l < p.U && z < (1u << (3 * l)) && p.wpre[upper_words(p.U)].x) average_cell(p, e, l, z);
+  }
+}
+
+// Levels min(l_hi, U - 1) .. 0, one CTA per stripe.
+__global__ void __launch_bounds__(1024) kb_upper_avg_top(const Stripe* __restrict__ stripes,
+                                                         const EmitJob* __restrict__ emits, int l_hi) {
+  pdl_enter();
+  const Stripe& p = stripes[blockIdx.x];
+  const EmitJob& e = emits[blockIdx.x];
+  if (!e.levels || p.U == 0 || p.wpre[upper_words(p.U)].x == 0) return;
+  for (int l = min(l_hi, p.U - 1); l >= 0; l--) {
+    for (uint32_t z = threadIdx.x; z < (1u << (3 * l)); z += 1024u) average_cell(p, e, l, z);
+    __syncthreads();
+  }
+}
+
+// Nodes of the stripe written before the children of cell a of level m < U.
+__device__ __forceinline__ uint32_t children_base(const Stripe& p, int m, uint32_t a) {
+  uint32_t s = 0;
+  for (int l = 1; l <= m + 1; l++) s += upper_rank(p, l, 8u * (a >> (3 * (m + 1 - l))));
+  for (int l = m + 2; l <= p.U; l++) s += upper_rank(p, l, (a + 1u) << (3 * (l - m)));
+  const uint2 v = brick_prefix(p, (a + 1u) << (3 * (p.U - m)));
+  return s + v.x + v.y;
+}
+
+// Data records of the stripe (-levels) before the average of cell z of level m < U.
+__device__ __forceinline__ uint32_t data_before(const Stripe& p, bool payload, int m, uint32_t z) {
+  uint32_t s = 0;
+  for (int l = 1; l <= m; l++) s += upper_rank(p, l, z >> (3 * (m - l)));
+  for (int l = m + 1; l <= p.U; l++) s += upper_rank(p, l, (z + 1u) << (3 * (l - m)));
+  const uint2 v = brick_prefix(p, (z + 1u) << (3 * (p.U - m)));
+  return s + (payload ? v.x : 0u) + v.y;
+}
+
+// Cell i of levels 0 .. U-1.
+__device__ __forceinline__ void upper_node(const Stripe& p, const EmitJob& e, uint64_t i) {
+  int m = 0;
+  while (i >= upper_cell(m + 1, 0)) m++;
+  if (m >= p.U) return;
+  const uint32_t z = (uint32_t)(i - upper_cell(m, 0));
+  if (!((p.ubits[upper_off(m) + (z >> 5)] >> (z & 31u)) & 1u)) return;
+  const uint32_t mask = upper_byte(p, m + 1, z);
+  const float* v = e.levels ? e.upper_cache + i * 6 : nullptr;
+  if (m == 0) {  // the stripe root, which the host writes
+    e.root_out[0] = mask;
+    if (v) {
+      for (int k = 0; k < 6; k++) e.root_out[1 + k] = __float_as_uint(v[k]);
+      store_data_record(e, e.data_base + e.data_span - 1, 0, v);
+    }
+    return;
+  }
+  const uint32_t sib = upper_byte(p, m, z >> 3) & ((1u << (z & 7u)) - 1u);
+  uint64_t di = 0;
+  if (v) {
+    di = e.data_base + data_before(p, !e.binary, m, z);
+    store_data_record(e, di, 0, v);
+  }
+  store_node_record(e, e.node_base + children_base(p, m - 1, z >> 3) + __popc(sib), di,
+                    e.node_base + children_base(p, m, z), child_offsets(mask));
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(kTreeThreads) kb_upper_nodes(const Stripe* __restrict__ stripes,
+                                                               const EmitJob* __restrict__ emits,
+                                                               const uint64_t* __restrict__ cta_beg, uint32_t n,
+                                                               Stripe p0, EmitJob e0) {
+  pdl_enter();
+  if constexpr (SINGLE) {
+    upper_node(p0, e0, (uint64_t)blockIdx.x * kTreeThreads + threadIdx.x);
+  } else {
+    __shared__ Stripe sp;
+    __shared__ EmitJob se;
+    uint64_t cta;
+    const uint32_t s = cta_stripe(cta_beg, n, cta);
+    stage(sp, stripes[s]);
+    stage(se, emits[s]);
+    __syncthreads();
+    upper_node(sp, se, cta * kTreeThreads + threadIdx.x);
+  }
+}
+
+}  // namespace
+
+// ===========================================================================
+// Launch wrappers
+// ===========================================================================
+namespace {
+Stripe stripe_or_zero(const Stripe* s) {
+  Stripe p;
+  std::memset(&p, 0, sizeof(p));
+  if (s) p = *s;
+  return p;
+}
+EmitJob emit_or_zero(const EmitJob* s) {
+  EmitJob e;
+  std::memset(&e, 0, sizeof(e));
+  if (s) e = *s;
+  return e;
+}
+}  // namespace
+
+void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const Stripe* single,
+                     cudaStream_t st) {
+  if (ctas == 0) return;
+  KScope k("bricks", st);
+  const Stripe p0 = stripe_or_zero(single);
+  launch_k(single ? kb_bricks<true> : kb_bricks<false>, dim3((unsigned)ctas), dim3(32 * kBrickCta), 0, st, stripes,
+           cta_beg, n, p0);
+}
+
+void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts, const uint64_t* tasks,
+                    uint64_t* tasks_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st) {
+  if (n == 0) return;
+  KScope k("upper", st);
+  // 128 threads cover level 4's 128 words at eight a thread with room for smaller CTAs to share an SM;
+  // larger stripes have 1,024 and 8,192 words to scan
+  if (max_upper >= 5) launch_k(kb_upper<1024>, dim3(n), dim3(1024), 0, st, stripes, counts, tasks, tasks_out, code, code_out);
+  else launch_k(kb_upper<128>, dim3(n), dim3(128), 0, st, stripes, counts, tasks, tasks_out, code, code_out);
+}
+
+void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
+                           uint64_t ctas, uint32_t ept, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
+  if (ctas == 0) return;
+  KScope k("leaf_payload", st);
+  launch_k(se ? kb_leaf_payload<true> : kb_leaf_payload<false>, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes,
+           emits, cta_beg, n, ept, stripe_or_zero(sp), emit_or_zero(se));
+}
+
+void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
+                   bool levels, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
+  if (ctas == 0) return;
+  KScope k("emit", st);
+  auto* kern = sp ? (levels ? kb_emit<true, true> : kb_emit<true, false>)
+                  : (levels ? kb_emit<false, true> : kb_emit<false, false>);
+  launch_k(kern, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes, emits, cta_beg, n, stripe_or_zero(sp),
+           emit_or_zero(se));
+}
+
+void launch_b_upper_avg(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st) {
+  if (n == 0 || max_upper == 0) return;
+  constexpr int kTop = 4;  // 4,096 cells: four per thread of one CTA
+  for (int l = max_upper - 1; l > kTop; l--) {
+    KScope k("upper_average", st);
+    launch_k(kb_upper_avg, dim3(1u << (3 * l - 8), n < 4096u ? n : 4096u), dim3(256), 0, st, stripes, emits, n, l);
+  }
+  KScope k("upper_average_top", st);
+  launch_k(kb_upper_avg_top, dim3(n), dim3(1024), 0, st, stripes, emits, kTop);
+}
+
+void launch_b_upper_nodes(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
+                          uint64_t ctas, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
+  if (ctas == 0) return;
+  KScope k("upper_nodes", st);
+  launch_k(sp ? kb_upper_nodes<true> : kb_upper_nodes<false>, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes,
+           emits, cta_beg, n, stripe_or_zero(sp), emit_or_zero(se));
+}
+
+}  // namespace ooc
