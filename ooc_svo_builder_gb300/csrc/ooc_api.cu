@@ -132,15 +132,11 @@ struct ooc_ctx {
   float phase_ms[kPhases] = {0, 0, 0, 0, 0, 0};
   unsigned long long launches = 0;
   ooc::LaunchState lstate;  // this context's launch count and timing hooks, installed per API call
-  DevBuf d_tris, d_hist, d_axis, d_upper, d_brick, d_innerlocal, d_uppercache, d_winners, d_taskoff,
-      d_taskpart, d_counter, d_nodes, d_data, d_recs, d_itemmask, d_itembox, d_leaf, d_touch, d_local, d_taskmap, d_woff;
-  uint64_t max_tasks = 0;  // most large-item warp tasks a sub-batch has had (sizes the task map)
-  // persistent phase A (ooc_tuning::persistent): its counters, its task map (all ones
-  // between launches: every entry a launch fills is emptied by the warp that reads it)
-  DevBuf d_pctr, d_pmap;
-  bool pmap_empty = false;
-  int persist_per_sm = -1;  // CTAs per SM of the persistent kernel for persist_lpl
-  uint32_t persist_lpl = 0;
+  DevBuf d_tris, d_hist, d_axis, d_upper, d_brick, d_innerlocal, d_uppercache, d_winners, d_large,
+      d_big, d_ctr, d_nodes, d_data, d_recs, d_itemmask, d_itembox, d_leaf, d_touch, d_local, d_woff;
+  // persistent occupancy passes (ooc_tuning::persistent): their counters, and the CTAs per SM
+  DevBuf d_pctr;
+  int persist_per_sm = -1;
   bool leaf_zero = true;  // d_leaf and d_touch hold only zeros (no sub-batch left them dirty)
   PinBuf h_misc, h_recs, h_tables1, h_tables2, h_words;
   // double-buffered outputs of pipelined sub-batches
@@ -812,11 +808,12 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   }
   uint32_t* upper = ensure<uint32_t>(c->d_upper, upper_w * 8);         // ubits, then upre
   uint2* brick = ensure<uint2>(c->d_brick, (pre_w + bricks) * 8 + bricks);  // wpre, then bpre, then bunits
-  uint64_t* task_off = ensure<uint64_t>(c->d_taskoff, (items + 1) * 8);
-  uint64_t* taskpart = ensure<uint64_t>(c->d_taskpart, scan_partials_needed(items + 1) * 8);
+  unsigned long long* large = ensure<unsigned long long>(c->d_large, items * 8);
+  const uint32_t big_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(items, 1), kMaxBig);
+  uint4* big = ensure<uint4>(c->d_big, (uint64_t)big_cap * sizeof(uint4));
+  unsigned long long* ctr = ensure<unsigned long long>(c->d_ctr, kLargeCtrWords * 8);
   uint64_t* item_mask = ensure<uint64_t>(c->d_itemmask, items * 8);
   uint64_t* item_box = ensure<uint64_t>(c->d_itembox, items * 8);
-  unsigned long long* counter = ensure<unsigned long long>(c->d_counter, 16);
 
   for (uint32_t s = 0; s < n; s++) {
     const StripeRef& r = sb[s];
@@ -852,15 +849,17 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     j.u = m.pl.u;
     j.unit_div = m.pl.unit_div;
     j.small_vol = c->tuning.small_vol;
-    j.lines_per_lane = c->tuning.lines_per_lane;
     j.leafbits = S.leaf;
     j.leaftouch = S.touch;
     j.wpre = S.wpre;
     j.leaflocal = S.local;
     j.leafwoff = S.woff;
-    j.task_off = task_off + item_beg[s];
-    j.task_flag = task_off + items;
-    j.task_counter = counter;
+    j.large = large;
+    j.big = big;
+    j.ctr = ctr;
+    j.big_cap = big_cap;
+    j.slice = 32u * c->tuning.lines_per_lane;
+    j.stripe = s;
     j.item_mask = m.pl.binary ? nullptr : item_mask + item_beg[s];
     j.item_box = m.pl.binary ? nullptr : item_box + item_beg[s];
   }
@@ -869,10 +868,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
 
   // persistent occupancy passes: the items of every stripe in chunks
   bool persist = c->tuning.persistent != 0 && !pieces;
-  if (persist && (c->persist_per_sm < 0 || c->persist_lpl != c->tuning.lines_per_lane)) {
-    c->persist_per_sm = persist_ctas_per_sm(c->tuning.lines_per_lane);
-    c->persist_lpl = c->tuning.lines_per_lane;
-  }
+  if (persist && c->persist_per_sm < 0) c->persist_per_sm = persist_ctas_per_sm();
   persist = persist && c->persist_per_sm > 0;
   std::vector<uint64_t> p_chunk;
   if (persist) p_chunk = cta_prefix(n, kPersistChunkItems, [&](uint32_t s) { return sb[s].n_items; });
@@ -880,7 +876,6 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   Uploader up1;
   const size_t o_vj = up1.add(vj.data(), n * sizeof(VoxJob));
   const size_t o_str = up1.add(stripe.data(), n * sizeof(Stripe));
-  const size_t o_beg = up1.add(item_beg.data(), (n + 1) * 8);
   const size_t o_cpi = up1.add(cp_items.data(), (n + 1) * 8);
   const size_t o_cpb = up1.add(cp_bricks.data(), (n + 1) * 8);
   size_t o_pc = 0;
@@ -889,68 +884,36 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   auto dp1 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t1 + off); };
   const VoxJob* d_vj = reinterpret_cast<const VoxJob*>(t1 + o_vj);
   const Stripe* d_str = reinterpret_cast<const Stripe*>(t1 + o_str);
-  const uint64_t* d_beg = reinterpret_cast<const uint64_t*>(t1 + o_beg);
 
   uint32_t* lvl = ensure_pinned<uint32_t>(c->h_misc, ((uint64_t)n * kCountWords + 64) * 4);  // counts of every stripe, then two totals
   uint32_t* lvl_dev = nullptr;  // the same pinned memory as the kernels address it
   ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&lvl_dev), lvl, 0), "mapped counts");
-  // Warp task -> item map, sized by the items and the most tasks a sub-batch has had.
-  // Built once the context has seen a sub-batch with many tasks: with few, the large
-  // items' search of the task offsets costs less than the map's launch.
-  constexpr uint64_t kMapMinTasks = 4096;
-  uint64_t* task_map = nullptr;
-  uint64_t map_cap = 0;
-  if (c->max_tasks >= kMapMinTasks) {
-    task_map = ensure<uint64_t>(c->d_taskmap, std::max<uint64_t>(items, c->max_tasks) * 8);
-    map_cap = c->d_taskmap.cap / 8;
-  }
   PersistJob pj;
   std::memset(&pj, 0, sizeof(pj));
-  bool any_payload_stripe = false;
-  for (uint32_t s = 0; s < n; s++) any_payload_stripe = any_payload_stripe || !meshes[sb[s].mesh].pl.binary;
   if (persist) {
-    // task entries: room for the most tasks seen so far, twice over; a chunk whose tasks
-    // do not fit walks them itself
-    const uint64_t cap = std::max<uint64_t>(std::max<uint64_t>(2 * c->max_tasks, items), 4096);
-    const size_t had = c->d_pmap.cap;
-    unsigned long long* pmap = ensure<unsigned long long>(c->d_pmap, cap * 8);
-    if (c->d_pmap.cap != had || !c->pmap_empty) {
-      ck(cudaMemsetAsync(pmap, 0xff, c->d_pmap.cap, st), "memset task entries");
-      c->pmap_empty = true;
-    }
     pj.jobs = d_vj;
-    pj.item_beg = d_beg;
     pj.n = n;
     pj.chunk_beg = dp1(o_pc);
     pj.ctr = ensure<unsigned long long>(c->d_pctr, kPersistCtrWords * 8);
-    pj.map = pmap;
-    pj.cap = c->d_pmap.cap / 8;
-    pj.lines_per_lane = c->tuning.lines_per_lane;
-    c->pmap_empty = false;  // until this launch is known to have ended without a timeout
+    pj.lists = lists_of(vj[0]);
   }
   c->leaf_zero = false;  // until the emission at the end of the sub-batch is queued
   run_launches(c, st, 0, [&] {
-    if (persist) {
+    {
       PhaseScope ph(c, PH_VOX, st);
-      ck(cudaMemsetAsync(task_off + items, 0, 8, st), "memset task_off");
-      ck(cudaMemsetAsync(pj.ctr, 0, kPersistCtrWords * 8, st), "memset persistent counters");
-      launch_b_persist(pj, c->num_sms, c->persist_per_sm, st);
-      if (any_payload_stripe) {  // the winner pass numbers the tasks by item
-        scan_u64_exclusive(task_off, items + 1, taskpart, st, true);
-        if (map_cap) launch_b_task_map(dp1(o_cpi), n, cp_items[n], d_beg, task_off, items, task_map, map_cap, st);
-      }
-    } else {
-      PhaseScope ph(c, PH_VOX, st);
-      ck(cudaMemsetAsync(task_off + items, 0, 8, st), "memset task_off");
-      if (pieces) {
+      ck(cudaMemsetAsync(ctr, 0, kLargeCtrWords * 8, st), "memset counters");
+      if (persist) {
+        ck(cudaMemsetAsync(pj.ctr, 0, kPersistCtrWords * 8, st), "memset persistent counters");
+        launch_b_persist(pj, c->num_sms, c->persist_per_sm, st);
+      } else if (pieces) {
         // each piece of the triangles as soon as its copy is done
         uint64_t beg = 0;
         for (const auto& pc : *pieces) {
           ck(cudaStreamWaitEvent(st, pc.second, 0), "wait piece");
           VoxJob jc = vj[0];
           jc.ibeg += beg;
+          jc.item0 = beg;
           jc.n_items = pc.first - beg;
-          jc.task_off += beg;
           if (jc.item_mask) jc.item_mask += beg;
           if (jc.item_box) jc.item_box += beg;
           launch_b_vox_small(nullptr, nullptr, 1, (jc.n_items + kChunk - 1) / kChunk, 0, &jc, st);
@@ -959,20 +922,17 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       } else {
         launch_b_vox_small(d_vj, dp1(o_cpi), n, cp_items[n], 0, n == 1 ? &vj[0] : nullptr, st);
       }
-      scan_u64_exclusive(task_off, items + 1, taskpart, st, true);
-      if (map_cap) launch_b_task_map(dp1(o_cpi), n, cp_items[n], d_beg, task_off, items, task_map, map_cap, st);
-      launch_b_vox_large(d_vj, d_beg, n, task_off, items, counter, 0, st, c->num_sms, (int)c->tuning.large_block,
-                         (int)c->tuning.large_ctas_per_sm, c->tuning.lines_per_lane, task_map, map_cap);
+      if (!persist)
+        launch_b_vox_large(d_vj, lists_of(vj[0]), 0, n == 1 ? &vj[0] : nullptr, st, c->num_sms,
+                           (int)c->tuning.large_block, (int)c->tuning.large_ctas_per_sm);
     }
     {
       PhaseScope ph(c, PH_PYR, st);
       launch_b_bricks(d_str, dp1(o_cpb), n, cp_bricks[n], n == 1 ? &stripe[0] : nullptr, st);
-      // the tasks of the sub-batch (sizes the task maps); the persistent kernel counts them itself
-      const uint64_t* tasks = persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTasksWord) : task_off + items;
       // The counts go straight into pinned host memory, written by the kernel: a copy on the
       // copy engine would queue behind the previous sub-batch's copy back, which the host
       // keeps refilling while it waits, and hold up the whole pipeline.
-      launch_b_upper(d_str, n, max_upper, lvl_dev, tasks, reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords),
+      launch_b_upper(d_str, n, max_upper, lvl_dev, ctr, reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords),
                      persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTimeoutWord) : nullptr,
                      reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords + 2), st);
     }
@@ -982,11 +942,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     uint64_t code;
     std::memcpy(&code, lvl + (uint64_t)n * kCountWords + 2, 8);
     if (code != 0) fail(OOC_ERR_DEVICE, "persistent voxelization: a wait ran out (code " + std::to_string(code) + ")");
-    c->pmap_empty = true;
   }
-  uint64_t tasks_seen;
-  std::memcpy(&tasks_seen, lvl + (uint64_t)n * kCountWords, 8);
-  c->max_tasks = std::max(c->max_tasks, tasks_seen);
+  uint64_t large_items;  // zero when there is none
+  std::memcpy(&large_items, lvl + (uint64_t)n * kCountWords, 8);
 
   // ---- counts, placement in the files ----
   std::vector<Placed> pl(n);
@@ -1180,9 +1138,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       PhaseScope ph(c, PH_VOX, st);
       ck(cudaMemsetAsync(winners, 0xff, total_leaves * 8, st), "memset winners");
       launch_b_vox_small(d_vj2, dp2(o_cpay), n, cp_pay[n], 1, n == 1 ? &vj[0] : nullptr, st);
-      if (tasks_seen)  // the count came back with the level counts
-        launch_b_vox_large(d_vj2, d_beg, n, task_off, items, counter, 1, st, c->num_sms, (int)c->tuning.large_block,
-                           (int)c->tuning.large_ctas_per_sm, c->tuning.lines_per_lane, task_map, map_cap);
+      if (large_items)
+        launch_b_vox_large(d_vj2, lists_of(vj[0]), 1, n == 1 ? &vj[0] : nullptr, st, c->num_sms,
+                           (int)c->tuning.large_block, (int)c->tuning.large_ctas_per_sm);
       launch_b_leaf_payload(d_str, d_ej, dp2(o_clp), n, cp_leafpay.beg[n], cp_leafpay.ept, sp1, se1, st);
     }
   });
@@ -1837,9 +1795,9 @@ void ooc_ctx_destroy(ooc_ctx* c) {
     if (rs) cudaStreamSynchronize(rs);
   if (c->h2d_stream) cudaStreamSynchronize(c->h2d_stream);
   DevBuf* bufs[] = {&c->d_tris, &c->d_hist, &c->d_axis, &c->d_upper, &c->d_brick, &c->d_innerlocal, &c->d_uppercache,
-                    &c->d_winners, &c->d_taskoff, &c->d_taskpart, &c->d_counter, &c->d_nodes,
+                    &c->d_winners, &c->d_large, &c->d_big, &c->d_ctr, &c->d_nodes,
                     &c->d_data, &c->d_recs, &c->d_itemmask, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_local,
-                    &c->d_taskmap, &c->d_woff, &c->d_pctr, &c->d_pmap, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
+                    &c->d_woff, &c->d_pctr, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
                     &c->d_group[1], &c->d_stream_mat, &c->d_stream_part, &c->d_stream_base, &c->d_part_off};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);

@@ -86,7 +86,6 @@ struct VoxJob {
   int sa[3], sb[3];         // stripe box in grid coordinates (inclusive)
   float u, unit_div;
   uint32_t small_vol;       // items with at most this many candidates (<= 64) run one per thread
-  uint32_t lines_per_lane;  // lines of a large item each lane of a warp task walks (task = 32 x this)
   uint32_t* leafbits;       // level-Ds words
   uint8_t* leaftouch;       // byte per 256-bit block of leafbits, set when a bit of the block is (may be NULL)
   // pass B (payload winners)
@@ -94,12 +93,31 @@ struct VoxJob {
   const uint32_t* leaflocal;// Stripe::local
   const uint64_t* leafwoff; // Stripe::woff
   unsigned long long* winners;  // per leaf: min of triangle index << 32 | its local Morton code
-  uint64_t* task_off;       // per item: exclusive prefix of warp tasks (n_items + 1)
-  uint64_t* task_flag;      // set to 1 by an item with tasks (the sub-batch's task_off[items]); may be NULL
-  unsigned long long* task_counter;
+  // the list of large items (shared by the stripes of a sub-batch)
+  unsigned long long* large; // items of one task each: item | stripe << 32 (room for every item)
+  uint4* big;               // the others: item, stripe, first task, tasks (big_cap entries)
+  unsigned long long* ctr;  // kCtr* counters
+  uint32_t big_cap;         // at most kMaxBig
+  uint32_t slice;           // lines of a task: 32 x lines_per_lane
+  uint32_t stripe;          // this job's index
+  uint64_t item0;           // number of the job's first item in its stripe (a piece of an upload)
   uint64_t* item_mask;      // per small item: which of its candidates passed (pass 0 -> pass 1); may be NULL
   uint64_t* item_box;       // per small item with a non-zero mask: its packed stripe-local box
 };
+
+// Counters of the large items' list, each on its own 128-byte line; all zero when pass 0 starts.
+constexpr int kCtrLarge = 0;   // items in `large`
+constexpr int kCtrBig = 16;    // entries and tasks of `big`
+constexpr int kCtrGrab = 32;   // taken so far: big tasks of pass 0, large items of pass 0, and the same of pass 1
+constexpr uint32_t kLargeCtrWords = 96;
+constexpr uint32_t kMaxBig = 1u << 16;  // entries of `big`
+struct LargeLists {
+  const unsigned long long* large;
+  const uint4* big;
+  unsigned long long* ctr;
+  uint32_t big_cap, slice;
+};
+inline LargeLists lists_of(const VoxJob& j) { return LargeLists{j.large, j.big, j.ctr, j.big_cap, j.slice}; }
 
 struct EmitJob {
   int binary;
@@ -177,9 +195,7 @@ struct LaunchScope {
   LaunchScope& operator=(const LaunchScope&) = delete;
 };
 
-// flag_last: data[n-1] is not an input but a flag; zero means every element is zero,
-// and the scan is left out.
-void scan_u64_exclusive(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st, bool flag_last = false);
+// Scan partials of a scan over n elements.
 uint64_t scan_partials_needed(uint64_t n);
 
 // n words from device memory into `dst`, mapped pinned host memory, by a kernel.
@@ -207,7 +223,6 @@ void launch_stream_group_chunk(const float* tris, int stride, uint64_t n, const 
 // entry point's launches); each returns the status of its own launch calls.
 cudaError_t launch_vox_small_occupancy(const VoxJob& j, cudaStream_t st);
 cudaError_t launch_vox_large_occupancy(const VoxJob& j, cudaStream_t st, int num_sms);
-cudaError_t scan_u64_exclusive_checked(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st);
 
 // src holds n entries of (index, `words` u64 values); dst[index*words + q] = value q.
 void launch_scatter_records(const uint64_t* src, uint64_t n, int words, uint64_t* dst, cudaStream_t st);
@@ -217,36 +232,24 @@ void launch_scatter_to(const uint64_t* src, uint64_t n, int words, cudaStream_t 
 // `single` (may be NULL): the job of a one-stripe launch, passed as a kernel parameter.
 void launch_b_vox_small(const VoxJob* jobs, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, int pass,
                         const VoxJob* single, cudaStream_t st);
-// Large items of every stripe; task_off is the batch-wide exclusive scan (total_items + 1 entries),
-// item_beg[s] the first batch item of stripe s (ascending).
-// map[t] = item | stripe << 32 for every warp task t, if they all fit in `cap` entries
-// (CTAs as for launch_b_vox_small: `cta_beg` over the stripes' items).
-void launch_b_task_map(const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const uint64_t* item_beg,
-                       const uint64_t* task_off, uint64_t total_items, uint64_t* map, uint64_t cap, cudaStream_t st);
-// `lines_per_lane` is every job's (it sizes each warp's shared list of lines); tasks find
-// their item in `map` when the tasks fit in `cap`, else by searching task_off.
-void launch_b_vox_large(const VoxJob* jobs, const uint64_t* item_beg, uint32_t n_stripes, const uint64_t* task_off,
-                        uint64_t total_items, unsigned long long* counter, int pass, cudaStream_t st, int num_sms,
-                        int block, int ctas_per_sm, uint32_t lines_per_lane, const uint64_t* map, uint64_t cap);
+// The listed large items of every stripe (`single`: the job of a one-stripe launch).
+void launch_b_vox_large(const VoxJob* jobs, const LargeLists& lists, int pass, const VoxJob* single, cudaStream_t st,
+                        int num_sms, int block, int ctas_per_sm);
 // The persistent occupancy kernel's inputs (ooc_tuning::persistent).
 struct PersistJob {
   const VoxJob* jobs;
-  const uint64_t* item_beg;   // n + 1: first item of each stripe in the sub-batch
   uint32_t n;                 // stripes
   const uint64_t* chunk_beg;  // n + 1: prefix of 256-item chunks per stripe
-  unsigned long long* ctr;    // 64 counters, four used: tickets, chunks done, tasks reserved, timeout code
-                              // (kCtr* in the kernel), each on its own 128-byte line
-  unsigned long long* map;    // cap task entries (item | task << 32), all ones when empty
-  uint64_t cap;
-  uint32_t lines_per_lane;
+  unsigned long long* ctr;    // kPersistCtrWords counters: tickets, chunks done, timeout code (kCtr* in the kernel),
+                              // each on its own 128-byte line
+  LargeLists lists;
 };
 // CTAs of the persistent kernel one SM holds (0 on an error).
-int persist_ctas_per_sm(uint32_t lines_per_lane);
+int persist_ctas_per_sm();
 void launch_b_persist(const PersistJob& pj, int num_sms, int ctas_per_sm, cudaStream_t st);
 constexpr uint64_t kPersistChunkItems = 256;  // items of a chunk unit
 constexpr uint32_t kPersistCtrWords = 64;     // counters of the persistent kernel
 constexpr uint32_t kPersistTimeoutWord = 48;  // where it records the code of a wait that ran out
-constexpr uint32_t kPersistTasksWord = 32;    // where it counts the tasks it found (queued or not)
 
 // ---- the octree (ooc_tree.cu) ----
 // `single` / `sp`, `se` (may be NULL): the stripe (and emit job) of a one-stripe launch, passed
@@ -261,9 +264,10 @@ inline uint32_t brick_ctas(const Stripe& s) {
 void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const Stripe* single,
                      cudaStream_t st);
 // One CTA per stripe: the upper levels' words and prefixes, and every stripe's counts (kCountWords each)
-// into `counts` (mapped pinned host memory), then *tasks and, when `code` is set, *code.
-void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts, const uint64_t* tasks,
-                    uint64_t* tasks_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st);
+// into `counts` (mapped pinned host memory), then the number of large items (`large_ctr`: kCtr*) and,
+// when `code` is set, *code.
+void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts,
+                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st);
 // The payloads of the stripes' leaves, into the data file: CTAs of kChunk threads, `ept` leaves each.
 void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
                            uint64_t ctas, uint32_t ept, const Stripe* sp, const EmitJob* se, cudaStream_t st);

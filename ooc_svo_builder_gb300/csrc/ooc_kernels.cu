@@ -31,13 +31,10 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-// `skip` (may be NULL): when it points at a zero, every element is zero and the
-// scan is left out (all zeros are their own exclusive scan).
 template <typename T>
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const T* __restrict__ in, uint64_t n,
-                                                              T* __restrict__ partials, const T* skip) {
+                                                              T* __restrict__ partials) {
   pdl_enter();
-  if (skip && *skip == T(0)) return;
   const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
   T v = 0;
 #pragma unroll
@@ -52,9 +49,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const T* __restric
 
 // Also partials[np] = the grand total.
 template <typename T>
-__global__ void __launch_bounds__(1024) k_scan_partials(T* partials, uint64_t np, const T* skip) {
+__global__ void __launch_bounds__(1024) k_scan_partials(T* partials, uint64_t np) {
   pdl_enter();
-  if (skip && *skip == T(0)) return;
   T carry = 0;
   for (uint64_t base = 0; base < np; base += blockDim.x) {
     const uint64_t i = base + threadIdx.x;
@@ -70,12 +66,8 @@ __global__ void __launch_bounds__(1024) k_scan_partials(T* partials, uint64_t np
 // Each thread scans SCAN_ITEMS consecutive elements staged through shared memory
 // (`partials` NULL: a single tile, nothing before it).
 template <typename T>
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(T* data, uint64_t n, const T* __restrict__ partials,
-                                                            const T* skip) {
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(T* data, uint64_t n, const T* __restrict__ partials) {
   pdl_enter();
-  // `skip` is read before any CTA writes: a scan that runs has a non-zero flag and a
-  // non-zero total, so a late CTA reading the written total skips nothing either
-  if (skip && *skip == T(0)) return;
   // the elements are counts: a zero total means all zero, which is already their scan
   if (partials && partials[gridDim.x] == T(0)) return;
   __shared__ T tile[SCAN_TILE + SCAN_TILE / 32];
@@ -113,25 +105,25 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_down(T* data, uint64_t n,
 }
 
 template <typename T>
-void scan_exclusive(T* data, uint64_t n, T* partials, cudaStream_t st, const T* skip = nullptr) {
+void scan_exclusive(T* data, uint64_t n, T* partials, cudaStream_t st) {
   if (n == 0) return;
   const unsigned nb = (unsigned)((n + SCAN_TILE - 1) / SCAN_TILE);
   if (nb == 1) {  // one tile: one launch
     KScope k("scan_down", st);
-    launch_k(k_scan_down<T>, dim3(1), dim3(SCAN_THREADS), 0, st, data, n, nullptr, skip);
+    launch_k(k_scan_down<T>, dim3(1), dim3(SCAN_THREADS), 0, st, data, n, nullptr);
     return;
   }
   {
     KScope k("scan_reduce", st);
-    launch_k(k_scan_reduce<T>, dim3(nb), dim3(SCAN_THREADS), 0, st, data, n, partials, skip);
+    launch_k(k_scan_reduce<T>, dim3(nb), dim3(SCAN_THREADS), 0, st, data, n, partials);
   }
   {
     KScope k("scan_partials", st);
-    launch_k(k_scan_partials<T>, dim3(1), dim3(1024), 0, st, partials, nb, skip);
+    launch_k(k_scan_partials<T>, dim3(1), dim3(1024), 0, st, partials, nb);
   }
   {
     KScope k("scan_down", st);
-    launch_k(k_scan_down<T>, dim3(nb), dim3(SCAN_THREADS), 0, st, data, n, partials, skip);
+    launch_k(k_scan_down<T>, dim3(nb), dim3(SCAN_THREADS), 0, st, data, n, partials);
   }
 }
 
@@ -431,34 +423,150 @@ __device__ __forceinline__ uint64_t item_lines(int W, const int lo[3], const int
   return W == 0 ? ey * ez : (W == 1 ? ex * ez : ex * ey);
 }
 
-// One line of a large item: pass 0 sets its bits, pass 1 offers the triangle
-// to every voxel it passes.  `dir` is the sign-carrying slope of the plane
-// value along the line (n_w * u) and `inv_dir` its reciprocal.
+// The list of large items.  Pass 0 appends every large item once: to `large` when its
+// lines make one task (at most `slice` lines), else to `big`, whose entries carry the number
+// of their first task so that several warps share the item.  A full `big` (ctr[kCtrBig]'s
+// count at its capacity) sends further items to `large`, where one warp walks them whole.
+// The lists serve both passes; their order does not matter to the result.
+//
+// kCtrBig packs the entries (low kBigCountBits bits) and the tasks (the others) reserved so
+// far, so one atomicAdd gives an entry and its first task in step.  A thread adds only after
+// it has read a count below the capacity, so the count passes the capacity by at most the
+// threads resident at once (below 2^19) and never reaches the tasks' bits.
+constexpr int kBigCountBits = 20;
+static_assert(kMaxBig + (1u << 19) < (1u << kBigCountBits), "the count stays in its bits");
+
+// The warp's lanes: item i of job j with `lines` lines (0: not a large item).  All 32 lanes call.
+__device__ __forceinline__ void append_large(const VoxJob& j, uint64_t i, uint32_t lines) {
+  const int lane = threadIdx.x & 31;
+  bool one = lines != 0;
+  if (lines > j.slice) {
+    const unsigned long long now = *reinterpret_cast<volatile unsigned long long*>(j.ctr + kCtrBig);
+    if ((now & ((1ull << kBigCountBits) - 1ull)) < j.big_cap) {
+      const uint32_t tasks = (lines + j.slice - 1u) / j.slice;
+      const unsigned long long got = atomicAdd(j.ctr + kCtrBig, ((unsigned long long)tasks << kBigCountBits) | 1ull);
+      const uint32_t slot = (uint32_t)got & ((1u << kBigCountBits) - 1u);
+      if (slot < j.big_cap) {
+        j.big[slot] = make_uint4((uint32_t)(j.item0 + i), j.stripe, (uint32_t)(got >> kBigCountBits), tasks);
+        one = false;
+      }
+    }
+  }
+  const uint32_t m = __ballot_sync(FULL, one);
+  if (!m) return;
+  unsigned long long at = 0;
+  const int leader = __ffs(m) - 1;
+  if (lane == leader) at = atomicAdd(j.ctr + kCtrLarge, (unsigned long long)__popc(m));
+  at = __shfl_sync(FULL, at, leader) + __popc(m & ((1u << lane) - 1u));
+  if (one) j.large[at] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
+}
+
+// A large item as the warp's lanes read it: the constants of the test arranged by the walk axis
+// w and the two across it, a and b (the first and second of the remaining axes).  Of the three
+// projections one depends on a and b only (the line's own test), one on a and w, one on b and w.
+// Sums of two products are commutative, so the arrangement changes no rounding.
+struct WalkItem {
+  float ea[3], eb[3], ed[3];     // line test: ea * a + eb * b + ed
+  float aw[3], af[3], ad[3];     // aw * w + af * a + ad
+  float bw[3], bf[3], bd[3];     // bw * w + bf * b + bd
+  float nw, na, nb, d1, d2;      // normal and plane offsets
+  float u, inv_dir;
+  int alo, blo, wlo, whi;        // clamped box
+  uint32_t local;                // stripe-local alo, blo, wlo, 10 bits each
+  uint32_t shape;                // lines along a (11 bits) | axis w << 11 | monotone << 13
+  uint32_t magic;                // floor(c / ea) = (c * magic) >> 32 for line numbers c < 2^20; 0: one line along a
+  uint32_t first;                // the first line of the task
+  uint32_t tri, stripe;
+  uint32_t pad;                  // 45 words: lanes reading different items hit different banks
+};
+static_assert(sizeof(WalkItem) == 45 * 4, "odd number of words");
+
+__device__ __forceinline__ void walk_setup(const VoxJob& j, const TriVerts& tv, uint64_t t, uint32_t stripe, uint32_t first,
+                                           int W, const int lo[3], const int hi[3], WalkItem& r) {
+  TriSetup s;
+  tri_setup(tv, j.u, s);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    if (W == 2) {  // a = x, b = y
+      r.ea[k] = s.xy[k][0], r.eb[k] = s.xy[k][1], r.ed[k] = s.dxy[k];
+      r.aw[k] = s.zx[k][0], r.af[k] = s.zx[k][1], r.ad[k] = s.dzx[k];
+      r.bw[k] = s.yz[k][1], r.bf[k] = s.yz[k][0], r.bd[k] = s.dyz[k];
+    } else if (W == 0) {  // a = y, b = z
+      r.ea[k] = s.yz[k][0], r.eb[k] = s.yz[k][1], r.ed[k] = s.dyz[k];
+      r.aw[k] = s.xy[k][0], r.af[k] = s.xy[k][1], r.ad[k] = s.dxy[k];
+      r.bw[k] = s.zx[k][1], r.bf[k] = s.zx[k][0], r.bd[k] = s.dzx[k];
+    } else {  // a = x, b = z
+      r.ea[k] = s.zx[k][1], r.eb[k] = s.zx[k][0], r.ed[k] = s.dzx[k];
+      r.aw[k] = s.xy[k][1], r.af[k] = s.xy[k][0], r.ad[k] = s.dxy[k];
+      r.bw[k] = s.yz[k][0], r.bf[k] = s.yz[k][1], r.bd[k] = s.dyz[k];
+    }
+  }
+  r.nw = W == 0 ? s.n[0] : (W == 1 ? s.n[1] : s.n[2]);
+  r.na = W == 0 ? s.n[1] : s.n[0];
+  r.nb = W == 2 ? s.n[1] : s.n[2];
+  r.d1 = s.d1;
+  r.d2 = s.d2;
+  r.u = j.u;
+  r.inv_dir = 1.0f / (r.nw * j.u);
+  const int ia = W == 0 ? 1 : 0, ib = W == 2 ? 1 : 2;
+  r.alo = ia ? lo[1] : lo[0];
+  r.blo = ib == 1 ? lo[1] : lo[2];
+  r.wlo = W == 0 ? lo[0] : (W == 1 ? lo[1] : lo[2]);
+  r.whi = W == 0 ? hi[0] : (W == 1 ? hi[1] : hi[2]);
+  const int sa = ia ? j.sa[1] : j.sa[0], sb = ib == 1 ? j.sa[1] : j.sa[2], sw = W == 0 ? j.sa[0] : (W == 1 ? j.sa[1] : j.sa[2]);
+  r.local = (uint32_t)(r.alo - sa) | ((uint32_t)(r.blo - sb) << 10) | ((uint32_t)(r.wlo - sw) << 20);
+  const uint32_t ea = (uint32_t)((ia ? hi[1] : hi[0]) - r.alo + 1);
+  const int top = max(hi[0], max(hi[1], hi[2]));
+  const bool mono = monotone_setup(s, fabsf(__fmul_rn((float)(top + 1), j.u)));
+  r.shape = ea | ((uint32_t)W << 11) | (mono ? 1u << 13 : 0u);
+  // ceil(2^32 / ea): its excess adds less than c / 2^32 <= 2^-12 < 1 / ea to the quotient
+  r.magic = ea > 1 ? (uint32_t)(0xffffffffu / ea) + 1u : 0u;
+  r.first = first;
+  r.tri = (uint32_t)t;
+  r.stripe = stripe;
+}
+
+// Line (ra, rb) of a large item: pass 0 sets its bits, pass 1 offers the triangle to every
+// voxel it passes.  The line's own projection has passed.
 template <int PASS>
-__device__ __forceinline__ void vox_line(const VoxJob& j, const TriSetup& s, uint32_t tri, int W, int ca, int cb,
-                                         int w0, int w1, bool mono, float dir, float inv_dir) {
-  const float fa = __fmul_rn((float)ca, j.u), fb = __fmul_rn((float)cb, j.u);
-  float px, py, pz;
-  auto corner = [&](int w) {
-    const float fw = __fmul_rn((float)w, j.u);
-    px = W == 0 ? fw : fa;
-    py = W == 1 ? fw : (W == 0 ? fa : fb);
-    pz = W == 2 ? fw : fb;
+__device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, uint32_t ra, uint32_t rb) {
+  const float u = r.u, fa = __fmul_rn((float)(r.alo + (int)ra), u), fb = __fmul_rn((float)(r.blo + (int)rb), u);
+  const uint32_t shape = r.shape;
+  const int W = (int)(shape >> 11) & 3, w0 = r.wlo, w1 = r.whi;
+  // n.p in the reference's order, (x + y) + z: the walk axis is z (q1 = x + y first) or one of the
+  // first two.  Adding the 0 changes only the sign of a zero, which no test sees.
+  const float nw = r.nw, d1 = r.d1, d2 = r.d2, pa = __fmul_rn(r.na, fa), pb = __fmul_rn(r.nb, fb);
+  const float q1 = W == 2 ? __fadd_rn(pa, pb) : pa, q2 = W == 2 ? 0.0f : pb;
+  float aw[3], fA[3], ad[3], bw[3], fB[3], bd[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    aw[k] = r.aw[k], fA[k] = __fmul_rn(r.af[k], fa), ad[k] = r.ad[k];
+    bw[k] = r.bw[k], fB[k] = __fmul_rn(r.bf[k], fb), bd[k] = r.bd[k];
+  }
+  auto at = [&](int w) { return __fmul_rn((float)w, u); };
+  auto rest = [&](float fw) {  // the two projections that depend on the walk coordinate
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(aw[k], fw), fA[k]), ad[k]) < 0.0f);
+      ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(bw[k], fw), fB[k]), bd[k]) < 0.0f);
+    }
+    return ok;
   };
-  corner(w0);  // the caller has passed the projection test that does not depend on the walk coordinate
-  // the two that do (with the plane test they complete the voxel test)
-  auto rest = [&]() {
-    return W == 2 ? (pass_yz(s, py, pz) && pass_zx(s, pz, px))
-                  : (W == 0 ? (pass_xy(s, px, py) && pass_zx(s, pz, px)) : (pass_xy(s, px, py) && pass_yz(s, py, pz)));
+  const bool up_side = nw * u > 0.0f;  // the plane value grows with w
+  auto side = [&](float fw) {  // plane_side
+    const float v = __fadd_rn(__fadd_rn(__fmul_rn(nw, fw), q1), q2);
+    const float a = __fadd_rn(v, d1), b = __fadd_rn(v, d2);
+    if (!(__fmul_rn(a, b) > 0.0f)) return 0;
+    return (a > 0.0f) == up_side ? 1 : -1;
   };
-  // stripe-local Morton bits of the two fixed coordinates; the walk axis adds its own
-  const int sw = W == 0 ? j.sa[0] : (W == 1 ? j.sa[1] : j.sa[2]);
-  const uint32_t la = (uint32_t)(ca - (W == 0 ? j.sa[1] : j.sa[0])), lb = (uint32_t)(cb - (W == 2 ? j.sa[1] : j.sa[2]));
-  const uint32_t mab = W == 0 ? (spread3_10(la) << 1) | (spread3_10(lb) << 2)
-                              : (W == 1 ? spread3_10(la) | (spread3_10(lb) << 2) : spread3_10(la) | (spread3_10(lb) << 1));
+  // stripe-local Morton bits: the fixed coordinates, and the walk coordinate moving by carries
+  const uint32_t la = (r.local & 1023u) + ra, lb = ((r.local >> 10) & 1023u) + rb, lw = r.local >> 20;
+  const uint32_t mab = (spread3_10(la) << (W == 0 ? 1 : 0)) | (spread3_10(lb) << (W == 2 ? 1 : 2));
+  const uint32_t wbits = 0x09249249u << W;
   uint32_t cur_w = 0xffffffffu, acc = 0;
-  auto emit = [&](int w) {
-    const uint32_t m = mab | (spread3_10((uint32_t)(w - sw)) << W);
+  auto emit = [&](uint32_t mw) {
+    const uint32_t m = mab | mw;
     if (PASS == 0) {
       const uint32_t wd = m >> 5;
       if (wd != cur_w) {
@@ -468,30 +576,26 @@ __device__ __forceinline__ void vox_line(const VoxJob& j, const TriSetup& s, uin
       }
       acc |= 1u << (m & 31);
     } else {
-      offer(j, m, tri);  // pass 0 set this voxel's bit
+      offer(j, m, r.tri);  // pass 0 set this voxel's bit
     }
   };
-  if (!mono) {  // every voxel of the line, complete test
-    for (int w = w0; w <= w1; w++) {
-      corner(w);
-      if (pass_z(s, plane_xy(s, px, py), px, py, pz) && rest()) emit(w);
+  if (!((shape >> 13) & 1u)) {  // every voxel of the line, complete test
+    uint32_t mw = spread3_10(lw) << W;
+    for (int w = w0; w <= w1; w++, mw = ((mw | ~wbits) + (1u << W)) & wbits) {
+      const float fw = at(w);
+      if (side(fw) == 0 && rest(fw)) emit(mw);
     }
   } else {
-    auto side = [&](int w) {
-      corner(w);
-      return plane_side(s, px, py, pz, dir);
-    };
     // start where the plane crosses the line's middle, then find one voxel of the run
-    const float off = (W == 0 ? 0.0f : s.n[0] * px) + (W == 1 ? 0.0f : s.n[1] * py) + (W == 2 ? 0.0f : s.n[2] * pz);
-    float west = -(off + 0.5f * (s.d1 + s.d2)) * inv_dir;
+    float west = -((pa + pb) + 0.5f * (d1 + d2)) * r.inv_dir;
     west = fminf(fmaxf(west, (float)w0), (float)w1);  // NaN becomes w0
     int start = (int)west, walk = 0;                   // walk: +1 up only, -1 down only, 0 both ways
-    const int g0 = side(start);
+    const int g0 = side(at(start));
     if (g0 < 0) {  // the run lies above: first w with side >= 0
       int lo = start, hi = -1, step = 1;
       for (;;) {
         const int nx = min(lo + step, w1);
-        if (side(nx) >= 0) {
+        if (side(at(nx)) >= 0) {
           hi = nx;
           break;
         }
@@ -501,17 +605,17 @@ __device__ __forceinline__ void vox_line(const VoxJob& j, const TriSetup& s, uin
       }
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (side(mid) >= 0) hi = mid;
+        if (side(at(mid)) >= 0) hi = mid;
         else lo = mid;
       }
-      if (side(hi) != 0) return;  // the run falls between two voxels
+      if (side(at(hi)) != 0) return;  // the run falls between two voxels
       start = hi;
       walk = 1;
     } else if (g0 > 0) {  // below: last w with side <= 0
       int hi = start, lo = -1, step = 1;
       for (;;) {
         const int nx = max(hi - step, w0);
-        if (side(nx) <= 0) {
+        if (side(at(nx)) <= 0) {
           lo = nx;
           break;
         }
@@ -521,21 +625,33 @@ __device__ __forceinline__ void vox_line(const VoxJob& j, const TriSetup& s, uin
       }
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (side(mid) <= 0) lo = mid;
+        if (side(at(mid)) <= 0) lo = mid;
         else hi = mid;
       }
-      if (side(lo) != 0) return;
+      if (side(at(lo)) != 0) return;
       start = lo;
       walk = -1;
     }
-    // px/py/pz hold `start`'s corner and its plane test passed
-    if (rest()) emit(start);
-    if (walk >= 0)
-      for (int w = start + 1; w <= w1 && side(w) == 0; w++)
-        if (rest()) emit(w);
-    if (walk <= 0)
-      for (int w = start - 1; w >= w0 && side(w) == 0; w--)
-        if (rest()) emit(w);
+    const uint32_t ms = spread3_10(lw + (uint32_t)(start - w0)) << W;
+    if (rest(at(start))) emit(ms);
+    if (walk >= 0) {
+      uint32_t mw = ms;
+      for (int w = start + 1; w <= w1; w++) {
+        const float fw = at(w);
+        if (side(fw) != 0) break;
+        mw = ((mw | ~wbits) + (1u << W)) & wbits;
+        if (rest(fw)) emit(mw);
+      }
+    }
+    if (walk <= 0) {
+      uint32_t mw = ms;
+      for (int w = start - 1; w >= w0; w--) {
+        const float fw = at(w);
+        if (side(fw) != 0) break;
+        mw = (mw - (1u << W)) & wbits;
+        if (rest(fw)) emit(mw);
+      }
+    }
   }
   if (PASS == 0 && acc) set_leaf(j, cur_w, acc);
 }
@@ -720,11 +836,11 @@ __device__ __forceinline__ uint64_t vox_small_factored(const VoxJob& j, const Tr
 }
 
 // Pass 0, one thread per item: items with at most small_vol (<= 64) candidates
-// are voxelized here and leave their pass mask; larger ones get a warp-task
-// count (32 x lines_per_lane lines per task).
-__device__ __forceinline__ uint64_t vox_small_occ_item(const VoxJob& j, uint64_t i, const TriVerts& tv) {
+// are voxelized here and leave their pass mask; returns the lines of a larger one.
+__device__ __forceinline__ uint32_t vox_small_occ_item(const VoxJob& j, uint64_t i, const TriVerts& tv) {
   int lo[3], hi[3];
-  uint64_t cost = 0, mask = 0;
+  uint32_t lines = 0;
+  uint64_t mask = 0;
   if (item_box(j, tv, lo, hi)) {
     const uint32_t bx = (uint32_t)(hi[0] - lo[0] + 1), by = (uint32_t)(hi[1] - lo[1] + 1),
                    bz = (uint32_t)(hi[2] - lo[2] + 1);
@@ -740,24 +856,18 @@ __device__ __forceinline__ uint64_t vox_small_occ_item(const VoxJob& j, uint64_t
                         ((uint64_t)(bz - 1) << 42);
       }
     } else {
-      const uint64_t per_task = 32ull * j.lines_per_lane;
-      cost = (item_lines(walk_axis(tv), lo, hi) + per_task - 1) / per_task;
+      lines = (uint32_t)item_lines(walk_axis(tv), lo, hi);
     }
   }
-  j.task_off[i] = cost;
-  if (cost && j.task_flag) *j.task_flag = 1ull;  // the sub-batch has tasks: its scan runs
   if (j.item_mask) j.item_mask[i] = mask;
-  return cost;
+  return lines;
 }
 
-__device__ __forceinline__ uint64_t vox_small_occ_item(const VoxJob& j, uint64_t i) {
-  return vox_small_occ_item(j, i, load_verts(j.tris, item_triangle(j, i), j.stride));
-}
-
-__global__ void k_vox_small_occ(VoxJob j) {
-  pdl_enter();
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < j.n_items) vox_small_occ_item(j, i);
+// Item i of job j (any i: past the last item nothing is done) by every lane of the warp.
+__device__ __forceinline__ void vox_small_occ(const VoxJob& j, uint64_t i) {
+  uint32_t lines = 0;
+  if (i < j.n_items) lines = vox_small_occ_item(j, i, load_verts(j.tris, item_triangle(j, i), j.stride));
+  append_large(j, i, lines);
 }
 
 // Pass 1 for small items: rank the voxels their pass mask names.
@@ -782,84 +892,141 @@ __device__ __forceinline__ void vox_small_win_item(const VoxJob& j, uint64_t i) 
 }
 
 
-// Lines 32*L*k .. 32*L*(k+1)-1 of large item i, L = lines_per_lane (lane, lane+32, ...).
-// The projection test that does not depend on the walk coordinate, for line (ca, cb).
-__device__ __forceinline__ bool line_passes(const VoxJob& j, const TriSetup& s, int W, int ca, int cb) {
-  const float fa = __fmul_rn((float)ca, j.u), fb = __fmul_rn((float)cb, j.u);
-  return W == 2 ? pass_xy(s, fa, fb) : (W == 0 ? pass_yz(s, fa, fb) : pass_zx(s, fb, fa));
-}
+// ---------------------------------------------------------------------------
+// Large items, several to a warp.  Up to kWalkItems lanes each set up one item (the set-up of
+// one item by all lanes cost a third of the whole pass); then the lines of all of them stand in
+// one row, 32 at a time are tested against their own projection, one per lane, and the ones that
+// pass go onto a stack from which 32 at a time are walked, one per lane.  So the lanes stay full
+// whatever the items' sizes.
+//
+// Bound by issue (no FMA).  Against one item per warp at a time: 8.8 -> 4.6 ms on the 20M-triangle
+// soup at gridsize 4096, 1.51 -> 0.89 ms on 4M triangles at gridsize 1024, and the list needs
+// neither a task count per item nor its scan (0.25 ms of the former).  Eight items a warp are 2 to
+// 4% slower, 32 (more shared memory) 7% slower on the batch of 128 meshes; 3 and 5 CTAs per SM 8% and 5%.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kWalkBits = 4, kWalkItems = 1u << kWalkBits;
+struct WalkScratch {
+  WalkItem item[kWalkItems];
+  uint32_t stack[64];  // item | ra << kWalkBits | rb << (kWalkBits + 10)
+};
 
-// Lines of a task, first tested by every lane against the projection that does not
-// depend on the walk coordinate; the lines that pass are packed into the warp's list
-// (`lines_smem`, 32 x lines_per_lane entries) and then walked one per lane, so lanes
-// do not idle beside lines outside the triangle.
-template <int PASS>
-__device__ __forceinline__ void vox_large_task(const VoxJob& j, uint64_t i, uint64_t k, int lane,
-                                               uint32_t* __restrict__ lines_smem) {
-  if (PASS == 1 && !j.winners) return;  // binary-mode stripe in a mixed batch: no winner pass
-  const uint64_t t = item_triangle(j, i);
-  const TriVerts tv = load_verts(j.tris, t, j.stride);
-  int lo[3], hi[3];
-  if (!item_box(j, tv, lo, hi)) return;  // cannot happen: the task count came from the same box
-  const int W = walk_axis(tv);
-  // lines of one item number at most 1024^2 (a stripe's face): 32-bit arithmetic
-  const uint32_t ea = (uint32_t)(W == 0 ? hi[1] - lo[1] + 1 : hi[0] - lo[0] + 1);  // first axis across the walk
-  const uint32_t lines = (uint32_t)item_lines(W, lo, hi);
-  const uint32_t c0 = (uint32_t)k * 32u * j.lines_per_lane + (uint32_t)lane;
-  TriSetup s;
-  tri_setup(tv, j.u, s);
-  const int top = max(hi[0], max(hi[1], hi[2]));
-  const bool mono = monotone_setup(s, fabsf(__fmul_rn((float)(top + 1), j.u)));
-  const float dir = (W == 0 ? s.n[0] : (W == 1 ? s.n[1] : s.n[2])) * j.u;
-  const float inv_dir = 1.0f / dir;
-  const int wlo = W == 0 ? lo[0] : (W == 1 ? lo[1] : lo[2]);
-  const int whi = W == 0 ? hi[0] : (W == 1 ? hi[1] : hi[2]);
-  const int alo = W == 0 ? lo[1] : lo[0], blo = W == 2 ? lo[1] : lo[2];
-  // all 32 lanes: test, then pack the passing lines as (ca - alo) | (cb - blo) << 16
+// The lanes with `has` (below kWalkItems): lines [first, first + most) of item `item` of stripe
+// `stripe`, or, when `parts` is not 0, part `first` of `parts` of its lines.
+template <int PASS, bool SINGLE>
+__device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, const VoxJob& j0, bool has, uint32_t item,
+                                           uint32_t stripe, uint32_t first, uint32_t most, uint32_t parts, int lane,
+                                           WalkScratch& sm) {
   const uint32_t lt = (1u << lane) - 1u;
-  const uint32_t first = (uint32_t)k * 32u * j.lines_per_lane;  // the task's first line (same for all lanes)
-  const uint32_t rounds = min(j.lines_per_lane, (lines - first + 31u) / 32u);
   uint32_t n = 0;
-#pragma unroll 1
-  for (uint32_t q = 0; q < rounds; q++) {
-    const uint32_t c = c0 + 32u * q;
-    const uint32_t ra = c % ea, rb = c / ea;
-    const bool ok = c < lines && line_passes(j, s, W, alo + (int)ra, blo + (int)rb);
-    const uint32_t vote = __ballot_sync(FULL, ok);
-    if (ok) lines_smem[n + __popc(vote & lt)] = ra | (rb << 16);
-    n += __popc(vote);
+  if (has) {
+    const VoxJob& j = SINGLE ? j0 : jobs[stripe];
+    if (PASS == 0 || j.winners) {  // (a binary stripe in a mixed batch has no winner pass)
+      const uint64_t t = item_triangle(j, item);
+      const TriVerts tv = load_verts(j.tris, t, j.stride);
+      int lo[3], hi[3];
+      if (item_box(j, tv, lo, hi)) {  // as when it was listed
+        const int W = walk_axis(tv);
+        const uint32_t lines = (uint32_t)item_lines(W, lo, hi);  // at most 1024^2 (a stripe's face)
+        if (parts) {  // whole rounds of 32 lines
+          most = (lines + 32u * parts - 1u) / (32u * parts) * 32u;
+          first *= most;
+        }
+        if (first < lines) {
+          n = min(most, lines - first);
+          walk_setup(j, tv, t, stripe, first, W, lo, hi, sm.item[lane]);
+        }
+      }
+    }
   }
+  const uint32_t incl = warp_inclusive(n), excl = incl - n, total = __shfl_sync(FULL, incl, 31);
   __syncwarp();
+  auto walk = [&](uint32_t e) {
+    const WalkItem& r = sm.item[e & (kWalkItems - 1u)];
+    walk_line<PASS>(SINGLE ? j0 : jobs[r.stripe], r, (e >> kWalkBits) & 1023u, e >> (kWalkBits + 10));
+  };
+  uint32_t cnt = 0;
 #pragma unroll 1
-  for (uint32_t q = (uint32_t)lane; q < n; q += 32u) {
-    const uint32_t r = lines_smem[q];
-    vox_line<PASS>(j, s, (uint32_t)t, W, alo + (int)(r & 0xffffu), blo + (int)(r >> 16), wlo, whi, mono, dir, inv_dir);
+  for (uint32_t r0 = 0; r0 < total; r0 += 32u) {
+    const uint32_t i = r0 + (uint32_t)lane;
+    uint32_t o = 0;  // its item: the first lane with incl > i
+#pragma unroll
+    for (uint32_t st = 16; st; st >>= 1) {
+      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
+      if (t <= i) o += st;
+    }
+    const uint32_t o_excl = __shfl_sync(FULL, excl, (int)o);
+    bool ok = i < total;
+    uint32_t e = 0;
+    if (ok) {
+      const WalkItem& r = sm.item[o];
+      const uint32_t c = i - o_excl + r.first, ea = r.shape & 2047u;
+      const uint32_t rb = r.magic ? __umulhi(c, r.magic) : c, ra = c - rb * ea;
+      const float fa = __fmul_rn((float)(r.alo + (int)ra), r.u), fb = __fmul_rn((float)(r.blo + (int)rb), r.u);
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(r.ea[k], fa), __fmul_rn(r.eb[k], fb)), r.ed[k]) < 0.0f);
+      e = o | (ra << kWalkBits) | (rb << (kWalkBits + 10));
+    }
+    const uint32_t vote = __ballot_sync(FULL, ok);
+    if (ok) sm.stack[cnt + __popc(vote & lt)] = e;
+    cnt += __popc(vote);
+    __syncwarp();
+    if (cnt >= 32u) {
+      cnt -= 32u;
+      walk(sm.stack[cnt + (uint32_t)lane]);
+      __syncwarp();
+    }
   }
-  __syncwarp();  // the list is free for the warp's next task
+  if ((uint32_t)lane < cnt) walk(sm.stack[lane]);
+  __syncwarp();  // the items and the stack are free for the warp's next ones
 }
 
-// Persistent warps pull 32-column tasks of large items from a global counter.
-template <int PASS>
-__global__ void __launch_bounds__(256, 4) k_vox_large(VoxJob j) {
-  pdl_enter();
-  extern __shared__ uint32_t lines_smem[];  // 32 x lines_per_lane per warp
-  const int lane = threadIdx.x & 31;
-  uint32_t* wl = lines_smem + (threadIdx.x >> 5) * 32u * j.lines_per_lane;
-  const uint64_t total = j.task_off[j.n_items];
-  if (total == 0) return;
-  for (;;) {
-    unsigned long long task = 0;
-    if (lane == 0) task = atomicAdd(j.task_counter, 1ull);
-    task = __shfl_sync(FULL, task, 0);
-    if (task >= total) break;
-    uint64_t lo_i = 0, hi_i = j.n_items;  // task_off[lo_i] <= task < task_off[hi_i]
-    while (hi_i - lo_i > 1) {
-      const uint64_t mid = (lo_i + hi_i) >> 1;
-      if (j.task_off[mid] <= task) lo_i = mid;
-      else hi_i = mid;
+// Persistent warps: first the tasks of the big items, one at a time (the longest work first),
+// then the others, as many at a time as leave every warp two helpings.
+template <int PASS, bool SINGLE>
+__device__ __forceinline__ void walk_lists(const VoxJob* __restrict__ jobs, const VoxJob& j0, const LargeLists& L, int lane,
+                                           WalkScratch& sm) {
+  const unsigned long long n = __ldcg(L.ctr + kCtrLarge), packed = __ldcg(L.ctr + kCtrBig);
+  const uint32_t nb = min((uint32_t)(packed & ((1u << kBigCountBits) - 1u)), L.big_cap);
+  if (nb) {
+    const uint4 end = __ldcg(L.big + nb - 1);
+    const uint64_t tasks = (uint64_t)end.z + end.w;
+    for (;;) {
+      unsigned long long t = 0;
+      if (lane == 0) t = atomicAdd(L.ctr + kCtrGrab + 32 * PASS, 1ull);
+      t = __shfl_sync(FULL, t, 0);
+      if (t >= tasks) break;
+      const uint32_t b = warp_search(nb, (uint32_t)t, lane, [&](uint32_t i) { return __ldcg(&L.big[i].z); });
+      const uint4 e = __ldcg(L.big + b);
+      const uint32_t k = (uint32_t)t - e.z;
+      if (k < e.w) walk_items<PASS, SINGLE>(jobs, j0, lane == 0, e.x, e.y, k * L.slice, L.slice, 0u, lane, sm);
     }
-    vox_large_task<PASS>(j, lo_i, task - j.task_off[lo_i], lane, wl);
   }
+  if (n == 0) return;
+  // Fewer items than warps: several warps share an item (up to 16, one per round of its 512 lines), so
+  // a handful of triangles takes one round and not sixteen (80 triangles at gridsize 64: 21 -> 10 us).  A
+  // warp's first helping is its number.
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t parts = (uint32_t)min(16ull, max(1ull, warps / n));
+  const uint64_t total = n * parts;
+  const uint32_t chunk = (uint32_t)min((unsigned long long)kWalkItems, n / (2 * warps) + 1);
+  uint64_t t = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk;
+  while (t < total) {
+    const bool has = (uint32_t)lane < chunk && t + (uint32_t)lane < total;
+    const uint64_t i = (t + (uint32_t)lane) / parts;
+    const unsigned long long e = has ? __ldcg(L.large + i) : 0ull;
+    walk_items<PASS, SINGLE>(jobs, j0, has, (uint32_t)e, (uint32_t)(e >> 32), (uint32_t)(t + (uint32_t)lane - i * parts), ~0u,
+                             parts > 1 ? parts : 0u, lane, sm);
+    if (lane == 0) t = (uint64_t)warps * chunk + atomicAdd(L.ctr + kCtrGrab + 16 + 32 * PASS, (unsigned long long)chunk);
+    t = __shfl_sync(FULL, t, 0);
+  }
+}
+
+template <int PASS, bool SINGLE>
+__global__ void __launch_bounds__(256, 4) kb_vox_large(const VoxJob* __restrict__ jobs, LargeLists lists, VoxJob j0) {
+  pdl_enter();
+  extern __shared__ __align__(16) unsigned char walk_smem[];
+  walk_lists<PASS, SINGLE>(jobs, j0, lists, threadIdx.x & 31, reinterpret_cast<WalkScratch*>(walk_smem)[threadIdx.x >> 5]);
 }
 
 // n words into `dst` (mapped pinned host memory): small results the host waits for
@@ -903,9 +1070,8 @@ __global__ void __launch_bounds__(kChunk, 4) kb_vox_small(const VoxJob* __restri
   pdl_enter();
   if constexpr (SINGLE) {
     const uint64_t i = (uint64_t)blockIdx.x * kChunk + threadIdx.x;
-    if (i >= j0.n_items) return;
-    if (PASS == 0) vox_small_occ_item(j0, i);
-    else vox_small_win_item(j0, i);
+    if (PASS == 0) vox_small_occ(j0, i);
+    else if (i < j0.n_items) vox_small_win_item(j0, i);
   } else {
     __shared__ VoxJob sj;
     uint64_t cta;
@@ -913,85 +1079,23 @@ __global__ void __launch_bounds__(kChunk, 4) kb_vox_small(const VoxJob* __restri
     stage(sj, jobs[s]);
     __syncthreads();
     const uint64_t i = cta * kChunk + threadIdx.x;
-    if (i >= sj.n_items) return;
-    if (PASS == 0) vox_small_occ_item(sj, i);
-    else vox_small_win_item(sj, i);
-  }
-}
-
-// The item and stripe of every warp task: map[t] = item | stripe << 32, one thread
-// per item writing its tasks' entries.  Written only when all tasks fit in `cap`.
-__global__ void __launch_bounds__(kChunk) kb_task_map(const uint64_t* __restrict__ cta_beg, uint32_t n,
-                                                      const uint64_t* __restrict__ item_beg,
-                                                      const uint64_t* __restrict__ task_off, uint64_t total_items,
-                                                      uint64_t* __restrict__ map, uint64_t cap) {
-  pdl_enter();
-  uint64_t cta;
-  const uint32_t s = cta_stripe(cta_beg, n, cta);
-  if (task_off[total_items] > cap) return;
-  const uint64_t i = item_beg[s] + cta * kChunk + threadIdx.x;
-  if (i >= item_beg[s + 1]) return;
-  for (uint64_t t = task_off[i], e = task_off[i + 1]; t < e; t++) map[t] = i | ((uint64_t)s << 32);
-}
-
-template <int PASS>
-__global__ void __launch_bounds__(256, 4) kb_vox_large(const VoxJob* __restrict__ jobs, const uint64_t* __restrict__ item_beg,
-                                                    uint32_t n_stripes, const uint64_t* __restrict__ task_off,
-                                                    uint64_t total_items, unsigned long long* counter,
-                                                    uint32_t lines_per_lane, const uint64_t* __restrict__ map,
-                                                    uint64_t cap) {
-  pdl_enter();
-  extern __shared__ uint32_t lines_smem[];  // 32 x lines_per_lane per warp (every job has this lines_per_lane)
-  const int lane = threadIdx.x & 31;
-  uint32_t* wl = lines_smem + (threadIdx.x >> 5) * 32u * lines_per_lane;
-  const uint64_t total = task_off[total_items];
-  if (total == 0) return;  // no large items in this launch: no counter traffic
-  for (;;) {
-    unsigned long long task = 0;
-    if (lane == 0) task = atomicAdd(counter, 1ull);
-    task = __shfl_sync(FULL, task, 0);
-    if (task >= total) break;
-    uint64_t lo_i = 0;
-    uint32_t s0 = 0;
-    if (total <= cap) {  // one load instead of two searches of dependent loads
-      const uint64_t v = map[task];
-      lo_i = (uint32_t)v;
-      s0 = (uint32_t)(v >> 32);
-    } else {
-      uint64_t hi_i = total_items;  // task_off[lo_i] <= task < task_off[hi_i]
-      while (hi_i - lo_i > 1) {
-        const uint64_t mid = (lo_i + hi_i) >> 1;
-        if (task_off[mid] <= task) lo_i = mid;
-        else hi_i = mid;
-      }
-      uint32_t s1 = n_stripes;  // item_beg[s0] <= lo_i < item_beg[s1]
-      while (s1 - s0 > 1) {
-        const uint32_t mid = (s0 + s1) >> 1;
-        if (item_beg[mid] <= lo_i) s0 = mid;
-        else s1 = mid;
-      }
-    }
-    vox_large_task<PASS>(jobs[s0], lo_i - item_beg[s0], task - task_off[lo_i], lane, wl);
+    if (PASS == 0) vox_small_occ(sj, i);
+    else if (i < sj.n_items) vox_small_win_item(sj, i);
   }
 }
 
 // ===========================================================================
 // Persistent occupancy passes (ooc_tuning::persistent): the small pass and the
-// large-triangle tasks of every stripe of a sub-batch in one launch.  Each warp
-// takes tickets from one counter and runs the unit its ticket names.  Tickets
-// come in this order:
-//   [0, C)          256-item chunks of the small pass, stripe by stripe;
-//   [C, C + T)      warp tasks of large items, in the order the chunks queued
-//                   them (T is final once every chunk is done).
-// A task waits only for chunks, whose tickets are smaller and held by running
-// warps already, so every wait ends whether or not the whole grid is resident.
-// Each wait is still bounded: past kPersistWaitNs it records its code in the
-// timeout counter and every warp stops.
+// large items of every stripe of a sub-batch in one launch.  Each warp takes
+// 256-item chunks of the small pass from one counter, stripe by stripe; when none
+// is left it waits until every chunk is done and joins the walk of the large
+// items.  The wait is for chunks that running warps hold already, so it ends
+// whether or not the whole grid is resident; it is still bounded: past
+// kPersistWaitNs it records its code in the timeout counter and every warp stops.
 // ===========================================================================
 // Counters, each on its own 128-byte line so the polls of waiting warps do not
 // queue behind the ticket atomics.
-constexpr int kCtrTicket = 0, kCtrChunksDone = 16, kCtrTasksQueued = kPersistTasksWord,
-              kCtrTimeout = kPersistTimeoutWord;
+constexpr int kCtrTicket = 0, kCtrChunksDone = 16, kCtrTimeout = kPersistTimeoutWord;
 static_assert(kPersistChunkItems == 32u * 8u, "a chunk is kPersistChunkRounds x 32 items");
 constexpr uint64_t kPersistWaitNs = 4000000000ull;  // a wait gives up after four seconds
 constexpr uint32_t kPersistChunkRounds = 8;          // a chunk is 8 x 32 items
@@ -1046,54 +1150,11 @@ __device__ __forceinline__ void stage_warp(T& dst, const T& src, int lane) {
   __syncwarp();
 }
 
-// 32 items of stripe s from item i0: the small pass, then their large items are
-// queued as warp tasks (or, when the task map is full, walked by this warp).
-__device__ __forceinline__ void persist_items(const PersistJob& pj, uint32_t s, uint64_t i0, int lane, const VoxJob& j,
-                                              uint32_t* __restrict__ wl) {
-  const uint64_t i = i0 + (uint64_t)lane;
-  uint32_t cost = 0;
-  if (i < j.n_items) cost = (uint32_t)vox_small_occ_item(j, i);
-  // warp-aggregated reservation of the items' tasks in the map
-  uint32_t excl = cost;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(FULL, excl, o);
-    if (lane >= o) excl += y;
-  }
-  const uint32_t total = __shfl_sync(FULL, excl, 31);
-  excl -= cost;
-  if (total == 0) return;
-  // One atomicAdd per 32 items (a compare-and-swap loop on this one counter
-  // stalled the whole grid).  Tasks reserved at or past `cap` have no entry:
-  // this warp walks them, and the warps that draw their tickets skip them.
-  unsigned long long base = 0;
-  if (lane == 0) base = atomicAdd(pj.ctr + kCtrTasksQueued, (unsigned long long)total);
-  base = __shfl_sync(FULL, base, 0);
-  __syncwarp();
-  const uint64_t ig = pj.item_beg[s] + i;  // the item's index in the sub-batch
-  uint32_t todo = __ballot_sync(FULL, cost != 0);
-  while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const uint32_t c = __shfl_sync(FULL, cost, src);
-    const uint64_t item = __shfl_sync(FULL, ig, src);
-    const uint64_t b = base + __shfl_sync(FULL, excl, src);
-    for (uint32_t k = (uint32_t)lane; k < c && b + k < pj.cap; k += 32u) {
-      volatile unsigned long long* e = reinterpret_cast<volatile unsigned long long*>(pj.map + b + k);
-      *e = item | ((uint64_t)k << 32);
-    }
-    const uint32_t walked_from = b >= pj.cap ? 0u : (pj.cap - b < c ? (uint32_t)(pj.cap - b) : c);
-    for (uint32_t k = walked_from; k < c; k++)
-      vox_large_task<0>(j, item - pj.item_beg[s], k, lane, wl);
-  }
-}
-
 __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
   pdl_enter();
-  extern __shared__ uint32_t lines_smem[];  // 32 x lines_per_lane per warp
   __shared__ VoxJob s_job[8];
+  __shared__ WalkScratch s_walk[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t* wl = lines_smem + (uint32_t)w * 32u * pj.lines_per_lane;
   const uint64_t C = pj.chunk_beg[pj.n];
   uint32_t job_s = ~0u;  // the stripe staged in s_job[w]
   for (;;) {
@@ -1102,67 +1163,32 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
       t = ld_acquire(pj.ctr + kCtrTimeout) != 0ull ? ~0ull : atomicAdd(pj.ctr + kCtrTicket, 1ull);
     t = __shfl_sync(FULL, t, 0);
     if (t == ~0ull) return;
-    if (t < C) {  // a chunk of kPersistChunkRounds x 32 items
-      const uint32_t s = find_stripe(pj.chunk_beg, pj.n, t);
-      if (s != job_s) {
-        stage_warp(s_job[w], pj.jobs[s], lane);
-        job_s = s;
-      }
-      const uint64_t c0 = (t - pj.chunk_beg[s]) * (32u * kPersistChunkRounds);
-      for (uint32_t q = 0; q < kPersistChunkRounds; q++) {
-        const uint64_t i0 = c0 + 32u * q;
-        if (i0 >= s_job[w].n_items) break;
-        persist_items(pj, s, i0, lane, s_job[w], wl);
-      }
-      // this chunk's queued tasks are visible before it counts as done
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) atomicAdd(pj.ctr + kCtrChunksDone, 1ull);
-      continue;
-    }
-    // a queued task, or (once every chunk is done and no task is left) the end
-    const uint64_t u = t - C;
-    // kind 1: task, 3: stop, 4: a task its chunk walks
-    unsigned long long kind = 0, entry = 0;
-    if (lane == 0) {
-      Backoff b;
-      for (;;) {
-        if (u < ld_acquire(pj.ctr + kCtrTasksQueued)) {
-          kind = 1;
-          break;
-        }
-        if (ld_acquire(pj.ctr + kCtrChunksDone) == C) {
-          kind = u < ld_acquire(pj.ctr + kCtrTasksQueued) ? 1 : 3;
-          break;
-        }
-        if (!b.pause(pj.ctr, 1u)) {
-          kind = 3;
-          break;
-        }
-      }
-      if (kind == 1 && u >= pj.cap) kind = 4;  // a task past the map: its chunk walks it
-      if (kind == 1) {  // the chunk that reserved entry u writes it right after
-        Backoff b2;
-        while ((entry = ld_acquire(pj.map + u)) == ~0ull)
-          if (!b2.pause(pj.ctr, 2u)) {
-            kind = 3;
-            break;
-          }
-        if (kind == 1) *reinterpret_cast<volatile unsigned long long*>(pj.map + u) = ~0ull;  // empty for the next launch
-      }
-    }
-    kind = __shfl_sync(FULL, kind, 0);
-    if (kind == 3) return;
-    if (kind == 4) continue;
-    entry = __shfl_sync(FULL, entry, 0);
-    const uint64_t item = (uint32_t)entry;
-    const uint32_t s = find_stripe(pj.item_beg, pj.n, item);
+    if (t >= C) break;
+    const uint32_t s = find_stripe(pj.chunk_beg, pj.n, t);  // a chunk of kPersistChunkRounds x 32 items
     if (s != job_s) {
+      __syncwarp();
       stage_warp(s_job[w], pj.jobs[s], lane);
       job_s = s;
     }
-    vox_large_task<0>(s_job[w], item - pj.item_beg[s], entry >> 32, lane, wl);
+    const uint64_t c0 = (t - pj.chunk_beg[s]) * (32u * kPersistChunkRounds);
+    for (uint32_t q = 0; q < kPersistChunkRounds; q++) {
+      const uint64_t i0 = c0 + 32u * q;
+      if (i0 >= s_job[w].n_items) break;
+      vox_small_occ(s_job[w], i0 + (uint64_t)lane);
+    }
+    // this chunk's listed items are visible before it counts as done
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) atomicAdd(pj.ctr + kCtrChunksDone, 1ull);
   }
+  bool ok = true;
+  if (lane == 0) {
+    Backoff b;
+    while (ld_acquire(pj.ctr + kCtrChunksDone) != C && ok) ok = b.pause(pj.ctr, 1u);
+  }
+  if (!__shfl_sync(FULL, ok, 0)) return;
+  __syncwarp();
+  walk_lists<0, false>(pj.jobs, s_job[w], pj.lists, lane, s_walk[w]);
 }
 
 }  // namespace
@@ -1171,12 +1197,6 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
 // Launch wrappers
 // ===========================================================================
 uint64_t scan_partials_needed(uint64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
-
-void scan_u64_exclusive(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st, bool flag_last) {
-  unsigned long long* d = reinterpret_cast<unsigned long long*>(data);
-  scan_exclusive<unsigned long long>(d, n, reinterpret_cast<unsigned long long*>(partials), st,
-                                     flag_last ? d + n - 1 : nullptr);
-}
 
 void launch_copy_words(const uint32_t* src, uint64_t n, uint32_t* dst, cudaStream_t st) {
   if (n == 0) return;
@@ -1239,54 +1259,24 @@ void launch_stream_group_chunk(const float* tris, int stride, uint64_t n, const 
 cudaError_t launch_vox_small_occupancy(const VoxJob& j, cudaStream_t st) {
   if (j.n_items == 0) return cudaSuccess;
   KScope k("vox_small_occupancy", st);
+  const VoxJob* jobs = nullptr;
+  const uint64_t* cta_beg = nullptr;
+  uint32_t n = 1;
   VoxJob arg = j;
-  void* args[] = {&arg};
-  return cudaLaunchKernel(reinterpret_cast<const void*>(&k_vox_small_occ), dim3(grid_for(j.n_items, 256)), dim3(256),
-                          args, 0, st);
+  void* args[] = {&jobs, &cta_beg, &n, &arg};
+  return cudaLaunchKernel(reinterpret_cast<const void*>(&kb_vox_small<0, true>), dim3(grid_for(j.n_items, kChunk)),
+                          dim3(kChunk), args, 0, st);
 }
 
 cudaError_t launch_vox_large_occupancy(const VoxJob& j, cudaStream_t st, int num_sms) {
   if (j.n_items == 0) return cudaSuccess;
-  const cudaError_t e = cudaMemsetAsync(j.task_counter, 0, sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
   KScope k("vox_large_occupancy", st);
+  const VoxJob* jobs = nullptr;
+  LargeLists lists = lists_of(j);
   VoxJob arg = j;
-  void* args[] = {&arg};
-  return cudaLaunchKernel(reinterpret_cast<const void*>(&k_vox_large<0>), dim3((unsigned)num_sms * 8), dim3(256), args,
-                          (size_t)256 * j.lines_per_lane * 4, st);
-}
-
-// scan_exclusive<uint64_t> with the status of every launch returned.
-cudaError_t scan_u64_exclusive_checked(uint64_t* data, uint64_t n, uint64_t* partials, cudaStream_t st) {
-  if (n == 0) return cudaSuccess;
-  const unsigned nb = (unsigned)((n + SCAN_TILE - 1) / SCAN_TILE);
-  const uint64_t* none = nullptr;  // no partials (one tile) / no skip flag
-  if (nb == 1) {
-    KScope k("scan_down", st);
-    void* args[] = {&data, &n, &none, &none};
-    return cudaLaunchKernel(reinterpret_cast<const void*>(&k_scan_down<uint64_t>), dim3(1), dim3(SCAN_THREADS), args,
-                            0, st);
-  }
-  cudaError_t e;
-  {
-    KScope k("scan_reduce", st);
-    void* args[] = {&data, &n, &partials, &none};
-    e = cudaLaunchKernel(reinterpret_cast<const void*>(&k_scan_reduce<uint64_t>), dim3(nb), dim3(SCAN_THREADS), args,
-                         0, st);
-  }
-  if (e != cudaSuccess) return e;
-  {
-    KScope k("scan_partials", st);
-    uint64_t np = nb;
-    void* args[] = {&partials, &np, &none};
-    e = cudaLaunchKernel(reinterpret_cast<const void*>(&k_scan_partials<uint64_t>), dim3(1), dim3(1024), args, 0, st);
-  }
-  if (e != cudaSuccess) return e;
-  KScope k("scan_down", st);
-  const uint64_t* cp = partials;
-  void* args[] = {&data, &n, &cp, &none};
-  return cudaLaunchKernel(reinterpret_cast<const void*>(&k_scan_down<uint64_t>), dim3(nb), dim3(SCAN_THREADS), args, 0,
-                          st);
+  void* args[] = {&jobs, &lists, &arg};
+  return cudaLaunchKernel(reinterpret_cast<const void*>(&kb_vox_large<0, true>), dim3((unsigned)num_sms * 4), dim3(256),
+                          args, 8 * sizeof(WalkScratch), st);
 }
 
 void launch_scatter_records(const uint64_t* src, uint64_t n, int words, uint64_t* dst, cudaStream_t st) {
@@ -1318,48 +1308,27 @@ void launch_b_vox_small(const VoxJob* jobs, const uint64_t* cta_beg, uint32_t n,
   }
 }
 
-void launch_b_task_map(const uint64_t* cta_beg, uint32_t n, uint64_t ctas, const uint64_t* item_beg,
-                       const uint64_t* task_off, uint64_t total_items, uint64_t* map, uint64_t cap, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k("task_map", st);
-  launch_k(kb_task_map, dim3((unsigned)ctas), dim3(kChunk), 0, st, cta_beg, n, item_beg, task_off, total_items, map,
-           cap);
-}
-
-void launch_b_vox_large(const VoxJob* jobs, const uint64_t* item_beg, uint32_t n_stripes, const uint64_t* task_off,
-                        uint64_t total_items, unsigned long long* counter, int pass, cudaStream_t st, int num_sms,
-                        int block, int ctas_per_sm, uint32_t lines_per_lane, const uint64_t* map, uint64_t cap) {
-  if (total_items == 0) return;
-  cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
-  const unsigned grid = (unsigned)num_sms * (unsigned)ctas_per_sm;
-  const size_t smem = (size_t)block * lines_per_lane * 4;  // each warp's list of passing lines
-  if (smem > (48u << 10)) {  // beyond the default dynamic limit (at most 256 x 64 x 4 = 64 KiB)
-    cudaFuncSetAttribute(kb_vox_large<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kb_vox_large<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+void launch_b_vox_large(const VoxJob* jobs, const LargeLists& lists, int pass, const VoxJob* single, cudaStream_t st,
+                        int num_sms, int block, int ctas_per_sm) {
   KScope k(pass == 0 ? "vox_large_occupancy" : "vox_large_winner", st);
-  if (pass == 0)
-    launch_k(kb_vox_large<0>, dim3(grid), dim3(block), smem, st, jobs, item_beg, n_stripes, task_off, total_items,
-             counter, lines_per_lane, map, cap);
-  else
-    launch_k(kb_vox_large<1>, dim3(grid), dim3(block), smem, st, jobs, item_beg, n_stripes, task_off, total_items,
-             counter, lines_per_lane, map, cap);
+  VoxJob j0;
+  std::memset(&j0, 0, sizeof(j0));
+  if (single) j0 = *single;
+  auto* kern = single ? (pass == 0 ? kb_vox_large<0, true> : kb_vox_large<1, true>)
+                      : (pass == 0 ? kb_vox_large<0, false> : kb_vox_large<1, false>);
+  launch_k(kern, dim3((unsigned)num_sms * (unsigned)ctas_per_sm), dim3(block), (size_t)(block / 32) * sizeof(WalkScratch), st,
+           jobs, lists, j0);
 }
 
-int persist_ctas_per_sm(uint32_t lines_per_lane) {
+int persist_ctas_per_sm() {
   int per_sm = 0;
-  const size_t smem = (size_t)256 * lines_per_lane * 4;
-  if (smem > (48u << 10) &&
-      cudaFuncSetAttribute(kb_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb_persist, 256, smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb_persist, 256, 0) != cudaSuccess) return 0;
   return per_sm;
 }
 
 void launch_b_persist(const PersistJob& pj, int num_sms, int ctas_per_sm, cudaStream_t st) {
   KScope k("persistent_occupancy", st);
-  const size_t smem = (size_t)256 * pj.lines_per_lane * 4;
-  launch_k(kb_persist, dim3((unsigned)(num_sms * ctas_per_sm)), dim3(256), smem, st, pj);
+  launch_k(kb_persist, dim3((unsigned)(num_sms * ctas_per_sm)), dim3(256), 0, st, pj);
 }
 
 }  // namespace ooc

@@ -99,6 +99,19 @@ __device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
   return (t * 0x00204081u) >> 28;
 }
 
+// The last index w < n of a non-decreasing array with at(w) <= r (at(0) <= r), by the whole
+// warp: every step reads 32 entries at once, so 8,192 words take three dependent loads.
+template <typename F>
+__device__ __forceinline__ uint32_t warp_search(uint32_t n, uint32_t r, int lane, F at) {
+  uint32_t lo = 0, step = 1;
+  while (step * 32u < n) step *= 32u;
+  for (;; step /= 32u) {
+    const uint32_t i = lo + (uint32_t)lane * step;
+    lo += (uint32_t)(__popc(__ballot_sync(FULL, i < n && at(i) <= r)) - 1) * step;
+    if (step == 1) return lo;
+  }
+}
+
 // ---- batched launches: a prefix of CTA counts maps each CTA to its stripe, whose
 // job the CTA copies into shared memory ----
 template <typename T>

@@ -7,9 +7,8 @@
 // pre-reserves all device memory, and latency-critical loops where an
 // allocation would synchronise the device.  This entry point takes the
 // triangles and the output bitfield from the caller and keeps the pass's only
-// scratch -- the per-triangle task offsets, their scan partials and the task
-// counter of the large-triangle kernel -- in a fixed-size array that lives in
-// this file as a static __device__ variable.  Every GPU that loads the library
+// scratch -- the list of the large triangles and its counters -- in a fixed-size
+// array that lives in this file as a static __device__ variable.  Every GPU that loads the library
 // holds that array (about 8.4 MB) until the process exits.
 #include <cuda_runtime.h>
 
@@ -24,9 +23,10 @@ namespace {
 using namespace ooc;
 
 constexpr uint64_t kMaxTris = OOC_NOALLOC_MAX_TRIANGLES;
-constexpr uint64_t kTaskWords = kMaxTris + 1;  // exclusive prefix of warp tasks, one entry per triangle + total
-constexpr uint64_t kPartialWords = (kTaskWords + 4095) / 4096 + 1;  // scan partials (4096-element tiles)
-constexpr uint64_t kScratchWords = kTaskWords + kPartialWords + 2;  // + task counter
+constexpr uint32_t kBig = 4096;  // entries of the big triangles' list (16 bytes each); past it one warp walks each
+constexpr uint64_t kBigWord = kLargeCtrWords, kLargeWord = kBigWord + 2 * kBig;
+constexpr uint64_t kScratchWords = kLargeWord + kMaxTris;
+static_assert(kBigWord % 2 == 0, "16-byte entries");
 
 // The scratch.  In host code this name is only a stand-in for the device
 // variable: its device address comes from cudaGetSymbolAddress below.
@@ -68,7 +68,6 @@ extern "C" int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, co
   const uint64_t words = voxels < 32 ? 1 : voxels / 32;
   if (occupancy_words < words) return OOC_ERR_INVALID;
 
-  if (scan_partials_needed(n_tris + 1) > kPartialWords) return OOC_ERR_LIMIT;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return OOC_ERR_DEVICE;
   unsigned long long* scratch = nullptr;
@@ -99,20 +98,20 @@ extern "C" int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, co
   j.u = u;
   j.unit_div = 1.0f / u;  // voxelizer.cpp:164
   j.small_vol = 64;
-  j.lines_per_lane = 16;
   j.leafbits = occupancy_device;
-  j.task_off = reinterpret_cast<uint64_t*>(scratch);
-  uint64_t* partials = reinterpret_cast<uint64_t*>(scratch + kTaskWords);
-  j.task_counter = scratch + kTaskWords + kPartialWords;
+  j.ctr = scratch;
+  j.big = reinterpret_cast<uint4*>(scratch + kBigWord);
+  j.large = scratch + kLargeWord;
+  j.big_cap = kBig;
+  j.slice = 512;
   j.item_mask = nullptr;
 
-  // What must start at zero: the output bits and the end of the task-offset
-  // scan (the other scratch entries are fully written before they are read).
-  // Every step's own status is checked; the first failure ends the call.
+  // What must start at zero: the output bits and the list's counters (its entries
+  // are written before they are read).  Every step's own status is checked; the
+  // first failure ends the call.
   if (cudaMemsetAsync(occupancy_device, 0, words * 4, st) != cudaSuccess) return OOC_ERR_DEVICE;
-  if (cudaMemsetAsync(j.task_off + n_tris, 0, 8, st) != cudaSuccess) return OOC_ERR_DEVICE;
+  if (cudaMemsetAsync(j.ctr, 0, kLargeCtrWords * 8, st) != cudaSuccess) return OOC_ERR_DEVICE;
   if (launch_vox_small_occupancy(j, st) != cudaSuccess) return OOC_ERR_DEVICE;
-  if (scan_u64_exclusive_checked(j.task_off, n_tris + 1, partials, st) != cudaSuccess) return OOC_ERR_DEVICE;
   if (launch_vox_large_occupancy(j, st, sms) != cudaSuccess) return OOC_ERR_DEVICE;
   return OOC_OK;
 }

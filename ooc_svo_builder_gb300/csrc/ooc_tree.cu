@@ -253,7 +253,8 @@ __device__ __forceinline__ uint32_t parent_word(const uint32_t w[8]) {
 // 256 words and fewer are left to the first warp, which needs no block barrier.
 template <int T>
 __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes, uint32_t* __restrict__ counts,
-                                              const uint64_t* __restrict__ tasks, uint64_t* __restrict__ tasks_out,
+                                              const unsigned long long* __restrict__ large_ctr,
+                                              uint64_t* __restrict__ large_out,
                                               const uint64_t* __restrict__ code, uint64_t* __restrict__ code_out) {
   pdl_enter();
   __shared__ Stripe sp;
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes
   stage(sp, stripes[blockIdx.x]);
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *tasks_out = *tasks;
+    *large_out = large_ctr[kCtrLarge] + large_ctr[kCtrBig];  // zero: none
     if (code) *code_out = *code;
   }
   uint32_t* out = counts + (uint64_t)blockIdx.x * kCountWords;
@@ -513,19 +514,6 @@ __device__ __forceinline__ void average_children(uint32_t mask, const float* chi
   out[3] = tx;
   out[4] = ty;
   out[5] = tz;
-}
-
-// The last index w < n of a non-decreasing array with at(w) <= r (at(0) <= r), by the whole
-// warp: every step reads 32 entries at once, so 8,192 words take three dependent loads.
-template <typename F>
-__device__ __forceinline__ uint32_t warp_search(uint32_t n, uint32_t r, int lane, F at) {
-  uint32_t lo = 0, step = 1;
-  while (step * 32u < n) step *= 32u;
-  for (;; step /= 32u) {
-    const uint32_t i = lo + (uint32_t)lane * step;
-    lo += (uint32_t)(__popc(__ballot_sync(FULL, i < n && at(i) <= r)) - 1) * step;
-    if (step == 1) return lo;
-  }
 }
 
 constexpr uint32_t kTreeThreads = 256;
@@ -1307,14 +1295,14 @@ void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n,
            cta_beg, n, p0);
 }
 
-void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts, const uint64_t* tasks,
-                    uint64_t* tasks_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st) {
+void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts,
+                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st) {
   if (n == 0) return;
   KScope k("upper", st);
   // 128 threads cover level 4's 128 words at eight a thread with room for smaller CTAs to share an SM;
   // larger stripes have 1,024 and 8,192 words to scan
-  if (max_upper >= 5) launch_k(kb_upper<1024>, dim3(n), dim3(1024), 0, st, stripes, counts, tasks, tasks_out, code, code_out);
-  else launch_k(kb_upper<128>, dim3(n), dim3(128), 0, st, stripes, counts, tasks, tasks_out, code, code_out);
+  if (max_upper >= 5) launch_k(kb_upper<1024>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
+  else launch_k(kb_upper<128>, dim3(n), dim3(128), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
 }
 
 void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
