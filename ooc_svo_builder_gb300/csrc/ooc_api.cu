@@ -151,7 +151,9 @@ struct ooc_ctx {
   std::vector<cudaEvent_t> up_events;    // recorded on h2d_stream as groups of meshes arrive
   DevBuf d_tables1, d_tables2;
   std::vector<DevBuf> d_mesh_items;
-  ooc_tuning tuning = {64, 16, 256, 4, 4ull << 30, 0, 8, 1, 0};  // launch choices (ooc_set_tuning / ooc_autotune)
+  // launch choices (ooc_set_tuning / ooc_autotune); for triangles of more than kSmallVol candidates the
+  // line walk costs less than one thread's share of a divergent warp
+  ooc_tuning tuning = {ooc::kSmallVol, 16, 256, 4, 4ull << 30, 0, 8, 1, 0};
   // executable graphs of captured launch sequences, by shape (launch count and kernels)
   std::vector<std::pair<uint64_t, cudaGraphExec_t>> graph_execs;
   DevBuf d_tune_arena;                               // autotuner outputs
@@ -2130,7 +2132,7 @@ int ooc_autotune(ooc_ctx* c, const ooc_mesh* sample, uint64_t n, ooc_tuning* bes
   rc = time_one(cur, cur_ms);  // warms the context's buffers too
   if (rc == OOC_OK) rc = time_one(cur, cur_ms);
   // one coordinate pass: each choice in turn, the others held at their best so far
-  const uint32_t lpl[] = {4, 8, 16, 32}, cps[] = {2, 4, 8}, blk[] = {128, 256}, svol[] = {16, 32, 48, 64}, gr[] = {0, 1},
+  const uint32_t lpl[] = {4, 8, 16, 32}, cps[] = {2, 4, 8}, blk[] = {128, 256}, svol[] = {8, 16, 32, 64}, gr[] = {0, 1},
                  ept[] = {1, 2, 4, 8}, pdl[] = {0, 1}, per[] = {0, 1};
   const uint64_t bud[] = {1ull << 30, 2ull << 30, 4ull << 30, 8ull << 30};
   auto try_values = [&](auto setter, const auto& values) {

@@ -97,7 +97,7 @@ extern "C" int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, co
   }
   j.u = u;
   j.unit_div = 1.0f / u;  // voxelizer.cpp:164
-  j.small_vol = 64;
+  j.small_vol = kSmallVol;
   j.leafbits = occupancy_device;
   j.ctr = scratch;
   j.big = reinterpret_cast<uint4*>(scratch + kBigWord);
