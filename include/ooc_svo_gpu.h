@@ -163,7 +163,8 @@ int ooc_arena_alloc(void* arena, uint64_t mesh, uint64_t nodes_bytes, uint64_t d
  * Launch choices of the voxelizer and the batch engine.  Every value gives the
  * same output; they only change speed. */
 typedef struct {
-  uint32_t small_vol;         /* triangles whose box has at most this many voxels run one per thread (1..64) */
+  uint32_t small_vol;         /* triangles whose box has at most this many voxels, and more than two along
+                                 one axis at most, run one per thread (1..64) */
   uint32_t lines_per_lane;    /* lines of a large triangle each lane of a warp task walks (1..64);
                                  the work-queue chunk is 32 x this many lines */
   uint32_t large_block;       /* threads per CTA of the large-triangle kernel: 64, 128 or 256 */

@@ -143,6 +143,27 @@ __device__ __forceinline__ float edge_offset(float a, float b, float va, float v
   return __fadd_rn(__fadd_rn(-dot2(a, b, va, vb), smax(0.0f, __fmul_rn(u, a))), smax(0.0f, __fmul_rn(u, b)));
 }
 
+// The edge functions of the three projections from the edges `e` and the normal s.n.
+__device__ __forceinline__ void edge_setup(const TriVerts& t, const float e[3][3], float u, TriSetup& s) {
+  const float fz = (s.n[2] < 0.0f) ? -1.0f : 1.0f;
+  const float fx = (s.n[0] < 0.0f) ? -1.0f : 1.0f;
+  const float fy = (s.n[1] < 0.0f) ? -1.0f : 1.0f;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    // XY: (-e.y, e.x), YZ: (-e.z, e.y), ZX: (-e.x, e.z); sign-flipped by n.
+    // Multiplying by +-1 is exact, like the reference's -1.0f * vec2.
+    s.xy[k][0] = __fmul_rn(fz, -e[k][1]);
+    s.xy[k][1] = __fmul_rn(fz, e[k][0]);
+    s.yz[k][0] = __fmul_rn(fx, -e[k][2]);
+    s.yz[k][1] = __fmul_rn(fx, e[k][1]);
+    s.zx[k][0] = __fmul_rn(fy, -e[k][0]);
+    s.zx[k][1] = __fmul_rn(fy, e[k][2]);
+    s.dxy[k] = edge_offset(s.xy[k][0], s.xy[k][1], t.v[k][0], t.v[k][1], u);
+    s.dyz[k] = edge_offset(s.yz[k][0], s.yz[k][1], t.v[k][1], t.v[k][2], u);
+    s.dzx[k] = edge_offset(s.zx[k][0], s.zx[k][1], t.v[k][2], t.v[k][0], u);
+  }
+}
+
 __device__ __forceinline__ void tri_setup(const TriVerts& t, float u, TriSetup& s) {
   float e[3][3];
 #pragma unroll
@@ -162,23 +183,7 @@ __device__ __forceinline__ void tri_setup(const TriVerts& t, float u, TriSetup& 
   s.d1 = dot3(s.n[0], s.n[1], s.n[2], __fsub_rn(cx, t.v[0][0]), __fsub_rn(cy, t.v[0][1]), __fsub_rn(cz, t.v[0][2]));
   s.d2 = dot3(s.n[0], s.n[1], s.n[2], __fsub_rn(__fsub_rn(u, cx), t.v[0][0]), __fsub_rn(__fsub_rn(u, cy), t.v[0][1]),
               __fsub_rn(__fsub_rn(u, cz), t.v[0][2]));
-  const float fz = (s.n[2] < 0.0f) ? -1.0f : 1.0f;
-  const float fx = (s.n[0] < 0.0f) ? -1.0f : 1.0f;
-  const float fy = (s.n[1] < 0.0f) ? -1.0f : 1.0f;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    // XY: (-e.y, e.x), YZ: (-e.z, e.y), ZX: (-e.x, e.z); sign-flipped by n.
-    // Multiplying by +-1 is exact, like the reference's -1.0f * vec2.
-    s.xy[k][0] = __fmul_rn(fz, -e[k][1]);
-    s.xy[k][1] = __fmul_rn(fz, e[k][0]);
-    s.yz[k][0] = __fmul_rn(fx, -e[k][2]);
-    s.yz[k][1] = __fmul_rn(fx, e[k][1]);
-    s.zx[k][0] = __fmul_rn(fy, -e[k][0]);
-    s.zx[k][1] = __fmul_rn(fy, e[k][2]);
-    s.dxy[k] = edge_offset(s.xy[k][0], s.xy[k][1], t.v[k][0], t.v[k][1], u);
-    s.dyz[k] = edge_offset(s.yz[k][0], s.yz[k][1], t.v[k][1], t.v[k][2], u);
-    s.dzx[k] = edge_offset(s.zx[k][0], s.zx[k][1], t.v[k][2], t.v[k][0], u);
-  }
+  edge_setup(t, e, u, s);
 }
 
 // XY projection tests for a column (x, y): they do not depend on z.

@@ -85,7 +85,7 @@ struct VoxJob {
   int pa[3], pb[3];         // partition box in grid coordinates (inclusive)
   int sa[3], sb[3];         // stripe box in grid coordinates (inclusive)
   float u, unit_div;
-  uint32_t small_vol;       // items with at most this many candidates (<= 64) run one per thread
+  uint32_t small_vol;       // small items have at most this many candidates (<= 64)
   uint32_t* leafbits;       // level-Ds words
   uint8_t* leaftouch;       // byte per 256-bit block of leafbits, set when a bit of the block is (may be NULL)
   // pass B (payload winners)

@@ -436,29 +436,46 @@ __device__ __forceinline__ uint64_t item_lines(int W, const int lo[3], const int
 constexpr int kBigCountBits = 20;
 static_assert(kMaxBig + (1u << 19) < (1u << kBigCountBits), "the count stays in its bits");
 
-// The warp's lanes: item i of job j with `lines` lines (0: not a large item).  All 32 lanes call.
+// Item i of job j with more than `slice` lines: whether it went to `big`.
+__device__ __forceinline__ bool append_big(const VoxJob& j, uint64_t i, uint32_t lines) {
+  const unsigned long long now = *reinterpret_cast<volatile unsigned long long*>(j.ctr + kCtrBig);
+  if ((now & ((1ull << kBigCountBits) - 1ull)) >= j.big_cap) return false;
+  const uint32_t tasks = (lines + j.slice - 1u) / j.slice;
+  const unsigned long long got = atomicAdd(j.ctr + kCtrBig, ((unsigned long long)tasks << kBigCountBits) | 1ull);
+  const uint32_t slot = (uint32_t)got & ((1u << kBigCountBits) - 1u);
+  if (slot >= j.big_cap) return false;
+  j.big[slot] = make_uint4((uint32_t)(j.item0 + i), j.stripe, (uint32_t)(got >> kBigCountBits), tasks);
+  return true;
+}
+
+// Every thread of a warp (CTA false) or of the CTA (of at most kChunk threads): item i of job j with
+// `lines` lines, 0 for an item that is not large.  One atomic per CTA: additions to one address
+// finish about 3 ns apart, and one per warp took all of the pass's time on the large soups (0.47 of
+// 0.47 ms for 4M triangles).
+template <bool CTA>
 __device__ __forceinline__ void append_large(const VoxJob& j, uint64_t i, uint32_t lines) {
-  const int lane = threadIdx.x & 31;
-  bool one = lines != 0;
-  if (lines > j.slice) {
-    const unsigned long long now = *reinterpret_cast<volatile unsigned long long*>(j.ctr + kCtrBig);
-    if ((now & ((1ull << kBigCountBits) - 1ull)) < j.big_cap) {
-      const uint32_t tasks = (lines + j.slice - 1u) / j.slice;
-      const unsigned long long got = atomicAdd(j.ctr + kCtrBig, ((unsigned long long)tasks << kBigCountBits) | 1ull);
-      const uint32_t slot = (uint32_t)got & ((1u << kBigCountBits) - 1u);
-      if (slot < j.big_cap) {
-        j.big[slot] = make_uint4((uint32_t)(j.item0 + i), j.stripe, (uint32_t)(got >> kBigCountBits), tasks);
-        one = false;
-      }
-    }
-  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool one = lines != 0 && !(lines > j.slice && append_big(j, i, lines));
   const uint32_t m = __ballot_sync(FULL, one);
-  if (!m) return;
   unsigned long long at = 0;
-  const int leader = __ffs(m) - 1;
-  if (lane == leader) at = atomicAdd(j.ctr + kCtrLarge, (unsigned long long)__popc(m));
-  at = __shfl_sync(FULL, at, leader) + __popc(m & ((1u << lane) - 1u));
-  if (one) j.large[at] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
+  if constexpr (CTA) {
+    __shared__ uint32_t s_cnt[kChunk / 32];
+    __shared__ unsigned long long s_at;
+    if (lane == 0) s_cnt[warp] = __popc(m);
+    const uint32_t total = (uint32_t)__syncthreads_count(one);
+    if (total == 0) return;
+    if (threadIdx.x == 0) s_at = atomicAdd(j.ctr + kCtrLarge, (unsigned long long)total);
+    uint32_t before = 0;
+    for (int k = 0; k < warp; k++) before += s_cnt[k];
+    __syncthreads();
+    at = s_at + before;
+  } else {
+    if (!m) return;
+    if (lane == 0) at = atomicAdd(j.ctr + kCtrLarge, (unsigned long long)__popc(m));
+    at = __shfl_sync(FULL, at, 0);
+  }
+  if (one)
+    j.large[at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
 }
 
 // A large item as the warp's lanes read it: the constants of the test arranged by the walk axis
@@ -665,32 +682,62 @@ __device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, ui
 // result gives the reference's verdict for every candidate, bit for bit; the
 // FP32 expressions are the reference's, operation by operation.  A candidate
 // passes when all seven pass (the reference's order of early exits only saves
-// work).  The pass mask of an item has bit (ix * by + iy) * bz + iz for box
-// coordinates (ix, iy, iz).
+// work).
+//
+// Small are the boxes of at most small_vol voxels that are at most two wide along two
+// axes; w is the third (the longest; z among equals), a and b are the ones that follow
+// it cyclically.  The edge tests are cyclic in (x, y, z), so with the coordinates rotated
+// to (a, b, w) they read the same for every w; the sums of three products keep the
+// reference's order (x + y) + z.  The pass mask of an item has bit (ia * bb + ib) * bw + iw.
+//
+// Bound by ALU instructions.  One body for every orientation, its voxels' bits merged into
+// one store per leaf word, took the pass from 86 to 90 us on a heightfield of 2M triangles,
+// where almost every box was already 2 x 2 x w, and from 485 to 246 us on 4M random
+// triangles and 282 to 173 us on 128 meshes (with append_large), where two boxes in three
+// were not and ran a voxel at a time.
 // ---------------------------------------------------------------------------
 
-// Sets a passing voxel's bit: bits of one leaf word are gathered in `acc`
-// while consecutive voxels stay in it.
-__device__ __forceinline__ void leaf_bit(const VoxJob& j, bool pass, uint32_t m, uint32_t& cur_w, uint32_t& acc) {
-  if (!pass) return;
-  const uint32_t w = m >> 5;
-  if (w != cur_w) {
-    if (acc) set_leaf(j, cur_w, acc);
-    cur_w = w;
-    acc = 0;
-  }
-  acc |= 1u << (m & 31);
+// p[0..2] of the rotated axes (a, b, w), summed in the reference's order: w = z: a, b, w are
+// x, y, z; w = x: y, z, x; w = y: z, x, y.
+__device__ __forceinline__ float sum3(int W, float pa, float pb, float pw) {
+  if (W == 2) return __fadd_rn(__fadd_rn(pa, pb), pw);
+  return W == 0 ? __fadd_rn(__fadd_rn(pw, pa), pb) : __fadd_rn(__fadd_rn(pb, pw), pa);
 }
 
-__device__ __forceinline__ uint64_t bit_if(bool p, uint32_t pos) { return p ? (1ull << (pos & 63u)) : 0ull; }
+// tri_setup with the coordinates rotated to (a, b, w).
+__device__ __forceinline__ void tri_setup_rotated(const TriVerts& t, float u, int W, TriSetup& s) {
+  float e[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    e[0][a] = __fsub_rn(t.v[1][a], t.v[0][a]);
+    e[1][a] = __fsub_rn(t.v[2][a], t.v[1][a]);
+    e[2][a] = __fsub_rn(t.v[0][a], t.v[2][a]);
+  }
+  s.n[0] = __fsub_rn(__fmul_rn(e[0][1], e[1][2]), __fmul_rn(e[0][2], e[1][1]));
+  s.n[1] = __fsub_rn(__fmul_rn(e[0][2], e[1][0]), __fmul_rn(e[0][0], e[1][2]));
+  s.n[2] = __fsub_rn(__fmul_rn(e[0][0], e[1][1]), __fmul_rn(e[0][1], e[1][0]));
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(sum3(W, __fmul_rn(s.n[0], s.n[0]), __fmul_rn(s.n[1], s.n[1]),
+                                                  __fmul_rn(s.n[2], s.n[2]))));
+#pragma unroll
+  for (int a = 0; a < 3; a++) s.n[a] = __fmul_rn(s.n[a], r);
+  float c1[3], c2[3];  // critical point and its opposite, minus the first vertex
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const float c = s.n[a] > 0.0f ? u : 0.0f;
+    c1[a] = __fmul_rn(s.n[a], __fsub_rn(c, t.v[0][a]));
+    c2[a] = __fmul_rn(s.n[a], __fsub_rn(__fsub_rn(u, c), t.v[0][a]));
+  }
+  s.d1 = sum3(W, c1[0], c1[1], c1[2]);
+  s.d2 = sum3(W, c2[0], c2[1], c2[2]);
+  edge_setup(t, e, u, s);
+}
 
-// Boxes at most two voxels wide in x and y (the common small triangle): z is
-// walked in 2 x 2 x 2 bricks, every test of a brick evaluated without
-// branches; slots outside the box are masked.  The Morton bits of a
-// coordinate + 1 come from the carry trick: setting every bit outside an
-// axis' positions makes +1 carry across them.
-__device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriSetup& s, const int lo[3], uint32_t bx,
-                                                     uint32_t by, uint32_t bz) {
+// A small box: w is walked in 2 x 2 x 2 bricks, every test of a brick evaluated without
+// branches; slots outside the box are masked.  (In the rotated coordinates x, y, z below
+// stand for a, b, w.)  The Morton bits of a coordinate + 1 come from the carry trick:
+// setting every bit outside an axis' positions makes +1 carry across them.
+__device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriSetup& s, int W, const int lo[3],
+                                                     const uint32_t local[3], uint32_t bx, uint32_t by, uint32_t bz) {
   const float px0 = __fmul_rn((float)lo[0], j.u), px1 = __fmul_rn((float)(lo[0] + 1), j.u);
   const float py0 = __fmul_rn((float)lo[1], j.u), py1 = __fmul_rn((float)(lo[1] + 1), j.u);
   // XY over the four columns (x_i, y_j)
@@ -704,12 +751,22 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
     c10 &= !(__fadd_rn(__fadd_rn(a1, b0), s.dxy[k]) < 0.0f);
     c11 &= !(__fadd_rn(__fadd_rn(a1, b1), s.dxy[k]) < 0.0f);
   }
-  // n.x * p.x + n.y * p.y per column, and the halves of the YZ and ZX dot products
-  // that do not depend on z
+  // the plane value's parts per column (see walk_line), and the halves of the YZ and ZX dot
+  // products that do not depend on z
   const float n0x0 = __fmul_rn(s.n[0], px0), n0x1 = __fmul_rn(s.n[0], px1);
   const float n1y0 = __fmul_rn(s.n[1], py0), n1y1 = __fmul_rn(s.n[1], py1);
-  const float q00 = __fadd_rn(n0x0, n1y0), q01 = __fadd_rn(n0x0, n1y1), q10 = __fadd_rn(n0x1, n1y0),
-              q11 = __fadd_rn(n0x1, n1y1);
+  // w = z: (x + y) + z, q the sum of the first two; otherwise (z + q) + r
+  const bool z_last = W == 2;
+  float q00, q01, q10, q11, r00 = 0.0f, r01 = 0.0f, r10 = 0.0f, r11 = 0.0f;
+  if (z_last) {
+    q00 = __fadd_rn(n0x0, n1y0), q01 = __fadd_rn(n0x0, n1y1), q10 = __fadd_rn(n0x1, n1y0), q11 = __fadd_rn(n0x1, n1y1);
+  } else if (W == 0) {
+    q00 = n0x0, q01 = n0x0, q10 = n0x1, q11 = n0x1;
+    r00 = n1y0, r01 = n1y1, r10 = n1y0, r11 = n1y1;
+  } else {
+    q00 = n1y0, q01 = n1y1, q10 = n1y0, q11 = n1y1;
+    r00 = n0x0, r01 = n0x0, r10 = n0x1, r11 = n0x1;
+  }
   float yz_y0[3], yz_y1[3], zx_x0[3], zx_x1[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
@@ -718,11 +775,16 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
     zx_x0[k] = __fmul_rn(s.zx[k][1], px0);
     zx_x1[k] = __fmul_rn(s.zx[k][1], px1);
   }
-  constexpr uint32_t XBITS = 0x09249249u, YBITS = 0x12492492u, ZBITS = 0x24924924u;
-  const uint32_t mx0 = spread3_10((uint32_t)(lo[0] - j.sa[0])), mx1 = ((mx0 | ~XBITS) + 1u) & XBITS;
-  const uint32_t my0 = spread3_10((uint32_t)(lo[1] - j.sa[1])) << 1, my1 = ((my0 | ~YBITS) + 2u) & YBITS;
-  uint32_t mz = spread3_10((uint32_t)(lo[2] - j.sa[2])) << 2;
-  uint32_t cur_w = 0xffffffffu, acc = 0;
+  // Morton bits: the rotated axes' shifts are 0, 1, 2 turned by W
+  const uint32_t xs = W == 2 ? 0u : (W == 0 ? 1u : 2u), ys = W == 2 ? 1u : (W == 0 ? 2u : 0u), zs = (uint32_t)W;
+  const uint32_t XBITS = 0x09249249u << xs, YBITS = 0x09249249u << ys, ZBITS = 0x09249249u << zs;
+  const uint32_t mx0 = spread3_10(local[0]) << xs, mx1 = ((mx0 | ~XBITS) + (1u << xs)) & XBITS;
+  const uint32_t my0 = spread3_10(local[1]) << ys, my1 = ((my0 | ~YBITS) + (1u << ys)) & YBITS;
+  const uint32_t z1 = 1u << zs;
+  uint32_t mz = spread3_10(local[2]) << zs;
+  // bits in their leaf words, and whether x, y + 1 lie in another word
+  const uint32_t mxy = mx0 | my0;
+  const bool sx = ((mx0 ^ mx1) >> 5) != 0, sy = ((my0 ^ my1) >> 5) != 0;
   uint64_t mask = 0;
   for (uint32_t zc = 0; zc < bz; zc += 2) {
     const bool z1ok = zc + 1 < bz;
@@ -745,129 +807,130 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
     }
     // the plane test: (n.p + d1) (n.p + d2) > 0 fails
     const float g0 = __fmul_rn(s.n[2], pz0), g1 = __fmul_rn(s.n[2], pz1);
-    auto plane = [&](float q, float g) {
-      const float nd = __fadd_rn(q, g);
-      return !(__fmul_rn(__fadd_rn(nd, s.d1), __fadd_rn(nd, s.d2)) > 0.0f);
+    float v000 = __fadd_rn(g0, q00), v001 = __fadd_rn(g1, q00), v010 = __fadd_rn(g0, q01), v011 = __fadd_rn(g1, q01);
+    float v100 = __fadd_rn(g0, q10), v101 = __fadd_rn(g1, q10), v110 = __fadd_rn(g0, q11), v111 = __fadd_rn(g1, q11);
+    if (!z_last) {
+      v000 = __fadd_rn(v000, r00), v001 = __fadd_rn(v001, r00), v010 = __fadd_rn(v010, r01), v011 = __fadd_rn(v011, r01);
+      v100 = __fadd_rn(v100, r10), v101 = __fadd_rn(v101, r10), v110 = __fadd_rn(v110, r11), v111 = __fadd_rn(v111, r11);
+    }
+    auto plane = [&](float nd) { return !(__fmul_rn(__fadd_rn(nd, s.d1), __fadd_rn(nd, s.d2)) > 0.0f); };
+    const bool p000 = c00 & y0z0 & z0x0 & plane(v000), p001 = c00 & y0z1 & z1x0 & plane(v001);
+    const bool p010 = c01 & y1z0 & z0x0 & plane(v010), p011 = c01 & y1z1 & z1x0 & plane(v011);
+    const bool p100 = c10 & y0z0 & z0x1 & plane(v100), p101 = c10 & y0z1 & z1x1 & plane(v101);
+    const bool p110 = c11 & y1z0 & z0x1 & plane(v110), p111 = c11 & y1z1 & z1x1 & plane(v111);
+    const uint32_t mz1 = ((mz | ~ZBITS) + z1) & ZBITS;
+    if (j.item_mask) {  // payload: two bits per column
+      const uint32_t c00b = (p000 ? 1u : 0u) | (p001 ? 2u : 0u), c01b = (p010 ? 1u : 0u) | (p011 ? 2u : 0u);
+      const uint32_t c10b = (p100 ? 1u : 0u) | (p101 ? 2u : 0u), c11b = (p110 ? 1u : 0u) | (p111 ? 2u : 0u);
+      uint64_t m = (uint64_t)c00b;
+      if (by > 1) m |= (uint64_t)c01b << bz;
+      if (bx > 1) m |= (uint64_t)c10b << (by * bz);
+      if (bx > 1 && by > 1) m |= (uint64_t)c11b << ((by + 1) * bz);
+      mask |= m << zc;
+    }
+    // The eight voxels' bits, merged along every axis whose + 1 stays in the word: one store per
+    // leaf word the brick touches (one to eight), the same slot in every lane.
+    const bool sz = ((mz ^ mz1) >> 5) != 0;
+    auto bit = [&](bool p, uint32_t m) { return p ? 1u << (m & 31u) : 0u; };
+    uint32_t b000 = bit(p000, mxy | mz), b001 = bit(p001, mxy | mz1);
+    uint32_t b010 = bit(p010, mx0 | my1 | mz), b011 = bit(p011, mx0 | my1 | mz1);
+    uint32_t b100 = bit(p100, mx1 | my0 | mz), b101 = bit(p101, mx1 | my0 | mz1);
+    uint32_t b110 = bit(p110, mx1 | my1 | mz), b111 = bit(p111, mx1 | my1 | mz1);
+    auto merge = [](bool apart, uint32_t& a, uint32_t& b) {
+      if (!apart) {
+        a |= b;
+        b = 0;
+      }
     };
-    const bool p000 = c00 & y0z0 & z0x0 & plane(q00, g0), p001 = c00 & y0z1 & z1x0 & plane(q00, g1);
-    const bool p010 = c01 & y1z0 & z0x0 & plane(q01, g0), p011 = c01 & y1z1 & z1x0 & plane(q01, g1);
-    const bool p100 = c10 & y0z0 & z0x1 & plane(q10, g0), p101 = c10 & y0z1 & z1x1 & plane(q10, g1);
-    const bool p110 = c11 & y1z0 & z0x1 & plane(q11, g0), p111 = c11 & y1z1 & z1x1 & plane(q11, g1);
-    const uint32_t mz1 = ((mz | ~ZBITS) + 4u) & ZBITS;
-    mask |= bit_if(p000, zc) | bit_if(p001, zc + 1) | bit_if(p010, bz + zc) | bit_if(p011, bz + zc + 1) |
-            bit_if(p100, by * bz + zc) | bit_if(p101, by * bz + zc + 1) | bit_if(p110, (by + 1) * bz + zc) |
-            bit_if(p111, (by + 1) * bz + zc + 1);
-    leaf_bit(j, p000, mx0 | my0 | mz, cur_w, acc);
-    leaf_bit(j, p001, mx0 | my0 | mz1, cur_w, acc);
-    leaf_bit(j, p010, mx0 | my1 | mz, cur_w, acc);
-    leaf_bit(j, p011, mx0 | my1 | mz1, cur_w, acc);
-    leaf_bit(j, p100, mx1 | my0 | mz, cur_w, acc);
-    leaf_bit(j, p101, mx1 | my0 | mz1, cur_w, acc);
-    leaf_bit(j, p110, mx1 | my1 | mz, cur_w, acc);
-    leaf_bit(j, p111, mx1 | my1 | mz1, cur_w, acc);
-    mz = ((mz1 | ~ZBITS) + 4u) & ZBITS;
+    merge(sz, b000, b001), merge(sz, b010, b011), merge(sz, b100, b101), merge(sz, b110, b111);
+    merge(sy, b000, b010), merge(sy, b001, b011), merge(sy, b100, b110), merge(sy, b101, b111);
+    merge(sx, b000, b100), merge(sx, b001, b101), merge(sx, b010, b110), merge(sx, b011, b111);
+    if (b000) set_leaf(j, (mxy | mz) >> 5, b000);
+    if (b001) set_leaf(j, (mxy | mz1) >> 5, b001);
+    if (b010) set_leaf(j, (mx0 | my1 | mz) >> 5, b010);
+    if (b100) set_leaf(j, (mx1 | my0 | mz) >> 5, b100);
+    if (b011 | b101 | b110 | b111) {
+      if (b011) set_leaf(j, (mx0 | my1 | mz1) >> 5, b011);
+      if (b101) set_leaf(j, (mx1 | my0 | mz1) >> 5, b101);
+      if (b110) set_leaf(j, (mx1 | my1 | mz) >> 5, b110);
+      if (b111) set_leaf(j, (mx1 | my1 | mz1) >> 5, b111);
+    }
+    mz = ((mz1 | ~ZBITS) + z1) & ZBITS;
   }
-  if (acc) set_leaf(j, cur_w, acc);
   return mask;
 }
 
-// Other small boxes (at most 64 voxels): the YZ verdicts over (y, z) and the
-// ZX verdicts over (z, x) as bit masks first, then per column the XY test and
-// per candidate the plane test.
-__device__ __forceinline__ uint64_t vox_small_factored(const VoxJob& j, const TriSetup& s, const int lo[3],
-                                                       uint32_t bx, uint32_t by, uint32_t bz) {
-  uint64_t yzm = 0;  // bit iy * bz + iz
-  for (uint32_t iy = 0; iy < by; iy++) {
-    const float py = __fmul_rn((float)(lo[1] + (int)iy), j.u);
-    const float a0 = __fmul_rn(s.yz[0][0], py), a1 = __fmul_rn(s.yz[1][0], py), a2 = __fmul_rn(s.yz[2][0], py);
-    for (uint32_t iz = 0; iz < bz; iz++) {
-      const float pz = __fmul_rn((float)(lo[2] + (int)iz), j.u);
-      const bool ok = !(__fadd_rn(__fadd_rn(a0, __fmul_rn(s.yz[0][1], pz)), s.dyz[0]) < 0.0f) &
-                      !(__fadd_rn(__fadd_rn(a1, __fmul_rn(s.yz[1][1], pz)), s.dyz[1]) < 0.0f) &
-                      !(__fadd_rn(__fadd_rn(a2, __fmul_rn(s.yz[2][1], pz)), s.dyz[2]) < 0.0f);
-      yzm |= bit_if(ok, iy * bz + iz);
-    }
-  }
-  uint64_t zxm = 0;  // bit ix * bz + iz
-  for (uint32_t ix = 0; ix < bx; ix++) {
-    const float px = __fmul_rn((float)(lo[0] + (int)ix), j.u);
-    const float b0 = __fmul_rn(s.zx[0][1], px), b1 = __fmul_rn(s.zx[1][1], px), b2 = __fmul_rn(s.zx[2][1], px);
-    for (uint32_t iz = 0; iz < bz; iz++) {
-      const float pz = __fmul_rn((float)(lo[2] + (int)iz), j.u);
-      const bool ok = !(__fadd_rn(__fadd_rn(__fmul_rn(s.zx[0][0], pz), b0), s.dzx[0]) < 0.0f) &
-                      !(__fadd_rn(__fadd_rn(__fmul_rn(s.zx[1][0], pz), b1), s.dzx[1]) < 0.0f) &
-                      !(__fadd_rn(__fadd_rn(__fmul_rn(s.zx[2][0], pz), b2), s.dzx[2]) < 0.0f);
-      zxm |= bit_if(ok, ix * bz + iz);
-    }
-  }
-  constexpr uint32_t XBITS = 0x09249249u, YBITS = 0x12492492u, ZBITS = 0x24924924u;
-  const uint32_t mz0 = spread3_10((uint32_t)(lo[2] - j.sa[2])) << 2;
-  const uint32_t my0 = spread3_10((uint32_t)(lo[1] - j.sa[1])) << 1;
-  uint32_t mx = spread3_10((uint32_t)(lo[0] - j.sa[0]));
-  const uint64_t zfull = bz >= 64 ? ~0ull : ((1ull << bz) - 1);
-  uint32_t cur_w = 0xffffffffu, acc = 0;
-  uint64_t mask = 0;
-  for (uint32_t ix = 0; ix < bx; ix++, mx = ((mx | ~XBITS) + 1u) & XBITS) {
-    const float px = __fmul_rn((float)(lo[0] + (int)ix), j.u);
-    const float n0px = __fmul_rn(s.n[0], px);
-    const uint64_t zx_col = (zxm >> ((ix * bz) & 63u)) & zfull;
-    uint32_t my = my0;
-    for (uint32_t iy = 0; iy < by; iy++, my = ((my | ~YBITS) + 2u) & YBITS) {
-      const uint64_t zb = zx_col & (yzm >> ((iy * bz) & 63u));
-      if (!zb) continue;
-      const float py = __fmul_rn((float)(lo[1] + (int)iy), j.u);
-      if (!pass_xy(s, px, py)) continue;
-      const float nxy = __fadd_rn(n0px, __fmul_rn(s.n[1], py));
-      const uint32_t mxy = mx | my;
-      const uint32_t cbase = (ix * by + iy) * bz;
-      uint32_t mz = mz0;
-      for (uint32_t iz = 0; iz < bz; iz++, mz = ((mz | ~ZBITS) + 4u) & ZBITS) {
-        if (!((zb >> iz) & 1u)) continue;
-        const float pz = __fmul_rn((float)(lo[2] + (int)iz), j.u);
-        const float nd = __fadd_rn(nxy, __fmul_rn(s.n[2], pz));
-        if (__fmul_rn(__fadd_rn(nd, s.d1), __fadd_rn(nd, s.d2)) > 0.0f) continue;
-        leaf_bit(j, true, mxy | mz, cur_w, acc);
-        mask |= 1ull << (cbase + iz);
-      }
-    }
-  }
-  if (acc) set_leaf(j, cur_w, acc);
-  return mask;
+// The grid box of an item and what the pass does with it.
+struct ItemBox {
+  int lo[3];
+  uint32_t b[3];  // extents
+  int W;          // small: the walk axis
+};
+enum ItemKind { ITEM_NONE = 0, ITEM_SMALL = 1, ITEM_LARGE = 2 };
+
+__device__ __forceinline__ ItemKind classify(const VoxJob& j, const TriVerts& tv, ItemBox& box, uint32_t& lines) {
+  int hi[3];
+  lines = 0;
+  if (!item_box(j, tv, box.lo, hi)) return ITEM_NONE;
+#pragma unroll
+  for (int a = 0; a < 3; a++) box.b[a] = (uint32_t)(hi[a] - box.lo[a] + 1);
+  const uint32_t b0 = box.b[0], b1 = box.b[1], b2 = box.b[2];
+  box.W = b2 >= b0 && b2 >= b1 ? 2 : (b0 >= b1 ? 0 : 1);
+  const uint32_t narrow = box.W == 2 ? max(b0, b1) : (box.W == 0 ? max(b1, b2) : max(b0, b2));
+  // extents are at most a stripe's 1024: the product fits 32 bits
+  if (narrow <= 2 && b0 * b1 * b2 <= j.small_vol) return ITEM_SMALL;
+  lines = (uint32_t)item_lines(walk_axis(tv), box.lo, hi);
+  return ITEM_LARGE;
 }
 
-// Pass 0, one thread per item: items with at most small_vol (<= 64) candidates
-// are voxelized here and leave their pass mask; returns the lines of a larger one.
-__device__ __forceinline__ uint32_t vox_small_occ_item(const VoxJob& j, uint64_t i, const TriVerts& tv) {
-  int lo[3], hi[3];
-  uint32_t lines = 0;
-  uint64_t mask = 0;
-  if (item_box(j, tv, lo, hi)) {
-    const uint32_t bx = (uint32_t)(hi[0] - lo[0] + 1), by = (uint32_t)(hi[1] - lo[1] + 1),
-                   bz = (uint32_t)(hi[2] - lo[2] + 1);
-    // extents are at most a stripe's 1024: the product fits 64 bits
-    if ((uint64_t)bx * by * bz <= j.small_vol) {
-      TriSetup s;
-      tri_setup(tv, j.u, s);
-      mask = (bx <= 2 && by <= 2) ? vox_small_bricks(j, s, lo, bx, by, bz) : vox_small_factored(j, s, lo, bx, by, bz);
-      if (j.item_mask && mask) {
-        // stripe-local box origin (10 bits per axis) and extents - 1 (6 bits each)
-        j.item_box[i] = (uint64_t)(lo[0] - j.sa[0]) | ((uint64_t)(lo[1] - j.sa[1]) << 10) |
-                        ((uint64_t)(lo[2] - j.sa[2]) << 20) | ((uint64_t)(bx - 1) << 30) | ((uint64_t)(by - 1) << 36) |
-                        ((uint64_t)(bz - 1) << 42);
-      }
-    } else {
-      lines = (uint32_t)item_lines(walk_axis(tv), lo, hi);
-    }
+// Voxelizes small item i; payload jobs get its pass mask and box.
+__device__ __forceinline__ void vox_small_item(const VoxJob& j, uint64_t i, const TriVerts& tv, const ItemBox& box) {
+  const int W = box.W;
+  TriVerts t = tv;
+  int lo[3] = {box.lo[0], box.lo[1], box.lo[2]};
+  uint32_t b[3] = {box.b[0], box.b[1], box.b[2]};
+  uint32_t local[3] = {(uint32_t)(lo[0] - j.sa[0]), (uint32_t)(lo[1] - j.sa[1]), (uint32_t)(lo[2] - j.sa[2])};
+  if (W != 2) {  // (a, b, w) = (y, z, x) or (z, x, y)
+    auto turn = [&](auto& x, auto& y, auto& z) {
+      const auto x0 = x, y0 = y, z0 = z;
+      x = W == 0 ? y0 : z0;
+      y = W == 0 ? z0 : x0;
+      z = W == 0 ? x0 : y0;
+    };
+#pragma unroll
+    for (int k = 0; k < 3; k++) turn(t.v[k][0], t.v[k][1], t.v[k][2]);
+    turn(lo[0], lo[1], lo[2]);
+    turn(b[0], b[1], b[2]);
+    turn(local[0], local[1], local[2]);
   }
-  if (j.item_mask) j.item_mask[i] = mask;
-  return lines;
+  TriSetup s;
+  tri_setup_rotated(t, j.u, W, s);
+  const uint64_t mask = vox_small_bricks(j, s, W, lo, local, b[0], b[1], b[2]);
+  if (j.item_mask) {
+    j.item_mask[i] = mask;
+    // Morton code of the box origin, extents along b (1 or 2) and w, walk axis
+    if (mask)
+      j.item_box[i] = (uint64_t)morton_local((uint32_t)(box.lo[0] - j.sa[0]), (uint32_t)(box.lo[1] - j.sa[1]),
+                                             (uint32_t)(box.lo[2] - j.sa[2])) |
+                      ((uint64_t)b[1] << 32) | ((uint64_t)b[2] << 34) | ((uint64_t)W << 41);
+  }
 }
 
-// Item i of job j (any i: past the last item nothing is done) by every lane of the warp.
+// Pass 0 for item i of job j (any i: past the last item nothing is done), one thread per item, by
+// every thread of the warp or (CTA) of the CTA.
+template <bool CTA>
 __device__ __forceinline__ void vox_small_occ(const VoxJob& j, uint64_t i) {
   uint32_t lines = 0;
-  if (i < j.n_items) lines = vox_small_occ_item(j, i, load_verts(j.tris, item_triangle(j, i), j.stride));
-  append_large(j, i, lines);
+  ItemKind kind = ITEM_NONE;
+  ItemBox box;
+  TriVerts tv;
+  if (i < j.n_items) {
+    tv = load_verts(j.tris, item_triangle(j, i), j.stride);
+    kind = classify(j, tv, box, lines);
+    if (kind != ITEM_SMALL && j.item_mask) j.item_mask[i] = 0;
+  }
+  if (kind == ITEM_SMALL) vox_small_item(j, i, tv, box);
+  append_large<CTA>(j, i, lines);  // last: its barrier then waits for little
 }
 
 // Pass 1 for small items: rank the voxels their pass mask names.
@@ -876,17 +939,22 @@ __device__ __forceinline__ void vox_small_win_item(const VoxJob& j, uint64_t i) 
   if (!mask) return;
   const uint32_t t = (uint32_t)item_triangle(j, i);
   const uint64_t box = j.item_box[i];
-  const uint32_t lx = (uint32_t)box & 1023u, ly = (uint32_t)(box >> 10) & 1023u, lz = (uint32_t)(box >> 20) & 1023u;
-  const uint32_t by = (uint32_t)(box >> 36 & 63u) + 1u, bz = (uint32_t)(box >> 42 & 63u) + 1u;
-  // q / d for q < 64, d <= 64 as (q * ceil(2^16 / d)) >> 16: the error of the rounded-up
-  // reciprocal adds less than q / 2^16 < 1/d, which never carries past the next integer
-  const uint32_t rz = (65535u + bz) / bz, ry = (65535u + by) / by;
+  const uint32_t m0 = (uint32_t)box & 0x3fffffffu;  // Morton code of the box origin
+  const uint32_t by = (uint32_t)(box >> 32) & 3u, bz = (uint32_t)(box >> 34) & 127u;
+  const uint32_t W = (uint32_t)(box >> 41) & 3u;  // the axes are turned so that it comes last (z below)
+  const uint32_t xs = W == 2 ? 0u : (W == 0 ? 1u : 2u), ys = W == 2 ? 1u : (W == 0 ? 2u : 0u);
+  const uint32_t XB = 0x09249249u << xs, YB = 0x09249249u << ys, ZB = 0x09249249u << W;
+  const uint32_t mx1 = ((m0 | ~XB) + (1u << xs)) & XB, my1 = ((m0 | ~YB) + (1u << ys)) & YB;
   while (mask) {
     const uint32_t q = (uint32_t)(__ffsll((long long)mask) - 1);
     mask &= mask - 1;
-    const uint32_t col = (q * rz) >> 16, z = q - col * bz;
-    const uint32_t x = (col * ry) >> 16, y = col - x * by;
-    const uint32_t m = morton_local(lx + x, ly + y, lz + z);
+    const uint32_t col = (q >= bz ? 1u : 0u) + (q >= 2u * bz ? 1u : 0u) + (q >= 3u * bz ? 1u : 0u);
+    uint32_t z = q - col * bz;  // below 64, its bits spread
+    z = (z | (z << 8)) & 0x300fu;
+    z = (z | (z << 4)) & 0x30c3u;
+    z = (z | (z << 2)) & 0x9249u;
+    const bool x = by == 2 ? col >= 2 : col != 0, y = by == 2 && (col & 1u);
+    const uint32_t m = (x ? mx1 : m0 & XB) | (y ? my1 : m0 & YB) | (((m0 | ~ZB) + (z << W)) & ZB);
     offer(j, m, t);
   }
 }
@@ -1064,14 +1132,29 @@ __global__ void k_scatter_to(const uint64_t* __restrict__ src, uint64_t n, int w
 // A one-stripe launch (SINGLE) takes the stripe's job as a kernel parameter
 // and indexes elements directly; a batch launch finds its stripe first and
 // stages the job in shared memory.
-template <int PASS, bool SINGLE>
-__global__ void __launch_bounds__(kChunk, 4) kb_vox_small(const VoxJob* __restrict__ jobs,
+template <bool SINGLE>
+__global__ void __launch_bounds__(kChunk, 3) kb_vox_occ(const VoxJob* __restrict__ jobs,
                                                        const uint64_t* __restrict__ cta_beg, uint32_t n, VoxJob j0) {
   pdl_enter();
   if constexpr (SINGLE) {
+    vox_small_occ<true>(j0, (uint64_t)blockIdx.x * kChunk + threadIdx.x);
+  } else {
+    __shared__ VoxJob sj;
+    uint64_t cta;
+    const uint32_t s = cta_stripe(cta_beg, n, cta);
+    stage(sj, jobs[s]);
+    __syncthreads();
+    vox_small_occ<true>(sj, cta * kChunk + threadIdx.x);
+  }
+}
+
+template <bool SINGLE>
+__global__ void __launch_bounds__(kChunk) kb_vox_win(const VoxJob* __restrict__ jobs, const uint64_t* __restrict__ cta_beg,
+                                                     uint32_t n, VoxJob j0) {
+  pdl_enter();
+  if constexpr (SINGLE) {
     const uint64_t i = (uint64_t)blockIdx.x * kChunk + threadIdx.x;
-    if (PASS == 0) vox_small_occ(j0, i);
-    else if (i < j0.n_items) vox_small_win_item(j0, i);
+    if (i < j0.n_items) vox_small_win_item(j0, i);
   } else {
     __shared__ VoxJob sj;
     uint64_t cta;
@@ -1079,8 +1162,7 @@ __global__ void __launch_bounds__(kChunk, 4) kb_vox_small(const VoxJob* __restri
     stage(sj, jobs[s]);
     __syncthreads();
     const uint64_t i = cta * kChunk + threadIdx.x;
-    if (PASS == 0) vox_small_occ(sj, i);
-    else if (i < sj.n_items) vox_small_win_item(sj, i);
+    if (i < sj.n_items) vox_small_win_item(sj, i);
   }
 }
 
@@ -1174,7 +1256,7 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
     for (uint32_t q = 0; q < kPersistChunkRounds; q++) {
       const uint64_t i0 = c0 + 32u * q;
       if (i0 >= s_job[w].n_items) break;
-      vox_small_occ(s_job[w], i0 + (uint64_t)lane);
+      vox_small_occ<false>(s_job[w], i0 + (uint64_t)lane);
     }
     // this chunk's listed items are visible before it counts as done
     __threadfence();
@@ -1264,7 +1346,7 @@ cudaError_t launch_vox_small_occupancy(const VoxJob& j, cudaStream_t st) {
   uint32_t n = 1;
   VoxJob arg = j;
   void* args[] = {&jobs, &cta_beg, &n, &arg};
-  return cudaLaunchKernel(reinterpret_cast<const void*>(&kb_vox_small<0, true>), dim3(grid_for(j.n_items, kChunk)),
+  return cudaLaunchKernel(reinterpret_cast<const void*>(&kb_vox_occ<true>), dim3(grid_for(j.n_items, kChunk)),
                           dim3(kChunk), args, 0, st);
 }
 
@@ -1299,13 +1381,8 @@ void launch_b_vox_small(const VoxJob* jobs, const uint64_t* cta_beg, uint32_t n,
   VoxJob j0;
   std::memset(&j0, 0, sizeof(j0));
   if (single) j0 = *single;
-  if (pass == 0) {
-    if (single) launch_k(kb_vox_small<0, true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, jobs, cta_beg, n, j0);
-    else launch_k(kb_vox_small<0, false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, jobs, cta_beg, n, j0);
-  } else {
-    if (single) launch_k(kb_vox_small<1, true>, dim3((unsigned)ctas), dim3(kChunk), 0, st, jobs, cta_beg, n, j0);
-    else launch_k(kb_vox_small<1, false>, dim3((unsigned)ctas), dim3(kChunk), 0, st, jobs, cta_beg, n, j0);
-  }
+  auto* kern = pass == 0 ? (single ? kb_vox_occ<true> : kb_vox_occ<false>) : (single ? kb_vox_win<true> : kb_vox_win<false>);
+  launch_k(kern, dim3((unsigned)ctas), dim3(kChunk), 0, st, jobs, cta_beg, n, j0);
 }
 
 void launch_b_vox_large(const VoxJob* jobs, const LargeLists& lists, int pass, const VoxJob* single, cudaStream_t st,
