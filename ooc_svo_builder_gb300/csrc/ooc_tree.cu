@@ -248,14 +248,17 @@ __device__ __forceinline__ uint32_t parent_word(const uint32_t w[8]) {
   return p;
 }
 
-// One CTA per stripe: the prefixes of level U, then the levels above it, each
-// thread on eight words.  Latency-bound (a few dependent block scans); levels of
-// 256 words and fewer are left to the first warp, which needs no block barrier.
-template <int T>
+// One CTA per stripe: the prefixes of level U, then the levels above it.  A warp takes
+// 32 K consecutive words of level U, a lane words 32 apart, so loads and stores are whole
+// lines (a thread on eight words in a row stored 4 bytes to a sector at a time: 20 us for
+// 8,192 words, now 9).  Latency-bound; the levels above have at most 1,024 words and sit in
+// shared memory, eight words to a thread, and those of 256 and fewer are left to the first
+// warp, which needs no block barrier.
+template <int T, int K>
 __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes, uint32_t* __restrict__ counts,
                                               const unsigned long long* __restrict__ large_ctr,
-                                              uint64_t* __restrict__ large_out,
-                                              const uint64_t* __restrict__ code, uint64_t* __restrict__ code_out) {
+                                              uint64_t* __restrict__ large_out, const uint64_t* __restrict__ code,
+                                              uint64_t* __restrict__ code_out) {
   pdl_enter();
   __shared__ Stripe sp;
   __shared__ uint32_t s_words[2][1024];
@@ -266,60 +269,76 @@ __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes
     if (code) *code_out = *code;
   }
   uint32_t* out = counts + (uint64_t)blockIdx.x * kCountWords;
-  const int U = sp.U;
+  const int U = sp.U, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t W = upper_words(U), off = upper_off(U);
   uint32_t carry_r = 0, carry_l = 0, carry_i = 0;
-  for (uint32_t base = 0; base < W; base += T * 8u) {
-    const uint32_t i0 = base + threadIdx.x * 8u;
-    uint32_t w[8], r = 0;
-    uint2 li[8];
-    uint32_t sl = 0, si = 0;
-    if (i0 + 8u <= W) {
-      const uint4* q = reinterpret_cast<const uint4*>(sp.ubits + off + i0);
-      const uint4 q0 = q[0], q1 = q[1];
-      w[0] = q0.x, w[1] = q0.y, w[2] = q0.z, w[3] = q0.w, w[4] = q1.x, w[5] = q1.y, w[6] = q1.z, w[7] = q1.w;
-      const uint4* v = reinterpret_cast<const uint4*>(sp.wpre + i0);
+  for (uint32_t base = 0; base < W; base += T * K) {
+    const uint32_t i0 = base + (uint32_t)warp * (32u * K) + (uint32_t)lane;
+    uint32_t w[K], r[K];
+    uint2 li[K];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const uint4 t = v[k];
-        li[2 * k] = make_uint2(t.x, t.y);
-        li[2 * k + 1] = make_uint2(t.z, t.w);
-      }
-    } else {
+    for (int k = 0; k < K; k++) {
+      const uint32_t i = i0 + 32u * k;
+      w[k] = i < W ? sp.ubits[off + i] : 0u;
+      li[k] = i < W ? sp.wpre[i] : make_uint2(0u, 0u);
+      r[k] = __popc(w[k]);
+    }
+    // exclusive within the warp's words: the 3 K scans side by side
+#pragma unroll 1
+    for (int d = 1; d < 32; d <<= 1) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        w[k] = i0 + k < W ? sp.ubits[off + i0 + k] : 0u;
-        li[k] = i0 + k < W ? sp.wpre[i0 + k] : make_uint2(0u, 0u);
+      for (int k = 0; k < K; k++) {
+        const uint32_t ur = __shfl_up_sync(FULL, r[k], d), ul = __shfl_up_sync(FULL, li[k].x, d),
+                       ui = __shfl_up_sync(FULL, li[k].y, d);
+        if (lane >= d) r[k] += ur, li[k].x += ul, li[k].y += ui;
       }
     }
+    uint32_t sum_r = 0, sum_l = 0, sum_i = 0;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      r += __popc(w[k]);
-      sl += li[k].x;
-      si += li[k].y;
+    for (int k = 0; k < K; k++) {
+      const uint32_t tr = __shfl_sync(FULL, r[k], 31), tl = __shfl_sync(FULL, li[k].x, 31),
+                     ti = __shfl_sync(FULL, li[k].y, 31);
+      const uint32_t er = __shfl_up_sync(FULL, r[k], 1), el = __shfl_up_sync(FULL, li[k].x, 1),
+                     ei = __shfl_up_sync(FULL, li[k].y, 1);
+      r[k] = sum_r + (lane ? er : 0u);
+      li[k] = make_uint2(sum_l + (lane ? el : 0u), sum_i + (lane ? ei : 0u));
+      sum_r += tr;
+      sum_l += tl;
+      sum_i += ti;
     }
-    unsigned long long tot;
-    uint32_t tot_r;
-    const unsigned long long ex = block_exclusive<unsigned long long>((unsigned long long)sl | ((unsigned long long)si << 32), tot);
-    uint32_t run_r = carry_r + block_exclusive<uint32_t>(r, tot_r);
-    uint32_t run_l = carry_l + (uint32_t)ex, run_i = carry_i + (uint32_t)(ex >> 32);
+    // across the warps
+    __shared__ uint32_t s_sum[3][33];
+    if (lane == 0) s_sum[0][warp] = sum_r, s_sum[1][warp] = sum_l, s_sum[2][warp] = sum_i;
+    __syncthreads();
+    if (warp < 3) {
+      const uint32_t v = lane < T / 32 ? s_sum[warp][lane] : 0u, inc = warp_inclusive(v);
+      s_sum[warp][lane] = inc - v;
+      if (lane == 31) s_sum[warp][32] = inc;
+    }
+    __syncthreads();
+    const uint32_t br = carry_r + s_sum[0][warp], bl = carry_l + s_sum[1][warp], bi = carry_i + s_sum[2][warp];
 #pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (i0 + k < W) {
-        sp.upre[off + i0 + k] = run_r;
-        sp.wpre[i0 + k] = make_uint2(run_l, run_i);
-        run_r += __popc(w[k]);
-        run_l += li[k].x;
-        run_i += li[k].y;
+    for (int k = 0; k < K; k++) {
+      const uint32_t i = i0 + 32u * k;
+      if (i < W) {
+        sp.upre[off + i] = br + r[k];
+        sp.wpre[i] = make_uint2(bl + li[k].x, bi + li[k].y);
       }
-    if (U > 0 && i0 < W) {
-      const uint32_t pw = parent_word(w);
-      sp.ubits[upper_off(U - 1) + i0 / 8u] = pw;
-      s_words[(U - 1) & 1][i0 / 8u] = pw;
+      if (U > 0) {  // eight words' parent word: four bits each
+        uint32_t pw = nonzero_bytes(w[k]) << (4 * (lane & 7));
+        pw |= __shfl_xor_sync(FULL, pw, 1);
+        pw |= __shfl_xor_sync(FULL, pw, 2);
+        pw |= __shfl_xor_sync(FULL, pw, 4);
+        if ((lane & 7) == 0 && i < W) {
+          sp.ubits[upper_off(U - 1) + i / 8u] = pw;
+          s_words[(U - 1) & 1][i / 8u] = pw;
+        }
+      }
     }
-    carry_r += tot_r;
-    carry_l += (uint32_t)tot;
-    carry_i += (uint32_t)(tot >> 32);
+    carry_r += s_sum[0][32];
+    carry_l += s_sum[1][32];
+    carry_i += s_sum[2][32];
+    __syncthreads();
   }
   if (threadIdx.x == 0) {  // the entries past the end
     sp.ubits[off + W] = 0u;
@@ -1301,8 +1320,13 @@ void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* 
   KScope k("upper", st);
   // 128 threads cover level 4's 128 words at eight a thread with room for smaller CTAs to share an SM;
   // larger stripes have 1,024 and 8,192 words to scan
-  if (max_upper >= 5) launch_k(kb_upper<1024>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
-  else launch_k(kb_upper<128>, dim3(n), dim3(128), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
+  // level U has 8192, 1024, 128, ... words: one round of one word a thread, or eight
+  if (max_upper >= 6)
+    launch_k(kb_upper<1024, 8>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
+  else if (max_upper == 5)
+    launch_k(kb_upper<1024, 1>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
+  else
+    launch_k(kb_upper<128, 1>, dim3(n), dim3(128), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
 }
 
 void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
