@@ -1046,9 +1046,16 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hr_dev), hr, 0), "mapped root info");
   hr[(uint64_t)n * 16] = 0;  // the layout check flag: the record kernels set it, in host memory
   auto bricks_of = [&](uint32_t s) -> uint64_t { return lvl[(uint64_t)s * kCountWords + 2 + stripe[s].U]; };  // non-empty
-  uint64_t total_bricks = 0;
+  uint64_t total_bricks = 0, total_records = 0;
   for (uint32_t s = 0; s < n; s++)
-    if (!pl[s].empty) total_bricks += bricks_of(s);
+    if (!pl[s].empty) total_bricks += bricks_of(s), total_records += pl[s].total;
+  // A warp's share of the emission, in records: as long as the SMs (24 warps each) get 2.7 rounds of
+  // warps about 1,024 to 4,096, as long as they get 8 up to 8,192.  Fewer repeat the warp's search
+  // and set-up more often, more leave SMs idle behind the last warps: at 1,024, 2,048, 4,096 and
+  // 8,192 the 4M soup at gridsize 1024 takes 725, 662, 637, 650 us, 128 meshes 719, 633, 573, 545 and
+  // 300k triangles at 2048 (8.6M records) 272, 307, 303, 303.
+  const uint64_t per_sm = total_records / c->num_sms;
+  const uint64_t share = std::clamp<uint64_t>(std::max(std::min<uint64_t>(per_sm / 64, 4096), per_sm / 192), 1024, 8192);
   std::vector<EmitJob> ej(n);
   for (uint32_t s = 0; s < n; s++) {
     const MeshWork& m = meshes[sb[s].mesh];
@@ -1094,10 +1101,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       e.data_win_len = q.data_span;
     }
     e.n_leaf = q.n_leaf;
-    // A warp's share: about 1,024 records, as long as 48 warps per SM have one.  Fewer repeat the
-    // warp's search and set-up more often; more leave SMs idle behind the warps of dense bricks.
+    // as long as 48 warps per SM have one
     e.bricks_per_warp = (uint32_t)std::max<uint64_t>(
-        1, std::min(q.total ? 1024 * bricks_of(s) / q.total : 1, total_bricks / ((uint64_t)c->num_sms * 48)));
+        1, std::min(q.total ? share * bricks_of(s) / q.total : 1, total_bricks / ((uint64_t)c->num_sms * 48)));
     if (!m.pl.binary) {
       e.winners = winners + leaf_at[s];
       vj[s].winners = winners + leaf_at[s];

@@ -105,10 +105,10 @@ struct VoxJob {
   uint64_t* item_box;       // per small item with a non-zero mask: its packed stripe-local box
 };
 
-// The default of ooc_tuning::small_vol.  Occupancy passes, small + large, in us at 64, 32, 16 and 8
-// candidates: 20k-triangle sphere at gridsize 256 49, 43, 34, 28; 4M soup at 1024 1731, 1534, 1515, 1516;
-// batch of 128 meshes 1271, 1146, 1083, 1083; heightfield of 2M triangles at 1024 94, 94, 93, 109 (its
-// boxes of 2 x 2 x 3 fit 12 voxels: the line walk is no match for the one-thread pass there).
+// The default of ooc_tuning::small_vol.  Occupancy passes, small + large, in us at 8, 12, 16 and 32
+// candidates: heightfield of 2M triangles at gridsize 1024 113, 100, 94, 95 (its boxes of 2 x 2 x 3 fit
+// 12 voxels: the line walk is no match for the one-thread pass there); 4M soup at 1024 1278, 1265, 1258,
+// 1260; batch of 128 meshes 984, 970, 972, 978; 20k-triangle sphere at 256 26 to 27 for all.
 constexpr uint32_t kSmallVol = 16;
 
 // Counters of the large items' list, each on its own 128-byte line; all zero when pass 0 starts.

@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kTreeThreads) kb_leaf_payload(const Stripe* __
 // ===========================================================================
 // Emission: the records of every brick's run and the brick's own.
 //
-// A warp takes consecutive non-empty bricks of the stripe and lays them out in
+// A warp takes consecutive non-empty bricks of the stripe, 32 at a time, and lays them out in
 // steps of eight units (a unit: 512 leaf bits, a child of a brick), four lanes to
 // a unit, whichever bricks the units belong to, so a step is full on sparse bricks
 // too.  A lane holds 128 leaf bits: two nodes of 64 (a run of their leaves and
@@ -609,17 +609,18 @@ __global__ void __launch_bounds__(kTreeThreads) kb_leaf_payload(const Stripe* __
 // the warp a few instructions (records stored by the lanes themselves took 2.2 times
 // as long on the 20M-triangle soup at gridsize 4096).
 //
-// Bound by latency and issue: about 800 warp instructions per step, DRAM at a
-// third of its rate.  The 20M-triangle soup (651M records, 15.6 GB) takes 6.8 ms;
-// the passes this replaced (keys, subtree sizes bottom-up, positions top-down and
-// leaf records, each over arrays of every node) took 19 ms.  On the 1024^3
-// heightfield it is 41 us instead of 190.
+// Bound by issue and latency on sparse bricks, by DRAM writes on dense ones.  The 20M-triangle soup at
+// gridsize 4096 (651M records, 15.6 GB) takes 4.8 ms, 3.2 TB/s; 4M triangles at 1024 (2.9 GB) 0.49 ms, 5.9
+// TB/s; the 1024^3 heightfield 33 us.  Taking the bricks word by word instead of 32 non-empty ones at a
+// time, loading a step's leaf words in the step, filling the window with a pattern worked out per word and
+// windows of 128 records on four CTAs per SM took 6.8, 0.73 and 0.043 ms; passes over arrays of every node
+// (keys, subtree sizes bottom-up, positions top-down, leaf records) 19 ms for the first.
 // ===========================================================================
 // A window holds kWindow records and a gap of up to two slots between the records of eight bricks.
-// CTAs per SM: three (no spills) took 10% longer on the large soups and 10% less on the heightfield,
-// where a warp has one or two bricks; five is within 2% of four.
-constexpr int kEmitCtas = 4;
-constexpr uint32_t kWindow = 128;
+// Three CTAs per SM with windows of 288, and four with 160 (all that shared memory holds): 489 and 541 us
+// on the 4M soup, 248 and 244 on 300k triangles with payload, 31 and 37 on the heightfield.
+constexpr int kEmitCtas = 3;
+constexpr uint32_t kWindow = 288;
 constexpr uint32_t kSlots = kWindow + 16;
 
 // A lane's words as the warp's lanes read them when they share out the step's parents of leaves.
@@ -634,6 +635,7 @@ struct __align__(16) WarpScratch {
   uint64_t win[kSlots * 3];
   LaneWords words[32];
   uint32_t gaps[8];
+  uint16_t units[256];  // of the word's bricks: brick | place in it << 5 | number in it << 8
 };
 
 // Bit position of the t-th (from 0) set bit of the 8-bit mask m.
@@ -715,35 +717,37 @@ __device__ __forceinline__ void average_records(const EmitJob& e, uint32_t n, Su
   s.average(n);
 }
 
-// What the layout of word w's bricks needs from memory, lane = brick.  Loaded before the
-// previous word is laid out: the marks come from DRAM, and the word's first use of them would
-// otherwise wait for two loads in a row.
-struct WordIn {
-  uint32_t bits;        // the word
-  uint2 wp, wn, bp;     // leaves and inner nodes before the word, before the next, and before the brick in the word
+// What the layout of up to 32 bricks, consecutive among the non-empty ones, needs from memory, lane =
+// brick.  Loaded before the bricks ahead of them are laid out: the marks come from DRAM, and the
+// first use of them would otherwise wait for several loads in a row.
+struct BrickIn {
+  uint32_t x;        // the brick (lanes below the number of bricks)
+  uint32_t bits;     // the non-empty bricks from its parent's first child on
+  uint2 pre;         // leaves and inner nodes before it
+  uint2 end;         // the same of the first brick past the last lane's (lane 0) and past its parent's (lane 1)
   uint32_t units;
   uint4 marks;
-  uint32_t up, upd;     // upper nodes recorded before the brick's parent's children; averaged before the brick (-levels)
+  uint32_t up, upd;  // upper nodes recorded before the brick's parent's children; averaged before the brick (-levels)
 };
 
 template <bool LEVELS>
-__device__ __forceinline__ WordIn load_word(const Stripe& p, uint32_t w, int lane) {
-  WordIn in;
+__device__ __forceinline__ BrickIn load_bricks(const Stripe& p, uint32_t x, uint32_t n, int lane) {
+  BrickIn in;
   const int U = p.U;
-  const uint32_t x = w * 32u + (uint32_t)lane, off = upper_off(U) + w;
-  in.bits = p.ubits[off];
-  const bool have = (in.bits >> lane) & 1u;
-  in.wp = p.wpre[w];
-  in.wn = p.wpre[w + 1];
-  in.bp = p.bpre[x];
+  const uint32_t off = upper_off(U) + (x >> 5), last = __shfl_sync(FULL, x, (int)n - 1);
+  const bool have = (uint32_t)lane < n;
+  in.x = x;
   in.units = have ? p.bunits[x] : 0u;
   in.marks = make_uint4(~0u, ~0u, ~0u, ~0u);
   if (have && p.touch) in.marks = reinterpret_cast<const uint4*>(p.touch)[x];
+  const uint32_t bits = p.ubits[off];
+  const uint2 wp = p.wpre[x >> 5], bp = p.bpre[x];
+  in.end = brick_prefix(p, lane == 0 ? last + 1u : (last | 7u) + 1u);
+  in.bits = bits >> (x & 24u);
+  in.pre = make_uint2(wp.x + bp.x, wp.y + bp.y);
   in.up = in.upd = 0;
   if (U) {
     const uint32_t pre = p.upre[off];
-    in.up = pre + __popc(in.bits & ((1u << (lane & ~7)) - 1u));
-    if (LEVELS) in.upd = pre + __popc(in.bits & ((1u << lane) - 1u));
 #pragma unroll
     for (int l = 1; l < kMaxUpper; l++)
       if (l < U) {
@@ -752,36 +756,42 @@ __device__ __forceinline__ WordIn load_word(const Stripe& p, uint32_t w, int lan
         in.up += ur + __popc(ub & ((1u << (anc & 24u)) - 1u));  // before its parent's children: whole bytes
         if (LEVELS) in.upd += ur + __popc(ub & ((1u << (anc & 31u)) - 1u));
       }
+    in.up += pre + __popc(bits & ((1u << (x & 24u)) - 1u));
+    if (LEVELS) in.upd += pre + __popc(bits & ((1u << (x & 31u)) - 1u));
   }
   return in;
 }
 
-// The bricks `rem` of word w.
+// n bricks (1 to 32).
 template <bool LEVELS>
-__device__ __forceinline__ void emit_word(const Stripe& p, const EmitJob& e, uint32_t w, uint32_t rem, const WordIn& in,
-                                          int lane, WarpScratch& sm, const uint64_t* __restrict__ lut) {
+__device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, uint32_t n, const BrickIn& in, int lane,
+                                            WarpScratch& sm, const uint64_t* __restrict__ lut) {
   const uint32_t le = (2u << lane) - 1u, lt = le >> 1;
   const int K = p.K, U = p.U;
   const bool pay = !e.binary;
   uint64_t* const nodes = e.node_win - (int64_t)(e.node_win_base - e.node_base) * 3;  // the stripe's records
   const uint64_t dbase = e.data_base;
   // ---- lane = brick x ----
-  const uint32_t x = w * 32u + (uint32_t)lane;
-  bool mine = (rem >> lane) & 1u;
-  const uint2 wn = in.wn;
-  const uint32_t lpre = in.wp.x + in.bp.x, ipre = in.wp.y + in.bp.y;
+  const uint32_t x = in.x;
+  bool mine = (uint32_t)lane < n;
+  const uint32_t lpre = in.pre.x, ipre = in.pre.y;
   uint32_t units = mine && K ? in.units : 0u;
   // leaf blocks that may have a bit
   const uint32_t blocks = nonzero_bytes(in.marks.x) | (nonzero_bytes(in.marks.y) << 4) | (nonzero_bytes(in.marks.z) << 8) |
                           (nonzero_bytes(in.marks.w) << 12);
   const uint32_t up = in.up, upd = in.upd;
-  const uint32_t sib = __popc((in.bits >> (lane & ~7)) & ((1u << (lane & 7)) - 1u));
+  const uint32_t sib = __popc(in.bits & ((1u << (x & 7u)) - 1u));
   const uint32_t start = up + lpre + ipre;  // stripe-relative, like all positions here
-  uint32_t nl = __shfl_down_sync(FULL, lpre, 1), ni = __shfl_down_sync(FULL, ipre, 1);  // before the next brick
-  const uint32_t pend = ((uint32_t)lane | 7u) + 1u;                                      // the parent's end
+  // before the next brick: the next lane's, or past the last's
+  uint32_t nl = __shfl_down_sync(FULL, lpre, 1), ni = __shfl_down_sync(FULL, ipre, 1);
+  const uint32_t pend = (uint32_t)lane - sib + (uint32_t)__popc(in.bits & 0xffu);  // the lane past its parent's children
   uint32_t pl = __shfl_sync(FULL, lpre, (int)(pend & 31u)), pi = __shfl_sync(FULL, ipre, (int)(pend & 31u));
-  if (lane == 31) nl = wn.x, ni = wn.y;
-  if (pend == 32u) pl = wn.x, pi = wn.y;
+  {
+    const uint32_t l0 = __shfl_sync(FULL, in.end.x, 0), i0 = __shfl_sync(FULL, in.end.y, 0);
+    const uint32_t l1 = __shfl_sync(FULL, in.end.x, 1), i1 = __shfl_sync(FULL, in.end.y, 1);
+    if ((uint32_t)lane + 1u >= n) nl = l0, ni = i0;
+    if (pend >= n) pl = l1, pi = i1;
+  }
   const uint32_t n3 = K == kBrickLevels ? __popc(units) : 0u;
   const uint32_t g3 = start + (nl - lpre) + (ni - ipre) - n3;  // where its children's group starts
   const uint32_t dpre = LEVELS ? (pay ? lpre : 0u) + ipre + upd : 0u;               // data records before its own
@@ -804,37 +814,46 @@ __device__ __forceinline__ void emit_word(const Stripe& p, const EmitJob& e, uin
   const uint32_t cnt = __popc(units);
   const uint32_t incl = warp_inclusive(cnt), excl = incl - cnt;
   const uint32_t total = __shfl_sync(FULL, incl, 31);
+  for (uint32_t m = units, k = 0; m; m &= m - 1, k++)
+    sm.units[excl + k] = (uint16_t)((uint32_t)lane | (((uint32_t)__ffs(m) - 1u) << 5) | (k << 8));
+  __syncwarp();
   uint32_t carry = 0;          // records | leaves << 16 of the last step's last brick so far
   uint32_t root_mask = units;  // of a one-brick stripe
   const uint32_t odd0 = (uint32_t)(reinterpret_cast<uintptr_t>(nodes) >> 3);
+  // A step's words, loaded while the step before is laid out: the lane's unit's entry of
+  // sm.units and its leaf words.
+  uint32_t un_next = 0, x_next = 0;
+  uint4 v_next = make_uint4(0u, 0u, 0u, 0u);
+  auto unit_word = [&](uint32_t xo, uint32_t un) {
+    return xo * 128u + ((un >> 5) & 7u) * 16u + (uint32_t)(lane & 3) * 4u;  // below 2^25
+  };
+  auto fetch = [&](uint32_t g) {
+    const uint32_t u = g + (uint32_t)(lane >> 2);
+    un_next = sm.units[min(u, total - 1u)];
+    const uint32_t o_blocks = __shfl_sync(FULL, blocks, (int)(un_next & 31u));
+    x_next = __shfl_sync(FULL, x, (int)(un_next & 31u));
+    const uint32_t word = unit_word(x_next, un_next);
+    v_next = make_uint4(0u, 0u, 0u, 0u);
+    if (u < total && ((o_blocks >> (((un_next >> 4) & 14u) + (uint32_t)((lane >> 1) & 1))) & 1u) &&
+        (K == kBrickLevels || word < leaf_words(p.depth)))
+      v_next = *reinterpret_cast<const uint4*>(p.leaf + word);
+  };
+  if (total) fetch(0);
   for (uint32_t g = 0; g < total; g += 8u) {
     // ---- four lanes = unit u ----
     const uint32_t u = g + (uint32_t)(lane >> 2);
     const bool valid = u < total;
-    uint32_t o = 0;  // its brick: the first lane with incl > u
-#pragma unroll
-    for (uint32_t st = 16; st; st >>= 1) {
-      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
-      if (t <= u) o += st;
-    }
-    const uint32_t o_first = __shfl_sync(FULL, excl, (int)o);
-    const uint32_t t3 = u - o_first;  // its number in the brick
-    const uint32_t q = select8(__shfl_sync(FULL, units, (int)o), t3) & 7u;
-    const uint32_t o_blocks = __shfl_sync(FULL, blocks, (int)o), o_start = __shfl_sync(FULL, start, (int)o);
+    const uint32_t un = un_next, xo = x_next;
+    const uint32_t o = un & 31u, q = (un >> 5) & 7u, t3 = un >> 8;  // its brick, place and number in the brick
+    const uint32_t o_first = u - t3;
+    const uint32_t o_start = __shfl_sync(FULL, start, (int)o);
     const uint32_t o_g3 = __shfl_sync(FULL, g3, (int)o);
     uint32_t o_lpre = 0, o_dpre = 0;
     if (!LEVELS && pay) o_lpre = __shfl_sync(FULL, lpre, (int)o);
     if (LEVELS) o_dpre = __shfl_sync(FULL, dpre, (int)o);
-    const uint32_t xo = w * 32u + o;
-    const uint32_t word = xo * 128u + q * 16u + (uint32_t)(lane & 3) * 4u;  // below 2^25
-    uint64_t a = 0, b = 0;
-    if (valid && ((o_blocks >> (2u * q + (uint32_t)((lane >> 1) & 1))) & 1u) && (K == kBrickLevels || word < leaf_words(p.depth))) {
-      uint4* src = reinterpret_cast<uint4*>(p.leaf + word);
-      const uint4 v = *src;
-      a = (uint64_t)v.x | ((uint64_t)v.y << 32);
-      b = (uint64_t)v.z | ((uint64_t)v.w << 32);
-      if (a | b) *src = make_uint4(0u, 0u, 0u, 0u);  // zero for the next build
-    }
+    const uint64_t a = (uint64_t)v_next.x | ((uint64_t)v_next.y << 32), b = (uint64_t)v_next.z | ((uint64_t)v_next.w << 32);
+    if (a | b) *reinterpret_cast<uint4*>(p.leaf + unit_word(xo, un)) = make_uint4(0u, 0u, 0u, 0u);  // zero for the next build
+    if (g + 8u < total) fetch(g + 8u);
     const uint32_t ca = __popcll(a), cb = __popcll(b);
     const uint32_t ma = K >= 2 ? nonzero_bytes64(a) : 0u, mb = K >= 2 ? nonzero_bytes64(b) : 0u;
     const uint32_t ka = __popc(ma), kb = __popc(mb), kc = ka + kb;
@@ -990,12 +1009,17 @@ __device__ __forceinline__ void emit_word(const Stripe& p, const EmitJob& e, uin
       uint64_t* const rec = sm.win;
       {  // every slot a leaf's record, two words at a time
         const uint32_t n4 = ((nrec + 2u * __popc(heads)) * 3u + 1u) / 2u;
-        uint32_t f = (2u * (uint32_t)lane) % 3u;  // the first word's place in its record; +64 words: one further
+        ulonglong2* const q = reinterpret_cast<ulonglong2*>(rec);
         const uint64_t lead = pay ? 0ull : 1ull;
-        for (uint32_t i = (uint32_t)lane; i < n4; i += 32u) {
-          reinterpret_cast<ulonglong2*>(rec)[i] =
-              make_ulonglong2(f == 0 ? lead : (f == 1 ? 0ull : ~0ull), f == 0 ? 0ull : (f == 1 ? ~0ull : lead));
-          f = f == 2 ? 0u : f + 1u;
+        // words 2 i and 2 i + 1 of the pattern lead, 0, ~0; 64 words on it is one word further
+        const uint32_t f = (2u * (uint32_t)lane) % 3u;
+        const ulonglong2 v0 = make_ulonglong2(f == 0 ? lead : (f == 1 ? 0ull : ~0ull), f == 0 ? 0ull : (f == 1 ? ~0ull : lead));
+        const ulonglong2 v1 = make_ulonglong2(f == 2 ? lead : (f == 0 ? 0ull : ~0ull), f == 2 ? 0ull : (f == 0 ? ~0ull : lead));
+        const ulonglong2 v2 = make_ulonglong2(f == 1 ? lead : (f == 2 ? 0ull : ~0ull), f == 1 ? 0ull : (f == 2 ? ~0ull : lead));
+        for (uint32_t i = (uint32_t)lane; i < n4; i += 96u) {
+          q[i] = v0;
+          if (i + 32u < n4) q[i + 32u] = v1;
+          if (i + 64u < n4) q[i + 64u] = v2;
         }
       }
       __syncwarp();
@@ -1107,38 +1131,62 @@ __device__ __forceinline__ void emit_word(const Stripe& p, const EmitJob& e, uin
 }
 
 // The bricks of the stripe's warp i: bricks_per_warp consecutive ones of its non-empty bricks.
+// The warp's share: non-empty bricks i * bricks_per_warp to the next warp's first.
 template <bool LEVELS>
 __device__ __forceinline__ void emit_warp(const Stripe& p, const EmitJob& e, uint64_t i, int lane, WarpScratch& sm,
                                           const uint64_t* __restrict__ lut) {
-  const uint32_t W = upper_words(p.U), off = upper_off(p.U), n = p.upre[off + W];
+  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t W = upper_words(p.U), off = upper_off(p.U), all = p.upre[off + W];
   const uint64_t r0 = i * e.bricks_per_warp;
-  if (r0 >= n) return;
-  uint32_t r = (uint32_t)r0;
-  const uint32_t r1 = (uint32_t)min((uint64_t)n, r0 + e.bricks_per_warp);
-  uint32_t w = warp_search(W, r, lane, [&](uint32_t i) { return p.upre[off + i]; });
-  WordIn in = load_word<LEVELS>(p, w, lane);
-  uint32_t rank = p.upre[off + w];  // of the word's first brick
-  for (;;) {
-    const uint32_t mine = rank + __popc(in.bits & ((1u << lane) - 1u));
-    const uint32_t rem = __ballot_sync(FULL, ((in.bits >> lane) & 1u) && mine >= r && mine < r1);
-    rank += __popc(in.bits);
-    uint32_t nw = w;
-    WordIn next = in;
-    const bool more = rank < r1;
-    if (more) {
-      for (nw = w + 1; nw < W; nw += 32u) {  // the next word with a brick: there is one
-        const uint32_t i = nw + (uint32_t)lane;
-        const uint32_t some = __ballot_sync(FULL, i < W && p.ubits[off + i] != 0u);
-        if (some) {
-          nw += (uint32_t)__ffs(some) - 1u;
+  if (r0 >= all) return;
+  uint32_t left = (uint32_t)min((uint64_t)all - r0, (uint64_t)e.bricks_per_warp);
+  // the word of the first, and the word's bricks from it on
+  uint32_t w = warp_search(W, (uint32_t)r0, lane, [&](uint32_t i) { return p.upre[off + i]; });
+  uint32_t first;
+  {
+    const uint32_t b = p.ubits[off + w], skip = (uint32_t)r0 - p.upre[off + w];
+    first = __ballot_sync(FULL, ((b >> lane) & 1u) && __popc(b & lt) >= skip);
+  }
+  // Lane k's brick: the k-th of the n next; w and first move past them.
+  uint32_t* const list = reinterpret_cast<uint32_t*>(sm.words);
+  auto next_bricks = [&](uint32_t n) {
+    uint32_t got = 0;
+    while (got < n && w < W) {
+      const uint32_t mine = w + (uint32_t)lane < W ? p.ubits[off + w + (uint32_t)lane] : 0u;
+      uint32_t some = __ballot_sync(FULL, (lane == 0 ? mine & first : mine) != 0u);
+      uint32_t to = w + 32u, to_first = ~0u;
+      while (some) {
+        const uint32_t k = (uint32_t)__ffs(some) - 1u;
+        some &= some - 1u;
+        const uint32_t b = __shfl_sync(FULL, mine, (int)k) & (k == 0 ? first : ~0u);
+        const uint32_t pos = got + __popc(b & lt);
+        const bool set = (b >> lane) & 1u;
+        if (set && pos < n) list[pos] = (w + k) * 32u + (uint32_t)lane;
+        got += __popc(b);
+        if (got >= n) {
+          to = w + k;
+          to_first = __ballot_sync(FULL, set && pos >= n);
           break;
         }
       }
-      if (nw < W) next = load_word<LEVELS>(p, nw, lane);
+      w = to;
+      first = to_first;
     }
-    emit_word<LEVELS>(p, e, w, rem, in, lane, sm, lut);
-    if (!more || nw >= W) break;
-    w = nw;
+    __syncwarp();
+    const uint32_t x = list[min((uint32_t)lane, n - 1u)];
+    __syncwarp();
+    return x;
+  };
+  uint32_t n = min(left, 32u);
+  BrickIn in = load_bricks<LEVELS>(p, next_bricks(n), n, lane);
+  for (;;) {
+    left -= n;
+    const uint32_t n_next = min(left, 32u);
+    BrickIn next = in;
+    if (n_next) next = load_bricks<LEVELS>(p, next_bricks(n_next), n_next, lane);
+    emit_bricks<LEVELS>(p, e, n, in, lane, sm, lut);
+    if (!n_next) break;
+    n = n_next;
     in = next;
   }
   bulk_wait_all();

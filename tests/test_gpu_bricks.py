@@ -31,3 +31,13 @@ def test_bricks(builder, N, payload, levels):
         d = octree.diff(got.tree, octree.Octree(N, nodes, data))
         assert not d, "\n".join(d)
         assert got.info["n_filled"] == info["n_filled"]
+
+
+@pytest.mark.parametrize("payload,levels", [(False, False), (True, False), (True, True)])
+def test_sparse_bricks(builder, payload, levels):
+    """Scattered points: a warp takes several groups of 32 bricks, each from many words, ending inside parents."""
+    at = np.random.default_rng(3).random((600000, 3), dtype=np.float32)
+    t = tri.pack(at, at, at, colors=[at, at, at] if payload else None)
+    got = builder.build(t, make_params(2048, 2048, geometry_only=not payload, levels=levels))
+    want = octree.Octree(2048, *pyoracle.build(t, 2048, 2048, levels=levels)[:2])
+    assert not octree.diff(got.tree, want)
