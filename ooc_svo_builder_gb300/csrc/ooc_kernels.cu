@@ -478,224 +478,14 @@ __device__ __forceinline__ void append_large(const VoxJob& j, uint64_t i, uint32
     j.large[at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
 }
 
-// A large item as the warp's lanes read it: the constants of the test arranged by the walk axis
-// w and the two across it, a and b (the first and second of the remaining axes).  Of the three
-// projections one depends on a and b only (the line's own test), one on a and w, one on b and w.
-// Sums of two products are commutative, so the arrangement changes no rounding.
-struct WalkItem {
-  float ea[3], eb[3], ed[3];     // line test: ea * a + eb * b + ed
-  float aw[3], af[3], ad[3];     // aw * w + af * a + ad
-  float bw[3], bf[3], bd[3];     // bw * w + bf * b + bd
-  float nw, na, nb, d1, d2;      // normal and plane offsets
-  float u, inv_dir;
-  int alo, blo, wlo, whi;        // clamped box
-  uint32_t local;                // stripe-local alo, blo, wlo, 10 bits each
-  uint32_t shape;                // lines along a (11 bits) | axis w << 11 | monotone << 13
-  uint32_t magic;                // floor(c / ea) = (c * magic) >> 32 for line numbers c < 2^20; 0: one line along a
-  uint32_t first;                // the first line of the task
-  uint32_t tri, stripe;
-  uint32_t pad;                  // 45 words: lanes reading different items hit different banks
-};
-static_assert(sizeof(WalkItem) == 45 * 4, "odd number of words");
-
-__device__ __forceinline__ void walk_setup(const VoxJob& j, const TriVerts& tv, uint64_t t, uint32_t stripe, uint32_t first,
-                                           int W, const int lo[3], const int hi[3], WalkItem& r) {
-  TriSetup s;
-  tri_setup(tv, j.u, s);
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    if (W == 2) {  // a = x, b = y
-      r.ea[k] = s.xy[k][0], r.eb[k] = s.xy[k][1], r.ed[k] = s.dxy[k];
-      r.aw[k] = s.zx[k][0], r.af[k] = s.zx[k][1], r.ad[k] = s.dzx[k];
-      r.bw[k] = s.yz[k][1], r.bf[k] = s.yz[k][0], r.bd[k] = s.dyz[k];
-    } else if (W == 0) {  // a = y, b = z
-      r.ea[k] = s.yz[k][0], r.eb[k] = s.yz[k][1], r.ed[k] = s.dyz[k];
-      r.aw[k] = s.xy[k][0], r.af[k] = s.xy[k][1], r.ad[k] = s.dxy[k];
-      r.bw[k] = s.zx[k][1], r.bf[k] = s.zx[k][0], r.bd[k] = s.dzx[k];
-    } else {  // a = x, b = z
-      r.ea[k] = s.zx[k][1], r.eb[k] = s.zx[k][0], r.ed[k] = s.dzx[k];
-      r.aw[k] = s.xy[k][1], r.af[k] = s.xy[k][0], r.ad[k] = s.dxy[k];
-      r.bw[k] = s.yz[k][0], r.bf[k] = s.yz[k][1], r.bd[k] = s.dyz[k];
-    }
-  }
-  r.nw = W == 0 ? s.n[0] : (W == 1 ? s.n[1] : s.n[2]);
-  r.na = W == 0 ? s.n[1] : s.n[0];
-  r.nb = W == 2 ? s.n[1] : s.n[2];
-  r.d1 = s.d1;
-  r.d2 = s.d2;
-  r.u = j.u;
-  r.inv_dir = 1.0f / (r.nw * j.u);
-  const int ia = W == 0 ? 1 : 0, ib = W == 2 ? 1 : 2;
-  r.alo = ia ? lo[1] : lo[0];
-  r.blo = ib == 1 ? lo[1] : lo[2];
-  r.wlo = W == 0 ? lo[0] : (W == 1 ? lo[1] : lo[2]);
-  r.whi = W == 0 ? hi[0] : (W == 1 ? hi[1] : hi[2]);
-  const int sa = ia ? j.sa[1] : j.sa[0], sb = ib == 1 ? j.sa[1] : j.sa[2], sw = W == 0 ? j.sa[0] : (W == 1 ? j.sa[1] : j.sa[2]);
-  r.local = (uint32_t)(r.alo - sa) | ((uint32_t)(r.blo - sb) << 10) | ((uint32_t)(r.wlo - sw) << 20);
-  const uint32_t ea = (uint32_t)((ia ? hi[1] : hi[0]) - r.alo + 1);
-  const int top = max(hi[0], max(hi[1], hi[2]));
-  const bool mono = monotone_setup(s, fabsf(__fmul_rn((float)(top + 1), j.u)));
-  r.shape = ea | ((uint32_t)W << 11) | (mono ? 1u << 13 : 0u);
-  // ceil(2^32 / ea): its excess adds less than c / 2^32 <= 2^-12 < 1 / ea to the quotient
-  r.magic = ea > 1 ? (uint32_t)(0xffffffffu / ea) + 1u : 0u;
-  r.first = first;
-  r.tri = (uint32_t)t;
-  r.stripe = stripe;
+// (x, y, z) -> (a, b, w): w the axis W, a and b the ones that follow it cyclically.
+template <typename T>
+__device__ __forceinline__ void turn(int W, T& x, T& y, T& z) {
+  const T x0 = x, y0 = y, z0 = z;
+  x = W == 2 ? x0 : (W == 0 ? y0 : z0);
+  y = W == 2 ? y0 : (W == 0 ? z0 : x0);
+  z = W == 2 ? z0 : (W == 0 ? x0 : y0);
 }
-
-// Line (ra, rb) of a large item: pass 0 sets its bits, pass 1 offers the triangle to every
-// voxel it passes.  The line's own projection has passed.
-template <int PASS>
-__device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, uint32_t ra, uint32_t rb) {
-  const float u = r.u, fa = __fmul_rn((float)(r.alo + (int)ra), u), fb = __fmul_rn((float)(r.blo + (int)rb), u);
-  const uint32_t shape = r.shape;
-  const int W = (int)(shape >> 11) & 3, w0 = r.wlo, w1 = r.whi;
-  // n.p in the reference's order, (x + y) + z: the walk axis is z (q1 = x + y first) or one of the
-  // first two.  Adding the 0 changes only the sign of a zero, which no test sees.
-  const float nw = r.nw, d1 = r.d1, d2 = r.d2, pa = __fmul_rn(r.na, fa), pb = __fmul_rn(r.nb, fb);
-  const float q1 = W == 2 ? __fadd_rn(pa, pb) : pa, q2 = W == 2 ? 0.0f : pb;
-  float aw[3], fA[3], ad[3], bw[3], fB[3], bd[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    aw[k] = r.aw[k], fA[k] = __fmul_rn(r.af[k], fa), ad[k] = r.ad[k];
-    bw[k] = r.bw[k], fB[k] = __fmul_rn(r.bf[k], fb), bd[k] = r.bd[k];
-  }
-  auto at = [&](int w) { return __fmul_rn((float)w, u); };
-  auto rest = [&](float fw) {  // the two projections that depend on the walk coordinate
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(aw[k], fw), fA[k]), ad[k]) < 0.0f);
-      ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(bw[k], fw), fB[k]), bd[k]) < 0.0f);
-    }
-    return ok;
-  };
-  const bool up_side = nw * u > 0.0f;  // the plane value grows with w
-  auto side = [&](float fw) {  // plane_side
-    const float v = __fadd_rn(__fadd_rn(__fmul_rn(nw, fw), q1), q2);
-    const float a = __fadd_rn(v, d1), b = __fadd_rn(v, d2);
-    if (!(__fmul_rn(a, b) > 0.0f)) return 0;
-    return (a > 0.0f) == up_side ? 1 : -1;
-  };
-  // stripe-local Morton bits: the fixed coordinates, and the walk coordinate moving by carries
-  const uint32_t la = (r.local & 1023u) + ra, lb = ((r.local >> 10) & 1023u) + rb, lw = r.local >> 20;
-  const uint32_t mab = (spread3_10(la) << (W == 0 ? 1 : 0)) | (spread3_10(lb) << (W == 2 ? 1 : 2));
-  const uint32_t wbits = 0x09249249u << W;
-  uint32_t cur_w = 0xffffffffu, acc = 0;
-  auto emit = [&](uint32_t mw) {
-    const uint32_t m = mab | mw;
-    if (PASS == 0) {
-      const uint32_t wd = m >> 5;
-      if (wd != cur_w) {
-        if (acc) set_leaf(j, cur_w, acc);
-        cur_w = wd;
-        acc = 0;
-      }
-      acc |= 1u << (m & 31);
-    } else {
-      offer(j, m, r.tri);  // pass 0 set this voxel's bit
-    }
-  };
-  if (!((shape >> 13) & 1u)) {  // every voxel of the line, complete test
-    uint32_t mw = spread3_10(lw) << W;
-    for (int w = w0; w <= w1; w++, mw = ((mw | ~wbits) + (1u << W)) & wbits) {
-      const float fw = at(w);
-      if (side(fw) == 0 && rest(fw)) emit(mw);
-    }
-  } else {
-    // start where the plane crosses the line's middle, then find one voxel of the run
-    float west = -((pa + pb) + 0.5f * (d1 + d2)) * r.inv_dir;
-    west = fminf(fmaxf(west, (float)w0), (float)w1);  // NaN becomes w0
-    int start = (int)west, walk = 0;                   // walk: +1 up only, -1 down only, 0 both ways
-    const int g0 = side(at(start));
-    if (g0 < 0) {  // the run lies above: first w with side >= 0
-      int lo = start, hi = -1, step = 1;
-      for (;;) {
-        const int nx = min(lo + step, w1);
-        if (side(at(nx)) >= 0) {
-          hi = nx;
-          break;
-        }
-        if (nx == w1) return;
-        lo = nx;
-        step <<= 1;
-      }
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (side(at(mid)) >= 0) hi = mid;
-        else lo = mid;
-      }
-      if (side(at(hi)) != 0) return;  // the run falls between two voxels
-      start = hi;
-      walk = 1;
-    } else if (g0 > 0) {  // below: last w with side <= 0
-      int hi = start, lo = -1, step = 1;
-      for (;;) {
-        const int nx = max(hi - step, w0);
-        if (side(at(nx)) <= 0) {
-          lo = nx;
-          break;
-        }
-        if (nx == w0) return;
-        hi = nx;
-        step <<= 1;
-      }
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (side(at(mid)) <= 0) lo = mid;
-        else hi = mid;
-      }
-      if (side(at(lo)) != 0) return;
-      start = lo;
-      walk = -1;
-    }
-    const uint32_t ms = spread3_10(lw + (uint32_t)(start - w0)) << W;
-    if (rest(at(start))) emit(ms);
-    if (walk >= 0) {
-      uint32_t mw = ms;
-      for (int w = start + 1; w <= w1; w++) {
-        const float fw = at(w);
-        if (side(fw) != 0) break;
-        mw = ((mw | ~wbits) + (1u << W)) & wbits;
-        if (rest(fw)) emit(mw);
-      }
-    }
-    if (walk <= 0) {
-      uint32_t mw = ms;
-      for (int w = start - 1; w >= w0; w--) {
-        const float fw = at(w);
-        if (side(fw) != 0) break;
-        mw = (mw - (1u << W)) & wbits;
-        if (rest(fw)) emit(mw);
-      }
-    }
-  }
-  if (PASS == 0 && acc) set_leaf(j, cur_w, acc);
-}
-
-// ---------------------------------------------------------------------------
-// Small items: the candidate tests by projection.  Of the seven tests of a
-// candidate voxel (voxelizer.cpp:266-287) the three XY edge tests depend only
-// on (x, y), the YZ tests only on (y, z), the ZX tests only on (z, x); only the
-// plane test depends on all three.  Each is a pure function of its
-// coordinates, so evaluating it once per distinct projection and reusing the
-// result gives the reference's verdict for every candidate, bit for bit; the
-// FP32 expressions are the reference's, operation by operation.  A candidate
-// passes when all seven pass (the reference's order of early exits only saves
-// work).
-//
-// Small are the boxes of at most small_vol voxels that are at most two wide along two
-// axes; w is the third (the longest; z among equals), a and b are the ones that follow
-// it cyclically.  The edge tests are cyclic in (x, y, z), so with the coordinates rotated
-// to (a, b, w) they read the same for every w; the sums of three products keep the
-// reference's order (x + y) + z.  The pass mask of an item has bit (ia * bb + ib) * bw + iw.
-//
-// Bound by ALU instructions.  One body for every orientation, its voxels' bits merged into
-// one store per leaf word, took the pass from 86 to 90 us on a heightfield of 2M triangles,
-// where almost every box was already 2 x 2 x w, and from 485 to 246 us on 4M random
-// triangles and 282 to 173 us on 128 meshes (with append_large), where two boxes in three
-// were not and ran a voxel at a time.
-// ---------------------------------------------------------------------------
 
 // p[0..2] of the rotated axes (a, b, w), summed in the reference's order: w = z: a, b, w are
 // x, y, z; w = x: y, z, x; w = y: z, x, y.
@@ -731,6 +521,262 @@ __device__ __forceinline__ void tri_setup_rotated(const TriVerts& t, float u, in
   s.d2 = sum3(W, c2[0], c2[1], c2[2]);
   edge_setup(t, e, u, s);
 }
+
+// Two floats that go through one instruction, each with its own rounding.  A packed product whose only
+// use is a packed sum is contracted to an FMA, whatever the compiler's flags and the .rn say (measured:
+// the results differ), so a product that goes into a sum is an FMA itself, with -0 (which changes no
+// product, signed zeros included) that the compiler cannot know: nz = minus_zero of a run-time value.
+struct F2 {
+  uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {  // never into a sum
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b, F2 nz) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(nz.v));
+  return r;
+}
+__device__ __forceinline__ F2 minus_zero(float finite) {
+  const float z = __fmul_rn(fabsf(finite), -0.0f);
+  return f2(z, z);
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ void split(F2 a, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+
+// A large item as the warp's lanes read it, in words of 16 bytes: the constants of the test with the
+// coordinates turned so that the walk axis w comes last (the edge tests are cyclic in the axes, and sums
+// of two products commutative, so that changes no rounding).  Of the three projections (a, b) is the
+// line's own test, (a, w) and (b, w) go through the walk as pairs.
+struct __align__(16) WalkItem {
+  F2 ea, eb;                   // line test ea * a + eb * b + ed: of edges 0 and 1
+  F2 ed;
+  float ea2, eb2;              // and of edge 2
+  float ed2, u;
+  int alo, blo;                // clamped box
+  uint32_t shape;              // lines along a (11 bits) | axis w << 11 | monotone << 13
+  uint32_t magic;              // floor(c / ea) = (c * magic) >> 32 for line numbers c < 2^20; 0: one line along a
+  uint32_t first;              // the first line of the task, less the lines of the items before it
+  uint32_t tri;
+  F2 w[3], f[3], d[3];         // edge k on (a, w) and (b, w): w * (w, w) + f * (a, b) + d
+  F2 dd;                       // the plane's offsets d1, d2
+  float nw, na, nb, inv_dir;   // normal
+  int wlo, whi;
+  uint32_t local;              // stripe-local alo, blo, wlo, 10 bits each
+  uint32_t stripe;
+};
+static_assert(sizeof(WalkItem) == 44 * 4, "eight lanes that read 16 bytes of eight items in a row hit different banks");
+
+__device__ __forceinline__ void walk_setup(const VoxJob& j, const TriVerts& tv, uint64_t t, uint32_t stripe, uint32_t first,
+                                           int W, const int lo[3], const int hi[3], WalkItem& r) {
+  TriVerts v = tv;
+  int l[3] = {lo[0], lo[1], lo[2]}, h[3] = {hi[0], hi[1], hi[2]}, o[3] = {j.sa[0], j.sa[1], j.sa[2]};
+#pragma unroll
+  for (int k = 0; k < 3; k++) turn(W, v.v[k][0], v.v[k][1], v.v[k][2]);
+  turn(W, l[0], l[1], l[2]);
+  turn(W, h[0], h[1], h[2]);
+  turn(W, o[0], o[1], o[2]);
+  const float u = j.u;
+  TriSetup s;
+  tri_setup_rotated(v, u, W, s);
+  r.ea = f2(s.xy[0][0], s.xy[1][0]), r.eb = f2(s.xy[0][1], s.xy[1][1]), r.ed = f2(s.dxy[0], s.dxy[1]);
+  r.ea2 = s.xy[2][0], r.eb2 = s.xy[2][1], r.ed2 = s.dxy[2];
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    r.w[k] = f2(s.zx[k][0], s.yz[k][1]), r.f[k] = f2(s.zx[k][1], s.yz[k][0]), r.d[k] = f2(s.dzx[k], s.dyz[k]);
+  r.dd = f2(s.d1, s.d2);
+  r.nw = s.n[2], r.na = s.n[0], r.nb = s.n[1];
+  r.u = u;
+  r.inv_dir = 1.0f / (s.n[2] * u);
+  r.alo = l[0], r.blo = l[1], r.wlo = l[2], r.whi = h[2];
+  r.local = (uint32_t)(l[0] - o[0]) | ((uint32_t)(l[1] - o[1]) << 10) | ((uint32_t)(l[2] - o[2]) << 20);
+  const uint32_t ea = (uint32_t)(h[0] - l[0] + 1);
+  const int top = max(hi[0], max(hi[1], hi[2]));
+  const bool mono = monotone_setup(s, fabsf(__fmul_rn((float)(top + 1), u)));
+  r.shape = ea | ((uint32_t)W << 11) | (mono ? 1u << 13 : 0u);
+  // ceil(2^32 / ea): its excess adds less than c / 2^32 <= 2^-12 < 1 / ea to the quotient
+  r.magic = ea > 1 ? (uint32_t)(0xffffffffu / ea) + 1u : 0u;
+  r.first = first;
+  r.tri = (uint32_t)t;
+  r.stripe = stripe;
+}
+
+// Line (ra, rb) of a large item: pass 0 sets its bits, pass 1 offers the triangle to every
+// voxel it passes.  The line's own projection has passed.
+template <int PASS>
+__device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, uint32_t ra, uint32_t rb) {
+  const float u = r.u, fa = __fmul_rn((float)(r.alo + (int)ra), u), fb = __fmul_rn((float)(r.blo + (int)rb), u);
+  const uint32_t shape = r.shape;
+  const int W = (int)(shape >> 11) & 3, w0 = r.wlo, w1 = r.whi;
+  // n.p in the reference's order, (x + y) + z: with w = z a + b first, with w = x (w + a) + b, with w = y
+  // (w + b) + a.  Adding the 0 changes only the sign of a zero, which no test sees.
+  const float nw = r.nw, pa = __fmul_rn(r.na, fa), pb = __fmul_rn(r.nb, fb);
+  const float q1 = W == 2 ? __fadd_rn(pa, pb) : (W == 0 ? pa : pb), q2 = W == 2 ? 0.0f : (W == 0 ? pb : pa);
+  const F2 dd = r.dd, fab = f2(fa, fb), nz = minus_zero(u);  // u: the unit length, finite
+  F2 cw[3], cf[3], cd[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) cw[k] = r.w[k], cf[k] = mul2(r.f[k], fab, nz), cd[k] = r.d[k];
+  auto at = [&](int w) { return __fmul_rn((float)w, u); };
+  auto rest = [&](float fw) {  // the two projections that depend on the walk coordinate; a NaN passes
+    const F2 ww = f2(fw, fw);
+    float m[6];
+#pragma unroll
+    for (int k = 0; k < 3; k++) split(add2(add2(mul2(cw[k], ww, nz), cf[k]), cd[k]), m[2 * k], m[2 * k + 1]);
+    return !(fminf(fminf(fminf(m[0], m[1]), fminf(m[2], m[3])), fminf(m[4], m[5])) < 0.0f);
+  };
+  const bool up_side = nw * u > 0.0f;  // the plane value grows with w
+  auto side = [&](float fw) {  // plane_side
+    const float v = __fadd_rn(__fadd_rn(__fmul_rn(nw, fw), q1), q2);
+    float a, b;
+    split(add2(f2(v, v), dd), a, b);
+    if (!(__fmul_rn(a, b) > 0.0f)) return 0;
+    return (a > 0.0f) == up_side ? 1 : -1;
+  };
+  // stripe-local Morton bits: the fixed coordinates, and the walk coordinate moving by carries
+  const uint32_t la = (r.local & 1023u) + ra, lb = ((r.local >> 10) & 1023u) + rb, lw = r.local >> 20;
+  const uint32_t mab = (spread3_10(la) << (W == 2 ? 0 : W + 1)) | (spread3_10(lb) << (W == 0 ? 2 : W - 1));
+  const uint32_t wbits = 0x09249249u << W;
+  auto emit = [&](uint32_t mw) {
+    const uint32_t m = mab | mw;
+    if (PASS == 0) set_leaf(j, m >> 5, 1u << (m & 31u));
+    else offer(j, m, r.tri);  // pass 0 set this voxel's bit
+  };
+  if (!((shape >> 13) & 1u)) {  // every voxel of the line, complete test
+    uint32_t mw = spread3_10(lw) << W;
+    for (int w = w0; w <= w1; w++, mw = ((mw | ~wbits) + (1u << W)) & wbits) {
+      const float fw = at(w);
+      if (side(fw) == 0 && rest(fw)) emit(mw);
+    }
+    return;
+  }
+  // Start at the voxel nearest to the middle of the run, which is at least one voxel long: only a run
+  // that the box cuts off, or rounding, leaves it outside (rounding down instead did for every fourth
+  // line of random triangles).
+  float d1, d2;
+  split(dd, d1, d2);
+  float west = -((pa + pb) + 0.5f * (d1 + d2)) * r.inv_dir;
+  west = fminf(fmaxf(west, (float)w0), (float)w1);  // NaN becomes w0
+  int start = (int)(west + 0.5f), walk = 0;                   // walk: +1 up only, -1 down only, 0 both ways
+  const int g0 = side(at(start));
+  if (g0 < 0) {  // the run lies above: first w with side >= 0
+    int lo = start, hi = -1, step = 1;
+    for (;;) {
+      const int nx = min(lo + step, w1);
+      if (side(at(nx)) >= 0) {
+        hi = nx;
+        break;
+      }
+      if (nx == w1) return;
+      lo = nx;
+      step <<= 1;
+    }
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (side(at(mid)) >= 0) hi = mid;
+      else lo = mid;
+    }
+    if (side(at(hi)) != 0) return;  // the run falls between two voxels
+    start = hi;
+    walk = 1;
+  } else if (g0 > 0) {  // below: last w with side <= 0
+    int hi = start, lo = -1, step = 1;
+    for (;;) {
+      const int nx = max(hi - step, w0);
+      if (side(at(nx)) <= 0) {
+        lo = nx;
+        break;
+      }
+      if (nx == w0) return;
+      hi = nx;
+      step <<= 1;
+    }
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (side(at(mid)) <= 0) lo = mid;
+      else hi = mid;
+    }
+    if (side(at(lo)) != 0) return;
+    start = lo;
+    walk = -1;
+  }
+  // that voxel and its neighbours, whose plane tests go through as a pair
+  const float fs = at(start);
+  float fu, fd, pu, pd;
+  const F2 f_ud = mul2(f2((float)(start + 1), (float)(start - 1)), f2(u, u));
+  split(f_ud, fu, fd);
+  {
+    const F2 v = add2(add2(mul2(f2(nw, nw), f_ud, nz), f2(q1, q1)), f2(q2, q2));
+    split(mul2(add2(v, f2(d1, d1)), add2(v, f2(d2, d2))), pu, pd);
+  }
+  const bool up = walk >= 0 && start < w1 && !(pu > 0.0f), down = walk <= 0 && start > w0 && !(pd > 0.0f);
+  const uint32_t ms = spread3_10(lw + (uint32_t)(start - w0)) << W;
+  uint32_t mu = ((ms | ~wbits) + (1u << W)) & wbits, md = (ms - (1u << W)) & wbits;
+  const bool on_s = rest(fs), on_u = up & rest(fu), on_d = down & rest(fd);
+  if (PASS == 0) {  // one store per leaf word
+    const uint32_t m0 = mab | ms, m1 = mab | mu, m2 = mab | md;
+    uint32_t b0 = on_s ? 1u << (m0 & 31u) : 0u, b1 = on_u ? 1u << (m1 & 31u) : 0u, b2 = on_d ? 1u << (m2 & 31u) : 0u;
+    if (((m0 ^ m1) >> 5) == 0) b0 |= b1, b1 = 0;
+    if (((m0 ^ m2) >> 5) == 0) b0 |= b2, b2 = 0;
+    if (b0) set_leaf(j, m0 >> 5, b0);
+    if (b1) set_leaf(j, m1 >> 5, b1);
+    if (b2) set_leaf(j, m2 >> 5, b2);
+  } else {
+    if (on_s) emit(ms);
+    if (on_u) emit(mu);
+    if (on_d) emit(md);
+  }
+  if (up)
+    for (int w = start + 2; w <= w1; w++) {
+      const float fw = at(w);
+      if (side(fw) != 0) break;
+      mu = ((mu | ~wbits) + (1u << W)) & wbits;
+      if (rest(fw)) emit(mu);
+    }
+  if (down)
+    for (int w = start - 2; w >= w0; w--) {
+      const float fw = at(w);
+      if (side(fw) != 0) break;
+      md = (md - (1u << W)) & wbits;
+      if (rest(fw)) emit(md);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Small items: the candidate tests by projection.  Of the seven tests of a
+// candidate voxel (voxelizer.cpp:266-287) the three XY edge tests depend only
+// on (x, y), the YZ tests only on (y, z), the ZX tests only on (z, x); only the
+// plane test depends on all three.  Each is a pure function of its
+// coordinates, so evaluating it once per distinct projection and reusing the
+// result gives the reference's verdict for every candidate, bit for bit; the
+// FP32 expressions are the reference's, operation by operation.  A candidate
+// passes when all seven pass (the reference's order of early exits only saves
+// work).
+//
+// Small are the boxes of at most small_vol voxels that are at most two wide along two
+// axes; w is the third (the longest; z among equals), a and b are the ones that follow
+// it cyclically.  The edge tests are cyclic in (x, y, z), so with the coordinates rotated
+// to (a, b, w) they read the same for every w; the sums of three products keep the
+// reference's order (x + y) + z.  The pass mask of an item has bit (ia * bb + ib) * bw + iw.
+//
+// Bound by ALU instructions.  One body for every orientation, its voxels' bits merged into
+// one store per leaf word, took the pass from 86 to 90 us on a heightfield of 2M triangles,
+// where almost every box was already 2 x 2 x w, and from 485 to 246 us on 4M random
+// triangles and 282 to 173 us on 128 meshes (with append_large), where two boxes in three
+// were not and ran a voxel at a time.
+// ---------------------------------------------------------------------------
 
 // A small box: w is walked in 2 x 2 x 2 bricks, every test of a brick evaluated without
 // branches; slots outside the box are masked.  (In the rotated coordinates x, y, z below
@@ -890,18 +936,12 @@ __device__ __forceinline__ void vox_small_item(const VoxJob& j, uint64_t i, cons
   int lo[3] = {box.lo[0], box.lo[1], box.lo[2]};
   uint32_t b[3] = {box.b[0], box.b[1], box.b[2]};
   uint32_t local[3] = {(uint32_t)(lo[0] - j.sa[0]), (uint32_t)(lo[1] - j.sa[1]), (uint32_t)(lo[2] - j.sa[2])};
-  if (W != 2) {  // (a, b, w) = (y, z, x) or (z, x, y)
-    auto turn = [&](auto& x, auto& y, auto& z) {
-      const auto x0 = x, y0 = y, z0 = z;
-      x = W == 0 ? y0 : z0;
-      y = W == 0 ? z0 : x0;
-      z = W == 0 ? x0 : y0;
-    };
+  if (W != 2) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) turn(t.v[k][0], t.v[k][1], t.v[k][2]);
-    turn(lo[0], lo[1], lo[2]);
-    turn(b[0], b[1], b[2]);
-    turn(local[0], local[1], local[2]);
+    for (int k = 0; k < 3; k++) turn(W, t.v[k][0], t.v[k][1], t.v[k][2]);
+    turn(W, lo[0], lo[1], lo[2]);
+    turn(W, b[0], b[1], b[2]);
+    turn(W, local[0], local[1], local[2]);
   }
   TriSetup s;
   tri_setup_rotated(t, j.u, W, s);
@@ -967,10 +1007,13 @@ __device__ __forceinline__ void vox_small_win_item(const VoxJob& j, uint64_t i) 
 // pass go onto a stack from which 32 at a time are walked, one per lane.  So the lanes stay full
 // whatever the items' sizes.
 //
-// Bound by issue (no FMA).  Against one item per warp at a time: 8.8 -> 4.6 ms on the 20M-triangle
-// soup at gridsize 4096, 1.51 -> 0.89 ms on 4M triangles at gridsize 1024, and the list needs
-// neither a task count per item nor its scan (0.25 ms of the former).  Eight items a warp are 2 to
-// 4% slower, 32 (more shared memory) 7% slower on the batch of 128 meshes; 3 and 5 CTAs per SM 8% and 5%.
+// Bound by issue (no FMA), the walk three fifths of it, the lines' tests a quarter.  4.2 ms on the
+// 20M-triangle soup at gridsize 4096 (8.8 with one item per warp at a time), 0.81 (1.51) ms on 4M triangles
+// at 1024, 0.63 + 0.58 ms for the two passes of 128 meshes.  Of the rest a start at the voxel nearest the
+// run's middle, the voxel's neighbours tested as a pair, two projections per instruction, setting up the
+// turned triangle and finding a line's item with one reduction gave 5.3 -> 4.2, 1.01 -> 0.81 and 0.80 ->
+// 0.63.  Eight items a warp are 2 to 4% slower; 32 are 2% faster on the soups and 5 to 15% slower on the
+// smaller calls; 3 and 5 CTAs per SM 8% and 5% slower.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kWalkBits = 4, kWalkItems = 1u << kWalkBits;
 struct WalkScratch {
@@ -984,55 +1027,54 @@ template <int PASS, bool SINGLE>
 __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, const VoxJob& j0, bool has, uint32_t item,
                                            uint32_t stripe, uint32_t first, uint32_t most, uint32_t parts, int lane,
                                            WalkScratch& sm) {
-  const uint32_t lt = (1u << lane) - 1u;
+  const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u;
   uint32_t n = 0;
+  uint64_t t = 0;
+  TriVerts tv;
+  int lo[3], hi[3], W = 0;
   if (has) {
     const VoxJob& j = SINGLE ? j0 : jobs[stripe];
     if (PASS == 0 || j.winners) {  // (a binary stripe in a mixed batch has no winner pass)
-      const uint64_t t = item_triangle(j, item);
-      const TriVerts tv = load_verts(j.tris, t, j.stride);
-      int lo[3], hi[3];
+      t = item_triangle(j, item);
+      tv = load_verts(j.tris, t, j.stride);
       if (item_box(j, tv, lo, hi)) {  // as when it was listed
-        const int W = walk_axis(tv);
+        W = walk_axis(tv);
         const uint32_t lines = (uint32_t)item_lines(W, lo, hi);  // at most 1024^2 (a stripe's face)
         if (parts) {  // whole rounds of 32 lines
           most = (lines + 32u * parts - 1u) / (32u * parts) * 32u;
           first *= most;
         }
-        if (first < lines) {
-          n = min(most, lines - first);
-          walk_setup(j, tv, t, stripe, first, W, lo, hi, sm.item[lane]);
-        }
+        if (first < lines) n = min(most, lines - first);
       }
     }
   }
   const uint32_t incl = warp_inclusive(n), excl = incl - n, total = __shfl_sync(FULL, incl, 31);
+  const uint32_t with = __ballot_sync(FULL, n != 0);
+  if (n) walk_setup(SINGLE ? j0 : jobs[stripe], tv, t, stripe, first - excl, W, lo, hi, sm.item[__popc(with & lt)]);
   __syncwarp();
   auto walk = [&](uint32_t e) {
     const WalkItem& r = sm.item[e & (kWalkItems - 1u)];
     walk_line<PASS>(SINGLE ? j0 : jobs[r.stripe], r, (e >> kWalkBits) & 1023u, e >> (kWalkBits + 10));
   };
-  uint32_t cnt = 0;
+  uint32_t cnt = 0, begun = 0;  // lines on the stack; items that began in an earlier round
 #pragma unroll 1
   for (uint32_t r0 = 0; r0 < total; r0 += 32u) {
     const uint32_t i = r0 + (uint32_t)lane;
-    uint32_t o = 0;  // its item: the first lane with incl > i
-#pragma unroll
-    for (uint32_t st = 16; st; st >>= 1) {
-      const uint32_t t = __shfl_sync(FULL, incl, (int)(o + st - 1));
-      if (t <= i) o += st;
-    }
-    const uint32_t o_excl = __shfl_sync(FULL, excl, (int)o);
+    const uint32_t starts = __reduce_or_sync(FULL, n && excl - r0 < 32u ? 1u << (excl - r0) : 0u);
+    const uint32_t o = begun + __popc(starts & le) - 1u;
+    begun += __popc(starts);
     bool ok = i < total;
     uint32_t e = 0;
     if (ok) {
       const WalkItem& r = sm.item[o];
-      const uint32_t c = i - o_excl + r.first, ea = r.shape & 2047u;
+      const uint32_t c = i + r.first, ea = r.shape & 2047u;
       const uint32_t rb = r.magic ? __umulhi(c, r.magic) : c, ra = c - rb * ea;
       const float fa = __fmul_rn((float)(r.alo + (int)ra), r.u), fb = __fmul_rn((float)(r.blo + (int)rb), r.u);
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        ok &= !(__fadd_rn(__fadd_rn(__fmul_rn(r.ea[k], fa), __fmul_rn(r.eb[k], fb)), r.ed[k]) < 0.0f);
+      float t0, t1;
+      const F2 nz = minus_zero(r.u);
+      split(add2(add2(mul2(r.ea, f2(fa, fa), nz), mul2(r.eb, f2(fb, fb), nz)), r.ed), t0, t1);
+      const float t2 = __fadd_rn(__fadd_rn(__fmul_rn(r.ea2, fa), __fmul_rn(r.eb2, fb)), r.ed2);
+      ok = !(fminf(fminf(t0, t1), t2) < 0.0f);  // a NaN passes
       e = o | (ra << kWalkBits) | (rb << (kWalkBits + 10));
     }
     const uint32_t vote = __ballot_sync(FULL, ok);
@@ -1056,37 +1098,49 @@ __device__ __forceinline__ void walk_lists(const VoxJob* __restrict__ jobs, cons
                                            WalkScratch& sm) {
   const unsigned long long n = __ldcg(L.ctr + kCtrLarge), packed = __ldcg(L.ctr + kCtrBig);
   const uint32_t nb = min((uint32_t)(packed & ((1u << kBigCountBits) - 1u)), L.big_cap);
+  uint64_t tasks = 0;
   if (nb) {
     const uint4 end = __ldcg(L.big + nb - 1);
-    const uint64_t tasks = (uint64_t)end.z + end.w;
-    for (;;) {
-      unsigned long long t = 0;
-      if (lane == 0) t = atomicAdd(L.ctr + kCtrGrab + 32 * PASS, 1ull);
-      t = __shfl_sync(FULL, t, 0);
-      if (t >= tasks) break;
-      const uint32_t b = warp_search(nb, (uint32_t)t, lane, [&](uint32_t i) { return __ldcg(&L.big[i].z); });
-      const uint4 e = __ldcg(L.big + b);
-      const uint32_t k = (uint32_t)t - e.z;
-      if (k < e.w) walk_items<PASS, SINGLE>(jobs, j0, lane == 0, e.x, e.y, k * L.slice, L.slice, 0u, lane, sm);
-    }
+    tasks = (uint64_t)end.z + end.w;
   }
-  if (n == 0) return;
   // Fewer items than warps: several warps share an item (up to 16, one per round of its 512 lines), so
   // a handful of triangles takes one round and not sixteen (80 triangles at gridsize 64: 21 -> 10 us).  A
   // warp's first helping is its number.
   const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  const uint32_t parts = (uint32_t)min(16ull, max(1ull, warps / n));
+  const uint32_t parts = n ? (uint32_t)min(16ull, max(1ull, warps / n)) : 1u;
   const uint64_t total = n * parts;
   const uint32_t chunk = (uint32_t)min((unsigned long long)kWalkItems, n / (2 * warps) + 1);
   uint64_t t = (uint64_t)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * chunk;
-  while (t < total) {
-    const bool has = (uint32_t)lane < chunk && t + (uint32_t)lane < total;
-    const uint64_t i = (t + (uint32_t)lane) / parts;
-    const unsigned long long e = has ? __ldcg(L.large + i) : 0ull;
-    walk_items<PASS, SINGLE>(jobs, j0, has, (uint32_t)e, (uint32_t)(e >> 32), (uint32_t)(t + (uint32_t)lane - i * parts), ~0u,
-                             parts > 1 ? parts : 0u, lane, sm);
-    if (lane == 0) t = (uint64_t)warps * chunk + atomicAdd(L.ctr + kCtrGrab + 16 + 32 * PASS, (unsigned long long)chunk);
-    t = __shfl_sync(FULL, t, 0);
+  bool big = tasks != 0;
+#pragma unroll 1
+  for (;;) {
+    bool has;
+    uint32_t item, stripe, first, most = ~0u, ps = 0;
+    if (big) {
+      unsigned long long g = 0;
+      if (lane == 0) g = atomicAdd(L.ctr + kCtrGrab + 32 * PASS, 1ull);
+      g = __shfl_sync(FULL, g, 0);
+      if (g >= tasks) {
+        big = false;
+        continue;
+      }
+      const uint4 e = __ldcg(L.big + warp_search(nb, (uint32_t)g, lane, [&](uint32_t i) { return __ldcg(&L.big[i].z); }));
+      const uint32_t k = (uint32_t)g - e.z;
+      has = lane == 0 && k < e.w;
+      item = e.x, stripe = e.y, first = k * L.slice, most = L.slice;
+    } else {
+      if (t >= total) break;
+      has = (uint32_t)lane < chunk && t + (uint32_t)lane < total;
+      const uint64_t i = (t + (uint32_t)lane) / parts;
+      const unsigned long long e = has ? __ldcg(L.large + i) : 0ull;
+      item = (uint32_t)e, stripe = (uint32_t)(e >> 32), first = (uint32_t)(t + (uint32_t)lane - i * parts);
+      if (parts > 1) ps = parts;
+    }
+    walk_items<PASS, SINGLE>(jobs, j0, has, item, stripe, first, most, ps, lane, sm);
+    if (!big) {
+      if (lane == 0) t = (uint64_t)warps * chunk + atomicAdd(L.ctr + kCtrGrab + 16 + 32 * PASS, (unsigned long long)chunk);
+      t = __shfl_sync(FULL, t, 0);
+    }
   }
 }
 
