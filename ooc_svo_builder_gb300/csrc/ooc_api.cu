@@ -142,6 +142,8 @@ struct ooc_ctx {
   // double-buffered outputs of pipelined sub-batches
   DevBuf d_out_nodes[2], d_out_data[2];
   PinBuf h_root[2];
+  PinBuf h_flag;        // the layout check's flag: the record kernels set it, in host memory
+  bool unfinished = false;  // a build was begun and has not come to its end
   D2HRing ring[2][2];  // [slot][OOC_STREAM_NODES / OOC_STREAM_DATA]
   cudaEvent_t ev_compute[2] = {nullptr, nullptr};
   cudaEvent_t ev_data[2] = {nullptr, nullptr};  // host output: a sub-batch's data file is final
@@ -617,12 +619,16 @@ uint64_t pyramid_words(int Ds) {
   return w;
 }
 
-// CTA prefix of one batched launch: stripe s gets ceil(count(s) / per_cta) CTAs.
+// CTA prefix of one batched launch: stripe s gets ceil(count(s) / per_cta) CTAs, and extra(s) more.
+template <typename F, typename G>
+std::vector<uint64_t> cta_prefix(uint32_t n, uint64_t per_cta, F count, G extra) {
+  std::vector<uint64_t> beg(n + 1, 0);
+  for (uint32_t s = 0; s < n; s++) beg[s + 1] = beg[s] + (count(s) + per_cta - 1) / per_cta + extra(s);
+  return beg;
+}
 template <typename F>
 std::vector<uint64_t> cta_prefix(uint32_t n, uint64_t per_cta, F count) {
-  std::vector<uint64_t> beg(n + 1, 0);
-  for (uint32_t s = 0; s < n; s++) beg[s + 1] = beg[s] + (count(s) + per_cta - 1) / per_cta;
-  return beg;
+  return cta_prefix(n, per_cta, count, [](uint32_t) -> uint64_t { return 0; });
 }
 
 // A per-leaf launch: its CTA prefix and the leaves each thread takes.  A thread takes as many
@@ -714,6 +720,14 @@ void alloc_through(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, s
   for (; os.alloc_next <= idx; os.alloc_next++) ensure_dest(c, st, meshes[os.alloc_next], os);
 }
 
+constexpr uint32_t kRootWords = 8;  // of a stripe's root in h_root: its average (with -levels)
+
+// The record kernels that have finished found no index out of range.
+void check_layout_flag(ooc_ctx* c) {
+  const uint32_t flag = *static_cast<volatile const uint32_t*>(c->h_flag.p);
+  if (flag != 0) fail(OOC_ERR_DEVICE, "internal layout check failed (flag " + std::to_string(flag) + ")");
+}
+
 // A launched sub-batch whose records are still on their way to the host.
 struct Pending {
   bool active = false;
@@ -721,8 +735,9 @@ struct Pending {
   std::vector<StripeRef> sb;
   std::vector<Placed> pl;
   std::vector<int> depth;
+  std::vector<uint32_t> root_mask;  // the stripe roots' children
   // how far the hand-over has got (finish_sub_batch resumes from here)
-  bool checked = false;  // the sub-batch's kernels are done and its layout flag is clear
+  bool checked = false;  // the sub-batch's kernels are done, or nothing of them is needed to hand it over
   uint32_t at = 0;       // stripe being handed over
   int stage = 0;         // 0 not started, 1 node bytes, 2 data bytes
   uint64_t cur = 0;      // next byte of the current range
@@ -1041,10 +1056,10 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     ensure<uint64_t>(c->d_out_nodes[slot], out_nodes * 24);
     ensure<unsigned char>(c->d_out_data[slot], out_data * 32);
   }
-  uint32_t* hr = ensure_pinned<uint32_t>(c->h_root[slot], ((uint64_t)n * 16 + 1) * 4);
-  uint32_t* hr_dev = nullptr;
+  uint32_t* hr = ensure_pinned<uint32_t>(c->h_root[slot], (uint64_t)n * kRootWords * 4);
+  uint32_t *hr_dev = nullptr, *flag_dev = nullptr;
   ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&hr_dev), hr, 0), "mapped root info");
-  hr[(uint64_t)n * 16] = 0;  // the layout check flag: the record kernels set it, in host memory
+  ck(cudaHostGetDevicePointer(reinterpret_cast<void**>(&flag_dev), c->h_flag.p, 0), "mapped flag");
   auto bricks_of = [&](uint32_t s) -> uint64_t { return lvl[(uint64_t)s * kCountWords + 2 + stripe[s].U]; };  // non-empty
   uint64_t total_bricks = 0, total_records = 0;
   for (uint32_t s = 0; s < n; s++)
@@ -1072,9 +1087,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     e.stride = vj[s].stride;
     e.unit_div = m.pl.unit_div;
     e.upper_cache = upper_cache ? upper_cache + cell_at[s] * 6 : nullptr;
-    e.root_out = hr_dev + (uint64_t)s * 16;
+    e.root_out = hr_dev + (uint64_t)s * kRootWords;
     e.n_tris = m.resident;
-    e.flag = hr_dev + (uint64_t)n * 16;
+    e.flag = flag_dev;
     e.node_base = q.node_base;
     e.data_base = q.data_base;
     e.data_span = q.data_span;
@@ -1123,7 +1138,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   for (uint32_t s = 0; s < n; s++) early_data = early_data && !meshes[sb[s].mesh].pl.levels;
   const std::vector<uint64_t> cp_emit = cta_prefix(n, kTreeWarpsPerCta, [&](uint32_t s) -> uint64_t {
     return live(s) ? (bricks_of(s) + ej[s].bricks_per_warp - 1) / ej[s].bricks_per_warp : 0;
-  });
+  }, [&](uint32_t s) -> uint64_t { return live(s) && !any_levels ? upper_node_ctas(stripe[s].U) : 0; });
   const std::vector<uint64_t> cp_upper = cta_prefix(n, kChunk, [&](uint32_t s) -> uint64_t {
     return live(s) ? upper_cell(stripe[s].U, 0) : 0;  // levels 0 .. U-1
   });
@@ -1159,8 +1174,10 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     {
       PhaseScope ph(c, PH_TREE, st);
       launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, sp1, se1, st);
-      if (any_levels) launch_b_upper_avg(d_str, d_ej, n, max_upper, st);
-      launch_b_upper_nodes(d_str, d_ej, dp2(o_un), n, cp_upper[n], sp1, se1, st);
+      if (any_levels) {
+        launch_b_upper_avg(d_str, d_ej, n, max_upper, st);
+        launch_b_upper_nodes(d_str, d_ej, dp2(o_un), n, cp_upper[n], sp1, se1, st);
+      }
     }
   });
   c->leaf_zero = true;
@@ -1180,14 +1197,20 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   }
   out_pending.active = true;
   out_pending.slot = slot;
-  out_pending.checked = false;
+  // With the records on the device the counts were all the host needs, unless it averages the stripe
+  // roots; the flag is looked at when the build has finished.
+  out_pending.checked = os.mode == OUT_CTX && (!any_levels || meshes[sb[0].mesh].pl.n_stripes == 1);
   out_pending.at = 0;
   out_pending.stage = 0;
   out_pending.cur = 0;
   out_pending.sb = sb;
   out_pending.pl = pl;
   out_pending.depth.resize(n);
-  for (uint32_t s = 0; s < n; s++) out_pending.depth[s] = stripe[s].depth;
+  out_pending.root_mask.resize(n);
+  for (uint32_t s = 0; s < n; s++) {
+    out_pending.depth[s] = stripe[s].depth;
+    out_pending.root_mask[s] = lvl[(uint64_t)s * kCountWords + kRootWord];
+  }
 }
 
 // Hand a sub-batch's stripes to their meshes, in file order.  With `block` it
@@ -1207,12 +1230,8 @@ bool finish_sub_batch(ooc_ctx* c, std::vector<MeshWork>& meshes, Pending& pd, co
       ck(e, "sub-batch");
     }
     ck(cudaGetLastError(), "sub-batch kernels");
-    const uint32_t* hr = static_cast<const uint32_t*>(c->h_root[slot].p);
-    if (hr[(uint64_t)n * 16] != 0)
-      fail(OOC_ERR_DEVICE, "internal layout check failed (flag " + std::to_string(hr[(uint64_t)n * 16]) + ")");
+    check_layout_flag(c);
     pd.checked = true;
-    pd.at = 0;
-    pd.stage = 0;
   }
   const uint32_t* hr = static_cast<const uint32_t*>(c->h_root[slot].p);
   for (; pd.at < n; pd.at++, pd.stage = 0) {
@@ -1249,21 +1268,17 @@ bool finish_sub_batch(ooc_ctx* c, std::vector<MeshWork>& meshes, Pending& pd, co
     }
     m.top.node_pos += q.node_span;
     m.top.data_pos += q.data_span;
-    const uint32_t* h_root = hr + (uint64_t)s * 16;
     TNode r;
-    const uint32_t mask = h_root[0];
-    float cf[6];
-    std::memcpy(cf, h_root + 1, sizeof(cf));
+    const uint32_t mask = pd.root_mask[s];
+    if (m.pl.levels) std::memcpy(r.cache, hr + (uint64_t)s * kRootWords, sizeof(r.cache));
     if (pd.depth[s] >= 1) {
       r.data = m.pl.levels ? q.data_base + q.data_span - 1 : 0;
       r.cb = q.node_base + q.total - 1 - (uint64_t)__builtin_popcount(mask);
       r.off = offsets_from_mask(mask);
-      if (m.pl.levels) std::memcpy(r.cache, cf, sizeof(cf));
     } else {
       r.data = m.pl.binary ? 1 : q.data_base;
       r.cb = 0;
       r.off = ~0ull;
-      if (!m.pl.binary) std::memcpy(r.cache, cf, sizeof(cf));
     }
     m.top.push(m.top.top, r);
   }
@@ -1587,25 +1602,36 @@ void fill_info(const MeshWork& m, ooc_build_info* info) {
   info->n_items = m.n_items;
 }
 
+// Where a kernel on `st` reads the records at `h` (pinned): there, or in a device copy.  A handful is
+// read over the link sooner than a copy is queued and done.
+const uint64_t* records_for_device(ooc_ctx* c, const uint64_t* h, size_t bytes, cudaStream_t st) {
+  if (bytes <= 16384) {
+    void* mapped = nullptr;
+    ck(cudaHostGetDevicePointer(&mapped, const_cast<uint64_t*>(h), 0), "mapped records");
+    return static_cast<const uint64_t*>(mapped);
+  }
+  uint64_t* d = ensure<uint64_t>(c->d_recs, bytes);
+  ck(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st), "records");
+  return d;
+}
+
 // Device mode: scatter the host-written records (top levels, header records) into the device files.
 void finish_device_output(ooc_ctx* c, cudaStream_t st, MeshWork& m, Emitter& out) {
   uint64_t* nodes = ensure_keep<uint64_t>(c->d_nodes, m.top.node_pos * 24, m.top.node_pos * 24, st);
   unsigned char* data = ensure_keep<unsigned char>(c->d_data, m.top.data_pos * 32, m.top.data_pos * 32, st);
-  const uint64_t nr = out.node_recs.size() / 4, dr = out.data_recs.size() / 5;
-  const size_t bytes = (out.node_recs.size() + out.data_recs.size()) * 8;
+  const size_t nw = out.node_recs.size(), bytes = (nw + out.data_recs.size()) * 8;
   uint64_t* h = ensure_pinned<uint64_t>(c->h_recs, bytes);
-  std::memcpy(h, out.node_recs.data(), out.node_recs.size() * 8);
-  std::memcpy(h + out.node_recs.size(), out.data_recs.data(), out.data_recs.size() * 8);
-  uint64_t* d = ensure<uint64_t>(c->d_recs, bytes);
-  ck(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st), "records");
-  launch_scatter_records(d, nr, 3, nodes, st);
-  launch_scatter_records(d + out.node_recs.size(), dr, 4, reinterpret_cast<uint64_t*>(data), st);
+  std::memcpy(h, out.node_recs.data(), nw * 8);
+  std::memcpy(h + nw, out.data_recs.data(), out.data_recs.size() * 8);
+  launch_scatter_records(records_for_device(c, h, bytes, st), nw / 4, out.data_recs.size() / 5, nodes,
+                         reinterpret_cast<uint64_t*>(data), st);
   c->res_nodes = m.top.node_pos;
   c->res_data = m.top.data_pos;
-  c->res_valid = true;
 }
 
-void finish_timing(ooc_ctx* c) {
+// The end of a build that succeeded.
+void finish_build(ooc_ctx* c) {
+  c->unfinished = false;
   for (float& v : c->phase_ms) v = 0.0f;
   if (c->timing) {
     for (const auto& m : c->marks) {
@@ -1651,11 +1677,14 @@ void begin_build(ooc_ctx* c) {
   c->stream_passes = 0;
   c->part_tris.clear();
   c->part_filled.clear();
-  // a build that failed part-way may have left copies queued into the staging buffers
-  ck(cudaStreamSynchronize(c->copy_stream), "cudaStreamSynchronize");
-  ck(cudaStreamSynchronize(c->ring_stream[0]), "cudaStreamSynchronize");
-  ck(cudaStreamSynchronize(c->ring_stream[1]), "cudaStreamSynchronize");
-  ck(cudaStreamSynchronize(c->h2d_stream), "cudaStreamSynchronize");
+  if (c->unfinished) {  // a build that failed part-way may have left copies queued into the staging buffers
+    ck(cudaStreamSynchronize(c->copy_stream), "cudaStreamSynchronize");
+    ck(cudaStreamSynchronize(c->ring_stream[0]), "cudaStreamSynchronize");
+    ck(cudaStreamSynchronize(c->ring_stream[1]), "cudaStreamSynchronize");
+    ck(cudaStreamSynchronize(c->h2d_stream), "cudaStreamSynchronize");
+  }
+  c->unfinished = true;
+  *ensure_pinned<volatile uint32_t>(c->h_flag, 4) = 0;
   c->err.clear();
   c->marks.clear();
   c->kmarks.clear();
@@ -1758,7 +1787,7 @@ int build_from_file_stream(ooc_ctx* c, const ooc_build_params* prm, const char* 
     ck(cudaStreamSynchronize(st), "build");
     ck(cudaGetLastError(), "build kernels");
     fill_info(meshes[0], info);
-    finish_timing(c);
+    finish_build(c);
   });
 }
 }  // namespace ooc
@@ -1810,7 +1839,7 @@ void ooc_ctx_destroy(ooc_ctx* c) {
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   PinBuf* pins[] = {&c->h_misc, &c->h_recs, &c->h_tables1, &c->h_tables2, &c->h_words, &c->h_stage[0],
-                    &c->h_stage[1]};
+                    &c->h_stage[1], &c->h_flag};
   for (PinBuf* b : pins)
     if (b->p) cudaFreeHost(b->p);
   for (cudaEvent_t e : c->ev_stage)
@@ -1992,7 +2021,7 @@ int ooc_build_batch(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_meshes, oo
       });
     }
     ck(cudaStreamSynchronize(st), "build");
-    finish_timing(c);
+    finish_build(c);
   });
 }
 
@@ -2040,10 +2069,8 @@ int ooc_build_batch_device(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_mes
           uint64_t* h = ensure_pinned<uint64_t>(c->h_recs, words * 8);
           std::memcpy(h, nrec.data(), nrec.size() * 8);
           std::memcpy(h + nrec.size(), drec.data(), drec.size() * 8);
-          uint64_t* d = ensure<uint64_t>(c->d_recs, words * 8);
-          ck(cudaMemcpyAsync(d, h, words * 8, cudaMemcpyHostToDevice, c->copy_stream), "records");
-          launch_scatter_to(d, nrec.size() / 4, 3, c->copy_stream);
-          launch_scatter_to(d + nrec.size(), drec.size() / 5, 4, c->copy_stream);
+          launch_scatter_records(records_for_device(c, h, words * 8, c->copy_stream), nrec.size() / 4, drec.size() / 5,
+                                 nullptr, nullptr, c->copy_stream);
         }
         // the meshes' stripes were finished before their sub-batch's event; the scatter is this stream's
         ck(cudaStreamSynchronize(c->copy_stream), "records");
@@ -2054,7 +2081,7 @@ int ooc_build_batch_device(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_mes
       });
     }
     ck(cudaStreamSynchronize(st), "build");
-    finish_timing(c);
+    finish_build(c);
   });
 }
 
@@ -2207,8 +2234,10 @@ int ooc_build_device(ooc_ctx* c, const ooc_build_params* prm, const float* tris_
     }
     ck(cudaStreamSynchronize(st), "build");
     ck(cudaGetLastError(), "build kernels");
+    check_layout_flag(c);
+    c->res_valid = true;
     fill_info(meshes[0], info);
-    finish_timing(c);
+    finish_build(c);
   });
 }
 
@@ -2238,7 +2267,7 @@ int ooc_build_from_device(ooc_ctx* c, const ooc_build_params* prm, const float* 
     ck(cudaStreamSynchronize(st), "build");
     ck(cudaGetLastError(), "build kernels");
     fill_info(meshes[0], info);
-    finish_timing(c);
+    finish_build(c);
   });
 }
 

@@ -73,7 +73,8 @@ struct Stripe {
 __host__ __device__ inline uint64_t touch_bytes(int depth) { return (leaf_blocks(depth) + 15) / 16 * 16; }
 
 // Words of a stripe's counts as the host reads them.
-constexpr uint32_t kCountWords = 16;  // [0] leaves, [1] inner nodes below the bricks, [2 + l] nodes of upper level l
+// [0] leaves, [1] inner nodes below the bricks, [2 + l] nodes of upper level l, [kRootWord] the root's child mask
+constexpr uint32_t kCountWords = 16, kRootWord = 15;
 
 // Inputs of the voxelization kernels for one stripe.
 struct VoxJob {
@@ -136,7 +137,7 @@ struct EmitJob {
   int stride;
   float unit_div;
   float* upper_cache;       // per cell of the upper levels and the bricks' children (upper_cell): its average; with -levels
-  uint32_t* root_out;       // 7 words for the host: the stripe root's child mask and its average
+  uint32_t* root_out;       // 6 words for the host: the stripe root's average; with -levels
   const unsigned long long* winners;  // per leaf: triangle << 32 | local Morton code
   uint64_t n_leaf;          // leaves of the stripe (payload)
   uint32_t bricks_per_warp; // of the emission
@@ -155,6 +156,9 @@ struct EmitJob {
 
 // Cell z of upper level l in the upper_cache.
 __host__ __device__ inline uint64_t upper_cell(int l, uint64_t z) { return ((1ull << (3 * l)) - 1) / 7 + z; }
+
+// CTAs of kTreeThreads threads over the cells above a stripe's bricks.
+__host__ __device__ inline uint32_t upper_node_ctas(int U) { return (uint32_t)((upper_cell(U, 0) + 255u) / 256u); }
 
 // Threads per CTA of the batched kernels; CTA b of a launch belongs to stripe s
 // when cta_beg[s] <= b < cta_beg[s+1] and handles that stripe's elements from
@@ -231,8 +235,10 @@ cudaError_t launch_vox_small_occupancy(const VoxJob& j, cudaStream_t st);
 cudaError_t launch_vox_large_occupancy(const VoxJob& j, cudaStream_t st, int num_sms);
 
 // src holds n entries of (index, `words` u64 values); dst[index*words + q] = value q.
-void launch_scatter_records(const uint64_t* src, uint64_t n, int words, uint64_t* dst, cudaStream_t st);
-void launch_scatter_to(const uint64_t* src, uint64_t n, int words, cudaStream_t st);
+// Node records (n of 3 words) and then data records (of 4) at `src`, each after one word that says where
+// it goes: its number in nodes or data or, without these, its address.
+void launch_scatter_records(const uint64_t* src, uint64_t n_nodes, uint64_t n_data, uint64_t* nodes, uint64_t* data,
+                            cudaStream_t st);
 
 // ---- batched launches: per-stripe jobs in device arrays; `cta_beg` (n + 1 entries) maps CTAs to stripes ----
 // `single` (may be NULL): the job of a one-stripe launch, passed as a kernel parameter.

@@ -1159,23 +1159,16 @@ __global__ void k_copy_words(const uint32_t* __restrict__ src, uint64_t n, uint3
     dst[i] = src[i];
 }
 
-__global__ void k_scatter_records(const uint64_t* __restrict__ src, uint64_t n, int words, uint64_t* __restrict__ dst) {
+// Records written on the host, at `src` device or mapped host memory (see launch_scatter_records).
+__global__ void k_scatter_records(const uint64_t* __restrict__ src, uint64_t n_nodes, uint64_t n_data,
+                                  uint64_t* __restrict__ nodes, uint64_t* __restrict__ data) {
   pdl_enter();
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t* s = src + i * (1 + words);
-  uint64_t* d = dst + s[0] * words;
-  for (int q = 0; q < words; q++) d[q] = s[1 + q];
-}
-
-// Records with their own destination: src[i] = {address, words...}.
-__global__ void k_scatter_to(const uint64_t* __restrict__ src, uint64_t n, int words) {
-  pdl_enter();
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t* s = src + i * (1 + words);
-  uint64_t* d = reinterpret_cast<uint64_t*>(s[0]);
-  for (int q = 0; q < words; q++) d[q] = s[1 + q];
+  if (i >= n_nodes + n_data) return;
+  const bool node = i < n_nodes;
+  const uint64_t* s = node ? src + i * 4 : src + n_nodes * 4 + (i - n_nodes) * 5;
+  uint64_t* d = nodes ? (node ? nodes + s[0] * 3 : data + s[0] * 4) : reinterpret_cast<uint64_t*>(s[0]);
+  for (int q = 0; q < (node ? 3 : 4); q++) d[q] = s[1 + q];
 }
 
 // ===========================================================================
@@ -1415,16 +1408,11 @@ cudaError_t launch_vox_large_occupancy(const VoxJob& j, cudaStream_t st, int num
                           args, 8 * sizeof(WalkScratch), st);
 }
 
-void launch_scatter_records(const uint64_t* src, uint64_t n, int words, uint64_t* dst, cudaStream_t st) {
-  if (n == 0) return;
+void launch_scatter_records(const uint64_t* src, uint64_t n_nodes, uint64_t n_data, uint64_t* nodes, uint64_t* data,
+                            cudaStream_t st) {
+  if (n_nodes + n_data == 0) return;
   KScope k("scatter_records", st);
-  launch_k(k_scatter_records, dim3(grid_for(n, 128)), dim3(128), 0, st, src, n, words, dst);
-}
-
-void launch_scatter_to(const uint64_t* src, uint64_t n, int words, cudaStream_t st) {
-  if (n == 0) return;
-  KScope k("scatter_records", st);
-  launch_k(k_scatter_to, dim3(grid_for(n, 128)), dim3(128), 0, st, src, n, words);
+  launch_k(k_scatter_records, dim3(grid_for(n_nodes + n_data, 128)), dim3(128), 0, st, src, n_nodes, n_data, nodes, data);
 }
 
 // ---- batched launch wrappers ----

@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes
         sp.upre[off + i] = br + r[k];
         sp.wpre[i] = make_uint2(bl + li[k].x, bi + li[k].y);
       }
+      if (U == 1 && i == 0) out[kRootWord] = w[k] & 0xffu;
       if (U > 0) {  // eight words' parent word: four bits each
         uint32_t pw = nonzero_bytes(w[k]) << (4 * (lane & 7));
         pw |= __shfl_xor_sync(FULL, pw, 1);
@@ -347,6 +348,15 @@ __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes
     out[0] = carry_l;
     out[1] = carry_i;
     out[2 + U] = carry_r;
+    if (U == 0) {  // the root's children, straight from the brick
+      uint32_t mask = 0;
+      if (sp.K == kBrickLevels) mask = sp.bunits[0];
+      else if (sp.K == 1) mask = sp.leaf[0] & 0xffu;
+      else if (sp.K == 2) mask = nonzero_bytes(sp.leaf[0]) | (nonzero_bytes(sp.leaf[1]) << 4);
+      else if (sp.K == 3)
+        for (int k = 0; k < 8; k++) mask |= (sp.leaf[2 * k] | sp.leaf[2 * k + 1]) ? 1u << k : 0u;
+      out[kRootWord] = mask;
+    }
   }
   __syncthreads();
   for (int l = U - 1; l >= 0; l--) {
@@ -375,6 +385,7 @@ __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes
         sp.upre[off + i0 + k] = run;
         run += __popc(w[k]);
       }
+    if (l == 1 && threadIdx.x == 0) out[kRootWord] = w[0] & 0xffu;
     if (l > 0 && i0 < W) {
       const uint32_t pw = parent_word(w);
       sp.ubits[upper_off(l - 1) + i0 / 8u] = pw;
@@ -818,7 +829,6 @@ __device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, u
     sm.units[excl + k] = (uint16_t)((uint32_t)lane | (((uint32_t)__ffs(m) - 1u) << 5) | (k << 8));
   __syncwarp();
   uint32_t carry = 0;          // records | leaves << 16 of the last step's last brick so far
-  uint32_t root_mask = units;  // of a one-brick stripe
   const uint32_t odd0 = (uint32_t)(reinterpret_cast<uintptr_t>(nodes) >> 3);
   // A step's words, loaded while the step before is laid out: the lane's unit's entry of
   // sm.units and its leaf words.
@@ -989,10 +999,7 @@ __device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, u
         for (int i = 0; i < 6; i++) c[i] = sa.v[i];
       }
     }
-    if (K < kBrickLevels) {
-      const uint32_t r = K == 3 ? m3 : (K == 2 ? ma : (uint32_t)a & 0xffu);
-      root_mask = __shfl_sync(FULL, r, 0);
-    } else if (last && valid) {  // the unit's own record
+    if (K == kBrickLevels && last && valid) {  // the unit's own record
       uint64_t* t = nodes + (uint64_t)(o_g3 + t3) * 3u;
       t[0] = LEVELS ? dbase + d3 : 0;
       t[1] = e.node_base + grp;
@@ -1112,20 +1119,17 @@ __device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, u
       }
       store_data_record(e, dbase + dtop, 0, s4.v);
       if (U == 0)
-        for (int i = 0; i < 6; i++) e.root_out[1 + i] = __float_as_uint(s4.v[i]);
+        for (int i = 0; i < 6; i++) e.root_out[i] = __float_as_uint(s4.v[i]);
     }
   }
   if (mine && p.touch) reinterpret_cast<uint4*>(p.touch)[x] = make_uint4(0u, 0u, 0u, 0u);  // zero for the next build
-  if (U == 0 && lane == 0) {  // the stripe root, which the host writes
-    e.root_out[0] = root_mask;
-    if (K == 0) {  // one voxel
-      p.leaf[0] = 0u;
-      if (pay) {
-        float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        uint32_t key;
-        leaf_value(e, 0, key, c);
-        for (int i = 0; i < 6; i++) e.root_out[1 + i] = __float_as_uint(c[i]);
-      }
+  if (K == 0 && lane == 0) {  // one voxel
+    p.leaf[0] = 0u;
+    if (LEVELS && pay) {
+      float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+      uint32_t key;
+      leaf_value(e, 0, key, c);
+      for (int i = 0; i < 6; i++) e.root_out[i] = __float_as_uint(c[i]);
     }
   }
 }
@@ -1192,6 +1196,70 @@ __device__ __forceinline__ void emit_warp(const Stripe& p, const EmitJob& e, uin
   bulk_wait_all();
 }
 
+// Nodes of the stripe written before the children of cell a of level m < U.
+__device__ __forceinline__ uint32_t children_base(const Stripe& p, int m, uint32_t a) {
+  uint32_t s = 0;
+  for (int l = 1; l <= m + 1; l++) s += upper_rank(p, l, 8u * (a >> (3 * (m + 1 - l))));
+  for (int l = m + 2; l <= p.U; l++) s += upper_rank(p, l, (a + 1u) << (3 * (l - m)));
+  const uint2 v = brick_prefix(p, (a + 1u) << (3 * (p.U - m)));
+  return s + v.x + v.y;
+}
+
+// Data records of the stripe (-levels) before the average of cell z of level m < U.
+__device__ __forceinline__ uint32_t data_before(const Stripe& p, bool payload, int m, uint32_t z) {
+  uint32_t s = 0;
+  for (int l = 1; l <= m; l++) s += upper_rank(p, l, z >> (3 * (m - l)));
+  for (int l = m + 1; l <= p.U; l++) s += upper_rank(p, l, (z + 1u) << (3 * (l - m)));
+  const uint2 v = brick_prefix(p, (z + 1u) << (3 * (p.U - m)));
+  return s + (payload ? v.x : 0u) + v.y;
+}
+
+// Cell i of levels 0 .. U-1.
+__device__ __forceinline__ void upper_node(const Stripe& p, const EmitJob& e, uint64_t i) {
+  int m = 0;
+  while (i >= upper_cell(m + 1, 0)) m++;
+  if (m >= p.U) return;
+  const uint32_t z = (uint32_t)(i - upper_cell(m, 0));
+  if (!((p.ubits[upper_off(m) + (z >> 5)] >> (z & 31u)) & 1u)) return;
+  const uint32_t mask = upper_byte(p, m + 1, z);
+  const float* v = e.levels ? e.upper_cache + i * 6 : nullptr;
+  if (m == 0) {  // the stripe root, which the host writes
+    if (v) {
+      for (int k = 0; k < 6; k++) e.root_out[k] = __float_as_uint(v[k]);
+      store_data_record(e, e.data_base + e.data_span - 1, 0, v);
+    }
+    return;
+  }
+  const uint32_t sib = upper_byte(p, m, z >> 3) & ((1u << (z & 7u)) - 1u);
+  uint64_t di = 0;
+  if (v) {
+    di = e.data_base + data_before(p, !e.binary, m, z);
+    store_data_record(e, di, 0, v);
+  }
+  store_node_record(e, e.node_base + children_base(p, m - 1, z >> 3) + __popc(sib), di,
+                    e.node_base + children_base(p, m, z), child_offsets(mask));
+}
+
+// CTA `cta` of a stripe.  Without -levels the first ones write the records above the bricks (which wait
+// for averages otherwise): a launch of their own took 7 us of a small call, and 0.1 of 12 ms on the
+// 20M-triangle soup.
+template <bool LEVELS>
+__device__ __forceinline__ void emit_cta(const Stripe& p, const EmitJob& e, uint64_t cta, WarpScratch* ws,
+                                         const uint64_t* lut) {
+  if (!LEVELS) {
+    const uint32_t upper = upper_node_ctas(p.U);
+    if (cta < upper) {
+      upper_node(p, e, cta * kTreeThreads + threadIdx.x);
+      return;
+    }
+    cta -= upper;
+  }
+  const uint32_t warp = threadIdx.x >> 5;
+  const uint64_t i = cta * kTreeWarps + warp;
+  if (LEVELS && e.levels) emit_warp<true>(p, e, i, threadIdx.x & 31, ws[warp], lut);
+  else emit_warp<false>(p, e, i, threadIdx.x & 31, ws[warp], lut);
+}
+
 template <bool SINGLE, bool LEVELS>
 __global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(const Stripe* __restrict__ stripes,
                                                                       const EmitJob* __restrict__ emits,
@@ -1199,14 +1267,13 @@ __global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(
                                                                       Stripe p0, EmitJob e0) {
   __shared__ uint64_t lut[256];  // child_offsets of every mask
   __shared__ WarpScratch ws[kTreeWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  static_assert(kTreeThreads == 256, "one table entry per thread");
+  static_assert(kTreeThreads == 256, "one table entry per thread, and upper_node_ctas");
   static_assert(kWindow % 2 == 0 && kSlots % 2 == 0, "windows start on 16 bytes, every window's parity is the same");
   lut[threadIdx.x] = child_offsets(threadIdx.x);
   pdl_enter();
   if constexpr (SINGLE) {
     __syncthreads();
-    emit_warp<LEVELS>(p0, e0, (uint64_t)blockIdx.x * kTreeWarps + (uint32_t)warp, lane, ws[warp], lut);
+    emit_cta<LEVELS>(p0, e0, blockIdx.x, ws, lut);
   } else {
     __shared__ Stripe sp;
     __shared__ EmitJob se;
@@ -1215,9 +1282,7 @@ __global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(
     stage(sp, stripes[s]);
     stage(se, emits[s]);
     __syncthreads();
-    const uint64_t i = cta * kTreeWarps + (uint32_t)warp;
-    if (LEVELS && se.levels) emit_warp<true>(sp, se, i, lane, ws[warp], lut);
-    else emit_warp<false>(sp, se, i, lane, ws[warp], lut);
+    emit_cta<LEVELS>(sp, se, cta, ws, lut);
   }
 }
 
@@ -1266,51 +1331,6 @@ __global__ void __launch_bounds__(1024) kb_upper_avg_top(const Stripe* __restric
     for (uint32_t z = threadIdx.x; z < (1u << (3 * l)); z += 1024u) average_cell(p, e, l, z);
     __syncthreads();
   }
-}
-
-// Nodes of the stripe written before the children of cell a of level m < U.
-__device__ __forceinline__ uint32_t children_base(const Stripe& p, int m, uint32_t a) {
-  uint32_t s = 0;
-  for (int l = 1; l <= m + 1; l++) s += upper_rank(p, l, 8u * (a >> (3 * (m + 1 - l))));
-  for (int l = m + 2; l <= p.U; l++) s += upper_rank(p, l, (a + 1u) << (3 * (l - m)));
-  const uint2 v = brick_prefix(p, (a + 1u) << (3 * (p.U - m)));
-  return s + v.x + v.y;
-}
-
-// Data records of the stripe (-levels) before the average of cell z of level m < U.
-__device__ __forceinline__ uint32_t data_before(const Stripe& p, bool payload, int m, uint32_t z) {
-  uint32_t s = 0;
-  for (int l = 1; l <= m; l++) s += upper_rank(p, l, z >> (3 * (m - l)));
-  for (int l = m + 1; l <= p.U; l++) s += upper_rank(p, l, (z + 1u) << (3 * (l - m)));
-  const uint2 v = brick_prefix(p, (z + 1u) << (3 * (p.U - m)));
-  return s + (payload ? v.x : 0u) + v.y;
-}
-
-// Cell i of levels 0 .. U-1.
-__device__ __forceinline__ void upper_node(const Stripe& p, const EmitJob& e, uint64_t i) {
-  int m = 0;
-  while (i >= upper_cell(m + 1, 0)) m++;
-  if (m >= p.U) return;
-  const uint32_t z = (uint32_t)(i - upper_cell(m, 0));
-  if (!((p.ubits[upper_off(m) + (z >> 5)] >> (z & 31u)) & 1u)) return;
-  const uint32_t mask = upper_byte(p, m + 1, z);
-  const float* v = e.levels ? e.upper_cache + i * 6 : nullptr;
-  if (m == 0) {  // the stripe root, which the host writes
-    e.root_out[0] = mask;
-    if (v) {
-      for (int k = 0; k < 6; k++) e.root_out[1 + k] = __float_as_uint(v[k]);
-      store_data_record(e, e.data_base + e.data_span - 1, 0, v);
-    }
-    return;
-  }
-  const uint32_t sib = upper_byte(p, m, z >> 3) & ((1u << (z & 7u)) - 1u);
-  uint64_t di = 0;
-  if (v) {
-    di = e.data_base + data_before(p, !e.binary, m, z);
-    store_data_record(e, di, 0, v);
-  }
-  store_node_record(e, e.node_base + children_base(p, m - 1, z >> 3) + __popc(sib), di,
-                    e.node_base + children_base(p, m, z), child_offsets(mask));
 }
 
 template <bool SINGLE>
