@@ -1139,16 +1139,12 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   const std::vector<uint64_t> cp_emit = cta_prefix(n, kTreeWarpsPerCta, [&](uint32_t s) -> uint64_t {
     return live(s) ? (bricks_of(s) + ej[s].bricks_per_warp - 1) / ej[s].bricks_per_warp : 0;
   }, [&](uint32_t s) -> uint64_t { return live(s) && !any_levels ? upper_node_ctas(stripe[s].U) : 0; });
-  const std::vector<uint64_t> cp_upper = cta_prefix(n, kChunk, [&](uint32_t s) -> uint64_t {
-    return live(s) ? upper_cell(stripe[s].U, 0) : 0;  // levels 0 .. U-1
-  });
   Uploader up2;
   const size_t o_vj2 = up2.add(vj.data(), n * sizeof(VoxJob));
   const size_t o_ej = up2.add(ej.data(), n * sizeof(EmitJob));
   const size_t o_cpay = up2.add(cp_pay.data(), (n + 1) * 8);
   const size_t o_clp = up2.add(cp_leafpay.beg.data(), (n + 1) * 8);
   const size_t o_em = up2.add(cp_emit.data(), (n + 1) * 8);
-  const size_t o_un = up2.add(cp_upper.data(), (n + 1) * 8);
   unsigned char* t2 = up2.run(c, c->d_tables2, c->h_tables2, st);
   auto dp2 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t2 + off); };
   const VoxJob* d_vj2 = reinterpret_cast<const VoxJob*>(t2 + o_vj2);
@@ -1173,11 +1169,8 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   run_launches(c, st, 2, [&] {
     {
       PhaseScope ph(c, PH_TREE, st);
-      launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, sp1, se1, st);
-      if (any_levels) {
-        launch_b_upper_avg(d_str, d_ej, n, max_upper, st);
-        launch_b_upper_nodes(d_str, d_ej, dp2(o_un), n, cp_upper[n], sp1, se1, st);
-      }
+      launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, c->num_sms, sp1, se1, st);
+      if (any_levels) launch_b_upper_levels(d_str, d_ej, n, max_upper, st);
     }
   });
   c->leaf_zero = true;

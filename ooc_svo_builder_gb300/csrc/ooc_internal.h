@@ -287,12 +287,9 @@ void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const ui
 // levels and the marks.  CTAs of kTreeWarpsPerCta warps of EmitJob::bricks_per_warp non-empty bricks each.
 constexpr uint32_t kTreeWarpsPerCta = 8;
 void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                   bool levels, const Stripe* sp, const EmitJob* se, cudaStream_t st);
-// Averages of the upper levels above the bricks (-levels): one launch per level of more than 4,096 cells
-// and one for the rest.
-void launch_b_upper_avg(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st);
-// The records of the upper levels above the bricks, and the stripe roots' child masks and averages.
-void launch_b_upper_nodes(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                          uint64_t ctas, const Stripe* sp, const EmitJob* se, cudaStream_t st);
+                   bool levels, int num_sms, const Stripe* sp, const EmitJob* se, cudaStream_t st);
+// With -levels in the batch: the averages of the levels above the bricks, one launch per level of more than
+// 4,096 cells and one for the rest, which also writes these levels' records and the roots' averages.
+void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st);
 
 }  // namespace ooc

@@ -516,36 +516,6 @@ __device__ __forceinline__ uint64_t child_offsets(uint32_t mask) {
   return off;
 }
 
-// OctreeBuilder.cpp:81-99: sum over the 8 slots in child order (null slots add
-// zero), divide by the non-null count, normalise the normal.  `child`: the
-// averages (or leaf values) of the children, one after another; NULL: all zero.
-__device__ __forceinline__ void average_children(uint32_t mask, const float* child, float out[6]) {
-  float acc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  float notnull = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    if ((mask >> k) & 1u) {
-      notnull = __fadd_rn(notnull, 1.0f);
-      if (child) {
-#pragma unroll
-        for (int q = 0; q < 6; q++) c[q] = child[q];
-        child += 6;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 6; q++) acc[q] = __fadd_rn(acc[q], c[q]);
-  }
-  out[0] = __fdiv_rn(acc[0], notnull);
-  out[1] = __fdiv_rn(acc[1], notnull);
-  out[2] = __fdiv_rn(acc[2], notnull);
-  float tx = __fdiv_rn(acc[3], notnull), ty = __fdiv_rn(acc[4], notnull), tz = __fdiv_rn(acc[5], notnull);
-  normalize3(tx, ty, tz);
-  out[3] = tx;
-  out[4] = ty;
-  out[5] = tz;
-}
-
 constexpr uint32_t kTreeThreads = 256;
 constexpr uint32_t kTreeWarps = kTreeThreads / 32;
 static_assert(kTreeWarps == kTreeWarpsPerCta, "the host sizes the launches");
@@ -1260,8 +1230,8 @@ __device__ __forceinline__ void emit_cta(const Stripe& p, const EmitJob& e, uint
   else emit_warp<false>(p, e, i, threadIdx.x & 31, ws[warp], lut);
 }
 
-template <bool SINGLE, bool LEVELS>
-__global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(const Stripe* __restrict__ stripes,
+template <bool SINGLE, bool LEVELS, int CTAS>
+__global__ void __launch_bounds__(kTreeThreads, CTAS) kb_emit(const Stripe* __restrict__ stripes,
                                                                       const EmitJob* __restrict__ emits,
                                                                       const uint64_t* __restrict__ cta_beg, uint32_t n,
                                                                       Stripe p0, EmitJob e0) {
@@ -1291,21 +1261,24 @@ __global__ void __launch_bounds__(kTreeThreads, LEVELS ? 2 : kEmitCtas) kb_emit(
 __device__ __forceinline__ void average_cell(const Stripe& p, const EmitJob& e, int l, uint32_t z) {
   if (!((p.ubits[upper_off(l) + (z >> 5)] >> (z & 31u)) & 1u)) return;
   const uint32_t mask = upper_byte(p, l + 1, z);
-  // the children's averages stand at their cells: gather them in child order
-  float child[48];
-  uint32_t c = 0;
+  const float2* src = reinterpret_cast<const float2*>(e.upper_cache + upper_cell(l + 1, (uint64_t)z * 8u) * 6);
+  float2 child[8][3];
+#pragma unroll
+  for (uint32_t k = 0; k < 8; k++)
+    if ((mask >> k) & 1u)
+      for (int q = 0; q < 3; q++) child[k][q] = src[k * 3 + q];
+  Sum s;
+  s.zero();
 #pragma unroll
   for (uint32_t k = 0; k < 8; k++)
     if ((mask >> k) & 1u) {
-      const float* src = e.upper_cache + upper_cell(l + 1, (uint64_t)z * 8u + k) * 6;
-      for (int q = 0; q < 6; q++) child[c * 6 + q] = src[q];
-      c++;
+      const float c[6] = {child[k][0].x, child[k][0].y, child[k][1].x, child[k][1].y, child[k][2].x, child[k][2].y};
+      s.add(c);
     }
-  float v[6];
-  average_children(mask, child, v);
-  float* out = e.upper_cache + upper_cell(l, z) * 6;
+  s.average(__popc(mask));
+  float2* out = reinterpret_cast<float2*>(e.upper_cache + upper_cell(l, z) * 6);
 #pragma unroll
-  for (int q = 0; q < 6; q++) out[q] = v[q];
+  for (int q = 0; q < 3; q++) out[q] = make_float2(s.v[2 * q], s.v[2 * q + 1]);
 }
 
 // Level l of the stripes that have it above their bricks, one thread per cell (grid.y: the stripes).
@@ -1320,37 +1293,36 @@ __global__ void __launch_bounds__(256) kb_upper_avg(const Stripe* __restrict__ s
   }
 }
 
-// Levels min(l_hi, U - 1) .. 0, one CTA per stripe.
-__global__ void __launch_bounds__(1024) kb_upper_avg_top(const Stripe* __restrict__ stripes,
-                                                         const EmitJob* __restrict__ emits, int l_hi) {
+// Levels min(l_hi, U - 1) .. 0 and then the records above the bricks, CTAS CTAs (a cluster) per stripe.
+// Bound by latency, level after level.  One CTA took 29 us for the 4,681 cells above the bricks of a
+// 512 stripe, most of it for the 4,096 of level 4, and another launch 8 us for their records.
+constexpr uint32_t kTopThreads = 512;  // the cells of level 3
+template <uint32_t CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kTopThreads)
+    kb_upper_top(const Stripe* __restrict__ stripes, const EmitJob* __restrict__ emits, int l_hi) {
   pdl_enter();
-  const Stripe& p = stripes[blockIdx.x];
-  const EmitJob& e = emits[blockIdx.x];
-  if (!e.levels || p.U == 0 || p.wpre[upper_words(p.U)].x == 0) return;
-  for (int l = min(l_hi, p.U - 1); l >= 0; l--) {
-    for (uint32_t z = threadIdx.x; z < (1u << (3 * l)); z += 1024u) average_cell(p, e, l, z);
-    __syncthreads();
+  const Stripe& p = stripes[blockIdx.x / CTAS];
+  const EmitJob& e = emits[blockIdx.x / CTAS];
+  if (p.U == 0 || p.wpre[upper_words(p.U)].x == 0) return;
+  const uint32_t t = (blockIdx.x % CTAS) * kTopThreads + threadIdx.x;
+  if (e.levels) {
+    auto sync = [] {
+      if (CTAS == 1) __syncthreads();
+      else asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    };
+    int l = min(l_hi, p.U - 1);
+    for (; l > 3; l--) {
+      for (uint32_t z = t; z < (1u << (3 * l)); z += CTAS * kTopThreads) average_cell(p, e, l, z);
+      sync();
+    }
+    if (t < kTopThreads)  // the cluster's first CTA
+      for (; l >= 0; l--) {
+        if (t < (1u << (3 * l))) average_cell(p, e, l, t);
+        __syncthreads();
+      }
+    sync();
   }
-}
-
-template <bool SINGLE>
-__global__ void __launch_bounds__(kTreeThreads) kb_upper_nodes(const Stripe* __restrict__ stripes,
-                                                               const EmitJob* __restrict__ emits,
-                                                               const uint64_t* __restrict__ cta_beg, uint32_t n,
-                                                               Stripe p0, EmitJob e0) {
-  pdl_enter();
-  if constexpr (SINGLE) {
-    upper_node(p0, e0, (uint64_t)blockIdx.x * kTreeThreads + threadIdx.x);
-  } else {
-    __shared__ Stripe sp;
-    __shared__ EmitJob se;
-    uint64_t cta;
-    const uint32_t s = cta_stripe(cta_beg, n, cta);
-    stage(sp, stripes[s]);
-    stage(se, emits[s]);
-    __syncthreads();
-    upper_node(sp, se, cta * kTreeThreads + threadIdx.x);
-  }
+  for (uint64_t i = t; i < upper_cell(p.U, 0); i += CTAS * kTopThreads) upper_node(p, e, i);
 }
 
 }  // namespace
@@ -1406,32 +1378,30 @@ void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const ui
 }
 
 void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                   bool levels, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
+                   bool levels, int num_sms, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
   if (ctas == 0) return;
   KScope k("emit", st);
-  auto* kern = sp ? (levels ? kb_emit<true, true> : kb_emit<true, false>)
-                  : (levels ? kb_emit<false, true> : kb_emit<false, false>);
+  // With -levels two CTAs fit an SM only with 128 registers a thread, some of them spilled: where one CTA
+  // per SM is all there is, the kernel that keeps everything (3,001 triangles at gridsize 128 45 and 35 us;
+  // the heightfield at 512, more CTAs than SMs, 51 and 63).
+  auto* kern = !levels ? (sp ? kb_emit<true, false, kEmitCtas> : kb_emit<false, false, kEmitCtas>)
+               : !sp   ? kb_emit<false, true, 2>
+                       : (ctas <= (uint64_t)num_sms ? kb_emit<true, true, 1> : kb_emit<true, true, 2>);
   launch_k(kern, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes, emits, cta_beg, n, stripe_or_zero(sp),
            emit_or_zero(se));
 }
 
-void launch_b_upper_avg(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st) {
+void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st) {
   if (n == 0 || max_upper == 0) return;
-  constexpr int kTop = 4;  // 4,096 cells: four per thread of one CTA
+  constexpr int kTop = 4;  // 4,096 cells: one per thread of eight CTAs
   for (int l = max_upper - 1; l > kTop; l--) {
     KScope k("upper_average", st);
     launch_k(kb_upper_avg, dim3(1u << (3 * l - 8), n < 4096u ? n : 4096u), dim3(256), 0, st, stripes, emits, n, l);
   }
-  KScope k("upper_average_top", st);
-  launch_k(kb_upper_avg_top, dim3(n), dim3(1024), 0, st, stripes, emits, kTop);
-}
-
-void launch_b_upper_nodes(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
-                          uint64_t ctas, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
-  if (ctas == 0) return;
-  KScope k("upper_nodes", st);
-  launch_k(sp ? kb_upper_nodes<true> : kb_upper_nodes<false>, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes,
-           emits, cta_beg, n, stripe_or_zero(sp), emit_or_zero(se));
+  KScope k("upper_top", st);
+  // up to level 2 (64 cells, U = 3) one CTA; a cluster's barriers cost more there
+  if (max_upper <= 3) launch_k(kb_upper_top<1>, dim3(n), dim3(kTopThreads), 0, st, stripes, emits, kTop);
+  else launch_k(kb_upper_top<8>, dim3(n * 8u), dim3(kTopThreads), 0, st, stripes, emits, kTop);
 }
 
 }  // namespace ooc
