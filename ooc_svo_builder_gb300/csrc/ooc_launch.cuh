@@ -124,20 +124,10 @@ __device__ __forceinline__ void stage(T& dst, const T& src) {
 
 // CTA b belongs to the stripe s with cta_beg[s] <= b < cta_beg[s+1]; it is
 // the stripe's CTA b - cta_beg[s] and covers the elements per CTA of its launch
-// from there.
+// from there.  Every warp searches by itself, 32 stripes a probe: one thread's bisection
+// held the CTA for up to ten loads in a row.
 __device__ __forceinline__ uint32_t cta_stripe(const uint64_t* __restrict__ cta_beg, uint32_t n, uint64_t& cta) {
-  __shared__ uint32_t s_stripe;
-  if (threadIdx.x == 0) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (cta_beg[mid] <= blockIdx.x) lo = mid;
-      else hi = mid;
-    }
-    s_stripe = lo;
-  }
-  __syncthreads();
-  const uint32_t s = s_stripe;
+  const uint32_t s = warp_search(n, blockIdx.x, threadIdx.x & 31, [&](uint32_t i) { return cta_beg[i]; });
   cta = (uint64_t)(blockIdx.x - cta_beg[s]);  // the CTA's index within its stripe
   return s;
 }

@@ -445,9 +445,8 @@ __device__ void payload_color(const TriVerts& tv, const float n[3], int x, int y
 
 // Colour, normal and local Morton code of leaf `li` (its index among the stripe's leaves).
 // Returns false (and flags) if the leaf has no winning triangle.
-__device__ bool leaf_value(const EmitJob& e, uint64_t li, uint32_t& key, float out[6]) {
-  const unsigned long long win = e.winners[li];  // triangle, Morton code
-  key = (uint32_t)win;
+__device__ bool leaf_value(const EmitJob& e, unsigned long long win, float out[6]) {
+  const uint32_t key = (uint32_t)win;
   uint32_t lx, ly, lz;
   morton_local_decode(key, lx, ly, lz);
   const int x = e.origin[0] + (int)lx, y = e.origin[1] + (int)ly, z = e.origin[2] + (int)lz;
@@ -547,12 +546,18 @@ __device__ __forceinline__ uint32_t inner_before(const Stripe& p, uint32_t key) 
   return s;
 }
 
-__device__ __forceinline__ void leaf_payload(const Stripe& p, const EmitJob& e, uint64_t i) {
-  if (i >= e.n_leaf) return;
-  float v[6];
-  uint32_t key;
-  if (!leaf_value(e, i, key, v)) return;
-  store_data_record(e, e.data_base + i + (e.levels ? inner_before(p, key) : 0u), e.stripe_base + key, v);
+// Leaves (cta * ept + k) * kTreeThreads + thread of the stripe; the next leaf's winner is loaded ahead.
+__device__ __forceinline__ void leaf_payload(const Stripe& p, const EmitJob& e, uint64_t cta, uint32_t ept) {
+  uint64_t i = cta * ept * kTreeThreads + threadIdx.x;
+  unsigned long long next = i < e.n_leaf ? e.winners[i] : 0ull;
+#pragma unroll 1
+  for (uint32_t k = 0; k < ept && i < e.n_leaf; k++, i += kTreeThreads) {
+    const unsigned long long win = next;
+    if (k + 1 < ept && i + kTreeThreads < e.n_leaf) next = e.winners[i + kTreeThreads];
+    float v[6];
+    const uint32_t key = (uint32_t)win;
+    if (leaf_value(e, win, v)) store_data_record(e, e.data_base + i + (e.levels ? inner_before(p, key) : 0u), e.stripe_base + key, v);
+  }
 }
 
 template <bool SINGLE>
@@ -562,7 +567,7 @@ __global__ void __launch_bounds__(kTreeThreads) kb_leaf_payload(const Stripe* __
                                                                 uint32_t ept, Stripe p0, EmitJob e0) {
   pdl_enter();
   if constexpr (SINGLE) {
-    for (uint32_t k = 0; k < ept; k++) leaf_payload(p0, e0, ((uint64_t)blockIdx.x * ept + k) * kTreeThreads + threadIdx.x);
+    leaf_payload(p0, e0, blockIdx.x, ept);
   } else {
     __shared__ Stripe sp;
     __shared__ EmitJob se;
@@ -571,7 +576,7 @@ __global__ void __launch_bounds__(kTreeThreads) kb_leaf_payload(const Stripe* __
     stage(sp, stripes[s]);
     stage(se, emits[s]);
     __syncthreads();
-    for (uint32_t k = 0; k < ept; k++) leaf_payload(sp, se, (cta * ept + k) * kTreeThreads + threadIdx.x);
+    leaf_payload(sp, se, cta, ept);
   }
 }
 
@@ -1097,8 +1102,7 @@ __device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, u
     p.leaf[0] = 0u;
     if (LEVELS && pay) {
       float c[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-      uint32_t key;
-      leaf_value(e, 0, key, c);
+      leaf_value(e, e.winners[0], c);
       for (int i = 0; i < 6; i++) e.root_out[i] = __float_as_uint(c[i]);
     }
   }
