@@ -145,104 +145,113 @@ __device__ __forceinline__ WorldBox tri_world_box(const float* __restrict__ tris
   return b;
 }
 
-// Per axis, the partitions j whose world slab [lo_j, hi_j] passes the
-// reference's inclusive test form one contiguous run [j0, j1].
-__device__ __forceinline__ bool axis_run(float lo, float hi, const float* __restrict__ alo,
-                                         const float* __restrict__ ahi, int PA, int& j0, int& j1) {
-  j0 = -1;
-  j1 = -2;
+// Per axis, the partitions j whose world slab [lo_j, hi_j] passes the reference's inclusive test,
+// !(hi < lo_j) && !(lo > hi_j), form one contiguous run [j0, j1]: the slabs' bounds grow with j, so what
+// fails the second test comes first and what fails the first comes last.  (A NaN passes everywhere.)
+__device__ __forceinline__ bool axis_run(float lo, float hi, const float* alo, const float* ahi, int PA, int& j0, int& j1) {
+  j0 = 0;
+  j1 = PA - 1;
   for (int j = 0; j < PA; j++) {
-    const bool ok = !(hi < alo[j]) && !(lo > ahi[j]);
-    if (ok) {
-      if (j0 < 0) j0 = j;
-      j1 = j;
-    }
+    j0 += lo > ahi[j] ? 1 : 0;
+    j1 -= hi < alo[j] ? 1 : 0;
   }
-  return j0 >= 0;
+  return j0 <= j1;
 }
 
-__global__ void k_part_count(const float* __restrict__ tris, int stride, uint64_t n_tris,
-                             const float* __restrict__ axis_lo, const float* __restrict__ axis_hi, int pa_bits,
-                             uint32_t n_parts, uint32_t* __restrict__ hist, int use_smem) {
+// The slabs' bounds of the three axes, lower and then upper, into shared memory.
+__device__ __forceinline__ void stage_axes(float* dst, const float* __restrict__ axis_lo, const float* __restrict__ axis_hi,
+                                           int PA) {
+  for (int i = threadIdx.x; i < 3 * PA; i += blockDim.x) {
+    dst[i] = axis_lo[i];
+    dst[3 * PA + i] = axis_hi[i];
+  }
+}
+
+// Per-axis partition runs of triangle t, packed 7 bits per bound with bit 63 set,
+// or 0 when the triangle passes no partition's box test.
+__device__ __forceinline__ uint64_t part_runs(const float* __restrict__ tris, int stride, uint64_t t, const float* axes,
+                                              int PA) {
+  const WorldBox b = tri_world_box(tris, t, stride);
+  int x0, x1, y0, y1, z0, z1;
+  const bool x = axis_run(b.lo[0], b.hi[0], axes, axes + 3 * PA, PA, x0, x1);
+  const bool y = axis_run(b.lo[1], b.hi[1], axes + PA, axes + 4 * PA, PA, y0, y1);
+  const bool z = axis_run(b.lo[2], b.hi[2], axes + 2 * PA, axes + 5 * PA, PA, z0, z1);
+  if (!(x && y && z)) return 0ull;
+  return (uint64_t)x0 | ((uint64_t)x1 << 7) | ((uint64_t)y0 << 14) | ((uint64_t)y1 << 21) | ((uint64_t)z0 << 28) |
+         ((uint64_t)z1 << 35) | (1ull << 63);
+}
+
+__device__ __forceinline__ int run_bound(uint64_t r, int k) { return (int)((r >> (7 * k)) & 127u); }
+
+template <typename F>
+__device__ __forceinline__ void each_part(uint64_t r, F f) {
+  if (!r) return;
+  for (int jx = run_bound(r, 0); jx <= run_bound(r, 1); jx++)
+    for (int jy = run_bound(r, 2); jy <= run_bound(r, 3); jy++)
+      for (int jz = run_bound(r, 4); jz <= run_bound(r, 5); jz++) f(morton_local(jx, jy, jz));
+}
+
+// Bound by the additions to the partitions' counters (64 of them on the 20M-triangle soup), which finish
+// about 3 ns apart each: a block adds a partition's triangles once, so it takes `per` times 256 of them.
+// The two passes of that soup take 0.20 + 0.27 ms with 4,096 triangles a block and 0.40 + 0.42 with 256.
+constexpr int kPartCta = 256, kPartMax = 16;  // 8 is the same
+
+__global__ void __launch_bounds__(kPartCta) k_part_count(const float* __restrict__ tris, int stride, uint64_t n_tris,
+                                                         const float* __restrict__ axis_lo,
+                                                         const float* __restrict__ axis_hi, int pa_bits,
+                                                         uint32_t n_parts, uint32_t* __restrict__ hist, int use_smem,
+                                                         int per) {
   pdl_enter();
-  extern __shared__ uint32_t sh[];
-  if (use_smem) {
-    for (uint32_t i = threadIdx.x; i < n_parts; i += blockDim.x) sh[i] = 0;
-    __syncthreads();
-  }
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n_tris) {
-    const int PA = 1 << pa_bits;
-    const WorldBox b = tri_world_box(tris, t, stride);
-    int x0, x1, y0, y1, z0, z1;
-    if (axis_run(b.lo[0], b.hi[0], axis_lo, axis_hi, PA, x0, x1) &&
-        axis_run(b.lo[1], b.hi[1], axis_lo + PA, axis_hi + PA, PA, y0, y1) &&
-        axis_run(b.lo[2], b.hi[2], axis_lo + 2 * PA, axis_hi + 2 * PA, PA, z0, z1)) {
-      for (int jx = x0; jx <= x1; jx++)
-        for (int jy = y0; jy <= y1; jy++)
-          for (int jz = z0; jz <= z1; jz++) {
-            const uint32_t p = morton_local(jx, jy, jz);
-            if (use_smem) atomicAdd(&sh[p], 1u);
-            else atomicAdd(&hist[p], 1u);
-          }
-    }
+  extern __shared__ float axes[];
+  const int PA = 1 << pa_bits;
+  uint32_t* const sh = reinterpret_cast<uint32_t*>(axes + 6 * PA);
+  stage_axes(axes, axis_lo, axis_hi, PA);
+  if (use_smem)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kPartCta) sh[i] = 0;
+  __syncthreads();
+  uint32_t* const to = use_smem ? sh : hist;
+  for (int k = 0; k < per; k++) {
+    const uint64_t t = ((uint64_t)blockIdx.x * per + k) * kPartCta + threadIdx.x;
+    if (t < n_tris) each_part(part_runs(tris, stride, t, axes, PA), [&](uint32_t p) { atomicAdd(&to[p], 1u); });
   }
   if (use_smem) {
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n_parts; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kPartCta)
       if (sh[i]) atomicAdd(&hist[i], sh[i]);
   }
 }
 
-__global__ void k_part_emit(const float* __restrict__ tris, int stride, uint64_t n_tris,
-                            const float* __restrict__ axis_lo, const float* __restrict__ axis_hi, int pa_bits,
-                            uint32_t n_parts, uint32_t* __restrict__ cursor, uint32_t* __restrict__ items,
-                            int use_smem) {
+__global__ void __launch_bounds__(kPartCta) k_part_emit(const float* __restrict__ tris, int stride, uint64_t n_tris,
+                                                        const float* __restrict__ axis_lo,
+                                                        const float* __restrict__ axis_hi, int pa_bits,
+                                                        uint32_t n_parts, uint32_t* __restrict__ cursor,
+                                                        uint32_t* __restrict__ items, int use_smem, int per) {
   pdl_enter();
-  extern __shared__ uint32_t sh[];  // [n_parts] counts, [n_parts] bases
-  uint32_t* cnt = sh;
-  uint32_t* base = sh + n_parts;
-  if (use_smem) {
-    for (uint32_t i = threadIdx.x; i < n_parts; i += blockDim.x) cnt[i] = 0;
-    __syncthreads();
-  }
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ uint64_t runs[];  // of the block's triangles
   const int PA = 1 << pa_bits;
-  int x0 = 0, x1 = -1, y0 = 0, y1 = -1, z0 = 0, z1 = -1;
-  bool hit = false;
-  if (t < n_tris) {
-    const WorldBox b = tri_world_box(tris, t, stride);
-    hit = axis_run(b.lo[0], b.hi[0], axis_lo, axis_hi, PA, x0, x1) &&
-          axis_run(b.lo[1], b.hi[1], axis_lo + PA, axis_hi + PA, PA, y0, y1) &&
-          axis_run(b.lo[2], b.hi[2], axis_lo + 2 * PA, axis_hi + 2 * PA, PA, z0, z1);
-  }
-  if (!use_smem) {
-    if (hit)
-      for (int jx = x0; jx <= x1; jx++)
-        for (int jy = y0; jy <= y1; jy++)
-          for (int jz = z0; jz <= z1; jz++) {
-            const uint32_t p = morton_local(jx, jy, jz);
-            items[atomicAdd(&cursor[p], 1u)] = (uint32_t)t;
-          }
-    return;
-  }
-  if (hit)
-    for (int jx = x0; jx <= x1; jx++)
-      for (int jy = y0; jy <= y1; jy++)
-        for (int jz = z0; jz <= z1; jz++) atomicAdd(&cnt[morton_local(jx, jy, jz)], 1u);
+  float* const axes = reinterpret_cast<float*>(runs + (use_smem ? per * kPartCta : 0));
+  uint32_t* const cnt = reinterpret_cast<uint32_t*>(axes + 6 * PA);  // their number per partition, then where they go
+  const uint64_t t0 = (uint64_t)blockIdx.x * per * kPartCta;
+  stage_axes(axes, axis_lo, axis_hi, PA);
+  if (use_smem)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kPartCta) cnt[i] = 0;
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n_parts; i += blockDim.x) {
-    base[i] = cnt[i] ? atomicAdd(&cursor[i], cnt[i]) : 0u;
-    cnt[i] = 0;
+  for (int i = threadIdx.x; i < per * kPartCta; i += kPartCta) {
+    const uint64_t r = t0 + i < n_tris ? part_runs(tris, stride, t0 + i, axes, PA) : 0ull;
+    if (use_smem) {
+      runs[i] = r;
+      each_part(r, [&](uint32_t p) { atomicAdd(&cnt[p], 1u); });
+    } else {
+      each_part(r, [&](uint32_t p) { items[atomicAdd(&cursor[p], 1u)] = (uint32_t)(t0 + i); });
+    }
   }
+  if (!use_smem) return;
   __syncthreads();
-  if (hit)
-    for (int jx = x0; jx <= x1; jx++)
-      for (int jy = y0; jy <= y1; jy++)
-        for (int jz = z0; jz <= z1; jz++) {
-          const uint32_t p = morton_local(jx, jy, jz);
-          items[base[p] + atomicAdd(&cnt[p], 1u)] = (uint32_t)t;
-        }
+  for (uint32_t i = threadIdx.x; i < n_parts; i += kPartCta)
+    if (cnt[i]) cnt[i] = atomicAdd(&cursor[i], cnt[i]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < per * kPartCta; i += kPartCta)
+    each_part(runs[i], [&](uint32_t p) { items[atomicAdd(&cnt[p], 1u)] = (uint32_t)(t0 + i); });
 }
 
 // ---------------------------------------------------------------------------
@@ -256,43 +265,24 @@ __global__ void k_part_emit(const float* __restrict__ tris, int stride, uint64_t
 // ---------------------------------------------------------------------------
 constexpr int kStreamCta = (int)kStreamCtaTris;
 
-// Per-axis partition runs of triangle t, packed 7 bits per bound with bit 63 set,
-// or 0 when the triangle passes no partition's box test.
-__device__ __forceinline__ uint64_t stream_runs(const float* __restrict__ tris, int stride, uint64_t t,
-                                                const float* __restrict__ axis_lo, const float* __restrict__ axis_hi,
-                                                int PA) {
-  const WorldBox b = tri_world_box(tris, t, stride);
-  int x0, x1, y0, y1, z0, z1;
-  if (!(axis_run(b.lo[0], b.hi[0], axis_lo, axis_hi, PA, x0, x1) &&
-        axis_run(b.lo[1], b.hi[1], axis_lo + PA, axis_hi + PA, PA, y0, y1) &&
-        axis_run(b.lo[2], b.hi[2], axis_lo + 2 * PA, axis_hi + 2 * PA, PA, z0, z1)))
-    return 0ull;
-  return (uint64_t)x0 | ((uint64_t)x1 << 7) | ((uint64_t)y0 << 14) | ((uint64_t)y1 << 21) | ((uint64_t)z0 << 28) |
-         ((uint64_t)z1 << 35) | (1ull << 63);
-}
-
-__device__ __forceinline__ int run_bound(uint64_t r, int k) { return (int)((r >> (7 * k)) & 127u); }
-
 __global__ void __launch_bounds__(kStreamCta) k_stream_count(const float* __restrict__ tris, int stride, uint64_t n,
                                                              const float* __restrict__ axis_lo,
                                                              const float* __restrict__ axis_hi, int pa_bits,
                                                              uint32_t p0, uint32_t gp, uint32_t* __restrict__ mat,
                                                              uint32_t n_cta) {
   pdl_enter();
-  extern __shared__ uint32_t cnt[];
+  extern __shared__ float axes[];
+  const int PA = 1 << pa_bits;
+  uint32_t* const cnt = reinterpret_cast<uint32_t*>(axes + 6 * PA);
+  stage_axes(axes, axis_lo, axis_hi, PA);
   for (uint32_t q = threadIdx.x; q < gp; q += kStreamCta) cnt[q] = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) mat[(uint64_t)gp * n_cta] = 0;  // the scan's total entry
   __syncthreads();
   const uint64_t t = (uint64_t)blockIdx.x * kStreamCta + threadIdx.x;
   if (t < n) {
-    const uint64_t r = stream_runs(tris, stride, t, axis_lo, axis_hi, 1 << pa_bits);
-    if (r)
-      for (int jx = run_bound(r, 0); jx <= run_bound(r, 1); jx++)
-        for (int jy = run_bound(r, 2); jy <= run_bound(r, 3); jy++)
-          for (int jz = run_bound(r, 4); jz <= run_bound(r, 5); jz++) {
-            const uint32_t q = morton_local(jx, jy, jz) - p0;
-            if (q < gp) atomicAdd(&cnt[q], 1u);
-          }
+    each_part(part_runs(tris, stride, t, axes, PA), [&](uint32_t p) {
+      if (p - p0 < gp) atomicAdd(&cnt[p - p0], 1u);
+    });
   }
   __syncthreads();
   for (uint32_t q = threadIdx.x; q < gp; q += kStreamCta) mat[(uint64_t)q * n_cta + blockIdx.x] = cnt[q];
@@ -307,9 +297,13 @@ __global__ void __launch_bounds__(kStreamCta) k_stream_emit(const float* __restr
                                                             uint32_t n_cta, const uint64_t* __restrict__ base,
                                                             float* __restrict__ out) {
   pdl_enter();
+  extern __shared__ float axes[];
   __shared__ uint64_t runs[kStreamCta];
+  const int PA = 1 << pa_bits;
+  stage_axes(axes, axis_lo, axis_hi, PA);
+  __syncthreads();
   const uint64_t t = (uint64_t)blockIdx.x * kStreamCta + threadIdx.x;
-  const uint64_t r = t < n ? stream_runs(tris, stride, t, axis_lo, axis_hi, 1 << pa_bits) : 0ull;
+  const uint64_t r = t < n ? part_runs(tris, stride, t, axes, PA) : 0ull;
   runs[threadIdx.x] = r;
   __syncthreads();
   if (!r) return;
@@ -1334,24 +1328,34 @@ void launch_copy_words(const uint32_t* src, uint64_t n, uint32_t* dst, cudaStrea
   launch_k(k_copy_words, dim3((unsigned)g), dim3(256), 0, st, src, n, dst);
 }
 
+// Rounds of kPartCta triangles a block takes: as many as leave eight blocks per SM, and runs that fit
+// beside the counters in 48 KB.
+static int part_rounds(uint64_t n_tris, size_t counters) {
+  return (int)std::min<uint64_t>(std::min<uint64_t>(kPartMax, (49152 - counters) / (kPartCta * 8)),
+                                 std::max<uint64_t>(1, n_tris / (152ull * 8 * kPartCta)));
+}
+
 void launch_part_count(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
                        int pa_bits, uint64_t n_parts, uint32_t* hist, cudaStream_t st) {
   if (n_tris == 0) return;
   const int use_smem = n_parts <= 4096;
-  const size_t smem = use_smem ? n_parts * sizeof(uint32_t) : 0;
+  const size_t smem = ((use_smem ? n_parts : 0) + 6ull * (1ull << pa_bits)) * sizeof(uint32_t);
+  const int per = part_rounds(n_tris, smem);
   KScope k("part_count", st);
-  launch_k(k_part_count, dim3(grid_for(n_tris, 256)), dim3(256), smem, st, tris, stride, n_tris, axis_lo, axis_hi,
-           pa_bits, (uint32_t)n_parts, hist, use_smem);
+  launch_k(k_part_count, dim3(grid_for(n_tris, kPartCta * per)), dim3(kPartCta), smem, st, tris, stride, n_tris, axis_lo,
+           axis_hi, pa_bits, (uint32_t)n_parts, hist, use_smem, per);
 }
 
 void launch_part_emit(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
                       int pa_bits, uint64_t n_parts, uint32_t* cursor, uint32_t* items, cudaStream_t st) {
   if (n_tris == 0) return;
   const int use_smem = n_parts <= 4096;
-  const size_t smem = use_smem ? 2 * n_parts * sizeof(uint32_t) : 0;
+  size_t smem = ((use_smem ? n_parts : 0) + 6ull * (1ull << pa_bits)) * sizeof(uint32_t);
+  const int per = part_rounds(n_tris, smem);
+  if (use_smem) smem += (size_t)per * kPartCta * 8;
   KScope k("part_emit", st);
-  launch_k(k_part_emit, dim3(grid_for(n_tris, 256)), dim3(256), smem, st, tris, stride, n_tris, axis_lo, axis_hi,
-           pa_bits, (uint32_t)n_parts, cursor, items, use_smem);
+  launch_k(k_part_emit, dim3(grid_for(n_tris, kPartCta * per)), dim3(kPartCta), smem, st, tris, stride, n_tris, axis_lo,
+           axis_hi, pa_bits, (uint32_t)n_parts, cursor, items, use_smem, per);
 }
 
 uint32_t stream_ctas(uint64_t n) { return (uint32_t)((n + kStreamCta - 1) / kStreamCta); }
@@ -1366,17 +1370,17 @@ void launch_stream_group_chunk(const float* tris, int stride, uint64_t n, const 
                                int pa_bits, uint32_t p0, uint32_t gp, uint32_t* mat, uint32_t* mat_partials,
                                uint64_t* base, float* out, cudaStream_t st) {
   if (n == 0 || gp == 0) return;
-  const uint32_t n_cta = stream_ctas(n);
+  const uint32_t n_cta = stream_ctas(n), axes = 6u << pa_bits;
   {
     KScope k("stream_count", st);
-    launch_k(k_stream_count, dim3(n_cta), dim3(kStreamCta), gp * sizeof(uint32_t), st, tris, stride, n, axis_lo,
+    launch_k(k_stream_count, dim3(n_cta), dim3(kStreamCta), (gp + axes) * sizeof(uint32_t), st, tris, stride, n, axis_lo,
              axis_hi, pa_bits, p0, gp, mat, n_cta);
   }
   scan_exclusive<uint32_t>(mat, (uint64_t)gp * n_cta + 1, mat_partials, st);
   {
     KScope k("stream_emit", st);
-    launch_k(k_stream_emit, dim3(n_cta), dim3(kStreamCta), 0, st, tris, stride, n, axis_lo, axis_hi, pa_bits, p0, gp,
-             mat, n_cta, base, out);
+    launch_k(k_stream_emit, dim3(n_cta), dim3(kStreamCta), axes * sizeof(float), st, tris, stride, n, axis_lo, axis_hi, pa_bits,
+             p0, gp, mat, n_cta, base, out);
   }
   KScope k("stream_advance", st);
   launch_k(k_stream_advance, dim3(grid_for(gp, 256)), dim3(256), 0, st, mat, n_cta, gp, base);
