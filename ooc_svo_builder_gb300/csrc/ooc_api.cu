@@ -137,6 +137,7 @@ struct ooc_ctx {
   // persistent occupancy passes (ooc_tuning::persistent): their counters, and the CTAs per SM
   DevBuf d_pctr;
   int persist_per_sm = -1;
+  bool ctr_zero = false;  // d_ctr holds only zeros
   bool leaf_zero = true;  // d_leaf and d_touch hold only zeros (no sub-batch left them dirty)
   PinBuf h_misc, h_recs, h_tables1, h_tables2, h_words;
   // double-buffered outputs of pipelined sub-batches
@@ -660,7 +661,9 @@ struct Uploader {
     parts.push_back({p, bytes});
     return off;
   }
-  unsigned char* run(ooc_ctx* c, DevBuf& dev, PinBuf& pin, cudaStream_t st) {
+  // `by_kernel`: a kernel reads the tables; a copy, sooner done by itself, would stand in the copy engine's
+  // queue behind the triangles of meshes that later sub-batches need.
+  unsigned char* run(DevBuf& dev, PinBuf& pin, bool by_kernel, cudaStream_t st) {
     size_t total = 0;
     for (auto& q : parts) total += (q.second + 255) / 256 * 256;
     unsigned char* h = ensure_pinned<unsigned char>(pin, total);
@@ -670,8 +673,13 @@ struct Uploader {
       if (q.second) std::memcpy(h + off, q.first, q.second);
       off += (q.second + 255) / 256 * 256;
     }
-    ck(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, st), "upload tables");
-    (void)c;
+    if (by_kernel) {
+      void* mapped = nullptr;
+      ck(cudaHostGetDevicePointer(&mapped, h, 0), "mapped tables");
+      launch_copy_words(static_cast<const uint32_t*>(mapped), total / 4, reinterpret_cast<uint32_t*>(d), st);
+    } else {
+      ck(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, st), "upload tables");
+    }
     return d;
   }
 };
@@ -829,6 +837,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   const uint32_t big_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(items, 1), kMaxBig);
   uint4* big = ensure<uint4>(c->d_big, (uint64_t)big_cap * sizeof(uint4));
   unsigned long long* ctr = ensure<unsigned long long>(c->d_ctr, kLargeCtrWords * 8);
+  if (!c->ctr_zero) ck(cudaMemsetAsync(ctr, 0, kLargeCtrWords * 8, st), "memset counters");
   uint64_t* item_mask = ensure<uint64_t>(c->d_itemmask, items * 8);
   uint64_t* item_box = ensure<uint64_t>(c->d_itembox, items * 8);
 
@@ -897,7 +906,9 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   const size_t o_cpb = up1.add(cp_bricks.data(), (n + 1) * 8);
   size_t o_pc = 0;
   if (persist) o_pc = up1.add(p_chunk.data(), (n + 1) * 8);
-  unsigned char* t1 = up1.run(c, c->d_tables1, c->h_tables1, st);
+  // a lone stripe's jobs are kernel parameters
+  const bool tables = n > 1 || persist, by_kernel = os.mode == OUT_DEST;
+  unsigned char* t1 = tables ? up1.run(c->d_tables1, c->h_tables1, by_kernel, st) : nullptr;
   auto dp1 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t1 + off); };
   const VoxJob* d_vj = reinterpret_cast<const VoxJob*>(t1 + o_vj);
   const Stripe* d_str = reinterpret_cast<const Stripe*>(t1 + o_str);
@@ -914,11 +925,10 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     pj.ctr = ensure<unsigned long long>(c->d_pctr, kPersistCtrWords * 8);
     pj.lists = lists_of(vj[0]);
   }
-  c->leaf_zero = false;  // until the emission at the end of the sub-batch is queued
+  c->leaf_zero = c->ctr_zero = false;  // until the emission at the end of the sub-batch is queued
   run_launches(c, st, 0, [&] {
     {
       PhaseScope ph(c, PH_VOX, st);
-      ck(cudaMemsetAsync(ctr, 0, kLargeCtrWords * 8, st), "memset counters");
       if (persist) {
         ck(cudaMemsetAsync(pj.ctr, 0, kPersistCtrWords * 8, st), "memset persistent counters");
         launch_b_persist(pj, c->num_sms, c->persist_per_sm, st);
@@ -951,7 +961,8 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       // keeps refilling while it waits, and hold up the whole pipeline.
       launch_b_upper(d_str, n, max_upper, lvl_dev, ctr, reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords),
                      persist ? reinterpret_cast<const uint64_t*>(pj.ctr + kPersistTimeoutWord) : nullptr,
-                     reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords + 2), st);
+                     reinterpret_cast<uint64_t*>(lvl_dev + (uint64_t)n * kCountWords + 2),
+                     n == 1 ? &stripe[0] : nullptr, st);
     }
   }, pieces != nullptr);  // waits on the upload stream are not captured
   wait_level_counts(st, idle);
@@ -1145,7 +1156,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   const size_t o_cpay = up2.add(cp_pay.data(), (n + 1) * 8);
   const size_t o_clp = up2.add(cp_leafpay.beg.data(), (n + 1) * 8);
   const size_t o_em = up2.add(cp_emit.data(), (n + 1) * 8);
-  unsigned char* t2 = up2.run(c, c->d_tables2, c->h_tables2, st);
+  unsigned char* t2 = n > 1 ? up2.run(c->d_tables2, c->h_tables2, by_kernel, st) : nullptr;
   auto dp2 = [&](size_t off) { return reinterpret_cast<const uint64_t*>(t2 + off); };
   const VoxJob* d_vj2 = reinterpret_cast<const VoxJob*>(t2 + o_vj2);
   const EmitJob* d_ej = reinterpret_cast<const EmitJob*>(t2 + o_ej);
@@ -1169,11 +1180,12 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   run_launches(c, st, 2, [&] {
     {
       PhaseScope ph(c, PH_TREE, st);
-      launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, c->num_sms, sp1, se1, st);
-      if (any_levels) launch_b_upper_levels(d_str, d_ej, n, max_upper, st);
+      launch_b_emit(d_str, d_ej, dp2(o_em), n, cp_emit[n], any_levels, c->num_sms, ctr, sp1, se1, st);
+      if (any_levels) launch_b_upper_levels(d_str, d_ej, n, max_upper, sp1, se1, st);
     }
   });
   c->leaf_zero = true;
+  c->ctr_zero = cp_emit[n] > 0;  // an emission clears them
   ck(cudaEventRecord(c->ev_compute[slot], st), "event");
   if (os.mode == OUT_HOST) {
     // The records travel to the host while the next sub-batch computes, on the slot's own
@@ -1551,6 +1563,18 @@ void build_meshes(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, co
     sb.clear();
     budget_words = 0;
   };
+  // Device destinations: the first sub-batch ends at the mesh with the first quarter of the triangles, so
+  // that the upload of the others has work beside it (128 meshes of 161 MB: 3.54 ms in one sub-batch; 3.34,
+  // 3.20, 3.08 and 3.23 with a half, third, quarter and eighth).  Another sub-batch costs about 0.15 ms: the
+  // upload of 32 MB.
+  size_t first_end = meshes.size();
+  if (os.mode == OUT_DEST) {
+    auto bytes = [](const MeshWork& m) { return m.n_tris * (m.pl.binary ? 9 : 21) * 4; };
+    uint64_t all = 0, acc = 0;
+    for (const MeshWork& m : meshes) all += bytes(m);
+    if (all >= 64ull << 20)
+      for (first_end = 0; acc < all / 4; first_end++) acc += bytes(meshes[first_end]);
+  }
   for (uint32_t mi = 0; mi < meshes.size(); mi++) {
     MeshWork& m = meshes[mi];
     for (uint64_t s = 0; s < m.pl.n_stripes; s++) {
@@ -1567,7 +1591,7 @@ void build_meshes(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, co
       // host output: the first sub-batch takes an eighth of the budget, so that the copy
       // back (the longer part of a large build) starts after a short first compute
       const uint64_t cap = (os.mode == OUT_HOST && k == 0) ? budget / 8 : budget;
-      if (!sb.empty() && budget_words + w > cap) flush();
+      if (!sb.empty() && (budget_words + w > cap || (k == 0 && mi >= first_end))) flush();
       sb.push_back(StripeRef{mi, s, part, ibeg, cnt});
       budget_words += w;
     }

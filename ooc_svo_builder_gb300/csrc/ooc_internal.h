@@ -279,7 +279,8 @@ void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n,
 // into `counts` (mapped pinned host memory), then the number of large items (`large_ctr`: kCtr*) and,
 // when `code` is set, *code.
 void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts,
-                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st);
+                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out,
+                    const Stripe* single, cudaStream_t st);
 // The payloads of the stripes' leaves, into the data file: CTAs of kChunk threads, `ept` leaves each.
 void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
                            uint64_t ctas, uint32_t ept, const Stripe* sp, const EmitJob* se, cudaStream_t st);
@@ -287,9 +288,11 @@ void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const ui
 // levels and the marks.  CTAs of kTreeWarpsPerCta warps of EmitJob::bricks_per_warp non-empty bricks each.
 constexpr uint32_t kTreeWarpsPerCta = 8;
 void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                   bool levels, int num_sms, const Stripe* sp, const EmitJob* se, cudaStream_t st);
+                   bool levels, int num_sms, unsigned long long* large_ctr, const Stripe* sp, const EmitJob* se,
+                   cudaStream_t st);
 // With -levels in the batch: the averages of the levels above the bricks, one launch per level of more than
 // 4,096 cells and one for the rest, which also writes these levels' records and the roots' averages.
-void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st);
+void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, const Stripe* sp,
+                           const EmitJob* se, cudaStream_t st);
 
 }  // namespace ooc

@@ -258,11 +258,12 @@ template <int T, int K>
 __global__ void __launch_bounds__(T) kb_upper(const Stripe* __restrict__ stripes, uint32_t* __restrict__ counts,
                                               const unsigned long long* __restrict__ large_ctr,
                                               uint64_t* __restrict__ large_out, const uint64_t* __restrict__ code,
-                                              uint64_t* __restrict__ code_out) {
+                                              uint64_t* __restrict__ code_out, const __grid_constant__ Stripe p0) {
   pdl_enter();
   __shared__ Stripe sp;
   __shared__ uint32_t s_words[2][1024];
-  stage(sp, stripes[blockIdx.x]);
+  if (stripes) stage(sp, stripes[blockIdx.x]);
+  else stage(sp, p0);
   __syncthreads();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *large_out = large_ctr[kCtrLarge] + large_ctr[kCtrBig];  // zero: none
@@ -1236,15 +1237,16 @@ __device__ __forceinline__ void emit_cta(const Stripe& p, const EmitJob& e, uint
 
 template <bool SINGLE, bool LEVELS, int CTAS>
 __global__ void __launch_bounds__(kTreeThreads, CTAS) kb_emit(const Stripe* __restrict__ stripes,
-                                                                      const EmitJob* __restrict__ emits,
-                                                                      const uint64_t* __restrict__ cta_beg, uint32_t n,
-                                                                      Stripe p0, EmitJob e0) {
+                                                              const EmitJob* __restrict__ emits,
+                                                              const uint64_t* __restrict__ cta_beg, uint32_t n,
+                                                              Stripe p0, EmitJob e0, unsigned long long* large_ctr) {
   __shared__ uint64_t lut[256];  // child_offsets of every mask
   __shared__ WarpScratch ws[kTreeWarps];
   static_assert(kTreeThreads == 256, "one table entry per thread, and upper_node_ctas");
   static_assert(kWindow % 2 == 0 && kSlots % 2 == 0, "windows start on 16 bytes, every window's parity is the same");
   lut[threadIdx.x] = child_offsets(threadIdx.x);
   pdl_enter();
+  if (blockIdx.x == 0 && threadIdx.x < kLargeCtrWords) large_ctr[threadIdx.x] = 0ull;  // for the next build
   if constexpr (SINGLE) {
     __syncthreads();
     emit_cta<LEVELS>(p0, e0, blockIdx.x, ws, lut);
@@ -1287,12 +1289,13 @@ __device__ __forceinline__ void average_cell(const Stripe& p, const EmitJob& e, 
 
 // Level l of the stripes that have it above their bricks, one thread per cell (grid.y: the stripes).
 __global__ void __launch_bounds__(256) kb_upper_avg(const Stripe* __restrict__ stripes, const EmitJob* __restrict__ emits,
-                                                    uint32_t n, int l) {
+                                                    uint32_t n, int l, const __grid_constant__ Stripe p0,
+                                                    const __grid_constant__ EmitJob e0) {
   pdl_enter();
   const uint32_t z = blockIdx.x * 256u + threadIdx.x;
   for (uint32_t s = blockIdx.y; s < n; s += gridDim.y) {
-    const Stripe& p = stripes[s];
-    const EmitJob& e = emits[s];
+    const Stripe& p = stripes ? stripes[s] : p0;
+    const EmitJob& e = stripes ? emits[s] : e0;
     if (e.levels && l < p.U && z < (1u << (3 * l)) && p.wpre[upper_words(p.U)].x) average_cell(p, e, l, z);
   }
 }
@@ -1303,10 +1306,11 @@ __global__ void __launch_bounds__(256) kb_upper_avg(const Stripe* __restrict__ s
 constexpr uint32_t kTopThreads = 512;  // the cells of level 3
 template <uint32_t CTAS>
 __global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(kTopThreads)
-    kb_upper_top(const Stripe* __restrict__ stripes, const EmitJob* __restrict__ emits, int l_hi) {
+    kb_upper_top(const Stripe* __restrict__ stripes, const EmitJob* __restrict__ emits, int l_hi,
+                 const __grid_constant__ Stripe p0, const __grid_constant__ EmitJob e0) {
   pdl_enter();
-  const Stripe& p = stripes[blockIdx.x / CTAS];
-  const EmitJob& e = emits[blockIdx.x / CTAS];
+  const Stripe& p = stripes ? stripes[blockIdx.x / CTAS] : p0;
+  const EmitJob& e = stripes ? emits[blockIdx.x / CTAS] : e0;
   if (p.U == 0 || p.wpre[upper_words(p.U)].x == 0) return;
   const uint32_t t = (blockIdx.x % CTAS) * kTopThreads + threadIdx.x;
   if (e.levels) {
@@ -1359,18 +1363,14 @@ void launch_b_bricks(const Stripe* stripes, const uint64_t* cta_beg, uint32_t n,
 }
 
 void launch_b_upper(const Stripe* stripes, uint32_t n, int max_upper, uint32_t* counts,
-                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out, cudaStream_t st) {
+                    const unsigned long long* large_ctr, uint64_t* large_out, const uint64_t* code, uint64_t* code_out,
+                    const Stripe* single, cudaStream_t st) {
   if (n == 0) return;
   KScope k("upper", st);
-  // 128 threads cover level 4's 128 words at eight a thread with room for smaller CTAs to share an SM;
-  // larger stripes have 1,024 and 8,192 words to scan
   // level U has 8192, 1024, 128, ... words: one round of one word a thread, or eight
-  if (max_upper >= 6)
-    launch_k(kb_upper<1024, 8>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
-  else if (max_upper == 5)
-    launch_k(kb_upper<1024, 1>, dim3(n), dim3(1024), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
-  else
-    launch_k(kb_upper<128, 1>, dim3(n), dim3(128), 0, st, stripes, counts, large_ctr, large_out, code, code_out);
+  auto* kern = max_upper >= 6 ? kb_upper<1024, 8> : (max_upper == 5 ? kb_upper<1024, 1> : kb_upper<128, 1>);
+  launch_k(kern, dim3(n), dim3(max_upper >= 5 ? 1024 : 128), 0, st, single ? nullptr : stripes, counts, large_ctr,
+           large_out, code, code_out, stripe_or_zero(single));
 }
 
 void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n,
@@ -1382,7 +1382,8 @@ void launch_b_leaf_payload(const Stripe* stripes, const EmitJob* emits, const ui
 }
 
 void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* cta_beg, uint32_t n, uint64_t ctas,
-                   bool levels, int num_sms, const Stripe* sp, const EmitJob* se, cudaStream_t st) {
+                   bool levels, int num_sms, unsigned long long* large_ctr, const Stripe* sp, const EmitJob* se,
+                   cudaStream_t st) {
   if (ctas == 0) return;
   KScope k("emit", st);
   // With -levels two CTAs fit an SM only with 128 registers a thread, some of them spilled: where one CTA
@@ -1392,20 +1393,24 @@ void launch_b_emit(const Stripe* stripes, const EmitJob* emits, const uint64_t* 
                : !sp   ? kb_emit<false, true, 2>
                        : (ctas <= (uint64_t)num_sms ? kb_emit<true, true, 1> : kb_emit<true, true, 2>);
   launch_k(kern, dim3((unsigned)ctas), dim3(kTreeThreads), 0, st, stripes, emits, cta_beg, n, stripe_or_zero(sp),
-           emit_or_zero(se));
+           emit_or_zero(se), large_ctr);
 }
 
-void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, cudaStream_t st) {
+void launch_b_upper_levels(const Stripe* stripes, const EmitJob* emits, uint32_t n, int max_upper, const Stripe* sp,
+                           const EmitJob* se, cudaStream_t st) {
   if (n == 0 || max_upper == 0) return;
   constexpr int kTop = 4;  // 4,096 cells: one per thread of eight CTAs
+  if (sp) stripes = nullptr;
   for (int l = max_upper - 1; l > kTop; l--) {
     KScope k("upper_average", st);
-    launch_k(kb_upper_avg, dim3(1u << (3 * l - 8), n < 4096u ? n : 4096u), dim3(256), 0, st, stripes, emits, n, l);
+    launch_k(kb_upper_avg, dim3(1u << (3 * l - 8), n < 4096u ? n : 4096u), dim3(256), 0, st, stripes, emits, n, l,
+             stripe_or_zero(sp), emit_or_zero(se));
   }
   KScope k("upper_top", st);
   // up to level 2 (64 cells, U = 3) one CTA; a cluster's barriers cost more there
-  if (max_upper <= 3) launch_k(kb_upper_top<1>, dim3(n), dim3(kTopThreads), 0, st, stripes, emits, kTop);
-  else launch_k(kb_upper_top<8>, dim3(n * 8u), dim3(kTopThreads), 0, st, stripes, emits, kTop);
+  const bool one = max_upper <= 3;
+  launch_k(one ? kb_upper_top<1> : kb_upper_top<8>, dim3(one ? n : n * 8u), dim3(kTopThreads), 0, st, stripes, emits, kTop,
+           stripe_or_zero(sp), emit_or_zero(se));
 }
 
 }  // namespace ooc
