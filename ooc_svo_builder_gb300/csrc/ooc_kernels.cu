@@ -792,28 +792,30 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
     c11 &= !(__fadd_rn(__fadd_rn(a1, b1), s.dxy[k]) < 0.0f);
   }
   // the plane value's parts per column (see walk_line), and the halves of the YZ and ZX dot
-  // products that do not depend on z
+  // products that do not depend on z; two sums go through one instruction (F2): the YZ and ZX
+  // tests of a z as one pair, the plane values of two z as another
   const float n0x0 = __fmul_rn(s.n[0], px0), n0x1 = __fmul_rn(s.n[0], px1);
   const float n1y0 = __fmul_rn(s.n[1], py0), n1y1 = __fmul_rn(s.n[1], py1);
   // w = z: (x + y) + z, q the sum of the first two; otherwise (z + q) + r
   const bool z_last = W == 2;
-  float q00, q01, q10, q11, r00 = 0.0f, r01 = 0.0f, r10 = 0.0f, r11 = 0.0f;
+  float q00, q01, q10, q11, r0 = 0.0f, r1 = 0.0f;
   if (z_last) {
     q00 = __fadd_rn(n0x0, n1y0), q01 = __fadd_rn(n0x0, n1y1), q10 = __fadd_rn(n0x1, n1y0), q11 = __fadd_rn(n0x1, n1y1);
   } else if (W == 0) {
     q00 = n0x0, q01 = n0x0, q10 = n0x1, q11 = n0x1;
-    r00 = n1y0, r01 = n1y1, r10 = n1y0, r11 = n1y1;
+    r0 = n1y0, r1 = n1y1;  // of y
   } else {
     q00 = n1y0, q01 = n1y1, q10 = n1y0, q11 = n1y1;
-    r00 = n0x0, r01 = n0x0, r10 = n0x1, r11 = n0x1;
+    r0 = n0x0, r1 = n0x1;  // of x
   }
-  float yz_y0[3], yz_y1[3], zx_x0[3], zx_x1[3];
+  const F2 nz = minus_zero(j.u);
+  F2 cz[3], c0[3], c1[3], cd[3];  // ZX and YZ: of z, of (x_0, y_0), of (x_1, y_1), rest
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    yz_y0[k] = __fmul_rn(s.yz[k][0], py0);
-    yz_y1[k] = __fmul_rn(s.yz[k][0], py1);
-    zx_x0[k] = __fmul_rn(s.zx[k][1], px0);
-    zx_x1[k] = __fmul_rn(s.zx[k][1], px1);
+    cz[k] = f2(s.zx[k][0], s.yz[k][1]);
+    c0[k] = f2(__fmul_rn(s.zx[k][1], px0), __fmul_rn(s.yz[k][0], py0));
+    c1[k] = f2(__fmul_rn(s.zx[k][1], px1), __fmul_rn(s.yz[k][0], py1));
+    cd[k] = f2(s.dzx[k], s.dyz[k]);
   }
   // Morton bits: the rotated axes' shifts are 0, 1, 2 turned by W
   const uint32_t xs = W == 2 ? 0u : (W == 0 ? 1u : 2u), ys = W == 2 ? 1u : (W == 0 ? 2u : 0u), zs = (uint32_t)W;
@@ -829,35 +831,44 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
   for (uint32_t zc = 0; zc < bz; zc += 2) {
     const bool z1ok = zc + 1 < bz;
     const float pz0 = __fmul_rn((float)(lo[2] + (int)zc), j.u), pz1 = __fmul_rn((float)(lo[2] + (int)zc + 1), j.u);
-    bool y0z0 = true, y0z1 = z1ok, y1z0 = true, y1z1 = z1ok;  // YZ over (y_j, z_k)
-    bool z0x0 = true, z0x1 = true, z1x0 = z1ok, z1x1 = z1ok;  // ZX over (z_k, x_i)
+    bool y0z0, y0z1, y1z0, y1z1;  // YZ over (y_j, z_k)
+    bool z0x0, z0x1, z1x0, z1x1;  // ZX over (z_k, x_i)
+    {
+      // dot((-e.x, e.z) * fy, (p.z, p.x)) + d and dot((-e.z, e.y) * fx, (p.y, p.z)) + d
+      const F2 pzz0 = f2(pz0, pz0), pzz1 = f2(pz1, pz1);
+      auto edges = [&](F2 pzz, const F2* c, bool& zx, bool& yz) {  // a NaN passes
+        float a[3], b[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-      // dot((-e.z, e.y) * fx, (p.y, p.z)) + d and dot((-e.x, e.z) * fy, (p.z, p.x)) + d
-      const float e0 = __fmul_rn(s.yz[k][1], pz0), e1 = __fmul_rn(s.yz[k][1], pz1);
-      y0z0 &= !(__fadd_rn(__fadd_rn(yz_y0[k], e0), s.dyz[k]) < 0.0f);
-      y0z1 &= !(__fadd_rn(__fadd_rn(yz_y0[k], e1), s.dyz[k]) < 0.0f);
-      y1z0 &= !(__fadd_rn(__fadd_rn(yz_y1[k], e0), s.dyz[k]) < 0.0f);
-      y1z1 &= !(__fadd_rn(__fadd_rn(yz_y1[k], e1), s.dyz[k]) < 0.0f);
-      const float f0 = __fmul_rn(s.zx[k][0], pz0), f1 = __fmul_rn(s.zx[k][0], pz1);
-      z0x0 &= !(__fadd_rn(__fadd_rn(f0, zx_x0[k]), s.dzx[k]) < 0.0f);
-      z0x1 &= !(__fadd_rn(__fadd_rn(f0, zx_x1[k]), s.dzx[k]) < 0.0f);
-      z1x0 &= !(__fadd_rn(__fadd_rn(f1, zx_x0[k]), s.dzx[k]) < 0.0f);
-      z1x1 &= !(__fadd_rn(__fadd_rn(f1, zx_x1[k]), s.dzx[k]) < 0.0f);
+        for (int k = 0; k < 3; k++) split(add2(add2(mul2(cz[k], pzz, nz), c[k]), cd[k]), a[k], b[k]);
+        zx = !(fminf(fminf(a[0], a[1]), a[2]) < 0.0f);
+        yz = !(fminf(fminf(b[0], b[1]), b[2]) < 0.0f);
+      };
+      edges(pzz0, c0, z0x0, y0z0);
+      edges(pzz0, c1, z0x1, y1z0);
+      edges(pzz1, c0, z1x0, y0z1);
+      edges(pzz1, c1, z1x1, y1z1);
+      y0z1 &= z1ok, y1z1 &= z1ok;
     }
     // the plane test: (n.p + d1) (n.p + d2) > 0 fails
-    const float g0 = __fmul_rn(s.n[2], pz0), g1 = __fmul_rn(s.n[2], pz1);
-    float v000 = __fadd_rn(g0, q00), v001 = __fadd_rn(g1, q00), v010 = __fadd_rn(g0, q01), v011 = __fadd_rn(g1, q01);
-    float v100 = __fadd_rn(g0, q10), v101 = __fadd_rn(g1, q10), v110 = __fadd_rn(g0, q11), v111 = __fadd_rn(g1, q11);
-    if (!z_last) {
-      v000 = __fadd_rn(v000, r00), v001 = __fadd_rn(v001, r00), v010 = __fadd_rn(v010, r01), v011 = __fadd_rn(v011, r01);
-      v100 = __fadd_rn(v100, r10), v101 = __fadd_rn(v101, r10), v110 = __fadd_rn(v110, r11), v111 = __fadd_rn(v111, r11);
-    }
-    auto plane = [&](float nd) { return !(__fmul_rn(__fadd_rn(nd, s.d1), __fadd_rn(nd, s.d2)) > 0.0f); };
-    const bool p000 = c00 & y0z0 & z0x0 & plane(v000), p001 = c00 & y0z1 & z1x0 & plane(v001);
-    const bool p010 = c01 & y1z0 & z0x0 & plane(v010), p011 = c01 & y1z1 & z1x0 & plane(v011);
-    const bool p100 = c10 & y0z0 & z0x1 & plane(v100), p101 = c10 & y0z1 & z1x1 & plane(v101);
-    const bool p110 = c11 & y1z0 & z0x1 & plane(v110), p111 = c11 & y1z1 & z1x1 & plane(v111);
+    const F2 g = mul2(f2(s.n[2], s.n[2]), f2(pz0, pz1), nz);
+    auto plane = [&](float q, float r, bool& z0, bool& z1) {
+      F2 v = add2(g, f2(q, q));
+      if (!z_last) v = add2(v, f2(r, r));
+      float a, b;
+      split(mul2(add2(v, f2(s.d1, s.d1)), add2(v, f2(s.d2, s.d2))), a, b);
+      z0 = !(a > 0.0f);
+      z1 = !(b > 0.0f);
+    };
+    bool v000, v001, v010, v011, v100, v101, v110, v111;
+    const bool of_y = W == 0;
+    plane(q00, r0, v000, v001);
+    plane(q01, of_y ? r1 : r0, v010, v011);
+    plane(q10, of_y ? r0 : r1, v100, v101);
+    plane(q11, r1, v110, v111);
+    const bool p000 = c00 & y0z0 & z0x0 & v000, p001 = c00 & y0z1 & z1x0 & v001;
+    const bool p010 = c01 & y1z0 & z0x0 & v010, p011 = c01 & y1z1 & z1x0 & v011;
+    const bool p100 = c10 & y0z0 & z0x1 & v100, p101 = c10 & y0z1 & z1x1 & v101;
+    const bool p110 = c11 & y1z0 & z0x1 & v110, p111 = c11 & y1z1 & z1x1 & v111;
     const uint32_t mz1 = ((mz | ~ZBITS) + z1) & ZBITS;
     if (j.item_mask) {  // payload: two bits per column
       const uint32_t c00b = (p000 ? 1u : 0u) | (p001 ? 2u : 0u), c01b = (p010 ? 1u : 0u) | (p011 ? 2u : 0u);
