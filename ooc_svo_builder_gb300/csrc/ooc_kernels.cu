@@ -608,10 +608,18 @@ __device__ __forceinline__ void walk_setup(const VoxJob& j, const TriVerts& tv, 
   r.stripe = stripe;
 }
 
+// spread3_10 of every coordinate, in shared memory: three lookups a line instead of three times eight
+// instructions (4.2 and 4.0 ms on the 20M-triangle soup).  By all threads of a CTA.
+__device__ __forceinline__ void fill_spread(uint32_t* spread) {
+  for (uint32_t i = threadIdx.x; i < 1024u; i += blockDim.x) spread[i] = spread3_10(i);
+  __syncthreads();
+}
+
 // Line (ra, rb) of a large item: pass 0 sets its bits, pass 1 offers the triangle to every
 // voxel it passes.  The line's own projection has passed.
 template <int PASS>
-__device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, uint32_t ra, uint32_t rb) {
+__device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, uint32_t ra, uint32_t rb,
+                                          const uint32_t* spread) {
   const float u = r.u, fa = __fmul_rn((float)(r.alo + (int)ra), u), fb = __fmul_rn((float)(r.blo + (int)rb), u);
   const uint32_t shape = r.shape;
   const int W = (int)(shape >> 11) & 3, w0 = r.wlo, w1 = r.whi;
@@ -641,7 +649,7 @@ __device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, ui
   };
   // stripe-local Morton bits: the fixed coordinates, and the walk coordinate moving by carries
   const uint32_t la = (r.local & 1023u) + ra, lb = ((r.local >> 10) & 1023u) + rb, lw = r.local >> 20;
-  const uint32_t mab = (spread3_10(la) << (W == 2 ? 0 : W + 1)) | (spread3_10(lb) << (W == 0 ? 2 : W - 1));
+  const uint32_t mab = (spread[la] << (W == 2 ? 0 : W + 1)) | (spread[lb] << (W == 0 ? 2 : W - 1));
   const uint32_t wbits = 0x09249249u << W;
   auto emit = [&](uint32_t mw) {
     const uint32_t m = mab | mw;
@@ -716,7 +724,7 @@ __device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, ui
     split(mul2(add2(v, f2(d1, d1)), add2(v, f2(d2, d2))), pu, pd);
   }
   const bool up = walk >= 0 && start < w1 && !(pu > 0.0f), down = walk <= 0 && start > w0 && !(pd > 0.0f);
-  const uint32_t ms = spread3_10(lw + (uint32_t)(start - w0)) << W;
+  const uint32_t ms = spread[lw + (uint32_t)(start - w0)] << W;
   uint32_t mu = ((ms | ~wbits) + (1u << W)) & wbits, md = (ms - (1u << W)) & wbits;
   const bool on_s = rest(fs), on_u = up & rest(fu), on_d = down & rest(fd);
   if (PASS == 0) {  // one store per leaf word
@@ -1012,9 +1020,9 @@ __device__ __forceinline__ void vox_small_win_item(const VoxJob& j, uint64_t i) 
 // pass go onto a stack from which 32 at a time are walked, one per lane.  So the lanes stay full
 // whatever the items' sizes.
 //
-// Bound by issue (no FMA), the walk three fifths of it, the lines' tests a quarter.  4.2 ms on the
-// 20M-triangle soup at gridsize 4096 (8.8 with one item per warp at a time), 0.81 (1.51) ms on 4M triangles
-// at 1024, 0.63 + 0.58 ms for the two passes of 128 meshes.  Of the rest a start at the voxel nearest the
+// Bound by issue (no FMA), the walk three fifths of it, the lines' tests a quarter.  4.0 ms on the
+// 20M-triangle soup at gridsize 4096 (8.8 with one item per warp at a time), 0.77 (1.51) ms on 4M triangles
+// at 1024, 0.65 + 0.60 ms for the two passes of 128 meshes.  Of the rest a start at the voxel nearest the
 // run's middle, the voxel's neighbours tested as a pair, two projections per instruction, setting up the
 // turned triangle and finding a line's item with one reduction gave 5.3 -> 4.2, 1.01 -> 0.81 and 0.80 ->
 // 0.63.  Eight items a warp are 2 to 4% slower; 32 are 2% faster on the soups and 5 to 15% slower on the
@@ -1031,7 +1039,7 @@ struct WalkScratch {
 template <int PASS, bool SINGLE>
 __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, const VoxJob& j0, bool has, uint32_t item,
                                            uint32_t stripe, uint32_t first, uint32_t most, uint32_t parts, int lane,
-                                           WalkScratch& sm) {
+                                           WalkScratch& sm, const uint32_t* spread) {
   const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u;
   uint32_t n = 0;
   uint64_t t = 0;
@@ -1059,7 +1067,7 @@ __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, cons
   __syncwarp();
   auto walk = [&](uint32_t e) {
     const WalkItem& r = sm.item[e & (kWalkItems - 1u)];
-    walk_line<PASS>(SINGLE ? j0 : jobs[r.stripe], r, (e >> kWalkBits) & 1023u, e >> (kWalkBits + 10));
+    walk_line<PASS>(SINGLE ? j0 : jobs[r.stripe], r, (e >> kWalkBits) & 1023u, e >> (kWalkBits + 10), spread);
   };
   uint32_t cnt = 0, begun = 0;  // lines on the stack; items that began in an earlier round
 #pragma unroll 1
@@ -1100,7 +1108,7 @@ __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, cons
 // then the others, as many at a time as leave every warp two helpings.
 template <int PASS, bool SINGLE>
 __device__ __forceinline__ void walk_lists(const VoxJob* __restrict__ jobs, const VoxJob& j0, const LargeLists& L, int lane,
-                                           WalkScratch& sm) {
+                                           WalkScratch& sm, const uint32_t* spread) {
   const unsigned long long n = __ldcg(L.ctr + kCtrLarge), packed = __ldcg(L.ctr + kCtrBig);
   const uint32_t nb = min((uint32_t)(packed & ((1u << kBigCountBits) - 1u)), L.big_cap);
   uint64_t tasks = 0;
@@ -1141,7 +1149,7 @@ __device__ __forceinline__ void walk_lists(const VoxJob* __restrict__ jobs, cons
       item = (uint32_t)e, stripe = (uint32_t)(e >> 32), first = (uint32_t)(t + (uint32_t)lane - i * parts);
       if (parts > 1) ps = parts;
     }
-    walk_items<PASS, SINGLE>(jobs, j0, has, item, stripe, first, most, ps, lane, sm);
+    walk_items<PASS, SINGLE>(jobs, j0, has, item, stripe, first, most, ps, lane, sm, spread);
     if (!big) {
       if (lane == 0) t = (uint64_t)warps * chunk + atomicAdd(L.ctr + kCtrGrab + 16 + 32 * PASS, (unsigned long long)chunk);
       t = __shfl_sync(FULL, t, 0);
@@ -1153,7 +1161,10 @@ template <int PASS, bool SINGLE>
 __global__ void __launch_bounds__(256, 4) kb_vox_large(const VoxJob* __restrict__ jobs, LargeLists lists, VoxJob j0) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char walk_smem[];
-  walk_lists<PASS, SINGLE>(jobs, j0, lists, threadIdx.x & 31, reinterpret_cast<WalkScratch*>(walk_smem)[threadIdx.x >> 5]);
+  __shared__ uint32_t s_spread[1024];
+  fill_spread(s_spread);
+  walk_lists<PASS, SINGLE>(jobs, j0, lists, threadIdx.x & 31, reinterpret_cast<WalkScratch*>(walk_smem)[threadIdx.x >> 5],
+                           s_spread);
 }
 
 // n words into `dst` (mapped pinned host memory): small results the host waits for
@@ -1288,6 +1299,8 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
   pdl_enter();
   __shared__ VoxJob s_job[8];
   __shared__ WalkScratch s_walk[8];
+  __shared__ uint32_t s_spread[1024];
+  fill_spread(s_spread);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint64_t C = pj.chunk_beg[pj.n];
   uint32_t job_s = ~0u;  // the stripe staged in s_job[w]
@@ -1322,7 +1335,7 @@ __global__ void __launch_bounds__(256, 4) kb_persist(PersistJob pj) {
   }
   if (!__shfl_sync(FULL, ok, 0)) return;
   __syncwarp();
-  walk_lists<0, false>(pj.jobs, s_job[w], pj.lists, lane, s_walk[w]);
+  walk_lists<0, false>(pj.jobs, s_job[w], pj.lists, lane, s_walk[w], s_spread);
 }
 
 }  // namespace
