@@ -132,8 +132,8 @@ struct ooc_ctx {
   float phase_ms[kPhases] = {0, 0, 0, 0, 0, 0};
   unsigned long long launches = 0;
   ooc::LaunchState lstate;  // this context's launch count and timing hooks, installed per API call
-  DevBuf d_tris, d_hist, d_axis, d_upper, d_brick, d_innerlocal, d_uppercache, d_winners, d_large,
-      d_big, d_ctr, d_nodes, d_data, d_recs, d_itemmask, d_itembox, d_leaf, d_touch, d_local, d_woff;
+  DevBuf d_tris, d_hist, d_axis, d_upper, d_brick, d_uppercache, d_winners, d_large,
+      d_big, d_ctr, d_nodes, d_data, d_recs, d_itemmask, d_itembox, d_leaf, d_touch, d_blocks;
   // persistent occupancy passes (ooc_tuning::persistent): their counters, and the CTAs per SM
   DevBuf d_pctr;
   int persist_per_sm = -1;
@@ -787,11 +787,10 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   // ---- geometry of every stripe ----
   std::vector<Stripe> stripe(n);
   std::vector<VoxJob> vj(n);
-  std::vector<uint64_t> item_beg(n + 1, 0), leaf_beg(n, 0), touch_beg(n, 0), local_beg(n, 0), upper_beg(n, 0),
+  std::vector<uint64_t> item_beg(n + 1, 0), leaf_beg(n, 0), touch_beg(n, 0), block_beg(n, 0), upper_beg(n, 0),
       word_beg(n, 0), brick_beg(n, 0);
-  uint64_t leaf_w = 0, tbytes = 0, nlocal = 0, upper_w = 0, pre_w = 0, bricks = 0, items = 0;
+  uint64_t leaf_w = 0, tbytes = 0, n_blocks = 0, upper_w = 0, pre_w = 0, bricks = 0, items = 0;
   int max_upper = 0;
-  bool payload_levels = false;
   for (uint32_t s = 0; s < n; s++) {
     const StripeRef& r = sb[s];
     const Plan& mp = meshes[r.mesh].pl;
@@ -806,9 +805,8 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     leaf_w += leaf_words(S.depth);
     touch_beg[s] = tbytes;
     if (S.depth >= kMarkDepth) tbytes += touch_bytes(S.depth);
-    local_beg[s] = nlocal;  // the ranks of leaf bits: payload stripes only
-    if (!mp.binary) nlocal += leaf_blocks(S.depth);
-    payload_levels = payload_levels || (!mp.binary && mp.levels);
+    block_beg[s] = n_blocks;  // the ranks of leaf bits: payload stripes only
+    if (!mp.binary) n_blocks += leaf_blocks(S.depth);
     upper_beg[s] = upper_w;
     upper_w += upper_off(S.U + 1);
     word_beg[s] = pre_w;  // one entry past the last word, in whole groups of eight
@@ -823,9 +821,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   if (leaf_w * 4 > c->d_leaf.cap || tbytes > c->d_touch.cap) c->leaf_zero = false;
   uint32_t* leaf = ensure<uint32_t>(c->d_leaf, leaf_w * 4);
   uint8_t* touch = ensure<uint8_t>(c->d_touch, tbytes);
-  uint32_t* local = nlocal ? ensure<uint32_t>(c->d_local, nlocal * 4) : nullptr;
-  uint64_t* woff = nlocal ? ensure<uint64_t>(c->d_woff, nlocal * 8) : nullptr;
-  uint16_t* inner_local = payload_levels ? ensure<uint16_t>(c->d_innerlocal, nlocal * 2) : nullptr;
+  LeafBlock* blocks = n_blocks ? ensure<LeafBlock>(c->d_blocks, n_blocks * sizeof(LeafBlock)) : nullptr;
   if (!c->leaf_zero) {
     ck(cudaMemsetAsync(leaf, 0, c->d_leaf.cap, st), "memset leaf levels");
     ck(cudaMemsetAsync(touch, 0, c->d_touch.cap, st), "memset leaf marks");
@@ -852,9 +848,8 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     S.wpre = brick + word_beg[s];
     S.bpre = brick + pre_w + brick_beg[s];
     S.bunits = reinterpret_cast<uint8_t*>(brick + pre_w + bricks) + brick_beg[s];
-    S.local = m.pl.binary ? nullptr : local + local_beg[s];
-    S.woff = m.pl.binary ? nullptr : woff + local_beg[s];
-    S.inner_local = !m.pl.binary && m.pl.levels ? inner_local + local_beg[s] : nullptr;
+    S.blocks = m.pl.binary ? nullptr : blocks + block_beg[s];
+    S.block_inner = m.pl.levels;
     VoxJob& j = vj[s];
     std::memset(&j, 0, sizeof(j));
     uint32_t pa[3], sa[3];
@@ -878,8 +873,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     j.leafbits = S.leaf;
     j.leaftouch = S.touch;
     j.wpre = S.wpre;
-    j.leaflocal = S.local;
-    j.leafwoff = S.woff;
+    j.blocks = S.blocks;
     j.large = large;
     j.big = big;
     j.ctr = ctr;
@@ -1848,10 +1842,10 @@ void ooc_ctx_destroy(ooc_ctx* c) {
   for (cudaStream_t rs : c->ring_stream)
     if (rs) cudaStreamSynchronize(rs);
   if (c->h2d_stream) cudaStreamSynchronize(c->h2d_stream);
-  DevBuf* bufs[] = {&c->d_tris, &c->d_hist, &c->d_axis, &c->d_upper, &c->d_brick, &c->d_innerlocal, &c->d_uppercache,
+  DevBuf* bufs[] = {&c->d_tris, &c->d_hist, &c->d_axis, &c->d_upper, &c->d_brick, &c->d_uppercache,
                     &c->d_winners, &c->d_large, &c->d_big, &c->d_ctr, &c->d_nodes,
-                    &c->d_data, &c->d_recs, &c->d_itemmask, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_local,
-                    &c->d_woff, &c->d_pctr, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
+                    &c->d_data, &c->d_recs, &c->d_itemmask, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_blocks,
+                    &c->d_pctr, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
                     &c->d_group[1], &c->d_stream_mat, &c->d_stream_part, &c->d_stream_base, &c->d_part_off};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);

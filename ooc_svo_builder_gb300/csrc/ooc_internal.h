@@ -45,6 +45,13 @@ __host__ __device__ inline uint32_t upper_words(int l) { return l < 2 ? 1u : 1u 
 __host__ __device__ inline uint64_t leaf_words(int depth) { return depth < 3 ? 8ull : 1ull << (3 * depth - 5); }
 __host__ __device__ inline uint64_t leaf_blocks(int depth) { return leaf_words(depth) / 8; }
 
+// What the rank of a leaf bit takes from its block of 256, in one load.
+struct __align__(16) LeafBlock {
+  uint64_t woff;   // byte k = set bits in the block's words 0..k-1
+  uint32_t local;  // set bits before the block within its 32 bricks
+  uint32_t inner;  // the leaves' parents and nodes of 64 leaf bits before the block within its brick
+};
+
 // The leaf levels and the marks live in buffers that are all zero between
 // builds: the voxelization of a stripe of 512^3 voxels and more marks every
 // 256-bit leaf block it sets a bit in (`touch`, one byte per block, written with
@@ -62,11 +69,8 @@ struct Stripe {
   uint2* wpre;       // .x leaves, .y inner nodes below the bricks (upper_words(U) + 1 entries)
   uint2* bpre;
   uint8_t* bunits;   // per brick: its child mask (1 for a brick of fewer levels); like bpre, whole words
-  // payload stripes, for the rank of a leaf bit (else NULL):
-  uint32_t* local;   // per leaf block: set bits before it within its 32 bricks (written for marked blocks)
-  uint64_t* woff;    // per leaf block: byte k = set bits in its words 0..k-1
-  uint16_t* inner_local;  // per leaf block, payload stripes with -levels (else NULL): the leaves' parents and nodes of
-                          // 64 leaf bits before it within its brick (written for marked blocks)
+  LeafBlock* blocks; // per leaf block of a payload stripe (else NULL; written for marked blocks)
+  int block_inner;   // whether LeafBlock::inner is wanted (-levels)
 };
 
 // Mark bytes of a stripe's leaf level, padded to 16 bytes.
@@ -91,8 +95,7 @@ struct VoxJob {
   uint8_t* leaftouch;       // byte per 256-bit block of leafbits, set when a bit of the block is (may be NULL)
   // pass B (payload winners)
   const uint2* wpre;        // Stripe::wpre
-  const uint32_t* leaflocal;// Stripe::local
-  const uint64_t* leafwoff; // Stripe::woff
+  const LeafBlock* blocks;  // Stripe::blocks
   unsigned long long* winners;  // per leaf: min of triangle index << 32 | its local Morton code
   // the list of large items (shared by the stripes of a sub-batch)
   unsigned long long* large; // items of one task each: item | stripe << 32 (room for every item)

@@ -378,8 +378,10 @@ __device__ __forceinline__ void set_leaf(const VoxJob& j, uint32_t w, uint32_t a
 // within the block (all from the brick pass), and one popcount.
 __device__ __forceinline__ uint32_t leaf_rank(const VoxJob& j, uint32_t b) {
   const uint32_t blk = b >> 8;
-  const uint32_t before = (uint32_t)(j.leafwoff[blk] >> (8 * ((b >> 5) & 7u))) & 0xffu;
-  return j.wpre[b >> 17].x + j.leaflocal[blk] + before + __popc(j.leafbits[b >> 5] & ((1u << (b & 31)) - 1u));
+  const uint4 r = __ldg(reinterpret_cast<const uint4*>(j.blocks) + blk);
+  const uint64_t woff = (uint64_t)r.x | ((uint64_t)r.y << 32);
+  const uint32_t before = (uint32_t)(woff >> (8 * ((b >> 5) & 7u))) & 0xffu;
+  return j.wpre[b >> 17].x + r.z + before + __popc(j.leafbits[b >> 5] & ((1u << (b & 31)) - 1u));
 }
 
 // Offers triangle t to voxel m: the smallest index wins, and the voxel's Morton code

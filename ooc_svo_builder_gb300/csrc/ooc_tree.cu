@@ -135,10 +135,6 @@ __device__ __forceinline__ WordCount count_bricks(const Stripe& p, uint32_t x0, 
     const uint32_t nonempty = __ballot_sync(FULL, l != 0);
     const uint32_t il = warp_inclusive(l), ii = warp_inclusive(in);
     const uint32_t el = carry_l + il - l, ei = carry_i + ii - in;
-    if (p.local && j < total) {
-      p.local[blk] = el;
-      p.woff[blk] = wo;
-    }
     const uint32_t src = excl - round;  // where this lane's brick starts, when it does in this round
     const uint32_t vl = __shfl_sync(FULL, el, (int)(src & 31u)), vi = __shfl_sync(FULL, ei, (int)(src & 31u));
     if (excl >= round && src < 32u) {
@@ -146,9 +142,11 @@ __device__ __forceinline__ WordCount count_bricks(const Stripe& p, uint32_t x0, 
       my_i = vi;
       if (!p.touch) seen = (nonempty >> src) & marked;
     }
-    if (p.inner_local) {
-      const uint32_t brick_i = __shfl_sync(FULL, my_i, (int)o);  // before the block's brick
-      if (j < total) p.inner_local[blk] = (uint16_t)(ei - brick_i);
+    if (p.blocks) {
+      uint32_t inner = 0;
+      if (p.block_inner) inner = ei - __shfl_sync(FULL, my_i, (int)o);  // after those before the block's brick
+      if (j < total)
+        reinterpret_cast<uint4*>(p.blocks)[blk] = make_uint4((uint32_t)wo, (uint32_t)(wo >> 32), el, inner);
     }
     carry_l += __shfl_sync(FULL, il, 31);
     carry_i += __shfl_sync(FULL, ii, 31);
@@ -209,10 +207,10 @@ __device__ __forceinline__ void count_cta(const Stripe& p, uint32_t cta) {
     }
     all |= s_bits[k] << (8 * k);
   }
-  if (p.local) {  // the blocks' ranks count from the word's start
+  if (p.blocks) {  // the blocks' ranks count from the word's start
     const uint32_t b0 = x0 * 16u, n = (uint32_t)min((uint64_t)128, leaf_blocks(p.depth) - min(leaf_blocks(p.depth), (uint64_t)b0));
     if (l)
-      for (uint32_t k = (uint32_t)lane; k < n; k += 32u) p.local[b0 + k] += l;
+      for (uint32_t k = (uint32_t)lane; k < n; k += 32u) p.blocks[b0 + k].local += l;
   }
   if (lane < 8) {
     p.bpre[x0 + (uint32_t)lane] = make_uint2(l + mine.l, i + mine.i);
@@ -531,7 +529,7 @@ static_assert(kTreeWarps == kTreeWarpsPerCta, "the host sizes the launches");
 // Inner nodes of the stripe whose regions end before leaf bit `key`.
 __device__ __forceinline__ uint32_t inner_before(const Stripe& p, uint32_t key) {
   const uint32_t x = p.K == kBrickLevels ? key >> 12 : 0u, blk = key >> 8;
-  uint32_t s = p.wpre[x >> 5].y + p.bpre[x].y + p.inner_local[blk];
+  uint32_t s = p.wpre[x >> 5].y + p.bpre[x].y + p.blocks[blk].inner;
   if (p.K == kBrickLevels) s += __popc(p.bunits[x] & ((1u << ((key >> 9) & 7u)) - 1u));  // nodes of 512 leaf bits
   for (int l = 1; l <= p.U; l++) s += upper_rank(p, l, x >> (3 * (p.U - l)));
   const uint4* q = reinterpret_cast<const uint4*>(p.leaf) + 2 * (uint64_t)blk;
