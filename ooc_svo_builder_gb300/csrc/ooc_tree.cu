@@ -73,6 +73,21 @@ __device__ __forceinline__ void raise_flag(const EmitJob& e, uint32_t code) {
 // leave most SMs idle for 16 rounds of loads: the CTA's four warps share a word,
 // eight bricks each (18 -> 10 us at gridsize 256).
 // ===========================================================================
+// Bit position of the t-th (from 0) set bit of the 8-bit mask m.
+__device__ __forceinline__ uint32_t select8(uint32_t m, uint32_t t) {
+  uint32_t pos = 0, c = __popc(m & 15u);
+  if (t >= c) {
+    t -= c;
+    pos = 4;
+  }
+  c = __popc((m >> pos) & 3u);
+  if (t >= c) {
+    t -= c;
+    pos += 2;
+  }
+  return pos + (t >= ((m >> pos) & 1u) ? 1u : 0u);
+}
+
 struct WordCount {
   uint32_t l, i;  // leaves and inner nodes below the bricks
 };
@@ -114,8 +129,8 @@ __device__ __forceinline__ WordCount count_bricks(const Stripe& p, uint32_t x0, 
     if (j < total) {
       uint32_t k = j - before;
       if (p.touch) {  // the k-th marked block
-        for (; k; k--) m &= m - 1;
-        k = (uint32_t)__ffs(m) - 1u;
+        const uint32_t c = __popc(m & 0xffu);
+        k = k < c ? select8(m & 0xffu, k) : 8u + select8(m >> 8, k - c);
       }
       blk = (uint64_t)(x0 + o) * 16u + k;
       const uint4* q = reinterpret_cast<const uint4*>(p.leaf) + 2 * blk;
@@ -133,23 +148,25 @@ __device__ __forceinline__ WordCount count_bricks(const Stripe& p, uint32_t x0, 
       }
     }
     const uint32_t nonempty = __ballot_sync(FULL, l != 0);
-    const uint32_t il = warp_inclusive(l), ii = warp_inclusive(in);
-    const uint32_t el = carry_l + il - l, ei = carry_i + ii - in;
+    // both counts in one scan: at most 32 x 256 leaves and 32 x 36 nodes
+    const uint32_t own = l | (in << 16), inc = warp_inclusive(own), before_own = inc - own;
+    const uint32_t el = carry_l + (before_own & 0xffffu);
     const uint32_t src = excl - round;  // where this lane's brick starts, when it does in this round
-    const uint32_t vl = __shfl_sync(FULL, el, (int)(src & 31u)), vi = __shfl_sync(FULL, ei, (int)(src & 31u));
+    const uint32_t at_src = __shfl_sync(FULL, before_own, (int)(src & 31u));
     if (excl >= round && src < 32u) {
-      my_l = vl;
-      my_i = vi;
+      my_l = carry_l + (at_src & 0xffffu);
+      my_i = carry_i + (at_src >> 16);
       if (!p.touch) seen = (nonempty >> src) & marked;
     }
     if (p.blocks) {
-      uint32_t inner = 0;
-      if (p.block_inner) inner = ei - __shfl_sync(FULL, my_i, (int)o);  // after those before the block's brick
+      uint32_t inner = 0;  // after those before the block's brick
+      if (p.block_inner) inner = carry_i + (before_own >> 16) - __shfl_sync(FULL, my_i, (int)o);
       if (j < total)
         reinterpret_cast<uint4*>(p.blocks)[blk] = make_uint4((uint32_t)wo, (uint32_t)(wo >> 32), el, inner);
     }
-    carry_l += __shfl_sync(FULL, il, 31);
-    carry_i += __shfl_sync(FULL, ii, 31);
+    const uint32_t all = __shfl_sync(FULL, inc, 31);
+    carry_l += all & 0xffffu;
+    carry_i += all >> 16;
   }
   if (excl >= total) {  // no block in this brick or after it
     my_l = carry_l;
@@ -622,21 +639,6 @@ struct __align__(16) WarpScratch {
   uint32_t gaps[8];
   uint16_t units[256];  // of the word's bricks: brick | place in it << 5 | number in it << 8
 };
-
-// Bit position of the t-th (from 0) set bit of the 8-bit mask m.
-__device__ __forceinline__ uint32_t select8(uint32_t m, uint32_t t) {
-  uint32_t pos = 0, c = __popc(m & 15u);
-  if (t >= c) {
-    t -= c;
-    pos = 4;
-  }
-  c = __popc((m >> pos) & 3u);
-  if (t >= c) {
-    t -= c;
-    pos += 2;
-  }
-  return pos + (t >= ((m >> pos) & 1u) ? 1u : 0u);
-}
 
 // Bulk copies of shared memory to global memory (both 16-byte aligned, a multiple of 16
 // bytes); a thread's copies since its last commit form a group.
