@@ -196,7 +196,7 @@ def cpu_port_time(tris, w, budget_s: float, max_runs: int, min_runs: int = 1):
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of a workload's dominant
 # kernel, from the ncu captures summarised under profiles/: (workload, kernel) -> (bytes, summary)
 NCU_TRAFFIC = {
-    ("heightfield1024", "vox_small_occupancy"): (179.5e6 + 34.5e6, "profiles/vox_small_heightfield1024.md"),
+    ("heightfield1024", "vox_small_occupancy"): (179.4e6 + 24.3e6, "profiles/heightfield1024.md"),
 }
 
 
@@ -205,8 +205,8 @@ def algorithmic_bytes(kernel: str, n_tris: int, info: dict, S: int, payload: boo
     tri_bytes = 84 if payload else 36
     leaf_words = S // 32
     if kernel == "vox_small_occupancy":
-        # vertices of every triangle (36 B) + its task count (8 B) + (payload) pass mask and box (16 B)
-        return n_tris * (36 + 8 + (16 if payload else 0))
+        # vertices of every triangle (36 B) + (payload) pass mask and box (16 B)
+        return n_tris * (36 + (16 if payload else 0))
     if kernel in ("vox_small_winner", "vox_large_occupancy", "vox_large_winner"):
         # vertices of every triangle (36 B) + the task count per item (8 B)
         return n_tris * (36 + 8)
