@@ -537,9 +537,9 @@ struct StreamSource {
 // The batch engine.  A batch is a list of meshes; every mesh is split into
 // stripes, and the stripes of all meshes run through one launch sequence (a
 // sub-batch when their occupancy pyramids exceed the memory budget).  Each
-// sub-batch synchronises with the host twice: after the level counts (to size
-// the per-node arrays and place every stripe's records in its file), and at
-// the end (root records for the host-side grouping).
+// sub-batch synchronises with the host after its counts (to size the outputs
+// and place every stripe's records in its file) and, unless the records stay on
+// the device, at its end.
 // ---------------------------------------------------------------------------
 struct MeshWork {
   const ooc_build_params* prm = nullptr;

@@ -540,8 +540,8 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b, F2 nz) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(nz.v));
   return r;
 }
-__device__ __forceinline__ F2 minus_zero(float finite) {
-  const float z = __fmul_rn(fabsf(finite), -0.0f);
+__device__ __forceinline__ F2 minus_zero(uint32_t small) {  // any run-time value below 2^31
+  const float z = __uint_as_float(0x80000000u | (small >> 31));
   return f2(z, z);
 }
 __device__ __forceinline__ F2 add2(F2 a, F2 b) {
@@ -629,7 +629,7 @@ __device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, ui
   // (w + b) + a.  Adding the 0 changes only the sign of a zero, which no test sees.
   const float nw = r.nw, pa = __fmul_rn(r.na, fa), pb = __fmul_rn(r.nb, fb);
   const float q1 = W == 2 ? __fadd_rn(pa, pb) : (W == 0 ? pa : pb), q2 = W == 2 ? 0.0f : (W == 0 ? pb : pa);
-  const F2 dd = r.dd, fab = f2(fa, fb), nz = minus_zero(u);  // u: the unit length, finite
+  const F2 dd = r.dd, fab = f2(fa, fb), nz = minus_zero(r.shape);
   F2 cw[3], cf[3], cd[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) cw[k] = r.w[k], cf[k] = mul2(r.f[k], fab, nz), cd[k] = r.d[k];
@@ -818,7 +818,7 @@ __device__ __forceinline__ uint64_t vox_small_bricks(const VoxJob& j, const TriS
     q00 = n1y0, q01 = n1y1, q10 = n1y0, q11 = n1y1;
     r0 = n0x0, r1 = n0x1;  // of x
   }
-  const F2 nz = minus_zero(j.u);
+  const F2 nz = minus_zero((uint32_t)j.stride);
   F2 cz[3], c0[3], c1[3], cd[3];  // ZX and YZ: of z, of (x_0, y_0), of (x_1, y_1), rest
 #pragma unroll
   for (int k = 0; k < 3; k++) {
@@ -1086,7 +1086,7 @@ __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, cons
       const uint32_t rb = r.magic ? __umulhi(c, r.magic) : c, ra = c - rb * ea;
       const float fa = __fmul_rn((float)(r.alo + (int)ra), r.u), fb = __fmul_rn((float)(r.blo + (int)rb), r.u);
       float t0, t1;
-      const F2 nz = minus_zero(r.u);
+      const F2 nz = minus_zero(r.shape);
       split(add2(add2(mul2(r.ea, f2(fa, fa), nz), mul2(r.eb, f2(fb, fb), nz)), r.ed), t0, t1);
       const float t2 = __fadd_rn(__fadd_rn(__fmul_rn(r.ea2, fa), __fmul_rn(r.eb2, fb)), r.ed2);
       ok = !(fminf(fminf(t0, t1), t2) < 0.0f);  // a NaN passes
