@@ -22,8 +22,8 @@
 #include <string>
 #include <vector>
 
-#include "ooc_device.cuh"
 #include "ooc_internal.h"
+#include "ooc_morton.h"
 #include "ooc_svo_gpu.h"
 
 namespace {
@@ -144,7 +144,7 @@ struct ooc_ctx {
   DevBuf d_out_nodes[2], d_out_data[2];
   PinBuf h_root[2];
   PinBuf h_flag;        // the layout check's flag: the record kernels set it, in host memory
-  bool unfinished = false;  // a build was begun and has not come to its end
+  cudaStream_t build_stream = nullptr;  // the stream the build queues on, once it does
   D2HRing ring[2][2];  // [slot][OOC_STREAM_NODES / OOC_STREAM_DATA]
   cudaEvent_t ev_compute[2] = {nullptr, nullptr};
   cudaEvent_t ev_data[2] = {nullptr, nullptr};  // host output: a sub-batch's data file is final
@@ -1490,6 +1490,7 @@ void finalize_mesh(MeshWork& m) {
 // that have just completed.
 void build_meshes(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, const OutSpec& os,
                   const std::function<void(const std::vector<size_t>&)>& on_done = nullptr) {
+  c->build_stream = st;
   if (c->d_mesh_items.size() < meshes.size()) c->d_mesh_items.resize(meshes.size());
   for (size_t i = 0; i < meshes.size(); i++) {
     MeshWork& m = meshes[i];
@@ -1642,7 +1643,6 @@ void finish_device_output(ooc_ctx* c, cudaStream_t st, MeshWork& m, Emitter& out
 
 // The end of a build that succeeded.
 void finish_build(ooc_ctx* c) {
-  c->unfinished = false;
   for (float& v : c->phase_ms) v = 0.0f;
   if (c->timing) {
     for (const auto& m : c->marks) {
@@ -1688,13 +1688,7 @@ void begin_build(ooc_ctx* c) {
   c->stream_passes = 0;
   c->part_tris.clear();
   c->part_filled.clear();
-  if (c->unfinished) {  // a build that failed part-way may have left copies queued into the staging buffers
-    ck(cudaStreamSynchronize(c->copy_stream), "cudaStreamSynchronize");
-    ck(cudaStreamSynchronize(c->ring_stream[0]), "cudaStreamSynchronize");
-    ck(cudaStreamSynchronize(c->ring_stream[1]), "cudaStreamSynchronize");
-    ck(cudaStreamSynchronize(c->h2d_stream), "cudaStreamSynchronize");
-  }
-  c->unfinished = true;
+  c->build_stream = nullptr;
   *ensure_pinned<volatile uint32_t>(c->h_flag, 4) = 0;
   c->err.clear();
   c->marks.clear();
@@ -1734,6 +1728,25 @@ int guarded(ooc_ctx* c, F&& f) {
   }
 }
 
+// The end of a build that failed: when its call returns nothing of it is queued any more, on the caller's
+// stream or the context's, so the caller's triangles and destinations are free and the context's buffers
+// can serve a build on another stream.  (Errors are the build's, which has reported its first.)
+void abandon_build(ooc_ctx* c) {
+  for (cudaStream_t st : {c->build_stream, c->copy_stream, c->ring_stream[0], c->ring_stream[1], c->h2d_stream})
+    if (st) cudaStreamSynchronize(st);
+}
+
+// Runs one build on `c`.
+template <typename F>
+int run_build(ooc_ctx* c, F&& f) {
+  const int rc = guarded(c, [&] {
+    begin_build(c);
+    f();
+  });
+  if (rc != OOC_OK && c) abandon_build(c);
+  return rc;
+}
+
 }  // namespace
 
 namespace ooc {
@@ -1771,8 +1784,7 @@ bool file_wants_stream(ooc_ctx* c, const ooc_build_params* prm, uint64_t n_tris)
 
 int build_from_file_stream(ooc_ctx* c, const ooc_build_params* prm, const char* tridata, uint64_t n_tris,
                            ooc_sink_fn sink, void* user, ooc_build_info* info) {
-  return guarded(c, [&] {
-    begin_build(c);
+  return run_build(c, [&] {
     check_params(prm, n_tris);
     if (!sink) fail(OOC_ERR_INVALID, "sink is NULL");
     cudaStream_t st = c->own_stream;
@@ -2010,8 +2022,7 @@ struct BatchInput {
 
 int ooc_build_batch(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_meshes, ooc_batch_sink_fn sink, void* user,
                     ooc_build_info* infos) {
-  return guarded(c, [&] {
-    begin_build(c);
+  return run_build(c, [&] {
     if (!sink) fail(OOC_ERR_INVALID, "sink is NULL");
     cudaStream_t st = c->own_stream;
     BatchInput b(c, meshes_in, n_meshes, false);
@@ -2038,8 +2049,7 @@ int ooc_build_batch(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_meshes, oo
 
 int ooc_build_batch_device(ooc_ctx* c, const ooc_mesh* meshes_in, uint64_t n_meshes, ooc_alloc_fn alloc,
                            ooc_ready_fn ready, void* user, ooc_build_info* infos) {
-  return guarded(c, [&] {
-    begin_build(c);
+  return run_build(c, [&] {
     if (!alloc) fail(OOC_ERR_INVALID, "alloc is NULL");
     cudaStream_t st = c->own_stream;
     BatchInput b(c, meshes_in, n_meshes, true);
@@ -2224,8 +2234,7 @@ int ooc_arena_alloc(void* arena, uint64_t mesh, uint64_t nodes_bytes, uint64_t d
 
 int ooc_build_device(ooc_ctx* c, const ooc_build_params* prm, const float* tris_device, uint64_t n_tris,
                      void* stream, ooc_build_info* info) {
-  return guarded(c, [&] {
-    begin_build(c);
+  return run_build(c, [&] {
     check_params(prm, n_tris);
     if (n_tris && !tris_device) fail(OOC_ERR_INVALID, "triangles are NULL");
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : c->own_stream;
@@ -2254,8 +2263,7 @@ int ooc_build_device(ooc_ctx* c, const ooc_build_params* prm, const float* tris_
 
 int ooc_build_from_device(ooc_ctx* c, const ooc_build_params* prm, const float* tris_device, uint64_t n_tris,
                           ooc_sink_fn sink, void* user, ooc_build_info* info) {
-  return guarded(c, [&] {
-    begin_build(c);
+  return run_build(c, [&] {
     check_params(prm, n_tris);
     if (!sink) fail(OOC_ERR_INVALID, "sink is NULL");
     if (n_tris && !tris_device) fail(OOC_ERR_INVALID, "triangles are NULL");

@@ -1,0 +1,112 @@
+// Builds that fail part-way, on the stand-in runtime of fake_cuda.h (test_failed_builds.py).
+// One argument: the property to check.  Every call is made to fail at each of its allocations
+// and of its callbacks in turn, on a context of its own.
+#include <algorithm>
+#include <string>
+
+#include "fake_cuda.h"
+
+namespace {
+
+int bad = 0;
+void expect(bool ok, const std::string& what) {
+  if (ok) return;
+  if (bad++ < 10) std::printf("%s\n", what.c_str());
+}
+
+ooc_build_params params(uint64_t grid, uint64_t limit, bool levels = false) {
+  ooc_build_params p;
+  std::memset(&p, 0, sizeof(p));
+  p.gridsize = grid;
+  p.memory_limit_mb = limit;
+  p.geometry_only = 1;
+  p.generate_levels = levels;
+  for (int a = 0; a < 3; a++) p.bbox_max[a] = 1.0f;
+  return p;
+}
+
+// What a call's callbacks do: the `left`-th from now on refuses.
+struct Callbacks {
+  long left = -1;
+  ooc_device_arena arena{};
+  int next() { return left >= 0 && left-- == 0 ? 1 : 0; }
+};
+int on_sink(void* u, int32_t, const void*, uint64_t) { return static_cast<Callbacks*>(u)->next(); }
+int on_batch_sink(void* u, uint64_t, int32_t, const void*, uint64_t) { return static_cast<Callbacks*>(u)->next(); }
+int on_alloc(void* u, uint64_t m, uint64_t nb, uint64_t db, void* st, void** n, void** d) {
+  Callbacks* c = static_cast<Callbacks*>(u);
+  return c->next() ? 1 : ooc_arena_alloc(&c->arena, m, nb, db, st, n, d);
+}
+int on_ready(void* u, uint64_t) { return static_cast<Callbacks*>(u)->next(); }
+
+// The calls: octree on the device, to a sink, batches to a sink and to device destinations; one stripe or
+// 64 in several sub-batches.
+constexpr int kCalls = 6;
+const char* const kNames[kCalls] = {"device", "device, 64 partitions", "device, 64 partitions, levels",
+                                    "sink, 64 partitions", "batch", "batch to device memory"};
+char arena_mem[1 << 20];
+
+int call(int which, ooc_ctx* c, cudaStream_t st, Callbacks& cb) {
+  static float tri[9] = {0.0f, 0.0f, 0.0f, 0.1f, 0.0f, 0.0f, 0.0f, 0.1f, 0.0f};
+  ooc_mesh m[3];
+  for (ooc_mesh& x : m) x.tris = tri, x.n_tris = 1, x.params = params(64, 2048);
+  m[1].params = params(256, 1);
+  ooc_set_batch_budget(c, 8 * 40000);  // about eight stripes of 64^3
+  cb.arena = ooc_device_arena{arena_mem, sizeof(arena_mem), 0};
+  const ooc_build_params one = params(64, 2048), many = params(256, 1), lev = params(256, 1, true);
+  switch (which) {
+    case 0: return ooc_build_device(c, &one, tri, 1, st, nullptr);
+    case 1: return ooc_build_device(c, &many, tri, 1, st, nullptr);
+    case 2: return ooc_build_device(c, &lev, tri, 1, st, nullptr);
+    case 3: return ooc_build(c, &many, tri, 1, on_sink, &cb, nullptr);
+    case 4: return ooc_build_batch(c, m, 3, on_batch_sink, &cb, nullptr);
+    default: return ooc_build_batch_device(c, m, 3, on_alloc, on_ready, &cb, nullptr);
+  }
+}
+
+// After a failure at every point of every call: `check(name of the point, context)`.
+template <typename F>
+void each_failure(F check) {
+  for (int which = 0; which < kCalls; which++)
+    for (int kind = 0; kind < 2; kind++) {  // allocations, callbacks
+      long at = 0;
+      for (;; at++) {
+        fake::last = cudaSuccess;
+        const cudaStream_t user = fake::new_stream();
+        ooc_ctx* c = nullptr;
+        expect(ooc_ctx_create(0, &c) == OOC_OK, "ooc_ctx_create");
+        Callbacks cb;
+        if (kind == 0) fake::fail_after = at;
+        else cb.left = at;
+        const int rc = call(which, c, user, cb);
+        const bool reached = (kind == 0 ? fake::fail_after : cb.left) < 0;
+        fake::fail_after = -1;
+        if (reached) {
+          expect(rc != OOC_OK, "a failure was not reported");
+          check(std::string(kNames[which]) + (kind ? ", callback " : ", allocation ") + std::to_string(at), c);
+        } else {
+          expect(rc == OOC_OK, std::string(kNames[which]) + " without a failure: " + ooc_last_error(c));
+        }
+        ooc_ctx_destroy(c);
+        cudaStreamDestroy(user);
+        if (!reached) break;
+      }
+      expect(at > (kind == 0 || which > 2 ? 3 : -1), std::string(kNames[which]) + ": too few points of failure");
+    }
+}
+
+void check_drained() {
+  each_failure([](const std::string& at, ooc_ctx*) {
+    expect(fake::queued() == 0, at + ": " + std::to_string(fake::queued()) + " operations still queued");
+  });
+}
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const std::string what = argc > 1 ? argv[1] : "";
+  if (what == "drained") check_drained();
+  else return 2;
+  std::printf("%d failures\n", bad);
+  return bad ? 1 : 0;
+}
