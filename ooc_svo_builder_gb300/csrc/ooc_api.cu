@@ -1730,10 +1730,12 @@ int guarded(ooc_ctx* c, F&& f) {
 
 // The end of a build that failed: when its call returns nothing of it is queued any more, on the caller's
 // stream or the context's, so the caller's triangles and destinations are free and the context's buffers
-// can serve a build on another stream.  (Errors are the build's, which has reported its first.)
+// can serve a build on another stream.  (Errors are the build's, which has reported its first.)  Its emission
+// may not have run, or have found a brick outside its window, whose bits and marks it then leaves.
 void abandon_build(ooc_ctx* c) {
   for (cudaStream_t st : {c->build_stream, c->copy_stream, c->ring_stream[0], c->ring_stream[1], c->h2d_stream})
     if (st) cudaStreamSynchronize(st);
+  if (c->build_stream) c->leaf_zero = c->ctr_zero = false;
 }
 
 // Runs one build on `c`.

@@ -101,11 +101,34 @@ void check_drained() {
   });
 }
 
+// A build that fails its layout check leaves the bits of what it did not write: the next one, whatever it
+// returns to, starts from clean buffers.
+void check_clean() {
+  for (int which = 0; which < kCalls; which++) {
+    const cudaStream_t user = fake::new_stream();
+    ooc_ctx* c = nullptr;
+    expect(ooc_ctx_create(0, &c) == OOC_OK, "ooc_ctx_create");
+    Callbacks cb;
+    fake::raise_flag = true;
+    expect(call(which, c, user, cb) == OOC_ERR_DEVICE, std::string(kNames[which]) + ": the flag was not reported");
+    fake::raise_flag = false;
+    for (int next = 0; next < kCalls; next++) {
+      fake::dirty = 0;
+      expect(call(next, c, user, cb) == OOC_OK, std::string(kNames[next]) + ": " + ooc_last_error(c));
+      expect(fake::dirty == 0, std::string(kNames[next]) + " after " + kNames[which] + " with its flag raised: " +
+                                   std::to_string(fake::dirty) + " stripes began with bits set");
+    }
+    ooc_ctx_destroy(c);
+    cudaStreamDestroy(user);
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "drained") check_drained();
+  else if (what == "clean") check_clean();
   else return 2;
   std::printf("%d failures\n", bad);
   return bad ? 1 : 0;
