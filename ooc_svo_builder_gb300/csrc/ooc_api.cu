@@ -1706,7 +1706,8 @@ void begin_build(ooc_ctx* c) {
   }
 }
 
-// Runs one API call on `c`: its launches report to c's own launch state.
+// Runs one API call on `c`: its launches report to c's own launch state.  A failure is reported by the
+// call's status; as the thread's last CUDA error it would fail the check at the end of the next build.
 template <typename F>
 int guarded(ooc_ctx* c, F&& f) {
   if (!c) return OOC_ERR_INVALID;
@@ -1718,12 +1719,15 @@ int guarded(ooc_ctx* c, F&& f) {
   } catch (const OocError& e) {
     c->err = e.msg;
     c->launches = c->lstate.launches;
+    cudaGetLastError();
     return e.code;
   } catch (const std::bad_alloc&) {
     c->err = "host allocation failed";
+    cudaGetLastError();
     return OOC_ERR_OOM;
   } catch (...) {
     c->err = "unexpected exception";
+    cudaGetLastError();
     return OOC_ERR_DEVICE;
   }
 }

@@ -123,12 +123,23 @@ void check_clean() {
   }
 }
 
+// The build after a failed one succeeds: the failure's error is not met again as that build's own.
+void check_recovered() {
+  each_failure([](const std::string& at, ooc_ctx* c) {
+    expect(fake::last == cudaSuccess, at + ": the error is still the thread's last one");
+    Callbacks cb;
+    for (int next = 0; next < kCalls; next++)
+      expect(call(next, c, nullptr, cb) == OOC_OK, std::string(kNames[next]) + " after " + at + ": " + ooc_last_error(c));
+  });
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "drained") check_drained();
   else if (what == "clean") check_clean();
+  else if (what == "recovered") check_recovered();
   else return 2;
   std::printf("%d failures\n", bad);
   return bad ? 1 : 0;
