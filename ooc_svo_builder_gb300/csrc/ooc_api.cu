@@ -1864,7 +1864,7 @@ void ooc_ctx_destroy(ooc_ctx* c) {
                     &c->d_winners, &c->d_large, &c->d_big, &c->d_ctr, &c->d_nodes,
                     &c->d_data, &c->d_recs, &c->d_itemmask, &c->d_itembox, &c->d_leaf, &c->d_touch, &c->d_blocks,
                     &c->d_pctr, &c->d_chunk[0], &c->d_chunk[1], &c->d_group[0],
-                    &c->d_group[1], &c->d_stream_mat, &c->d_stream_part, &c->d_stream_base, &c->d_part_off};
+                    &c->d_group[1], &c->d_stream_mat, &c->d_stream_part, &c->d_stream_base, &c->d_part_off, &c->d_tune_arena};
   for (DevBuf* b : bufs)
     if (b->p) cudaFree(b->p);
   PinBuf* pins[] = {&c->h_misc, &c->h_recs, &c->h_tables1, &c->h_tables2, &c->h_words, &c->h_stage[0],

@@ -133,6 +133,23 @@ void check_recovered() {
   });
 }
 
+// A destroyed context has given back its memory, streams, events and graphs.
+void check_freed() {
+  const cudaStream_t user = fake::new_stream();
+  ooc_ctx* c = nullptr;
+  expect(ooc_ctx_create(0, &c) == OOC_OK, "ooc_ctx_create");
+  Callbacks cb;
+  for (int which = 0; which < kCalls; which++) expect(call(which, c, user, cb) == OOC_OK, kNames[which]);
+  static float tri[9] = {0.0f, 0.0f, 0.0f, 0.1f, 0.0f, 0.0f, 0.0f, 0.1f, 0.0f};
+  const ooc_mesh m = {tri, 1, params(64, 2048)};
+  expect(ooc_autotune(c, &m, 1, nullptr) == OOC_OK, "ooc_autotune");
+  ooc_ctx_destroy(c);
+  cudaStreamDestroy(user);
+  expect(fake::device.empty(), std::to_string(fake::device.size()) + " device allocations left");
+  expect(fake::pinned.empty(), std::to_string(fake::pinned.size()) + " pinned allocations left");
+  expect(fake::streams.empty() && fake::events == 0 && fake::execs == 0, "streams, events or graphs left");
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -140,6 +157,7 @@ int main(int argc, char** argv) {
   if (what == "drained") check_drained();
   else if (what == "clean") check_clean();
   else if (what == "recovered") check_recovered();
+  else if (what == "freed") check_freed();
   else return 2;
   std::printf("%d failures\n", bad);
   return bad ? 1 : 0;

@@ -31,6 +31,7 @@ def check(tmp_path_factory):
     "drained",  # nothing of a failed call is still queued, on any stream, when it returns
     "clean",    # the build after one whose layout check failed starts from clean buffers
     "recovered",  # every kind of build succeeds after a failure
+    "freed",    # a destroyed context has given everything back
 ])
 def test_failed_builds(check, what):
     p = subprocess.run([check, what], capture_output=True, text=True, timeout=300)
