@@ -136,9 +136,12 @@ int ooc_build_from_device(ooc_ctx* ctx, const ooc_build_params* params, const fl
  * files are written straight into device memory that the caller provides:
  * `alloc` is called once per mesh, in mesh order, as soon as the mesh's sizes
  * are known and before any of its records are written.  It returns two device
- * pointers (8-byte aligned) through `nodes` and `data`; `stream` is the
- * cudaStream_t the library writes them on, so memory allocated stream-ordered
- * on it (cudaMallocAsync) may be used.  `ready` (may be NULL) is called once
+ * pointers through `nodes` (8-byte aligned) and `data` (16-byte aligned; 8
+ * will do where the file holds only its header records, as it does with
+ * geometry_only and without generate_levels); `stream` is the cudaStream_t the
+ * library writes them on (with generate_levels it also reads the data records
+ * back there), so memory allocated stream-ordered on it (cudaMallocAsync) may
+ * be used.  `ready` (may be NULL) is called once
  * per mesh, in mesh order, when every byte of its files has been written.  The
  * files are byte-identical to what ooc_build writes for that mesh alone.
  * Both callbacks return 0, or non-zero to abort the call. */
@@ -148,9 +151,10 @@ typedef int (*ooc_ready_fn)(void* user, uint64_t mesh);
 int ooc_build_batch_device(ooc_ctx* ctx, const ooc_mesh* meshes, uint64_t n_meshes, ooc_alloc_fn alloc,
                            ooc_ready_fn ready, void* user, ooc_build_info* infos);
 
-/* A bump allocator over one caller-owned device buffer, usable as `alloc`
- * with `user` = the arena: each file starts on a 256-byte boundary; a full
- * arena fails the call with OOC_ERR_OOM. */
+/* A bump allocator over one caller-owned device buffer (`base` 16-byte
+ * aligned), usable as `alloc` with `user` = the arena: each file starts on a
+ * 256-byte boundary of the buffer; a full arena fails the call with
+ * OOC_ERR_OOM. */
 typedef struct {
   void* base;
   uint64_t capacity;

@@ -712,6 +712,9 @@ void ensure_dest(ooc_ctx* c, cudaStream_t st, MeshWork& m, const OutSpec& os) {
     fail(OOC_ERR_OOM, "destination allocation failed for mesh " + std::to_string(m.index));
   if ((reinterpret_cast<uintptr_t>(dn) | reinterpret_cast<uintptr_t>(dd)) & 7)
     fail(OOC_ERR_INVALID, "destinations must be 8-byte aligned");
+  // the stripes' data records are written (and with -levels read) 16 bytes at a time; the header records are not
+  if ((reinterpret_cast<uintptr_t>(dd) & 15) && m.total_data > (m.pl.binary ? 2u : 1u))
+    fail(OOC_ERR_INVALID, "a data file of more than its header records needs a 16-byte aligned destination");
   m.dst_nodes = dn;
   m.dst_data = dd;
   m.dst_ready = true;

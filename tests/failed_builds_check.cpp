@@ -150,6 +150,39 @@ void check_freed() {
   expect(fake::streams.empty() && fake::events == 0 && fake::execs == 0, "streams, events or graphs left");
 }
 
+// Destinations of a batch: `nodes` needs 8 bytes, `data` 16 where the file holds more than header records.
+struct Offsets {
+  uint64_t nodes, data;
+};
+int offset_alloc(void* u, uint64_t, uint64_t nb, uint64_t, void*, void** n, void** d) {
+  const Offsets* o = static_cast<Offsets*>(u);
+  char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(arena_mem) + 255) / 256 * 256);
+  *n = base + o->nodes;
+  *d = base + (nb + 511) / 256 * 256 + o->data;
+  return 0;
+}
+void check_aligned() {
+  static float tri[21] = {0.0f, 0.0f, 0.0f, 0.1f, 0.0f, 0.0f, 0.0f, 0.1f, 0.0f};
+  for (int payload = 0; payload < 2; payload++)
+    for (int levels = 0; levels < 2; levels++)
+      for (uint64_t count = 0; count < 2; count++)
+        for (uint64_t nodes : {0, 4, 8, 16})
+          for (uint64_t data : {0, 4, 8, 16}) {
+            ooc_ctx* c = nullptr;
+            expect(ooc_ctx_create(0, &c) == OOC_OK, "ooc_ctx_create");
+            ooc_mesh m = {tri, count, params(64, 2048, levels)};
+            m.params.geometry_only = !payload;
+            Offsets o{nodes, data};
+            const bool records = count && (payload || levels);
+            const int want = nodes % 8 || data % (records ? 16 : 8) ? OOC_ERR_INVALID : OOC_OK;
+            const int got = ooc_build_batch_device(c, &m, 1, offset_alloc, nullptr, &o, nullptr);
+            expect(got == want, "payload " + std::to_string(payload) + ", levels " + std::to_string(levels) + ", " +
+                                    std::to_string(count) + " triangles, nodes at " + std::to_string(nodes) + ", data at " +
+                                    std::to_string(data) + ": status " + std::to_string(got));
+            ooc_ctx_destroy(c);
+          }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -158,6 +191,7 @@ int main(int argc, char** argv) {
   else if (what == "clean") check_clean();
   else if (what == "recovered") check_recovered();
   else if (what == "freed") check_freed();
+  else if (what == "aligned") check_aligned();
   else return 2;
   std::printf("%d failures\n", bad);
   return bad ? 1 : 0;

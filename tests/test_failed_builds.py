@@ -32,6 +32,7 @@ def check(tmp_path_factory):
     "clean",    # the build after one whose layout check failed starts from clean buffers
     "recovered",  # every kind of build succeeds after a failure
     "freed",    # a destroyed context has given everything back
+    "aligned",  # destinations that the records' stores cannot reach are refused, the others are not
 ])
 def test_failed_builds(check, what):
     p = subprocess.run([check, what], capture_output=True, text=True, timeout=300)
