@@ -305,11 +305,11 @@ int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, const float* 
 
 /* ---- Serving loop (no counterpart in the reference) ----
  * Requests (meshes) are admitted by their computed HBM footprint against
- * `memory_budget`: their triangles, the occupancy pyramids of their stripes,
- * and per-node arrays plus output records for an upper bound on their nodes
- * (a tree whose L leaves are at depth D has at most min(8^l, L) nodes at level
- * l, and L is at most the summed grid boxes of the triangles, clamped to the
- * grid).  Footprints are computed by sizing threads of the server, so a
+ * `memory_budget`: their triangles, every stripe's arrays, their (triangle,
+ * stripe) items, and the output records of an upper bound on their nodes (a
+ * tree whose L leaves are at depth D has at most min(8^l, L) nodes at level l,
+ * and L is at most the summed per-triangle bounds on the voxels set), once more
+ * for a mesh of several stripes, whose records wait for its sizes.  Footprints are computed by sizing threads of the server, so a
  * submission returns at once; a request whose footprint exceeds the whole
  * budget completes, without running, with status OOC_ERR_LIMIT.  Requests are
  * admitted in submission order.  Requests run in

@@ -607,11 +607,6 @@ struct Placed {  // a stripe after the level counts
   uint64_t out_node_off = 0, out_data_off = 0;  // host mode: offsets in the batch output buffers
 };
 
-// Stripes of 512^3 voxels and more mark their leaf blocks; smaller leaf
-// levels are read and zeroed whole (their marks would cost the voxelization
-// more than they save).
-constexpr int kMarkDepth = 9;
-
 // Words of a stripe's whole occupancy pyramid, every level padded to 256-bit blocks: what a
 // stripe counts against the batch budget.
 uint64_t pyramid_words(int Ds) {
@@ -791,8 +786,8 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   std::vector<Stripe> stripe(n);
   std::vector<VoxJob> vj(n);
   std::vector<uint64_t> item_beg(n + 1, 0), leaf_beg(n, 0), touch_beg(n, 0), block_beg(n, 0), upper_beg(n, 0),
-      word_beg(n, 0), brick_beg(n, 0);
-  uint64_t leaf_w = 0, tbytes = 0, n_blocks = 0, upper_w = 0, pre_w = 0, bricks = 0, items = 0;
+      word_beg(n, 0), brick_beg(n, 0), cell_at(n, 0);
+  uint64_t leaf_w = 0, tbytes = 0, n_blocks = 0, upper_w = 0, pre_w = 0, bricks = 0, cells = 0, items = 0;
   int max_upper = 0;
   for (uint32_t s = 0; s < n; s++) {
     const StripeRef& r = sb[s];
@@ -804,18 +799,21 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     S.U = S.depth - S.K;
     S.n_bricks = 1u << (3 * S.U);
     max_upper = std::max(max_upper, S.U);
+    const StripeSizes z = stripe_sizes(S.depth, !mp.binary, mp.levels != 0);
     leaf_beg[s] = leaf_w;
-    leaf_w += leaf_words(S.depth);
+    leaf_w += z.leaf;
     touch_beg[s] = tbytes;
-    if (S.depth >= kMarkDepth) tbytes += touch_bytes(S.depth);
-    block_beg[s] = n_blocks;  // the ranks of leaf bits: payload stripes only
-    if (!mp.binary) n_blocks += leaf_blocks(S.depth);
+    tbytes += z.touch;
+    block_beg[s] = n_blocks;
+    n_blocks += z.blocks;
     upper_beg[s] = upper_w;
-    upper_w += upper_off(S.U + 1);
-    word_beg[s] = pre_w;  // one entry past the last word, in whole groups of eight
-    pre_w += (upper_words(S.U) + 8) / 8 * 8;
+    upper_w += z.upper;
+    word_beg[s] = pre_w;
+    pre_w += z.words;
     brick_beg[s] = bricks;
-    bricks += std::max<uint32_t>(S.n_bricks, 32);  // whole words
+    bricks += z.bricks;
+    cell_at[s] = cells;
+    cells += z.cells;
     item_beg[s] = items;
     items += r.n_items;
   }
@@ -974,8 +972,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   // ---- counts, placement in the files ----
   std::vector<Placed> pl(n);
   uint64_t total_nodes = 0, total_leaves = 0;
-  std::vector<uint64_t> leaf_at(n, 0), cell_at(n, 0);  // the stripes' places in the per-leaf arrays
-  uint64_t cells = 0;
+  std::vector<uint64_t> leaf_at(n, 0);  // the stripes' places in the per-leaf array
   bool any_levels = false;
   for (uint32_t s = 0; s < n; s++) {
     const uint32_t* o = lvl + (uint64_t)s * kCountWords;
@@ -996,11 +993,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
       leaf_at[s] = total_leaves;
       total_leaves += q.n_leaf;
     }
-    if (m.pl.levels) {
-      any_levels = true;
-      cell_at[s] = cells;
-      cells += upper_cell(stripe[s].U + (stripe[s].K == kBrickLevels ? 2 : 1), 0);  // with the bricks' children
-    }
+    any_levels = any_levels || m.pl.levels;
     total_nodes += q.total;
   }
   if (total_nodes >> 32) fail(OOC_ERR_LIMIT, "more than 2^32 nodes in one sub-batch; lower the batch budget");
@@ -1025,7 +1018,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
   }
   // ---- per-leaf arrays and output windows ----
   const bool any_payload = total_leaves != 0;
-  float* upper_cache = any_levels ? ensure<float>(c->d_uppercache, cells * 24) : nullptr;
+  float* upper_cache = any_levels ? ensure<float>(c->d_uppercache, cells * kCellBytes) : nullptr;
   unsigned long long* winners = any_payload ? ensure<unsigned long long>(c->d_winners, total_leaves * 8) : nullptr;
   uint64_t out_nodes = 0, out_data = 0;
   if (os.mode == OUT_DEST) {

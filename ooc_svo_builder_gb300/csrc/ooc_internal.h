@@ -76,6 +76,44 @@ struct Stripe {
 // Mark bytes of a stripe's leaf level, padded to 16 bytes.
 __host__ __device__ inline uint64_t touch_bytes(int depth) { return (leaf_blocks(depth) + 15) / 16 * 16; }
 
+// Stripes of 512^3 voxels and more mark their leaf blocks; smaller leaf
+// levels are read and zeroed whole (their marks would cost the voxelization
+// more than they save).
+constexpr int kMarkDepth = 9;
+
+// Cell z of upper level l in the upper_cache.
+__host__ __device__ inline uint64_t upper_cell(int l, uint64_t z) { return ((1ull << (3 * l)) - 1) / 7 + z; }
+
+// Elements of a stripe's arrays in a sub-batch's buffers: what the engine allocates and what the
+// serving loop admits a request for.
+struct StripeSizes {
+  uint64_t leaf;    // words
+  uint64_t touch;   // bytes
+  uint64_t blocks;  // the ranks of leaf bits: payload stripes only
+  uint64_t upper;   // words of ubits, and as many of upre
+  uint64_t words;   // wpre: one entry past the last word, in whole groups of eight
+  uint64_t bricks;  // bpre and bunits: whole words
+  uint64_t cells;   // with -levels: averages of the upper levels, the bricks and the bricks' children
+};
+inline StripeSizes stripe_sizes(int depth, bool payload, bool levels) {
+  const int K = depth < kBrickLevels ? depth : kBrickLevels, U = depth - K;
+  StripeSizes z;
+  z.leaf = leaf_words(depth);
+  z.touch = depth >= kMarkDepth ? touch_bytes(depth) : 0;
+  z.blocks = payload ? leaf_blocks(depth) : 0;
+  z.upper = upper_off(U + 1);
+  z.words = (upper_words(U) + 8) / 8 * 8;
+  z.bricks = U < 2 ? 32 : 1ull << (3 * U);
+  z.cells = levels ? upper_cell(U + (K == kBrickLevels ? 2 : 1), 0) : 0;
+  return z;
+}
+constexpr uint64_t kCellBytes = 24;
+inline uint64_t stripe_bytes(const StripeSizes& z) {
+  return z.leaf * 4 + z.touch + z.blocks * sizeof(LeafBlock) + z.upper * 8 + (z.words + z.bricks) * 8 + z.bricks +
+         z.cells * kCellBytes;
+}
+constexpr uint64_t kItemBytes = 24;  // an item's place in the list of large items, its pass mask and its box
+
 // Words of a stripe's counts as the host reads them.
 // [0] leaves, [1] inner nodes below the bricks, [2 + l] nodes of upper level l, [kRootWord] the root's child mask
 constexpr uint32_t kCountWords = 16, kRootWord = 15;
@@ -156,9 +194,6 @@ struct EmitJob {
   uint64_t data_base;       // file index of the stripe's first data record
   uint64_t data_span;       // data records of the stripe
 };
-
-// Cell z of upper level l in the upper_cache.
-__host__ __device__ inline uint64_t upper_cell(int l, uint64_t z) { return ((1ull << (3 * l)) - 1) / 7 + z; }
 
 // CTAs of kTreeThreads threads over the cells above a stripe's bricks.
 __host__ __device__ inline uint32_t upper_node_ctas(int U) { return (uint32_t)((upper_cell(U, 0) + 255u) / 256u); }

@@ -17,7 +17,6 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
-#include <cmath>
 #include <condition_variable>
 #include <cstdlib>
 #include <cstring>
@@ -28,15 +27,15 @@
 #include <unordered_map>
 #include <vector>
 
+#include "ooc_admission.h"
 #include "ooc_extents.h"
-#include "ooc_footprint.h"
 #include "ooc_svo_gpu.h"
 
 namespace {
 
 using Clock = std::chrono::steady_clock;
 using ooc::Extents;
-using ooc::voxel_bound;
+using ooc::footprint;
 
 // Pinned host memory for host results.  With ooc_server_config::host_pool_mb
 // the server pins that much once, at creation, and carves each result's blocks
@@ -212,50 +211,9 @@ bool valid(const ooc_mesh& m) {
   return ooc_estimate_partitions(N, p.memory_limit_mb) <= (1ull << 21);
 }
 
-// HBM a request may hold while it is in flight: its triangles, the occupancy
-// pyramids of its stripes, and per-node arrays plus output records for an upper
-// bound on its nodes.  A tree with L leaves at depth D has at most min(8^l, L)
-// nodes at level l.  The leaves are at most the summed per-triangle bounds on the
-// voxels a triangle can set: the voxels of its grid box (voxelizer.cpp:189-204
-// tests no other), and, for a triangle with a finite plane, the voxels that
-// overlap it (the Schwarz-Seidel test is the triangle-box overlap test): their
-// centres lie within the triangle grown by a cube of side u, so the voxels
-// themselves lie within the triangle grown by a ball of radius sqrt(3) u, whose
-// volume is 2 r A + (pi / 2) r^2 L + (4 / 3) pi r^3 for area A and perimeter L
-// (Steiner's formula for a flat convex body).  A node costs at most kNodeBytes:
-// its 24-byte record and 32-byte data record, its key, subtree sizes and
-// starts, first child and winner (7 x 4 bytes) and its -levels cache (24
-// bytes), with room for the batch's job tables.
-constexpr uint64_t kNodeBytes = 120;
 constexpr uint64_t kDeliverPiece = 16ull << 20;  // bytes per copy of a host result's copy back
 constexpr std::chrono::seconds kPinWait{10};     // a host result waits this long for pinned memory
 constexpr int kSizers = 4;  // threads that compute the footprints of submitted requests
-
-uint64_t footprint(const ooc_mesh& m) {
-  const ooc_build_params& p = m.params;
-  const uint64_t N = p.gridsize;
-  const uint64_t stride = p.geometry_only ? 9 : 21;
-  uint64_t bytes = m.n_tris * stride * 4;
-  int D = 0;
-  while ((1ull << D) < N) D++;
-  const uint64_t P = ooc_estimate_partitions(N, p.memory_limit_mb);
-  int kP = 0;
-  while ((1ull << (3 * kP)) < P) kP++;
-  const int Ds = std::min(D - kP, 10);
-  uint64_t words = 0;
-  for (int l = 0; l <= Ds; l++) words += (((1ull << (3 * l)) + 31) / 32 + 7) / 8 * 8;
-  const uint64_t stripes = (N * N * N) >> (3 * Ds);
-  bytes += words * 4 * stripes;
-  const float unit_div = 1.0f / ((p.bbox_max[0] - p.bbox_min[0]) / (float)N);
-  const double cells = (double)N * (double)N * (double)N;
-  double leaves = 0.0;
-  for (uint64_t t = 0; t < m.n_tris && leaves < cells; t++) leaves += voxel_bound(m.tris + t * stride, unit_div, N);
-  leaves = std::min(leaves, cells);
-  double nodes = 0.0;
-  for (int l = 0; l <= D; l++) nodes += std::min(std::ldexp(1.0, 3 * l), leaves);
-  bytes += (uint64_t)std::min(nodes * (double)kNodeBytes, 1.8e19);
-  return bytes;
-}
 
 }  // namespace
 

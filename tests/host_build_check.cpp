@@ -1,10 +1,10 @@
-// Builds that fail part-way, on the stand-in runtime of fake_cuda.h (test_failed_builds.py).
-// One argument: the property to check.  Every call is made to fail at each of its allocations
-// and of its callbacks in turn, on a context of its own.
+// The host side of a build on the stand-in runtime of fake_cuda.h (test_host_build.py).  One
+// argument: the property to check.
 #include <algorithm>
 #include <string>
 
 #include "fake_cuda.h"
+#include "ooc_admission.h"
 
 namespace {
 
@@ -183,6 +183,58 @@ void check_aligned() {
           }
 }
 
+// What the serving loop admits a request for covers what a build of it allocates and its result.
+int sized_alloc(void* u, uint64_t, uint64_t nb, uint64_t db, void*, void** n, void** d) {
+  *static_cast<uint64_t*>(u) = nb + db;
+  *n = arena_mem;
+  *d = arena_mem + (nb + 255) / 256 * 256;
+  return 0;
+}
+void check_admitted() {
+  static float small[21] = {0.5f, 0.5f, 0.5f, 0.505f, 0.5f, 0.5f, 0.5f, 0.505f, 0.5f};
+  static float wide[21] = {0.0f, 0.0f, 0.0f, 1.0f, 1.0f, 0.9f, 0.1f, 1.0f, 1.0f};
+  for (int payload = 0; payload < 2; payload++)
+    for (int levels = 0; levels < 2; levels++)
+      for (const auto& [grid, limit] : {std::pair<uint64_t, uint64_t>{1, 2048}, {8, 2048}, {64, 2048}, {256, 2048}, {512, 2048},
+                                        {1024, 2048}, {2048, 16384}, {64, 1}, {128, 1}, {256, 1}, {512, 17}}) {
+        const bool parts = ooc_estimate_partitions(grid, limit) > 1;
+        ooc_ctx* c = nullptr;
+        expect(ooc_ctx_create(0, &c) == OOC_OK, "ooc_ctx_create");
+        ooc_mesh m = {parts ? wide : small, 1, params(grid, limit, levels)};  // the stand-in bins it everywhere
+        m.params.geometry_only = !payload;
+        ooc_set_batch_budget(c, 64 << 20);  // the octree of several stripes is parked
+        uint64_t files = 0;
+        fake::device_peak = fake::device_bytes;
+        expect(ooc_build_batch_device(c, &m, 1, sized_alloc, nullptr, &files, nullptr) == OOC_OK, ooc_last_error(c));
+        const uint64_t held = fake::device_peak + files, admitted = ooc::footprint(m);
+        const std::string at = "gridsize " + std::to_string(grid) + ", payload " + std::to_string(payload) + ", levels " +
+                               std::to_string(levels) + ": " + std::to_string(held) + " bytes held, admitted for " +
+                               std::to_string(admitted);
+        expect(held <= admitted, at);
+        if (grid == 1024) expect(admitted <= held + held / 16, at + ", far more");
+        ooc_ctx_destroy(c);
+      }
+  // the bound on a triangle's partitions against the test that bins it
+  std::srand(1);
+  const uint64_t N = 1024, per = 8, side = N / per;
+  const float u = 1.0f / (float)N;
+  for (int k = 0; k < 20000; k++) {
+    float v[9];
+    for (float& x : v) {
+      x = (float)std::rand() / (float)RAND_MAX * 1.4f - 0.2f;
+      if (std::rand() % 3 == 0) x = (float)(std::rand() % (int)(per + 1)) * (float)side * u;  // on a slab's bound
+    }
+    uint64_t n = 1;
+    for (int a = 0; a < 3; a++) {
+      const float lo = std::min(v[a], std::min(v[3 + a], v[6 + a])), hi = std::max(v[a], std::max(v[3 + a], v[6 + a]));
+      uint64_t on = 0;
+      for (uint64_t j = 0; j < per; j++) on += !(hi < (float)(j * side) * u) && !(lo > (float)((j + 1) * side) * u);
+      n *= on;
+    }
+    expect((double)n <= ooc::partition_bound(v, 1.0f / u, side, per), "partition_bound");
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -192,6 +244,7 @@ int main(int argc, char** argv) {
   else if (what == "recovered") check_recovered();
   else if (what == "freed") check_freed();
   else if (what == "aligned") check_aligned();
+  else if (what == "admitted") check_admitted();
   else return 2;
   std::printf("%d failures\n", bad);
   return bad ? 1 : 0;
