@@ -876,6 +876,7 @@ void run_sub_batch(ooc_ctx* c, cudaStream_t st, std::vector<MeshWork>& meshes, c
     j.wpre = S.wpre;
     j.blocks = S.blocks;
     j.large = large;
+    j.large_cap = items;
     j.big = big;
     j.ctr = ctr;
     j.big_cap = big_cap;

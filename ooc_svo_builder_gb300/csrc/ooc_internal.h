@@ -136,7 +136,8 @@ struct VoxJob {
   const LeafBlock* blocks;  // Stripe::blocks
   unsigned long long* winners;  // per leaf: min of triangle index << 32 | its local Morton code
   // the list of large items (shared by the stripes of a sub-batch)
-  unsigned long long* large; // items of one task each: item | stripe << 32 (room for every item)
+  unsigned long long* large; // items of one task each: item | stripe << 32
+  uint64_t large_cap;       // entries of `large`: at least the items
   uint4* big;               // the others: item, stripe, first task, tasks (big_cap entries)
   unsigned long long* ctr;  // kCtr* counters
   uint32_t big_cap;         // at most kMaxBig
@@ -163,9 +164,10 @@ struct LargeLists {
   const unsigned long long* large;
   const uint4* big;
   unsigned long long* ctr;
+  uint64_t large_cap;
   uint32_t big_cap, slice;
 };
-inline LargeLists lists_of(const VoxJob& j) { return LargeLists{j.large, j.big, j.ctr, j.big_cap, j.slice}; }
+inline LargeLists lists_of(const VoxJob& j) { return LargeLists{j.large, j.big, j.ctr, j.large_cap, j.big_cap, j.slice}; }
 
 struct EmitJob {
   int binary;

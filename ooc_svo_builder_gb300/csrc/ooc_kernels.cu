@@ -423,7 +423,10 @@ __device__ __forceinline__ uint64_t item_lines(int W, const int lo[3], const int
 // lines make one task (at most `slice` lines), else to `big`, whose entries carry the number
 // of their first task so that several warps share the item.  A full `big` (ctr[kCtrBig]'s
 // count at its capacity) sends further items to `large`, where one warp walks them whole.
-// The lists serve both passes; their order does not matter to the result.
+// The lists serve both passes; their order does not matter to the result.  Calls of the allocation-free
+// pass that overlap share its lists and find each other's counts and items there, which may cost them
+// voxels but no access out of range: additions past a list's end are dropped, and so are items that the
+// job does not have.
 //
 // kCtrBig packs the entries (low kBigCountBits bits) and the tasks (the others) reserved so
 // far, so one atomicAdd gives an entry and its first task in step.  A thread adds only after
@@ -470,8 +473,8 @@ __device__ __forceinline__ void append_large(const VoxJob& j, uint64_t i, uint32
     if (lane == 0) at = atomicAdd(j.ctr + kCtrLarge, (unsigned long long)__popc(m));
     at = __shfl_sync(FULL, at, 0);
   }
-  if (one)
-    j.large[at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
+  at += __popc(m & ((1u << lane) - 1u));
+  if (one && at < j.large_cap) j.large[at] = (uint32_t)(j.item0 + i) | ((unsigned long long)j.stripe << 32);
 }
 
 // (x, y, z) -> (a, b, w): w the axis W, a and b the ones that follow it cyclically.
@@ -1049,7 +1052,7 @@ __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, cons
   int lo[3], hi[3], W = 0;
   if (has) {
     const VoxJob& j = SINGLE ? j0 : jobs[stripe];
-    if (PASS == 0 || j.winners) {  // (a binary stripe in a mixed batch has no winner pass)
+    if (item < j.n_items && (PASS == 0 || j.winners)) {  // (a binary stripe in a mixed batch has no winner pass)
       t = item_triangle(j, item);
       tv = load_verts(j.tris, t, j.stride);
       if (item_box(j, tv, lo, hi)) {  // as when it was listed
@@ -1111,7 +1114,7 @@ __device__ __forceinline__ void walk_items(const VoxJob* __restrict__ jobs, cons
 template <int PASS, bool SINGLE>
 __device__ __forceinline__ void walk_lists(const VoxJob* __restrict__ jobs, const VoxJob& j0, const LargeLists& L, int lane,
                                            WalkScratch& sm, const uint32_t* spread) {
-  const unsigned long long n = __ldcg(L.ctr + kCtrLarge), packed = __ldcg(L.ctr + kCtrBig);
+  const unsigned long long n = min(__ldcg(L.ctr + kCtrLarge), (unsigned long long)L.large_cap), packed = __ldcg(L.ctr + kCtrBig);
   const uint32_t nb = min((uint32_t)(packed & ((1u << kBigCountBits) - 1u)), L.big_cap);
   uint64_t tasks = 0;
   if (nb) {

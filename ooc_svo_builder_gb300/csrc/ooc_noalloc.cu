@@ -102,6 +102,7 @@ extern "C" int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, co
   j.ctr = scratch;
   j.big = reinterpret_cast<uint4*>(scratch + kBigWord);
   j.large = scratch + kLargeWord;
+  j.large_cap = kMaxTris;
   j.big_cap = kBig;
   j.slice = 512;
   j.item_mask = nullptr;
