@@ -1300,7 +1300,7 @@ void bin_mesh(ooc_ctx* c, cudaStream_t st, MeshWork& m, DevBuf& items_buf) {
   ck(cudaMemcpyAsync(d_axis, axis.data(), axis.size() * 4, cudaMemcpyHostToDevice, st), "axis boxes");
   uint32_t* hist = ensure<uint32_t>(c->d_hist, pl.P * 4);
   ck(cudaMemsetAsync(hist, 0, pl.P * 4, st), "memset hist");
-  launch_part_count(m.d_tris, stride, m.n_tris, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, st);
+  launch_part_count(m.d_tris, stride, m.n_tris, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, c->num_sms, st);
   const uint32_t* h = read_back_words(c, hist, pl.P, st);
   ck(cudaStreamSynchronize(st), "binning");
   m.part_off.assign(pl.P + 1, 0);
@@ -1315,7 +1315,7 @@ void bin_mesh(ooc_ctx* c, cudaStream_t st, MeshWork& m, DevBuf& items_buf) {
   uint32_t* items = ensure<uint32_t>(items_buf, acc * 4);
   ck(cudaMemcpyAsync(hist, m.part_off.data(), pl.P * 4, cudaMemcpyHostToDevice, st), "cursors");
   ck(cudaStreamSynchronize(st), "cursors");  // part_off is reused on the host
-  launch_part_emit(m.d_tris, stride, m.n_tris, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, items, st);
+  launch_part_emit(m.d_tris, stride, m.n_tris, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, items, c->num_sms, st);
   m.items = items;
 }
 
@@ -1402,7 +1402,7 @@ void stream_count(ooc_ctx* c, cudaStream_t st, MeshWork& m) {
   ck(cudaMemsetAsync(hist, 0, pl.P * 4, st), "memset hist");
   const int stride = pl.binary ? 9 : 21;
   stream_pass(c, st, *m.src, std::max<uint64_t>(1, kStreamChunkBytes / m.src->rec), [&](const float* d, uint64_t n) {
-    launch_part_count(d, stride, n, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, st);
+    launch_part_count(d, stride, n, d_axis, d_axis + 3 * PA, pl.kP, pl.P, hist, c->num_sms, st);
   });
   const uint32_t* h = read_back_words(c, hist, pl.P, st);
   ck(cudaStreamSynchronize(st), "counts");

@@ -110,84 +110,8 @@ __device__ __forceinline__ void edge_setup(const TriVerts& t, const float e[3][3
   }
 }
 
-__device__ __forceinline__ void tri_setup(const TriVerts& t, float u, TriSetup& s) {
-  float e[3][3];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    e[0][a] = __fsub_rn(t.v[1][a], t.v[0][a]);
-    e[1][a] = __fsub_rn(t.v[2][a], t.v[1][a]);
-    e[2][a] = __fsub_rn(t.v[0][a], t.v[2][a]);
-  }
-  s.n[0] = __fsub_rn(__fmul_rn(e[0][1], e[1][2]), __fmul_rn(e[0][2], e[1][1]));
-  s.n[1] = __fsub_rn(__fmul_rn(e[0][2], e[1][0]), __fmul_rn(e[0][0], e[1][2]));
-  s.n[2] = __fsub_rn(__fmul_rn(e[0][0], e[1][1]), __fmul_rn(e[0][1], e[1][0]));
-  normalize3(s.n[0], s.n[1], s.n[2]);
-  // critical point and plane offsets
-  const float cx = (s.n[0] > 0.0f) ? u : 0.0f;
-  const float cy = (s.n[1] > 0.0f) ? u : 0.0f;
-  const float cz = (s.n[2] > 0.0f) ? u : 0.0f;
-  s.d1 = dot3(s.n[0], s.n[1], s.n[2], __fsub_rn(cx, t.v[0][0]), __fsub_rn(cy, t.v[0][1]), __fsub_rn(cz, t.v[0][2]));
-  s.d2 = dot3(s.n[0], s.n[1], s.n[2], __fsub_rn(__fsub_rn(u, cx), t.v[0][0]), __fsub_rn(__fsub_rn(u, cy), t.v[0][1]),
-              __fsub_rn(__fsub_rn(u, cz), t.v[0][2]));
-  edge_setup(t, e, u, s);
-}
-
-// XY projection tests for a column (x, y): they do not depend on z.
-__device__ __forceinline__ bool pass_xy(const TriSetup& s, float px, float py) {
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (__fadd_rn(dot2(s.xy[k][0], s.xy[k][1], px, py), s.dxy[k]) < 0.0f) return false;
-  return true;
-}
-
-// Plane test + YZ and ZX projection tests at one voxel (voxelizer.cpp:266-287);
-// the XY tests are evaluated once per column by pass_xy.
-__device__ __forceinline__ bool pass_z(const TriSetup& s, float nxy, float px, float py, float pz) {
-  const float nDOTp = __fadd_rn(nxy, __fmul_rn(s.n[2], pz));
-  if (__fmul_rn(__fadd_rn(nDOTp, s.d1), __fadd_rn(nDOTp, s.d2)) > 0.0f) return false;
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (__fadd_rn(dot2(s.yz[k][0], s.yz[k][1], py, pz), s.dyz[k]) < 0.0f) return false;
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (__fadd_rn(dot2(s.zx[k][0], s.zx[k][1], pz, px), s.dzx[k]) < 0.0f) return false;
-  return true;
-}
-
-// n.x*p.x + n.y*p.y, the part of dot(n, p) that is constant along a z column.
-__device__ __forceinline__ float plane_xy(const TriSetup& s, float px, float py) {
-  return __fadd_rn(__fmul_rn(s.n[0], px), __fmul_rn(s.n[1], py));
-}
-
-// The projection tests that do not depend on x (YZ) and on y (ZX).
-__device__ __forceinline__ bool pass_yz(const TriSetup& s, float py, float pz) {
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (__fadd_rn(dot2(s.yz[k][0], s.yz[k][1], py, pz), s.dyz[k]) < 0.0f) return false;
-  return true;
-}
-__device__ __forceinline__ bool pass_zx(const TriSetup& s, float pz, float px) {
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    if (__fadd_rn(dot2(s.zx[k][0], s.zx[k][1], pz, px), s.dzx[k]) < 0.0f) return false;
-  return true;
-}
-
-// Where the plane test of voxel p stands along axis w, whose normal component is nw:
-// 0 it passes, -1 the passing run lies at larger w, +1 at smaller w.  Every
-// operand of the test is a rounded sum or product of one monotone input, so
-// along any line the rounded plane value moves monotonically with the sign of
-// nw, the two offsets keep their order, and the passing voxels form one run;
-// outside it both factors have the sign that says which side it is on.
-__device__ __forceinline__ int plane_side(const TriSetup& s, float px, float py, float pz, float nw) {
-  const float nDOTp = __fadd_rn(plane_xy(s, px, py), __fmul_rn(s.n[2], pz));
-  const float a = __fadd_rn(nDOTp, s.d1), b = __fadd_rn(nDOTp, s.d2);
-  if (!(__fmul_rn(a, b) > 0.0f)) return 0;
-  return ((a > 0.0f) == (nw > 0.0f)) ? 1 : -1;
-}
-
-// True when the monotone-run argument above holds for this triangle: every
-// constant of the test finite and small enough that no sum or product of the
+// True when the voxels of a line that pass the plane test form one run (walk_line):
+// every constant of the test finite and small enough that no sum or product of the
 // test overflows or turns into NaN (voxel coordinates are below 2^60 too).
 __device__ __forceinline__ bool monotone_setup(const TriSetup& s, float coord_max) {
   const float lim = 1.0e18f;

@@ -15,7 +15,6 @@ namespace ooc {
 // occupancy bitfield (128 MiB) is about the size of the GB300's 129 MB L2, so
 // the voxelization atomics mostly stay on chip.
 constexpr int kMaxStripeDepth = 10;
-constexpr int kMaxLevels = kMaxStripeDepth + 1;
 
 // A stripe's octree is cut into bricks: the nodes kBrickLevels levels above the
 // leaves (16^3 voxels, 4,096 leaf bits; a stripe of depth 4 or less is one
@@ -251,9 +250,9 @@ uint64_t scan_partials_needed(uint64_t n);
 // n words from device memory into `dst`, mapped pinned host memory, by a kernel.
 void launch_copy_words(const uint32_t* src, uint64_t n, uint32_t* dst, cudaStream_t st);
 void launch_part_count(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
-                       int pa_bits, uint64_t n_parts, uint32_t* hist, cudaStream_t st);
+                       int pa_bits, uint64_t n_parts, uint32_t* hist, int num_sms, cudaStream_t st);
 void launch_part_emit(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
-                      int pa_bits, uint64_t n_parts, uint32_t* cursor, uint32_t* items, cudaStream_t st);
+                      int pa_bits, uint64_t n_parts, uint32_t* cursor, uint32_t* items, int num_sms, cudaStream_t st);
 
 // Out-of-core binning of one chunk of the triangle stream for the partition group
 // [p0, p0 + gp) (gp <= kStreamMaxGroup): the chunk's records of each group partition q
@@ -274,7 +273,6 @@ void launch_stream_group_chunk(const float* tris, int stride, uint64_t n, const 
 cudaError_t launch_vox_small_occupancy(const VoxJob& j, cudaStream_t st);
 cudaError_t launch_vox_large_occupancy(const VoxJob& j, cudaStream_t st, int num_sms);
 
-// src holds n entries of (index, `words` u64 values); dst[index*words + q] = value q.
 // Node records (n of 3 words) and then data records (of 4) at `src`, each after one word that says where
 // it goes: its number in nodes or data or, without these, its address.
 void launch_scatter_records(const uint64_t* src, uint64_t n_nodes, uint64_t n_data, uint64_t* nodes, uint64_t* data,

@@ -396,14 +396,14 @@ __device__ __forceinline__ uint64_t item_triangle(const VoxJob& j, uint64_t i) {
 
 // ---------------------------------------------------------------------------
 // Large items walk lines along the axis of their largest normal component.  On
-// every line the voxels that pass the plane test form one run (plane_side), so
+// every line the voxels that pass the plane test form one run (walk_line), so
 // a line costs its run plus a few probes instead of its whole length; every
 // voxel of the run still gets the complete test, so the result is the
 // reference's candidate loop (voxelizer.cpp:257-305) voxel for voxel.
 // ---------------------------------------------------------------------------
 
-// Axis of the largest component of cross(e0, e1); the item count and the tasks
-// call this same function, so they agree on the lines of every item.
+// Axis of the largest component of cross(e0, e1); the listing of the items and the
+// walk call this same function, so they agree on the lines of every item.
 __device__ __forceinline__ int walk_axis(const TriVerts& t) {
   const float e0x = t.v[1][0] - t.v[0][0], e0y = t.v[1][1] - t.v[0][1], e0z = t.v[1][2] - t.v[0][2];
   const float e1x = t.v[2][0] - t.v[1][0], e1y = t.v[2][1] - t.v[1][1], e1z = t.v[2][2] - t.v[1][2];
@@ -493,7 +493,7 @@ __device__ __forceinline__ float sum3(int W, float pa, float pb, float pw) {
   return W == 0 ? __fadd_rn(__fadd_rn(pw, pa), pb) : __fadd_rn(__fadd_rn(pb, pw), pa);
 }
 
-// tri_setup with the coordinates rotated to (a, b, w).
+// The constants of the test (voxelizer.cpp:207-254) with the coordinates rotated to (a, b, w).
 __device__ __forceinline__ void tri_setup_rotated(const TriVerts& t, float u, int W, TriSetup& s) {
   float e[3][3];
 #pragma unroll
@@ -645,7 +645,11 @@ __device__ __forceinline__ void walk_line(const VoxJob& j, const WalkItem& r, ui
     return !(fminf(fminf(fminf(m[0], m[1]), fminf(m[2], m[3])), fminf(m[4], m[5])) < 0.0f);
   };
   const bool up_side = nw * u > 0.0f;  // the plane value grows with w
-  auto side = [&](float fw) {  // plane_side
+  // Where the plane test of voxel w stands: 0 it passes, -1 the passing run lies at larger w, +1 at
+  // smaller w.  Every operand of the test is a rounded sum or product of one monotone input, so along the
+  // line the rounded plane value moves monotonically, the two offsets keep their order, and the passing
+  // voxels form one run; outside it both factors have the sign that says which side it is on.
+  auto side = [&](float fw) {
     const float v = __fadd_rn(__fadd_rn(__fmul_rn(nw, fw), q1), q2);
     float a, b;
     split(add2(f2(v, v), dd), a, b);
@@ -1359,28 +1363,28 @@ void launch_copy_words(const uint32_t* src, uint64_t n, uint32_t* dst, cudaStrea
 
 // Rounds of kPartCta triangles a block takes: as many as leave eight blocks per SM, and runs that fit
 // beside the counters in 48 KB.
-static int part_rounds(uint64_t n_tris, size_t counters) {
+static int part_rounds(uint64_t n_tris, size_t counters, int num_sms) {
   return (int)std::min<uint64_t>(std::min<uint64_t>(kPartMax, (49152 - counters) / (kPartCta * 8)),
-                                 std::max<uint64_t>(1, n_tris / (152ull * 8 * kPartCta)));
+                                 std::max<uint64_t>(1, n_tris / ((uint64_t)num_sms * 8 * kPartCta)));
 }
 
 void launch_part_count(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
-                       int pa_bits, uint64_t n_parts, uint32_t* hist, cudaStream_t st) {
+                       int pa_bits, uint64_t n_parts, uint32_t* hist, int num_sms, cudaStream_t st) {
   if (n_tris == 0) return;
   const int use_smem = n_parts <= 4096;
   const size_t smem = ((use_smem ? n_parts : 0) + 6ull * (1ull << pa_bits)) * sizeof(uint32_t);
-  const int per = part_rounds(n_tris, smem);
+  const int per = part_rounds(n_tris, smem, num_sms);
   KScope k("part_count", st);
   launch_k(k_part_count, dim3(grid_for(n_tris, kPartCta * per)), dim3(kPartCta), smem, st, tris, stride, n_tris, axis_lo,
            axis_hi, pa_bits, (uint32_t)n_parts, hist, use_smem, per);
 }
 
 void launch_part_emit(const float* tris, int stride, uint64_t n_tris, const float* axis_lo, const float* axis_hi,
-                      int pa_bits, uint64_t n_parts, uint32_t* cursor, uint32_t* items, cudaStream_t st) {
+                      int pa_bits, uint64_t n_parts, uint32_t* cursor, uint32_t* items, int num_sms, cudaStream_t st) {
   if (n_tris == 0) return;
   const int use_smem = n_parts <= 4096;
   size_t smem = ((use_smem ? n_parts : 0) + 6ull * (1ull << pa_bits)) * sizeof(uint32_t);
-  const int per = part_rounds(n_tris, smem);
+  const int per = part_rounds(n_tris, smem, num_sms);
   if (use_smem) smem += (size_t)per * kPartCta * 8;
   KScope k("part_emit", st);
   launch_k(k_part_emit, dim3(grid_for(n_tris, kPartCta * per)), dim3(kPartCta), smem, st, tris, stride, n_tris, axis_lo,

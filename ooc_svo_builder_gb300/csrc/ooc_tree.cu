@@ -459,7 +459,7 @@ __device__ void payload_color(const TriVerts& tv, const float n[3], int x, int y
   }
 }
 
-// Colour, normal and local Morton code of leaf `li` (its index among the stripe's leaves).
+// Colour and normal of the leaf whose winner (triangle << 32 | local Morton code) is `win`.
 // Returns false (and flags) if the leaf has no winning triangle.
 __device__ bool leaf_value(const EmitJob& e, unsigned long long win, float out[6]) {
   const uint32_t key = (uint32_t)win;
@@ -637,7 +637,7 @@ struct __align__(16) WarpScratch {
   uint64_t win[kSlots * 3];
   LaneWords words[32];
   uint32_t gaps[8];
-  uint16_t units[256];  // of the word's bricks: brick | place in it << 5 | number in it << 8
+  uint16_t units[256];  // of the 32 bricks in hand: brick | place in it << 5 | number in it << 8
 };
 
 // Bulk copies of shared memory to global memory (both 16-byte aligned, a multiple of 16
@@ -1109,8 +1109,7 @@ __device__ __forceinline__ void emit_bricks(const Stripe& p, const EmitJob& e, u
   }
 }
 
-// The bricks of the stripe's warp i: bricks_per_warp consecutive ones of its non-empty bricks.
-// The warp's share: non-empty bricks i * bricks_per_warp to the next warp's first.
+// The share of the stripe's warp i: bricks_per_warp consecutive ones of its non-empty bricks.
 template <bool LEVELS>
 __device__ __forceinline__ void emit_warp(const Stripe& p, const EmitJob& e, uint64_t i, int lane, WarpScratch& sm,
                                           const uint64_t* __restrict__ lut) {

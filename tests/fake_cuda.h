@@ -272,13 +272,13 @@ void launch_copy_words(const uint32_t* src, uint64_t n, uint32_t* dst, cudaStrea
   fake::put(st, [=] { std::memcpy(dst, src, n * 4); });
 }
 void launch_part_count(const float*, int, uint64_t n_tris, const float*, const float*, int, uint64_t n_parts, uint32_t* hist,
-                       cudaStream_t st) {
+                       int, cudaStream_t st) {
   fake::put(st, [=] {
     for (uint64_t p = 0; p < n_parts; p++) hist[p] += (uint32_t)n_tris;  // every triangle in every partition
   });
 }
 void launch_part_emit(const float*, int, uint64_t, const float*, const float*, int, uint64_t, uint32_t*, uint32_t*,
-                      cudaStream_t st) {
+                      int, cudaStream_t st) {
   fake::put(st, [] {});
 }
 void launch_stream_bases(const uint32_t*, uint32_t, uint32_t, uint64_t*, cudaStream_t) {}
