@@ -200,16 +200,20 @@ NCU_TRAFFIC = {
 }
 
 
-def algorithmic_bytes(kernel: str, n_tris: int, info: dict, S: int, payload: bool) -> float:
-    """Minimum DRAM bytes one launch of `kernel` must move for this workload."""
+def algorithmic_bytes(kernel: str, n_tris: int, n_large: int, info: dict, S: int, payload: bool) -> float:
+    """Minimum DRAM bytes one launch of `kernel` must move for this workload, `n_large` of whose triangles
+    are walked line by line."""
     tri_bytes = 84 if payload else 36
     leaf_words = S // 32
     if kernel == "vox_small_occupancy":
         # vertices of every triangle (36 B) + (payload) pass mask and box (16 B)
         return n_tris * (36 + (16 if payload else 0))
-    if kernel in ("vox_small_winner", "vox_large_occupancy", "vox_large_winner"):
-        # vertices of every triangle (36 B) + the task count per item (8 B)
-        return n_tris * (36 + 8)
+    if kernel == "vox_small_winner":  # pass mask and box of every triangle, the winner of every leaf
+        return n_tris * 16 + info["n_filled"] * 8
+    if kernel == "vox_large_occupancy":  # list entry and vertices of the large triangles
+        return n_large * (8 + 36)
+    if kernel == "vox_large_winner":
+        return n_large * (8 + 36) + info["n_filled"] * 8
     if kernel == "bricks":  # marks of every leaf block, and the marked blocks (at least one per 256 voxels)
         return leaf_words / 8 + info["n_filled"] / 256 * 32
     if kernel == "leaf_payload":
@@ -219,16 +223,19 @@ def algorithmic_bytes(kernel: str, n_tris: int, info: dict, S: int, payload: boo
     return 0.0
 
 
-def small_candidates(tris: np.ndarray, gridsize: int, small_vol: int = 64) -> int:
-    """Candidate voxels of the triangles the one-thread-per-triangle pass voxelizes: the sum of
-    their clamped grid-box volumes (voxelizer.cpp:199-204, boxes of at most `small_vol` voxels).
-    Meshes in the unit cube, so unit_div = gridsize."""
+def split_triangles(tris: np.ndarray, gridsize: int, small_vol: int):
+    """(candidate voxels of the triangles that the one-thread-per-triangle pass voxelizes, number of the
+    triangles that it lists for the line walk).  Small is a clamped grid box (voxelizer.cpp:199-204) of at
+    most `small_vol` voxels with at most one extent above two.  Meshes in the unit cube, so unit_div =
+    gridsize; the boxes are those of the whole grid, not cut at stripes."""
     v = tris[:, :9].reshape(-1, 3, 3).astype(np.float32)
     g = np.float32(gridsize)
     lo = np.clip((v.min(axis=1) * g).astype(np.int64), 0, gridsize - 1)
     hi = np.clip((v.max(axis=1) * g).astype(np.int64), 0, gridsize - 1)
-    vol = np.prod(hi - lo + 1, axis=1)
-    return int(vol[vol <= small_vol].sum())
+    ext = hi - lo + 1
+    vol = np.prod(ext, axis=1)
+    small = (vol <= small_vol) & ((ext > 2).sum(axis=1) <= 1)
+    return int(vol[small].sum()), int((~small).sum())
 
 
 def run_ours(args, world, rank, local):
@@ -349,14 +356,16 @@ def run_ours(args, world, rank, local):
             shutil.rmtree(tmp, ignore_errors=True)
     stripes = e2e_info["n_stripes"]
     h2d = T * tris.shape[1] * 4
-    # the stripe spans are copied back; header records and the stripe roots are written on the host
+    # the stripe spans are copied back; header records and the stripe roots are written on the host, the roots
+    # from the stripes' counts (16 words each)
     payload = w["payload"]
-    d2h = (e2e_info["n_nodes"] - stripes) * 24 + (e2e_info["n_data"] - (1 if payload else 2)) * 32 + stripes * 36
+    d2h = (e2e_info["n_nodes"] - stripes) * 24 + (e2e_info["n_data"] - (1 if payload else 2)) * 32 + stripes * 64
 
     # ---- roofline of the dominant kernel ----
     peaks = measured_peaks()
     S = min(w["gridsize"] ** 3, 1 << 30)
-    alg = algorithmic_bytes(dominant, T, info, S, payload) if dominant else 0.0
+    candidates, n_large = split_triangles(tris, w["gridsize"], int(b.tuning().small_vol))
+    alg = algorithmic_bytes(dominant, T, n_large, info, S, payload) if dominant else 0.0
     per_launch_ms = dom_ms / dom_n if dom_n else float("nan")
     launches_per_build = kt.get(dominant, (0, 1))[1] if dominant else 1
     alg_per_launch = alg / max(1, launches_per_build)
@@ -373,7 +382,7 @@ def run_ours(args, world, rank, local):
     # FMA (SMs x 128 lanes x the measured SM clock) against the 47 flops of the full
     # Schwarz-Seidel test per candidate voxel (voxelizer.cpp:266-287).
     if dominant == "vox_small_occupancy" and dom_n and clocks.get("sm_mhz"):
-        flops = 47.0 * small_candidates(tris, w["gridsize"]) / max(1, launches_per_build)
+        flops = 47.0 * candidates / max(1, launches_per_build)
         fp32_peak = sm_count * 128 * clocks["sm_mhz"] * 1e6 / 1e12
         fp32_achieved = flops / (per_launch_ms / 1e3) / 1e12
         roofline["fp32"] = {"bound": "fp32 issue (no FMA)", "achieved": fp32_achieved, "peak": fp32_peak,
