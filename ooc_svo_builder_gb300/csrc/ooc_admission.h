@@ -12,24 +12,15 @@
 
 namespace ooc {
 
-// An upper bound on the partitions of `side`^3 voxels, `per_axis` along each axis, whose inclusive box test
-// triangle v passes (partitioner.cpp:101-149).  A twentieth of a voxel covers the rounding of the
-// slabs' bounds.
-inline double partition_bound(const float* v, float unit_div, uint64_t side, uint64_t per_axis) {
-  constexpr double slack = 0.05;
-  double n = 1.0;
-  for (int a = 0; a < 3; a++) {
-    const double lo = (double)std::min(v[a], std::min(v[3 + a], v[6 + a])) * unit_div - slack;
-    const double hi = (double)std::max(v[a], std::max(v[3 + a], v[6 + a])) * unit_div + slack;
-    if (!std::isfinite(lo) || !std::isfinite(hi)) {
-      n *= (double)per_axis;
-      continue;
-    }
-    const double j0 = std::max(std::ceil(lo / (double)side) - 1.0, 0.0);
-    const double j1 = std::min(std::floor(hi / (double)side), (double)per_axis - 1.0);
-    n *= std::max(j1 - j0 + 1.0, 0.0);
-  }
-  return n;
+// An upper bound on the (triangle, partition) pairs of n triangles whose clamped grid boxes hold `boxes` voxels
+// together, with P partitions of `side`^3 voxels (the inclusive box test, partitioner.cpp:101-149).  A box of
+// e voxels along an axis reaches at most e / side + 2 partitions along it, the slabs' rounded bounds included;
+// the product over the axes is at most 8 + box (12 / side + 6 / side^2 + 1 / side^3), every extent being at
+// least one.  It takes a sum from the pass over the triangles: requests wait behind that pass, and working
+// each triangle's partitions out cost the serving loop 2 to 10% of its capacity.
+inline double pair_bound(double n, double boxes, uint64_t side, uint64_t P) {
+  const double r = 1.0 / (double)side;
+  return std::min(n * (double)P, 8.0 * n + boxes * r * (12.0 + r * (6.0 + r)));
 }
 
 // HBM a request may hold while it is in flight: its triangles; every stripe's arrays (stripe_bytes) and job
@@ -52,12 +43,15 @@ inline uint64_t footprint(const ooc_mesh& m) {
   const uint64_t stripes = (N * N * N) >> (3 * Ds);
   const float unit_div = 1.0f / ((p.bbox_max[0] - p.bbox_min[0]) / (float)N);
   const double cells = (double)N * (double)N * (double)N;
-  double leaves = 0.0, pairs = P > 1 ? 0.0 : (double)m.n_tris;
-  for (uint64_t t = 0; t < m.n_tris && (leaves < cells || P > 1); t++) {
+  double leaves = 0.0, boxes = 0.0;
+  const double enough = P > 1 ? HUGE_VAL : cells;
+  for (uint64_t t = 0; t < m.n_tris && leaves < enough; t++) {
     const float* v = m.tris + t * stride;
-    if (leaves < cells) leaves += voxel_bound(v, unit_div, N);
-    if (P > 1) pairs += partition_bound(v, unit_div, N >> kP, 1ull << kP);
+    const double box = box_voxels(v, unit_div, N);
+    boxes += box;
+    leaves += box_or_grown(v, unit_div, box);
   }
+  const double pairs = P > 1 ? pair_bound((double)m.n_tris, boxes, N >> kP, P) : (double)m.n_tris;
   leaves = std::min(leaves, cells);
   double nodes = 0.0;
   for (int l = 0; l <= D; l++) nodes += std::min(std::ldexp(1.0, 3 * l), leaves);

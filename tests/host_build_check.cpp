@@ -216,7 +216,7 @@ void check_admitted() {
       }
   // the bound on a triangle's partitions against the test that bins it
   std::srand(1);
-  const uint64_t N = 1024, per = 8, side = N / per;
+  const uint64_t N = 512, per = 8, side = N / per;
   const float u = 1.0f / (float)N;
   for (int k = 0; k < 20000; k++) {
     float v[9];
@@ -224,6 +224,8 @@ void check_admitted() {
       x = (float)std::rand() / (float)RAND_MAX * 1.4f - 0.2f;
       if (std::rand() % 3 == 0) x = (float)(std::rand() % (int)(per + 1)) * (float)side * u;  // on a slab's bound
     }
+    if (k % 2)  // a small box
+      for (int q = 3; q < 9; q++) v[q] = v[q % 3] + (float)(std::rand() % 257 - 128) / 128.0f * u * (float)(1 + 30 * (q % 3 == k % 3));
     uint64_t n = 1;
     for (int a = 0; a < 3; a++) {
       const float lo = std::min(v[a], std::min(v[3 + a], v[6 + a])), hi = std::max(v[a], std::max(v[3 + a], v[6 + a]));
@@ -231,7 +233,7 @@ void check_admitted() {
       for (uint64_t j = 0; j < per; j++) on += !(hi < (float)(j * side) * u) && !(lo > (float)((j + 1) * side) * u);
       n *= on;
     }
-    expect((double)n <= ooc::partition_bound(v, 1.0f / u, side, per), "partition_bound");
+    expect((double)n <= ooc::pair_bound(1.0, ooc::box_voxels(v, 1.0f / u, N), side, per * per * per), "pair_bound");
   }
 }
 
