@@ -202,7 +202,7 @@ uint64_t ooc_batch_budget(const ooc_ctx* ctx);
 /* Same path from triangles already in device memory; the octree stays in
  * device memory (see ooc_result_device).  `stream` is a cudaStream_t (NULL:
  * the context's own stream); all work is ordered on it and the call returns
- * after the stream has drained. */
+ * after the stream has drained, also when it fails. */
 int ooc_build_device(ooc_ctx* ctx, const ooc_build_params* params, const float* tris_device, uint64_t n_tris,
                      void* stream, ooc_build_info* info);
 
@@ -297,7 +297,8 @@ int ooc_kernel_time(const ooc_ctx* ctx, int32_t index, const char** name, float*
  * (cudaGetSymbolAddress) with that device current; make that first call
  * before any stream capture.  All calls on a device share the one scratch
  * array, which keeps the last call's contents: calls that may overlap on the
- * GPU (different streams without ordering between them) race. */
+ * GPU (different streams without ordering between them) race: their output
+ * may lack voxels. */
 #define OOC_NOALLOC_MAX_TRIANGLES 1048576
 #define OOC_NOALLOC_MAX_GRIDSIZE 1024
 int ooc_voxelize_occupancy_noalloc(const ooc_build_params* params, const float* tris_device, uint64_t n_tris,
